@@ -46,6 +46,15 @@ bool is_device_ptr(const void* p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Points x centroids x padded dimensions from which the tensor cores make the
+// assignment.  A training call (20 passes over the same points) gains from
+// about 5e8 on: 10k x 1000 x 128 6.4 -> 2.5 ms, 100k x 300 x 32 6.5 -> 4.8 ms,
+// but 10k x 100 x 128 2.1 -> 3.3 ms (five small launches a pass against one).
+// A single pass (add) has its scratch allocation to earn back: 200k x 1024 x
+// 128 8.1 -> 6.4 ms, 100k x 500 x 128 3.2 -> 3.7 ms.
+constexpr double kAssignTcTrain = 5.0e8;
+constexpr double kAssignTcAdd = 1.5e10;
+
 int pow2_floor(long long x) {
   int p = 1;
   while (static_cast<long long>(p) * 2 <= x && p < (1 << 30)) p <<= 1;
@@ -231,6 +240,110 @@ class IndexCore {
     ++launches_;
   }
 
+  // ---- nearest-centroid assignment -----------------------------------------
+
+  // Buffers of one train or add call's assignments on the tensor cores (one
+  // allocation); `on` is false where the exact kernel does them (small
+  // problems, no memory for the buffers, or a wait that gave up).  One
+  // Assigner serves one set of points.
+  struct Assigner {
+    bool on = false;
+    size_t chunk = 0;              // points per launch
+    size_t split_at = ~size_t(0);  // first point of the chunk xsplit holds
+    DevBuf<unsigned char> mem;
+    unsigned char *xsplit = nullptr, *csplit = nullptr;
+    float *xnorm = nullptr, *cnorm = nullptr, *mu = nullptr;
+    int2* pairs = nullptr;
+    int *exact = nullptr, *ctl = nullptr, *err = nullptr;
+  };
+
+  // For assignments of n points, at most `max_chunk` of them at a time, on the
+  // tensor cores from `min_work` on.
+  void assign_setup(Assigner& as, size_t n, size_t max_chunk, double min_work) {
+    if (static_cast<double>(n) * nlist_ * dpad_ < min_work) return;
+    const size_t kpad = static_cast<size_t>(assign_kpad(static_cast<int>(dpad_)));
+    as.chunk = std::min<size_t>(n, std::max<size_t>(128, max_chunk));
+    size_t total = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+      size_t off = 0;
+      auto carve = [&](auto*& p, size_t count) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(as.mem.p + off);
+        off += (count * sizeof(*p) + 255) / 256 * 256;
+      };
+      carve(as.xsplit, as.chunk * 4 * kpad);
+      carve(as.csplit, nlist_ * 4 * kpad);
+      carve(as.xnorm, as.chunk);
+      carve(as.cnorm, (nlist_ + 127) / 128 * 128);
+      carve(as.mu, dpad_);
+      carve(as.pairs, as.chunk);
+      carve(as.exact, as.chunk);
+      carve(as.ctl, 4);
+      carve(as.err, 1);
+      total = off;
+      if (pass == 0) {
+        try {
+          as.mem.reserve(total);
+        } catch (const Error& e) {
+          if (e.code != HB_ERR_NOMEM) throw;
+          cudaGetLastError();
+          return;
+        }
+      }
+    }
+    HB_CUDA(cudaMemsetAsync(as.err, 0, sizeof(int), st_));
+    launch_column_mean(cent_.p, static_cast<int>(nlist_), static_cast<int>(dpad_), as.mu, st_);
+    ++launches_;
+    as.on = true;
+  }
+
+  // arg[i] = the nearest centroid of x row i (the reference's strict '<' scan
+  // in centroid order), dist (optional) its exact distance.
+  void assign_rows(Assigner& as, const float* x, size_t n, int32_t* arg, float* dist) {
+    const int dp = static_cast<int>(dpad_), nl = static_cast<int>(nlist_);
+    if (!as.on) {
+      launch_l2_argmin(x, static_cast<int>(n), cent_.p, nl, dp, arg, dist, st_);
+      ++launches_;
+      return;
+    }
+    for (size_t b = 0; b < n; b += as.chunk) {
+      const size_t m = std::min(as.chunk, n - b);
+      if (as.split_at != b) {  // one chunk in all: split once for every iteration
+        launch_split_points(x + b * dpad_, m, dp, as.mu, as.xsplit, as.xnorm, st_);
+        ++launches_;
+        as.split_at = b;
+      }
+      AssignArgs a{};
+      a.x = x + b * dpad_;
+      a.n = static_cast<int>(m);
+      a.dpad = dp;
+      a.cent = cent_.p;
+      a.nlist = nl;
+      a.mu = as.mu;
+      a.xsplit = as.xsplit;
+      a.xnorm = as.xnorm;
+      a.csplit = as.csplit;
+      a.cnorm = as.cnorm;
+      a.pairs = as.pairs;
+      a.exact_list = as.exact;
+      a.ctl = as.ctl;
+      a.err = as.err;
+      a.arg = arg + b;
+      a.dist = dist ? dist + b : nullptr;
+      launches_ += launch_assign_tc(a, num_sms_, st_);
+    }
+  }
+
+  // Waits for the assignments; true (and the exact kernel from now on) when a
+  // bounded device wait gave up and they have to be made again.
+  bool assign_gave_up(Assigner& as) {
+    if (!as.on) return false;
+    HB_CUDA(cudaMemcpyAsync(err_host_, as.err, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    HB_CUDA(cudaStreamSynchronize(st_));
+    if (*err_host_ == 0) return false;
+    as.on = false;
+    return true;
+  }
+
   // ---- train: src/Index.cpp:381-425 + src/Clustering.cpp:14-152 ------------
 
   void train(size_t n, const float* x, bool lite) {
@@ -275,29 +388,39 @@ class IndexCore {
       xall.release();
       pts = xs.p;
     }
-    {
-      DevBuf<int64_t> cidx;
-      cidx.reserve(nlist_);
-      HB_CUDA(cudaMemcpyAsync(cidx.p, init.data(), nlist_ * sizeof(int64_t), cudaMemcpyHostToDevice, st_));
+    DevBuf<int64_t> cidx;
+    cidx.reserve(nlist_);
+    HB_CUDA(cudaMemcpyAsync(cidx.p, init.data(), nlist_ * sizeof(int64_t), cudaMemcpyHostToDevice, st_));
+    auto seed_centroids = [&]() {
       launch_gather_rows(pts, cidx.p, nlist_, static_cast<int>(dpad_), cent_.p, st_);
       ++launches_;
-      HB_CUDA(cudaStreamSynchronize(st_));
-    }
+    };
     DevBuf<int32_t> assign, counts;
     DevBuf<double> sums;
     assign.reserve(m);
     counts.reserve(nlist_);
     sums.reserve(nlist_ * dpad_);
-    for (int it = 0; it < niter; ++it) {
-      launch_l2_argmin(pts, static_cast<int>(m), cent_.p, static_cast<int>(nlist_), static_cast<int>(dpad_), assign.p,
-                       nullptr, st_);
-      HB_CUDA(cudaMemsetAsync(sums.p, 0, nlist_ * dpad_ * sizeof(double), st_));
-      HB_CUDA(cudaMemsetAsync(counts.p, 0, nlist_ * sizeof(int32_t), st_));
-      launch_kmeans_accumulate(pts, assign.p, m, static_cast<int>(d_), static_cast<int>(dpad_), sums.p, counts.p,
-                               st_);
-      launch_kmeans_update(sums.p, counts.p, static_cast<int>(nlist_), static_cast<int>(d_), static_cast<int>(dpad_),
-                           cent_.p, st_);
-      launches_ += 3;
+    Assigner as;
+    auto iterate = [&]() {
+      for (int it = 0; it < niter; ++it) {
+        assign_rows(as, pts, m, assign.p, nullptr);
+        HB_CUDA(cudaMemsetAsync(sums.p, 0, nlist_ * dpad_ * sizeof(double), st_));
+        HB_CUDA(cudaMemsetAsync(counts.p, 0, nlist_ * sizeof(int32_t), st_));
+        launch_kmeans_accumulate(pts, assign.p, m, static_cast<int>(d_), static_cast<int>(dpad_), sums.p, counts.p,
+                                 st_);
+        launch_kmeans_update(sums.p, counts.p, static_cast<int>(nlist_), static_cast<int>(d_), static_cast<int>(dpad_),
+                             cent_.p, st_);
+        launches_ += 2;
+      }
+    };
+    seed_centroids();
+    // The sample is split once for every iteration while its split rows fit
+    // 2 GiB.
+    assign_setup(as, m, (size_t(1) << 29) / static_cast<size_t>(assign_kpad(static_cast<int>(dpad_))), kAssignTcTrain);
+    iterate();
+    if (assign_gave_up(as)) {
+      seed_centroids();
+      iterate();
     }
     HB_CUDA(cudaStreamSynchronize(st_));
     trained_ = true;
@@ -319,8 +442,12 @@ class IndexCore {
     DevBuf<float> dist;
     assign.reserve(n);
     dist.reserve(n);
-    launch_l2_argmin(xpad.p, static_cast<int>(n), cent_.p, static_cast<int>(nlist_), static_cast<int>(dpad_), assign.p,
-                     dist.p, st_);
+    {
+      Assigner as;
+      assign_setup(as, n, size_t(1) << 17, kAssignTcAdd);
+      assign_rows(as, xpad.p, n, assign.p, dist.p);
+      if (assign_gave_up(as)) assign_rows(as, xpad.p, n, assign.p, dist.p);
+    }
     DevBuf<uint64_t> k0, k1;
     DevBuf<uint32_t> v0, v1;
     k0.reserve(n);
@@ -344,7 +471,7 @@ class IndexCore {
     otmp.reserve(ob);
     launch_list_offsets(assign.p, n, static_cast<int>(nlist_), list_off_.p, otmp.p, ob, st_);
     launch_row_norms(codes_.p, n, static_cast<int>(d_), static_cast<int>(dpad_), norms_.p, st_);
-    launches_ += 6;
+    launches_ += 5;
     host_off_.resize(nlist_ + 1);
     HB_CUDA(cudaMemcpyAsync(host_off_.data(), list_off_.p, (nlist_ + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
                             st_));

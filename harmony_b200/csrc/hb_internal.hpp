@@ -88,6 +88,37 @@ void launch_l2_matrix(const float* q, int nq, const float* rows, int nrows, int 
 void launch_l2_argmin(const float* q, int nq, const float* rows, int nrows, int dpad, int32_t* arg,
                       float* dist, cudaStream_t st);
 
+// The same for the queries sel[0 .. *nsel) (device; at most nmax) only.
+void launch_l2_argmin_list(const float* q, const int* sel, const int* nsel, int nmax, const float* rows, int nrows,
+                           int dpad, int32_t* arg, int num_sms, cudaStream_t st);
+
+// k_assign.cu: launch_l2_argmin's result through the tensor cores (3-term BF16
+// split, exact FP32 comparison of the close calls).
+struct AssignArgs {
+  const float* x;        // n x dpad points
+  int n;
+  int dpad;
+  const float* cent;     // nlist x dpad
+  int nlist;
+  const float* mu;       // dpad: the vector subtracted from points and centroids
+  const void* xsplit;    // n x 2*kpad BF16 [hi | lo] of x - mu (launch_split_points)
+  const float* xnorm;    // n: ||x - mu||^2
+  void* csplit;          // scratch, nlist x 2*kpad BF16
+  float* cnorm;          // scratch, nlist rounded up to 128
+  void* pairs;           // scratch, n x 8 bytes
+  int* exact_list;       // scratch, n
+  int* ctl;              // scratch, 4 ints: pairs, exact points, max ||c - mu||^2 (bits)
+  int* err;              // non-zero after a bounded wait gave up
+  int32_t* arg;          // out, n
+  float* dist;           // out, n (optional): exact distance to the centroid
+};
+int assign_kpad(int dpad);
+void launch_column_mean(const float* x, int rows, int dpad, float* mu, cudaStream_t st);
+void launch_split_points(const float* x, size_t n, int dpad, const float* mu, void* out, float* norm,
+                         cudaStream_t st);
+// Returns the number of this library's kernels it launched.
+int launch_assign_tc(const AssignArgs& a, int num_sms, cudaStream_t st);
+
 // Scan modes: the reference's three per-candidate accumulations.
 enum ScanMode : int { SCAN_PLAIN = 0, SCAN_CHUNK4 = 1, SCAN_DIMBLOCK = 2 };
 

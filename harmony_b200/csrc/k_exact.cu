@@ -211,12 +211,15 @@ __global__ void __launch_bounds__(kThreads) l2_matrix_kernel(const float* __rest
 // double-buffered tile; lexicographic (distance, row) minimum = the
 // reference's strict '<' scan in row order.  Distances >= FLT_MAX never
 // win; a query with no admissible row gets row 0 (Clustering's initial
-// closest_centroid, src/Clustering.cpp:103-104).
-template <int TV, int QT>
+// closest_centroid, src/Clustering.cpp:103-104).  LIST: the queries are
+// sel[0 .. *nsel), the CTAs striding over groups of QG of them (their number
+// is known on the device only).
+template <int TV, int QT, bool LIST>
 __global__ void __launch_bounds__(kThreads) l2_argmin_kernel(const float* __restrict__ q, int nq,
                                                              const float* __restrict__ rows, int nrows,
                                                              int dpad, int32_t* __restrict__ arg,
-                                                             float* __restrict__ dist) {
+                                                             float* __restrict__ dist, const int* __restrict__ sel,
+                                                             const int* __restrict__ nsel) {
   constexpr int G = kThreads / TV;
   constexpr int QG = G * QT;
   extern __shared__ __align__(16) float smem[];
@@ -224,56 +227,66 @@ __global__ void __launch_bounds__(kThreads) l2_argmin_kernel(const float* __rest
   float* sr0 = smem;
   float* sr1 = smem + TV * lds;
   float* sq = smem + 2 * TV * lds;
-  const int q0 = blockIdx.x * QG;
-  load_rows_async(sq, dpad, q + static_cast<size_t>(q0) * dpad, QG, nq - q0, dpad);
-  load_rows_async(sr0, lds, rows, TV, nrows, dpad);
-  cp_async_commit();
+  const int total = LIST ? *nsel : nq;
   const int r = threadIdx.x % TV;
   const int g = threadIdx.x / TV;
-  uint64_t best[QT];
-#pragma unroll
-  for (int i = 0; i < QT; ++i) best[i] = kEmpty;
-  const int ntiles = (nrows + TV - 1) / TV;
-  for (int t = 0; t < ntiles; ++t) {
-    float* cur = (t & 1) ? sr1 : sr0;
-    float* nxt = (t & 1) ? sr0 : sr1;
-    if (t + 1 < ntiles) {
-      const int rn = (t + 1) * TV;
-      load_rows_async(nxt, lds, rows + static_cast<size_t>(rn) * dpad, TV, nrows - rn, dpad);
+  for (int q0 = blockIdx.x * QG; q0 < total; q0 += gridDim.x * QG) {
+    if (LIST) {
+      const int cpr = dpad >> 2;
+      for (int idx = threadIdx.x; idx < QG * cpr; idx += kThreads) {
+        const int e = idx / cpr, c = idx - e * cpr;
+        const bool ok = q0 + e < total;
+        cp_async16(sq + e * dpad + c * 4, ok ? q + static_cast<size_t>(sel[q0 + e]) * dpad + c * 4 : q, ok);
+      }
+    } else {
+      load_rows_async(sq, dpad, q + static_cast<size_t>(q0) * dpad, QG, nq - q0, dpad);
     }
+    load_rows_async(sr0, lds, rows, TV, nrows, dpad);
     cp_async_commit();
-    cp_async_wait<1>();
-    __syncthreads();
-    float acc[QT];
-    dist_plain<QT>(cur + r * lds, sq + g * QT * dpad, dpad, dpad, acc);
-    const int row = t * TV + r;
-    if (row < nrows) {
+    uint64_t best[QT];
 #pragma unroll
-      for (int i = 0; i < QT; ++i)
-        if (acc[i] < FLT_MAX) {
-          const uint64_t key = make_key(acc[i], static_cast<uint32_t>(row));
-          best[i] = key < best[i] ? key : best[i];
-        }
-    }
-    __syncthreads();
-  }
-  // Reduce over the TV threads of each query group through shared memory
-  // (the row tiles are free now): red[(g * QT + i) * TV + r].
-  uint64_t* red = reinterpret_cast<uint64_t*>(sr0);
+    for (int i = 0; i < QT; ++i) best[i] = kEmpty;
+    const int ntiles = (nrows + TV - 1) / TV;
+    for (int t = 0; t < ntiles; ++t) {
+      float* cur = (t & 1) ? sr1 : sr0;
+      float* nxt = (t & 1) ? sr0 : sr1;
+      if (t + 1 < ntiles) {
+        const int rn = (t + 1) * TV;
+        load_rows_async(nxt, lds, rows + static_cast<size_t>(rn) * dpad, TV, nrows - rn, dpad);
+      }
+      cp_async_commit();
+      cp_async_wait<1>();
+      __syncthreads();
+      float acc[QT];
+      dist_plain<QT>(cur + r * lds, sq + g * QT * dpad, dpad, dpad, acc);
+      const int row = t * TV + r;
+      if (row < nrows) {
 #pragma unroll
-  for (int i = 0; i < QT; ++i) red[(g * QT + i) * TV + r] = best[i];
-  __syncthreads();
-  if (threadIdx.x < QG) {
-    uint64_t v = kEmpty;
-    for (int rr = 0; rr < TV; ++rr) {
-      const uint64_t o = red[threadIdx.x * TV + rr];
-      v = o < v ? o : v;
+        for (int i = 0; i < QT; ++i)
+          if (acc[i] < FLT_MAX) {
+            const uint64_t key = make_key(acc[i], static_cast<uint32_t>(row));
+            best[i] = key < best[i] ? key : best[i];
+          }
+      }
+      __syncthreads();
     }
-    const int qi = q0 + threadIdx.x;
-    if (qi < nq) {
+    // Reduce over the TV threads of each query group through shared memory
+    // (the row tiles are free now): red[(g * QT + i) * TV + r].
+    uint64_t* red = reinterpret_cast<uint64_t*>(sr0);
+#pragma unroll
+    for (int i = 0; i < QT; ++i) red[(g * QT + i) * TV + r] = best[i];
+    __syncthreads();
+    if (threadIdx.x < QG && q0 + static_cast<int>(threadIdx.x) < total) {
+      uint64_t v = kEmpty;
+      for (int rr = 0; rr < TV; ++rr) {
+        const uint64_t o = red[threadIdx.x * TV + rr];
+        v = o < v ? o : v;
+      }
+      const int qi = LIST ? sel[q0 + threadIdx.x] : q0 + static_cast<int>(threadIdx.x);
       arg[qi] = v == kEmpty ? 0 : static_cast<int32_t>(key_tie(v));
       if (dist) dist[qi] = v == kEmpty ? FLT_MAX : key_dist(v);
     }
+    __syncthreads();  // the tiles are reused by the next group
   }
 }
 
@@ -676,15 +689,23 @@ void matrix_launch(const float* q, int nq, const float* rows, int nrows, int dpa
 
 template <int TV, int QT>
 void argmin_launch(const float* q, int nq, const float* rows, int nrows, int dpad, int32_t* arg,
-                   float* dist, cudaStream_t st) {
+                   float* dist, const int* sel, const int* nsel, int max_ctas, cudaStream_t st) {
   constexpr int QG = (kThreads / TV) * QT;
   const size_t smem = (2 * static_cast<size_t>(TV) * (dpad + 4) + static_cast<size_t>(QG) * dpad) * 4;
   // The final reduction reuses the first row tile (kThreads * QT * 8 bytes,
   // below TV * (dpad + 4) * 4 for every shape launched here).
-  HB_CUDA(cudaFuncSetAttribute(l2_argmin_kernel<TV, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem)));
   dim3 grid((nq + QG - 1) / QG);
-  l2_argmin_kernel<TV, QT><<<grid, kThreads, smem, st>>>(q, nq, rows, nrows, dpad, arg, dist);
+  if (sel) {
+    HB_CUDA(cudaFuncSetAttribute(l2_argmin_kernel<TV, QT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(smem)));
+    grid.x = std::min<unsigned>(grid.x, static_cast<unsigned>(max_ctas));
+    l2_argmin_kernel<TV, QT, true><<<grid, kThreads, smem, st>>>(q, nq, rows, nrows, dpad, arg, dist, sel, nsel);
+  } else {
+    HB_CUDA(cudaFuncSetAttribute(l2_argmin_kernel<TV, QT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(smem)));
+    l2_argmin_kernel<TV, QT, false><<<grid, kThreads, smem, st>>>(q, nq, rows, nrows, dpad, arg, dist, nullptr,
+                                                                  nullptr);
+  }
   HB_CUDA(cudaGetLastError());
 }
 
@@ -701,15 +722,27 @@ void launch_l2_matrix(const float* q, int nq, const float* rows, int nrows, int 
   else matrix_launch<32, 2>(q, nq, rows, nrows, dpad, D, ldD, st);
 }
 
-void launch_l2_argmin(const float* q, int nq, const float* rows, int nrows, int dpad, int32_t* arg,
-                      float* dist, cudaStream_t st) {
+namespace {
+void argmin_dispatch(const float* q, int nq, const float* rows, int nrows, int dpad, int32_t* arg, float* dist,
+                     const int* sel, const int* nsel, int max_ctas, cudaStream_t st) {
   if (nq <= 0) return;
   HB_CHECK(nrows > 0, HB_ERR_STATE, "no centroids");
   HB_CHECK(dpad <= 1024, HB_ERR_INVALID, "dimension above 1024 is not supported");
-  if (dpad <= 128) argmin_launch<128, 8>(q, nq, rows, nrows, dpad, arg, dist, st);
-  else if (dpad <= 256) argmin_launch<64, 8>(q, nq, rows, nrows, dpad, arg, dist, st);
-  else if (dpad <= 512) argmin_launch<32, 4>(q, nq, rows, nrows, dpad, arg, dist, st);
-  else argmin_launch<16, 1>(q, nq, rows, nrows, dpad, arg, dist, st);
+  if (dpad <= 128) argmin_launch<128, 8>(q, nq, rows, nrows, dpad, arg, dist, sel, nsel, max_ctas, st);
+  else if (dpad <= 256) argmin_launch<64, 8>(q, nq, rows, nrows, dpad, arg, dist, sel, nsel, max_ctas, st);
+  else if (dpad <= 512) argmin_launch<32, 4>(q, nq, rows, nrows, dpad, arg, dist, sel, nsel, max_ctas, st);
+  else argmin_launch<16, 1>(q, nq, rows, nrows, dpad, arg, dist, sel, nsel, max_ctas, st);
+}
+}  // namespace
+
+void launch_l2_argmin(const float* q, int nq, const float* rows, int nrows, int dpad, int32_t* arg,
+                      float* dist, cudaStream_t st) {
+  argmin_dispatch(q, nq, rows, nrows, dpad, arg, dist, nullptr, nullptr, 0, st);
+}
+
+void launch_l2_argmin_list(const float* q, const int* sel, const int* nsel, int nmax, const float* rows, int nrows,
+                           int dpad, int32_t* arg, int num_sms, cudaStream_t st) {
+  argmin_dispatch(q, nmax, rows, nrows, dpad, arg, nullptr, sel, nsel, 2 * std::max(1, num_sms), st);
 }
 
 // ----------------------------------------------------------------------------
