@@ -709,6 +709,7 @@ class IndexCore {
     }
     int64_t tot = 0, mx = 0, mt = 0;
     for (int i = 0; i < last_nb_; ++i) {
+      if (cnt[i] >= kBoundOutOfRange) cnt[i] -= kBoundOutOfRange;  // a mark, not rows
       tot += cnt[i];
       mx = std::max<int64_t>(mx, cnt[i]);
       mt += m[i];

@@ -244,6 +244,7 @@ struct TcArgs {
   long long wait_budget;       // clock cycles a bounded mbarrier wait spends before giving up
 };
 constexpr int kRerankMaxCap = 8192;  // largest candidate buffer per query
+constexpr int kBoundOutOfRange = 1 << 29;  // added to the candidate count of a query outside the error bound's range
 constexpr int kFilterMaxK = 256;     // largest k of the bounded scan (its seed samples <= 256 rows)
 constexpr long long kDefaultWaitBudget = 2000000000LL;  // clock cycles before a device wait gives up
 size_t scan_bf16_smem_bytes(int kpad, int stages);

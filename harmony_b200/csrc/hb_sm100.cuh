@@ -115,6 +115,19 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }
 
+// True in one lane of the (converged) warp.  tcgen05.mma takes its
+// descriptors from uniform registers: a warp that runs its issue loop
+// converged, with only the instructions under this predicate, keeps them
+// there, while a loop run by one lane moves every operand over (about 90
+// cycles per instruction).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
+// A value every lane holds, in the form the compiler knows to be uniform.
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // ---- tcgen05 ----------------------------------------------------------------
 
 // Allocates `ncols` TMEM columns (power of two >= 32); the base address is

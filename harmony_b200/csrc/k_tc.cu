@@ -20,7 +20,9 @@
 //   | d(x) - D |                             <= (d + 3) u D
 // so |w(x) - d(x)| <= eps(q, l) = 1.0625 * (2 (2^-8 + 2^-10 + 2^-16) Q R
 // + (d + 3) u (Q^2 + R^2) + (d + 5) u (Q + R)^2), a bound per (query, list)
-// (d may be replaced by dpad >= d).  Residuals keep Q and R at the scale of
+// (d may be replaced by dpad >= d; 1e-30 is added for products the tensor
+// cores may flush to zero, and where eps is past 1e23 -- squares past about
+// 1e28 -- or NaN the query is searched exactly).  Residuals keep Q and R at the scale of
 // a list's spread, not of the data's distance from the origin.  Each row
 // therefore has a lower bound lb(x) = w(x) - eps(q, l_x) and an upper bound
 // ub(x) = w(x) + eps(q, l_x) of its distance (rounded outwards).  Let U be
@@ -55,18 +57,34 @@
 // bound.  The builders form the A tile, BF16(q - c_l) for the item's list,
 // from the FP32 queries.
 //
-// Warp roles (512 threads, 128 registers each), all running ahead of each
+// Warp roles (608 threads, 96 registers each), all running ahead of each
 // other through mbarriers, with no CTA-wide barrier between items:
 //   warps 0-11  three epilogue groups (each four warps = the four TMEM lane
 //               quarters); tile t of the CTA's global tile sequence goes to
 //               group t % 3 and accumulator t % 4 (three groups keep more
 //               warps on the epilogue, which bounds the kernel);
-//   warp 12     TMA producer of the B tiles;
-//   warp 13     MMA issuer; it also copies each tile's 128 row norms
-//               (a padded per-tile norm array) next to the accumulator;
-//   warps 14-15 item builders: fetch the next item from the global work
-//               counter, gather its BF16 query rows and bounds and write its
-//               A tile into the second A buffer while the current item runs.
+//   warps 12-15 item builders: form the item's A tile and its queries' bounds
+//               in the second A buffer while the current item runs, each warp
+//               a quarter of the rows;
+//   warp 16     TMA producer of the B tiles and of each tile's 128 row norms
+//               (a padded per-tile norm array);
+//   warp 17     MMA issuer (the warp converged, one lane issuing);
+//   warp 18     item fetcher: takes items from the global work counter and
+//               finds their list and queries two items ahead of the builders.
+// What bounds it: cycle counters in an instrumented copy (10M x 128, 10k
+// queries, nprobe 40, k 10) put the epilogue first (a group is busy 65 % of
+// the time, about 290 cycles per 32-column chunk and 2000 per chunk with an
+// admission, whose code is out of the instruction cache), then the tensor
+// pipe (34 %).  With two builder warps that also fetched the items, builders
+// were busy all the time on short lists, and a loop of one lane over the MMAs
+// took 97 cycles per instruction; splitting the builders' work over four
+// warps and a fetcher, nine shuffles for eight row sums, the converged issue
+// loop and two-column arithmetic took this search from 1404 to 1164 us, a
+// batch of 10k queries on 1M x 128 (nprobe 64, k 100) from 2224 to 1630 us and
+// 777 queries with their own nprobe on 4M x 96 from 804 to 611 us.
+// More than 16 warps hold the kernel to 96 registers per thread (five warps
+// on one SM sub-partition); a spill there costs more than the warps give, so
+// the builders keep one batch of rows in flight.
 // Every mbarrier wait is bounded (TcArgs::wait_budget cycles); on a timeout
 // the kernel records an error, the roles stop taking work, copies and MMAs
 // in flight are drained and TMEM is freed.
@@ -77,6 +95,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "hb_device.cuh"
 #include "hb_internal.hpp"
@@ -90,13 +109,15 @@ using namespace sm100;
 
 constexpr int kGroups = 3;                         // epilogue warpgroups, tile t -> group t % 3
 constexpr int kEpiThreads = 128;                   // threads per epilogue group (= queries per item)
-constexpr int kBuildWarps = 2;
-constexpr int kProdWarp = kGroups * 4, kMmaWarp = kGroups * 4 + 1, kBuildWarp0 = kGroups * 4 + 2;
-constexpr int kTcThreads = (kBuildWarp0 + kBuildWarps) * 32;
+constexpr int kBuildWarps = 4;                     // builder w forms A rows 32 w .. 32 w + 31
+constexpr int kBuildWarp0 = kGroups * 4;
+constexpr int kProdWarp = kBuildWarp0 + kBuildWarps, kMmaWarp = kProdWarp + 1, kFetchWarp = kProdWarp + 2;
+constexpr int kTcThreads = (kFetchWarp + 1) * 32;
 constexpr int kTile = 128;     // rows per B tile, queries per item (M)
 constexpr int kMaxStages = 4;
 constexpr int kAcc = 4;                            // TMEM accumulators of 128 columns, tile t -> t % 4
-constexpr size_t kSmemCap = 225 * 1024;            // dynamic shared memory budget
+constexpr int kNormSlots = 8;                      // tiles whose row norms sit in shared memory
+constexpr size_t kSmemCap = 226 * 1024;            // dynamic shared memory budget
 constexpr int kTightK = kFilterTightK;             // largest k whose bound tightens during the scan
 constexpr int kStage = 8;                          // admitted keys staged per epilogue thread before a flush
 
@@ -107,7 +128,20 @@ __device__ __forceinline__ float pair_eps(float cd, float R, int d) {
   const float Q = sqrtf(cd) * 1.0001f + 1e-30f;
   const float u = 5.9604645e-8f;  // 2^-24
   const float c1 = 0.00390625f + 0.0009765625f + 1.52587890625e-5f;
-  return 1.0625f * (2.0f * c1 * Q * R + (d + 3) * u * (R * R + Q * Q) + (d + 5) * u * (Q + R) * (Q + R));
+  return 1.0625f * (2.0f * c1 * Q * R + (d + 3) * u * (R * R + Q * Q) + (d + 5) * u * (Q + R) * (Q + R)) + 1e-30f;
+}
+
+// (a, b) <- n - 2 (a, b), both halves rounded on their own.
+__device__ __forceinline__ void fma2_m2(uint32_t& a, uint32_t& b, uint64_t n) {
+  asm("{\n .reg .b64 t, m;\n mov.b64 t, {%0, %1};\n mov.b64 m, {%3, %3};\n fma.rn.f32x2 t, t, m, %2;\n"
+      " mov.b64 {%0, %1}, t;\n}\n"
+      : "+r"(a), "+r"(b)
+      : "l"(n), "r"(0xC0000000u));
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float d;
+  asm("min.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
 }
 
 struct ItemDesc {
@@ -121,13 +155,17 @@ struct TcShared {
   uint64_t empty[kMaxStages];
   uint64_t accf[kAcc];
   uint64_t acce[kAcc];
-  uint64_t normf[kAcc];
+  uint64_t normf[kNormSlots];
   uint64_t itemf[2];
   uint64_t aempty[2];
+  uint64_t ffull[2];
+  uint64_t ffree[2];
   uint64_t drain;
   uint32_t tmem;
-  ItemDesc desc[2];
+  ItemDesc desc[2];   // the items of the two A buffers
+  ItemDesc fdesc[2];  // items fetched ahead of the builders
 };
+static_assert(kNormSlots >= kMaxStages + kAcc, "a norm slot is free when its stage is (see the producer)");
 
 // Next work item from the global counter, by one warp: lane 0 takes the
 // item, the warp finds its list with a 32-way search of item_off (three
@@ -184,16 +222,16 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const uint32_t tile_bytes = static_cast<uint32_t>(kpad / 64) * kblk_bytes;
   uint8_t* Abuf = smem;                                    // [2] A tiles
   uint8_t* stages = smem + 2 * tile_bytes;                 // [S] B tiles
-  float* nrm = reinterpret_cast<float*>(stages + static_cast<size_t>(S) * tile_bytes);  // [kAcc][128]
-  int* meta_q = reinterpret_cast<int*>(nrm + kAcc * kTile);                 // [2][128]
+  float* nrm = reinterpret_cast<float*>(stages + static_cast<size_t>(S) * tile_bytes);  // [kNormSlots][128]
+  int* meta_q = reinterpret_cast<int*>(nrm + kNormSlots * kTile);           // [2][128]
   float* meta_thr = reinterpret_cast<float*>(meta_q + 2 * kTile);           // [2][128]
   float* meta_eps = meta_thr + 2 * kTile;                                   // [2][128] eps(q, l)
   float* meta_cd = meta_eps + 2 * kTile;                                    // [2][128] ||q - c_l||^2
-  float* s_cent = meta_cd + 2 * kTile;                                      // [2][128] the item's centroid
-  uint64_t* staging = reinterpret_cast<uint64_t*>(s_cent + 2 * kTile);      // [kGroups][kStage][128]
+  int* fetch_q = reinterpret_cast<int*>(meta_cd + 2 * kTile);               // [2][128] queries fetched ahead
+  uint64_t* staging = reinterpret_cast<uint64_t*>(fetch_q + 2 * kTile);     // [kGroups][kStage][128]
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
+  const int warp = warp_uniform(tid >> 5), lane = tid & 31;
   int* err = a.err;
 
   if (warp == kMmaWarp) tmem_alloc(&sh.tmem, 512);
@@ -205,9 +243,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     for (int b = 0; b < kAcc; ++b) {
       mbar_init(&sh.accf[b], 1);
       mbar_init(&sh.acce[b], kEpiThreads);
-      mbar_init(&sh.normf[b], 1);
     }
+    for (int b = 0; b < kNormSlots; ++b) mbar_init(&sh.normf[b], 1);
     for (int i = 0; i < 2; ++i) {
+      mbar_init(&sh.ffull[i], 32);
+      mbar_init(&sh.ffree[i], kBuildWarps);
       mbar_init(&sh.itemf[i], kBuildWarps * 32);
       // A buffer / item slot free: the MMA warp's commit, the producer and
       // every epilogue thread.
@@ -223,90 +263,135 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const uint32_t tmem = sh.tmem;
   const int64_t total_items = a.item_off[a.nlist];
 
-  if (warp >= kBuildWarp0) {
-    // ---- item builders ---------------------------------------------------
-    const int bt = tid - kBuildWarp0 * 32;
-    constexpr int kBt = kBuildWarps * 32;
-    const int bw = bt >> 5;  // builder warp
-    ItemDesc nd;
-    nd.ntiles = -1;
-    if (bw == 0) nd = fetch_item(a, total_items, lane);
+  if (warp == kFetchWarp) {
+    // ---- item fetcher: two items ahead of the builders ---------------------
+    // The counter, the search of the item's list and its query list are a
+    // chain of a dozen dependent loads (about 6000 cycles), here off the
+    // builders' path.
+    for (uint32_t it = 0;; ++it) {
+      const int fb = static_cast<int>(it & 1u);
+      bool ok = mbar_wait(&sh.ffree[fb], ((it >> 1) & 1u) ^ 1u, err, 35, budget);
+      ok = __all_sync(0xffffffffu, ok);
+      ItemDesc d;
+      d.ntiles = -1;
+      if (ok) d = fetch_item(a, total_items, lane);
+      if (d.ntiles >= 0) {
+        // Row r holds the group's query (r % 32) * 4 + r / 32, so the queries
+        // of a partial group spread over the four warps of an epilogue group
+        // and over the builders.
+        const int64_t qbase = a.list_qoff[d.list] + static_cast<int64_t>(d.group) * kTile;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = 4 * lane + u;
+          fetch_q[fb * kTile + 32 * u + lane] =
+              i < d.qcnt ? static_cast<int>(static_cast<uint32_t>(a.list_q[qbase + i]) >> 16) : -1;
+        }
+      }
+      if (lane == 0) sh.fdesc[fb] = d;
+      mbar_arrive(&sh.ffull[fb]);
+      if (d.ntiles < 0) break;
+    }
+  } else if (warp >= kBuildWarp0 && warp < kBuildWarp0 + kBuildWarps) {
+    // ---- item builders: warp bw, A rows 32 bw .. 32 bw + 31 ------------------
+    const int bw = warp - kBuildWarp0;
+    const int c0 = 4 * lane;
+    const bool col_in = c0 < a.dpad, col_k = c0 < kpad;
+    // Byte offset of this lane's four columns in A row 0, the 16-byte piece
+    // taken with the row's swizzle below.
+    const uint32_t col_off = static_cast<uint32_t>(c0 >> 6) * kblk_bytes + static_cast<uint32_t>((c0 & 7) * 2);
+    const uint32_t piece = static_cast<uint32_t>((c0 & 63) >> 3);
     for (uint32_t it = 0;; ++it) {
       const int ab = static_cast<int>(it & 1u);
-      if (bt == 0) {
-        if (!mbar_wait(&sh.aempty[ab], ((it >> 1) & 1u) ^ 1u, err, 31, budget)) nd.ntiles = -1;
-        sh.desc[ab] = nd;
-      }
-      asm volatile("bar.sync 3, %0;\n" ::"n"(kBt) : "memory");
-      const ItemDesc d = sh.desc[ab];
+      bool ok = mbar_wait(&sh.ffull[ab], (it >> 1) & 1u, err, 36, budget);
+      ok = __all_sync(0xffffffffu, ok);
+      ItemDesc d = sh.fdesc[ab];
+      if (!ok) d.ntiles = -1;
+      int my_q = -1;
+      uint32_t my_thr = 0u;
+      float4 cv = make_float4(0.f, 0.f, 0.f, 0.f), xa[8];
+      float Rl = 0.0f;
+      // Eight rows of a batch: their loads in flight together.
+      auto load8 = [&](int base, float4(&x)[8]) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int q = __shfl_sync(0xffffffffu, my_q, base + j);
+          x[j] = q >= 0 && col_in ? __ldg(reinterpret_cast<const float4*>(a.q + static_cast<size_t>(q) * a.dpad + c0))
+                                  : cv;  // q - c = 0 for a padding column
+        }
+      };
       if (d.ntiles >= 0) {
-        const int64_t qbase = a.list_qoff[d.list] + static_cast<int64_t>(d.group) * kTile;
-        float* cen = s_cent + ab * kTile;
-        for (int c = bt; c < kpad; c += kBt) cen[c] = c < a.dpad ? a.cent[static_cast<size_t>(d.list) * a.dpad + c] : 0.0f;
-        // Row r holds the group's query (r % 32) * 4 + r / 32, so the queries
-        // of a partial group spread over the four epilogue warps.  Two rows
-        // per thread, their loads issued together.
-        int q2[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = bt + h * kBt;
-          const int i = (r & 31) * 4 + (r >> 5);
-          q2[h] = i < d.qcnt ? static_cast<int>(static_cast<uint32_t>(a.list_q[qbase + i]) >> 16) : -1;
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = bt + h * kBt;
-          const int q = q2[h];
-          // The query's bound as other items have lowered it so far.
-          meta_q[ab * kTile + r] = q;
-          meta_thr[ab * kTile + r] =
-              q >= 0 ? ordered_to_float(*reinterpret_cast<volatile uint32_t*>(a.thr + q)) : -INFINITY;
-        }
-        asm volatile("bar.sync 3, %0;\n" ::"n"(kBt) : "memory");
-        // A row r = BF16(q - c_l) of the row's query, and ||q - c_l||^2: a
-        // warp per row (lane = 4 consecutive columns), 16 rows in flight.
+        my_q = fetch_q[ab * kTile + 32 * bw + lane];
+        if (col_in) cv = *reinterpret_cast<const float4*>(a.cent + static_cast<size_t>(d.list) * a.dpad + c0);
+        Rl = a.rmax[d.list];
+        // The query's bound as other items have lowered it so far.
+        if (my_q >= 0) my_thr = *reinterpret_cast<volatile uint32_t*>(a.thr + my_q);
+        load8(0, xa);
+      }
+      // A buffer ab, its meta data and its descriptor are free.
+      ok = mbar_wait(&sh.aempty[ab], ((it >> 1) & 1u) ^ 1u, err, 31, budget);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) d.ntiles = -1;
+      if (bw == 0 && lane == 0) sh.desc[ab] = d;
+      if (d.ntiles >= 0) {
+        meta_q[ab * kTile + 32 * bw + lane] = my_q;
+        meta_thr[ab * kTile + 32 * bw + lane] = my_q >= 0 ? ordered_to_float(my_thr) : -INFINITY;
+        // A row r = BF16(q - c_l) of the row's query, and ||q - c_l||^2, eight
+        // rows at a time (lane = 4 consecutive columns), the next eight
+        // loading meanwhile.  Rows without a query are left as they are:
+        // their TMEM lanes belong to no query and the epilogue ignores them.
         uint8_t* A = Abuf + ab * tile_bytes;
-        const int c0 = 4 * lane;
-        const bool col_in = c0 < a.dpad, col_k = c0 < kpad;
-        const float4 cv = col_k ? *reinterpret_cast<const float4*>(cen + c0) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float Rl = a.rmax[d.list];
-        constexpr int kRowsInFlight = 8;
-        // Rows without a query are left as they are: their TMEM lanes belong
-        // to no query and the epilogue ignores them.  A block's rows with a
-        // query come first (query (r % 32) * 4 + r / 32 grows with r % 32).
-        for (int r0 = bw; r0 < kTile; r0 += kBuildWarps * kRowsInFlight) {
-          if (meta_q[ab * kTile + r0] < 0) continue;
-          float4 x[kRowsInFlight];
+        auto batch = [&](int base, const float4(&x)[8]) {
+          float cds[8];
+          const uint32_t row_off = static_cast<uint32_t>(32 * bw + base) * 128u + col_off;
 #pragma unroll
-          for (int j = 0; j < kRowsInFlight; ++j) {
-            const int q = meta_q[ab * kTile + r0 + j * kBuildWarps];
-            x[j] = q >= 0 && col_in ? __ldg(reinterpret_cast<const float4*>(a.q + static_cast<size_t>(q) * a.dpad + c0))
-                                    : cv;  // q - c = 0 for a padding column
-          }
-#pragma unroll
-          for (int j = 0; j < kRowsInFlight; ++j) {
-            const int r = r0 + j * kBuildWarps;
-            if (meta_q[ab * kTile + r] < 0) break;
+          for (int j = 0; j < 8; ++j) {
             const float v0 = x[j].x - cv.x, v1 = x[j].y - cv.y, v2 = x[j].z - cv.z, v3 = x[j].w - cv.w;
-            float cd = fmaf(v3, v3, fmaf(v2, v2, fmaf(v1, v1, v0 * v0)));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) cd += __shfl_xor_sync(0xffffffffu, cd, o);
+            cds[j] = fmaf(v3, v3, fmaf(v2, v2, fmaf(v1, v1, v0 * v0)));
             if (col_k) {
               __nv_bfloat162 p01 = __floats2bfloat162_rn(v0, v1), p23 = __floats2bfloat162_rn(v2, v3);
-              *reinterpret_cast<uint2*>(A + sw128_offset_bf16(r, c0, kblk_bytes)) =
+              *reinterpret_cast<uint2*>(A + row_off + j * 128 + ((piece ^ static_cast<uint32_t>(j)) << 4)) =
                   make_uint2(*reinterpret_cast<uint32_t*>(&p01), *reinterpret_cast<uint32_t*>(&p23));
             }
-            if (lane == 0) {
-              meta_cd[ab * kTile + r] = cd;
-              meta_eps[ab * kTile + r] = pair_eps(cd, Rl, a.dpad);  // eps(q, l) of this row's query
-            }
           }
+          // The eight rows' sums over the lanes in nine shuffles (each step
+          // halves the rows a lane carries; five shuffles a row would be
+          // forty), ending with row (lane >> 2)'s in every fourth lane, where
+          // its eps is formed.
+          const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0, h4 = (lane & 4) != 0;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            cds[j] = (h16 ? cds[j + 4] : cds[j]) + __shfl_xor_sync(0xffffffffu, h16 ? cds[j] : cds[j + 4], 16);
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            cds[j] = (h8 ? cds[j + 2] : cds[j]) + __shfl_xor_sync(0xffffffffu, h8 ? cds[j] : cds[j + 2], 8);
+          float cd = (h4 ? cds[1] : cds[0]) + __shfl_xor_sync(0xffffffffu, h4 ? cds[0] : cds[1], 4);
+          cd += __shfl_xor_sync(0xffffffffu, cd, 2);
+          cd += __shfl_xor_sync(0xffffffffu, cd, 1);
+          const int q = __shfl_sync(0xffffffffu, my_q, base + (lane >> 2));
+          if ((lane & 3) == 0 && q >= 0) {
+            const int r = 32 * bw + base + (lane >> 2);
+            const float eps = pair_eps(cd, Rl, a.dpad);  // eps(q, l) of this row's query
+            meta_cd[ab * kTile + r] = cd;
+            meta_eps[ab * kTile + r] = eps;
+            // Outside the bound's range (squares past about 1e28, infinities
+            // and NaN in the query or the list, all of which show in eps):
+            // marked as overflowed, so the query is searched exactly.
+            if (!(eps < 1e23f)) atomicMax(a.cand_cnt + q, kBoundOutOfRange);
+          }
+        };
+        // Rows with a query come first in every 32.
+        const unsigned have = __ballot_sync(0xffffffffu, my_q >= 0);
+#pragma unroll 1
+        for (int base = 0; base < 32 && ((have >> base) & 1u); base += 8) {
+          batch(base, xa);
+          if (base < 24) load8(base + 8, xa);
         }
         fence_proxy_async_smem();
       }
       mbar_arrive(&sh.itemf[ab]);
       if (d.ntiles < 0) break;
-      if (bw == 0) nd = fetch_item(a, total_items, lane);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.ffree[ab]);
     }
   } else if (warp == kProdWarp) {
     // ---- TMA producer ------------------------------------------------------
@@ -330,6 +415,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           mbar_arrive_expect_tx(&sh.full[s], tile_bytes);
           const int r = d.row0 + t * kTile;
           for (int kb = 0; kb < kpad / 64; ++kb) tma_load_2d(dst + kb * kblk_bytes, &tmap, kb * 64, r, &sh.full[s]);
+          // The tile's 128 row norms (a padded per-tile array) into slot
+          // p_idx % kNormSlots.  Its last reader is done: stage s was free, so
+          // the MMAs of tile p_idx - S were issued, after the epilogue had
+          // released the accumulator -- and the norms -- of tile
+          // p_idx - S - kAcc >= p_idx - kNormSlots.
+          const uint32_t ns = p_idx % kNormSlots;
+          mbar_arrive_expect_tx(&sh.normf[ns], kTile * 4);
+          bulk_load(nrm + ns * kTile, a.tile_norm + (d.tile0 + t) * kTile, kTile * 4, &sh.normf[ns]);
         }
         if (!ok) break;
       }
@@ -338,59 +431,63 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       for (uint32_t i = first; i < p_idx; ++i)
         mbar_wait(&sh.full[i % static_cast<uint32_t>(S)], (i / static_cast<uint32_t>(S)) & 1u, nullptr, 0,
                   200000000LL);
+      for (uint32_t i = p_idx > kNormSlots ? p_idx - kNormSlots : 0u; i < p_idx; ++i)
+        mbar_wait(&sh.normf[i % kNormSlots], (i / kNormSlots) & 1u, nullptr, 0, 200000000LL);
     }
   } else if (warp == kMmaWarp) {
-    // ---- MMA issuer (+ per-tile norms) --------------------------------------
-    if (lane == 0) {
-      const uint32_t idesc = idesc_bf16_f32(kTile, kTile);
-      const int nk = kpad / 16;
-      uint32_t m_idx = 0;
-      for (uint32_t it = 0;; ++it) {
-        const int ab = static_cast<int>(it & 1u);
-        if (!mbar_wait(&sh.itemf[ab], (it >> 1) & 1u, err, 33, budget)) break;
-        const ItemDesc d = sh.desc[ab];
-        if (d.ntiles < 0) break;
+    // ---- MMA issuer: the warp converged, one lane issuing --------------------
+    const uint32_t idesc = idesc_bf16_f32(kTile, kTile);
+    const uint32_t tm = static_cast<uint32_t>(warp_uniform(static_cast<int>(tmem)));
+    const uint32_t a_base = static_cast<uint32_t>(warp_uniform(static_cast<int>(smem_u32(Abuf))));
+    const uint32_t b_base = static_cast<uint32_t>(warp_uniform(static_cast<int>(smem_u32(stages))));
+    uint32_t m_idx = 0;
+    uint32_t s = 0, sp = 0;  // stage of tile m_idx and its phase parity
+    // One tile's MMAs.
+    auto issue = [&](auto nk, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc) {
+#pragma unroll
+      for (int k = 0; k < decltype(nk)::value; ++k) {
+        // The start-address field is (address >> 4) in the low 14 bits.
+        const uint64_t off16 = static_cast<uint64_t>((k >> 2) * (kTile * 128 / 16) + (k & 3) * 2);
+        mma_bf16(d_tmem, a_desc + off16, b_desc + off16, idesc, k > 0 ? 1u : 0u);
+      }
+    };
+    for (uint32_t it = 0;; ++it) {
+      const uint32_t ab = it & 1u;
+      bool ok = mbar_wait(&sh.itemf[ab], (it >> 1) & 1u, err, 33, budget);
+      const int ntiles = warp_uniform(sh.desc[ab].ntiles);
+      if (!__all_sync(0xffffffffu, ok) || ntiles < 0) break;
+      tc_fence_after();
+      const uint64_t a_desc = desc_sw128(a_base + ab * tile_bytes);
+      for (int t = 0; t < ntiles; ++t, ++m_idx) {
+        ok = mbar_wait(&sh.full[s], sp, err, 12, budget);
+        const uint32_t b = m_idx % kAcc;
+        ok = ok && mbar_wait(&sh.acce[b], ((m_idx / kAcc) & 1u) ^ 1u, err, 13, budget);
+        if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_after();
-        const uint64_t a_desc = desc_sw128(smem_u32(Abuf + ab * tile_bytes));
-        bool ok = true;
-        for (int t = 0; t < d.ntiles; ++t, ++m_idx) {
-          const int s = static_cast<int>(m_idx % static_cast<uint32_t>(S));
-          if (!mbar_wait(&sh.full[s], (m_idx / static_cast<uint32_t>(S)) & 1u, err, 12, budget)) {
-            ok = false;
-            break;
-          }
-          const int b = static_cast<int>(m_idx % kAcc);
-          if (!mbar_wait(&sh.acce[b], ((m_idx / kAcc) & 1u) ^ 1u, err, 13, budget)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          mbar_arrive_expect_tx(&sh.normf[b], kTile * 4);
-          bulk_load(nrm + b * kTile, a.tile_norm + (d.tile0 + t) * kTile, kTile * 4, &sh.normf[b]);
-          const uint64_t b_desc = desc_sw128(smem_u32(stages + s * tile_bytes));
-          const uint32_t d_tmem = tmem + static_cast<uint32_t>(b * kTile);
-          for (int k = 0; k < nk; ++k) {
-            // The start-address field is (address >> 4) in the low 14 bits.
-            const uint64_t off16 = (static_cast<uint32_t>(k >> 2) * kblk_bytes + static_cast<uint32_t>(k & 3) * 32u) >> 4;
-            mma_bf16(d_tmem, a_desc + off16, b_desc + off16, idesc, k > 0 ? 1u : 0u);
-          }
+        const uint64_t b_desc = desc_sw128(b_base + s * tile_bytes);
+        if (elect_one()) {
+          if (kpad == 128)
+            issue(std::integral_constant<int, 8>{}, tm + b * kTile, a_desc, b_desc);
+          else
+            issue(std::integral_constant<int, 4>{}, tm + b * kTile, a_desc, b_desc);
           mma_commit(&sh.empty[s]);
           mma_commit(&sh.accf[b]);
         }
-        // A buffer ab is free once these MMAs have completed.
-        mma_commit(&sh.aempty[ab]);
-        if (!ok) break;
+        __syncwarp();
+        if (++s == static_cast<uint32_t>(S)) {
+          s = 0;
+          sp ^= 1u;
+        }
       }
-      // Drain: every MMA done before TMEM is released, and the last norm copy
-      // of each accumulator landed (at most one per accumulator is pending:
-      // the next one waits for the epilogue to release the accumulator).
-      mma_commit(&sh.drain);
-      mbar_wait(&sh.drain, 0, nullptr, 0, 200000000LL);
-      for (int b = 0; b < kAcc; ++b) {
-        const uint32_t copies = m_idx > static_cast<uint32_t>(b) ? (m_idx - static_cast<uint32_t>(b) + kAcc - 1) / kAcc : 0u;
-        if (copies) mbar_wait(&sh.normf[b], (copies - 1u) & 1u, nullptr, 0, 200000000LL);
-      }
+      // A buffer ab is free once these MMAs have completed.
+      if (elect_one()) mma_commit(&sh.aempty[ab]);
+      __syncwarp();
+      if (!__all_sync(0xffffffffu, ok)) break;
     }
+    // Drain: every MMA done before TMEM is released.
+    if (elect_one()) mma_commit(&sh.drain);
+    __syncwarp();
+    mbar_wait(&sh.drain, 0, nullptr, 0, 200000000LL);
   } else {
     // ---- epilogue: thread = query (TMEM lane etid) ---------------------------
     const int grp = warp >> 2;
@@ -423,16 +520,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         return fminf(__fadd_ru(__fsub_ru(te, cd), 1e-6f * (fminf(fabsf(te), 1e30f) + cd)), FLT_MAX);
       };
       float thr_s = shifted(thr);
-      // The KT smallest upper bounds this thread knows for the query,
-      // ascending, and the k-th of them (KT = 0: no tightening).  A published
-      // U says that k rows have upper bounds <= U, so U may stand in for k of
-      // them: the k-th of a mix of stand-ins and real values is the k-th of k
-      // distinct rows or U itself.  Only a value under the current k-th
-      // changes the set.
+      // The k smallest upper bounds this thread knows for the query,
+      // ascending, in the last k of KT places (the others hold -inf, which no
+      // insertion moves), so the k-th is the last place whatever k is (KT = 0:
+      // no tightening).  A published U says that k rows have upper bounds
+      // <= U, so U may stand in for k of them: the k-th of a mix of stand-ins
+      // and real values is the k-th of k distinct rows or U itself.  Only a
+      // value under the current k-th changes the set.
       float best[KB];
-      float kth_loc = thr < FLT_MAX ? thr : INFINITY;
+      const float top0 = thr < FLT_MAX ? thr : INFINITY;
 #pragma unroll
-      for (int i = 0; i < KB; ++i) best[i] = kth_loc;
+      for (int i = 0; i < KB; ++i) best[i] = i >= KB - a.k ? top0 : -INFINITY;
       uint64_t* cbuf = a.cand + static_cast<size_t>(my_q < 0 ? 0 : my_q) * a.cap;
       uint32_t* ubuf = a.cand_ub + static_cast<size_t>(my_q < 0 ? 0 : my_q) * a.cap;
       // Admitted keys (lower bound, position) wait here (stride kEpiThreads:
@@ -473,24 +571,40 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         pend = false;
         ns = 0;
       };
+      // Admission of one column value under the bound.
+      auto admit = [&](float wv, uint32_t pos) {
+        stage((static_cast<uint64_t>(ordered_bits(wv)) << 32) | pos);
+        const float ub = __fadd_ru(wv, eps);
+        if (KT > 0 && ub < best[KB - 1]) {
+          float v = ub;
+#pragma unroll
+          for (int i = 0; i < KB; ++i) {
+            const float o = best[i];
+            best[i] = fminf(o, v);
+            v = fmaxf(o, v);
+          }
+          if (best[KB - 1] < thr) {
+            thr = best[KB - 1];
+            thr_s = shifted(thr);
+            atomicMin(a.thr + my_q, ordered_bits(thr));  // shared at once (no return value used)
+          }
+        }
+      };
       // One 32-column chunk of the accumulator in r: w' = ||r||^2 - 2 q'.r
-      // (rows past the list carry an infinite norm), their minimum against
-      // the bound, and the admission of the columns under it.
+      // (rows past the list carry an infinite norm) two columns per
+      // instruction, their minimum (three-input minima) against the bound, and
+      // the admission of the columns under it.
       auto chunk = [&](uint32_t(&r)[32], const float* nb, uint32_t pos0) {
-        const float4* n4 = reinterpret_cast<const float4*>(nb);
+        const ulonglong2* n2 = reinterpret_cast<const ulonglong2*>(nb);
         float mn = INFINITY;
 #pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          const float4 nv = n4[j4];
-          const float v0 = fmaf(-2.0f, __uint_as_float(r[4 * j4 + 0]), nv.x);
-          const float v1 = fmaf(-2.0f, __uint_as_float(r[4 * j4 + 1]), nv.y);
-          const float v2 = fmaf(-2.0f, __uint_as_float(r[4 * j4 + 2]), nv.z);
-          const float v3 = fmaf(-2.0f, __uint_as_float(r[4 * j4 + 3]), nv.w);
-          r[4 * j4 + 0] = __float_as_uint(v0);
-          r[4 * j4 + 1] = __float_as_uint(v1);
-          r[4 * j4 + 2] = __float_as_uint(v2);
-          r[4 * j4 + 3] = __float_as_uint(v3);
-          mn = fminf(mn, fminf(fminf(v0, v1), fminf(v2, v3)));
+        for (int g = 0; g < 8; ++g) {
+          uint32_t* v = r + 4 * g;
+          const ulonglong2 nv = n2[g];
+          fma2_m2(v[0], v[1], nv.x);
+          fma2_m2(v[2], v[3], nv.y);
+          mn = min3(mn, __uint_as_float(v[0]), __uint_as_float(v[1]));
+          mn = min3(mn, __uint_as_float(v[2]), __uint_as_float(v[3]));
         }
         if (my_q >= 0 && mn <= thr_s) {
           uint32_t mq[4] = {0u, 0u, 0u, 0u};
@@ -510,31 +624,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             for (int i = 0; i < 4; ++i) t4[i] = (j & 4) ? t8[2 * i + 1] : t8[2 * i];
 #pragma unroll
             for (int i = 0; i < 2; ++i) t2[i] = (j & 8) ? t4[2 * i + 1] : t4[2 * i];
-            const float wv = cd + __uint_as_float((j & 16) ? t2[1] : t2[0]);
-            stage((static_cast<uint64_t>(ordered_bits(wv)) << 32) | (pos0 + static_cast<uint32_t>(j)));
-            const float ub = __fadd_ru(wv, eps);
-            if (KT > 0 && ub < kth_loc) {
-              // Insert into the ascending KT smallest upper bounds; their k-th
-              // is a new U.
-              float v = ub;
-#pragma unroll
-              for (int i = 0; i < KB; ++i) {
-                const float o = best[i];
-                best[i] = fminf(o, v);
-                v = fmaxf(o, v);
-              }
-              // best is ascending: its k-th entry is the largest of the first k
-              // (a max, so the array stays in registers).
-              float kth = best[0];
-#pragma unroll
-              for (int i = 1; i < KB; ++i) kth = i < a.k ? fmaxf(kth, best[i]) : kth;
-              kth_loc = kth;
-              if (kth < thr) {
-                thr = kth;
-                thr_s = shifted(thr);
-                atomicMin(a.thr + my_q, ordered_bits(thr));  // shared at once (no return value used)
-              }
-            }
+            admit(cd + __uint_as_float((j & 16) ? t2[1] : t2[0]), pos0 + static_cast<uint32_t>(j));
           }
         }
       };
@@ -546,21 +636,22 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const uint32_t gt = G + static_cast<uint32_t>(t);  // the CTA's global tile index
         const int b = static_cast<int>(gt % kAcc);
         const uint32_t par = (gt / kAcc) & 1u;
-        ok = ok && mbar_wait(&sh.accf[b], par, err, 14, budget) && mbar_wait(&sh.normf[b], par, err, 15, budget);
+        const uint32_t nslot = gt % kNormSlots;
+        ok = ok && mbar_wait(&sh.accf[b], par, err, 14, budget) &&
+             mbar_wait(&sh.normf[nslot], (gt / kNormSlots) & 1u, err, 15, budget);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
         if (my_q >= 0 && ordered_to_float(g_thr) < thr) {
           thr = ordered_to_float(g_thr);
           thr_s = shifted(thr);
           if (KT > 0) {
-            kth_loc = fminf(kth_loc, thr);
 #pragma unroll
-            for (int i = 0; i < KB; ++i) best[i] = fminf(best[i], kth_loc);
+            for (int i = 0; i < KB; ++i) best[i] = fminf(best[i], thr);
           }
         }
         g_thr = my_q >= 0 ? *reinterpret_cast<volatile uint32_t*>(a.thr + my_q) : 0u;
         if (ok && warp_on) {
-          const float* nb = nrm + b * kTile;
+          const float* nb = nrm + nslot * kTile;
           const uint32_t col = tmem + lane_base + static_cast<uint32_t>(b * kTile);
           const uint32_t pos_t = static_cast<uint32_t>(d.row0 + t * kTile);
           // One register set (a second one, to load the next chunk while this
@@ -1125,7 +1216,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 size_t scan_bf16_smem_bytes(int kpad, int stages) {
   const size_t tile = static_cast<size_t>(kpad / 64) * kTile * 128;
-  return 1024 + tile * (2 + stages) + static_cast<size_t>(kAcc) * kTile * 4 + 2 * kTile * (4 + 4 + 4 + 4 + 4) +
+  return 1024 + tile * (2 + stages) + static_cast<size_t>(kNormSlots) * kTile * 4 + 2 * kTile * (4 + 4 + 4 + 4 + 4) +
          static_cast<size_t>(kGroups) * kStage * kEpiThreads * 8;
 }
 
