@@ -54,6 +54,14 @@ bool is_device_ptr(const void* p) {
 // 128 8.1 -> 6.4 ms, 100k x 500 x 128 3.2 -> 3.7 ms.
 constexpr double kAssignTcTrain = 5.0e8;
 constexpr double kAssignTcAdd = 1.5e10;
+// (query, row) pairs from which a plain FP32 search takes the bounded scan
+// instead of the exact scan: below it the exact scan's fewer kernels win.
+// Lists of 600 and 1000 rows, k 10 and 20: 9.6e4 pairs 189 -> 204 us, 1.6e5
+// 229 -> 171, 3.8e5 282 -> 218; k 100: 1.5e5 205 -> 242 us, 2.5e5 338 -> 324,
+// 3.8e5 296 -> 230.  Short lists (100 rows) keep the exact scan's items small:
+// 2.6e5 pairs 148 -> 181 us, 1.0e6 254 -> 194.
+constexpr double kScreenPairs = 2.0e5, kScreenPairsShort = 8.0e5;
+constexpr double kScreenShortRows = 256.0;
 
 int pow2_floor(long long x) {
   int p = 1;
@@ -777,6 +785,9 @@ class IndexCore {
     if (cand_path_)
       HB_CHECK(static_cast<int>(k) <= R, HB_ERR_INVALID,
                "BF16 search supports k up to " + std::to_string(kCandMaxR));
+    // FP32 plain scans take the bounded tensor-core scan too where it serves
+    // (screen_batch); the result is the exact scan's either way.
+    screen_ = !bf16 && exact_k && screen_possible(static_cast<int>(k));
     int mode = SCAN_PLAIN;
     size_t P = nprobe_;
     int W = 1, B = 1;
@@ -838,8 +849,12 @@ class IndexCore {
     const bool dev_in = is_device_ptr(q);
     size_t bs = std::min<size_t>(nq, batch_limit(P, k));
     if (cand_path_ && P > 0) bs = std::min(bs, cand_batch_limit(P));
-    if (bf16 && !cand_path_)
-      bs = std::min(bs, std::max<size_t>(1, (size_t(1) << 30) / (static_cast<size_t>(filter_cap(k)) * 8)));
+    const size_t bounded_bs = std::max<size_t>(1, (size_t(1) << 30) / (static_cast<size_t>(filter_cap(k)) * 8));
+    if (bf16 && !cand_path_) bs = std::min(bs, bounded_bs);
+    screen_ = screen_ && mode == SCAN_PLAIN && P > 0 &&
+              screen_pays(static_cast<int>(std::min(bs, bounded_bs)), static_cast<int>(P)) &&
+              !(p.use_graph && nq <= bs && nq > bounded_bs);  // a graph is one batch
+    if (screen_) bs = std::min(bs, bounded_bs);
     const int warm_lists = p.warmup_lists;
     const int warm_size = p.warmup_list_size > 0 ? p.warmup_list_size : static_cast<int>(k);
     // DIVIDE_DIM query blocks cover queries [0, B * (nq / B)); the rest stay
@@ -947,10 +962,11 @@ class IndexCore {
       cut_src_ = npqin_.p;
     }
     cut_b0_ = 0;
+    if (screen_) screen_ = screen_reserve(nb, k);
     char key[256];
-    std::snprintf(key, sizeof(key), "%d/%d/%d/%d/%d/%d/%d/%08x/%d/%d/%d/%d/%d", nb, k, P, R, p.precision, p.mode,
+    std::snprintf(key, sizeof(key), "%d/%d/%d/%d/%d/%d/%d/%08x/%d/%d/%d/%d/%d/%d", nb, k, P, R, p.precision, p.mode,
                   cut_mode_, cut_mode_ == 1 ? *reinterpret_cast<const uint32_t*>(&cut_thr_) : 0u, cut_cap_,
-                  seed_rows_, coarse_kind_, coarse_margin_, static_cast<int>(nprobe_));
+                  seed_rows_, coarse_kind_, coarse_margin_, static_cast<int>(nprobe_), screen_ ? 1 : 0);
     auto it = graphs_.find(key);
     if (it != graphs_.end() && it->second.gen != devbuf_generation().load()) {
       cudaGraphExecDestroy(it->second.exec);
@@ -958,7 +974,7 @@ class IndexCore {
       it = graphs_.end();
     }
     if (it != graphs_.end()) {
-      if (bf16) HB_CUDA(cudaMemsetAsync(err_dev_.p, 0, sizeof(int), st_));
+      if (bf16 || screen_) HB_CUDA(cudaMemsetAsync(err_dev_.p, 0, sizeof(int), st_));
       HB_CUDA(cudaGraphLaunch(it->second.exec, st_));
       launches_ += it->second.launches;
     } else {
@@ -998,7 +1014,9 @@ class IndexCore {
     }
     if (bf16 && !cand_path_) {
       bf16_err_check();
-      fix_overflow(nb, P, k, dout_.p, iout_.p);
+      last_overflow_ = fix_overflow(nb, P, k, dout_.p, iout_.p);
+    } else if (screen_) {
+      screen_finish(nb, P, k, dout_.p, iout_.p);
     }
     HB_CUDA(cudaMemcpyAsync(D, dout_.p, static_cast<size_t>(nb) * k * sizeof(float), cudaMemcpyDefault, st_));
     HB_CUDA(cudaMemcpyAsync(I, iout_.p, static_cast<size_t>(nb) * k * sizeof(int64_t), cudaMemcpyDefault, st_));
@@ -1412,7 +1430,73 @@ class IndexCore {
         ++launches_;
       }
     }
+    if (screen_ && screen_batch(nb, P, k, Dd, Id)) return;
     scan_exact_from(nb, P, k, qpad_.p, probes_.p, mode, cut, need_tops ? tops_.p : nullptr, W, B, qblock, Dd, Id);
+  }
+
+  // ---- FP32 searches on the bounded scan ------------------------------------
+  // The bounded scan decides which rows can be among the k nearest and
+  // recomputes those with the exact FP32 loop; every distance returned is that
+  // loop's, and so is the order (see k_tc.cu).  It serves plain FP32 searches
+  // of d <= 128 and k <= 256 as well, as the tensor-core coarse quantizer
+  // serves the probes.  Queries outside its error bound's range or with too
+  // many candidates are searched with the exact scan, and so is the whole
+  // batch when its buffers cannot be had or a device wait gave up.
+  bool screen_possible(int k) const {
+    return bf16_ready_ && kpad_ <= 128 && k <= kFilterMaxK && ntotal_ < (size_t(1) << 31) - 8192;
+  }
+  bool screen_pays(int nb, int P) const {
+    const double avg = static_cast<double>(ntotal_) / static_cast<double>(std::max<size_t>(nlist_, 1));
+    return static_cast<double>(nb) * P * avg >= (avg < kScreenShortRows ? kScreenPairsShort : kScreenPairs);
+  }
+
+  bool screen_reserve(int nb, int k) {
+    try {
+      bounded_reserve(nb, filter_cap(k), scr_cnt_, scr_m_);
+      return true;
+    } catch (const Error& e) {
+      if (e.code != HB_ERR_NOMEM) throw;
+      cudaGetLastError();
+      cbuf_.release();  // the exact scan's buffers need the memory
+      cbuf_ub_.release();
+      return false;
+    }
+  }
+
+  bool screen_batch(int nb, int P, int k, float* Dd, int64_t* Id) {
+    screen_ = screen_reserve(nb, k);
+    if (!screen_) return false;
+    const int cap = filter_cap(k);
+    const int cr = std::max(128, chunk_rows_for(nb, P, 128));
+    filter_pipeline(nb, P, k, cap, cr, scan_bf16_stages(kpad_), scr_cnt_.p, scr_m_.p, kDefaultWaitBudget, Dd, Id);
+    if (!capturing_) screen_finish(nb, P, k, Dd, Id);
+    return true;
+  }
+
+  // After a screened batch: queries left to the exact scan, or all of them
+  // when a wait gave up.
+  void screen_finish(int nb, int P, int k, float* Dd, int64_t* Id) {
+    HB_CUDA(cudaMemcpyAsync(err_host_, err_dev_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    HB_CUDA(cudaStreamSynchronize(st_));
+    if (*err_host_ != 0)
+      scan_exact_from(nb, P, k, qpad_.p, probes_.p, SCAN_PLAIN, false, nullptr, 1, 1, 0, Dd, Id);
+    else
+      fix_overflow(nb, P, k, Dd, Id);
+  }
+
+  // Per-batch buffers of the bounded scan (counts and re-ranked rows in the
+  // caller's own), and its error flag cleared.
+  void bounded_reserve(int nb, int cap, DevBuf<int>& cnt, DevBuf<int>& m) {
+    err_dev_.reserve(1);
+    HB_CUDA(cudaMemsetAsync(err_dev_.p, 0, sizeof(int), st_));
+    thr_.reserve(nb);
+    cnt.reserve(nb);
+    m.reserve(nb);
+    cflag_.reserve(nb);
+    over_list_.reserve(2 * static_cast<size_t>(nb));
+    over_n_.reserve(2);
+    cbuf_.reserve(static_cast<size_t>(nb) * cap);
+    cbuf_ub_.reserve(static_cast<size_t>(nb) * cap);
   }
 
   // The exact list scan and merge of nb queries (qpad, nb x dpad) over the
@@ -1498,18 +1582,9 @@ class IndexCore {
     }
     probes_.reserve(static_cast<size_t>(nb) * P);
     coarse_and_cut(nb, P);
-    err_dev_.reserve(1);
-    HB_CUDA(cudaMemsetAsync(err_dev_.p, 0, sizeof(int), st_));
     const int cap = filter_cap(k);
-    thr_.reserve(nb);
-    ccnt_.reserve(nb);
-    cflag_.reserve(nb);
-    rr_m_.reserve(nb);
-    over_list_.reserve(2 * static_cast<size_t>(nb));
+    bounded_reserve(nb, cap, ccnt_, rr_m_);
     last_nb_ = nb;
-    over_n_.reserve(2);
-    cbuf_.reserve(static_cast<size_t>(nb) * cap);
-    cbuf_ub_.reserve(static_cast<size_t>(nb) * cap);
     const int cr0 = std::max(128, chunk_rows_for(nb, P, 128));
     const int s0 = scan_bf16_stages(kpad_);
     const TuneKey key = tune_key(nb, P, k);
@@ -1517,10 +1592,10 @@ class IndexCore {
     const auto it = tune_.find(key);
     const int cr = it != tune_.end() ? it->second.chunk_rows : cr0;
     const int stages = it != tune_.end() ? it->second.stages : s0;
-    filter_pipeline(nb, P, k, cap, cr, stages, Dd, Id);
+    filter_pipeline(nb, P, k, cap, cr, stages, ccnt_.p, rr_m_.p, wait_budget_, Dd, Id);
     if (!capturing_) {
       bf16_err_check();
-      fix_overflow(nb, P, k, Dd, Id);
+      last_overflow_ = fix_overflow(nb, P, k, Dd, Id);
     }
   }
 
@@ -1530,11 +1605,12 @@ class IndexCore {
   // scan runs in two stages: every query's nearest list first, whose k-th
   // admitted value bounds the second stage over the other lists.  Every
   // (cr, stages) gives the same result.
-  void filter_pipeline(int nb, int P, int k, int cap, int cr, int stages, float* Dd, int64_t* Id) {
+  void filter_pipeline(int nb, int P, int k, int cap, int cr, int stages, int* cnt, int* rr_m, long long budget,
+                       float* Dd, int64_t* Id) {
     HB_CUDA(cudaMemsetAsync(over_n_.p, 0, 2 * sizeof(int), st_));
     {
       Scope sc(this, "query_prep");
-      launch_query_prep(nb, thr_.p, ccnt_.p, st_);
+      launch_query_prep(nb, thr_.p, cnt, st_);
     }
     list_cnt_.reserve(nlist_);
     list_cursor_.reserve(nlist_);
@@ -1588,12 +1664,12 @@ class IndexCore {
     a.rmax = rmax_.p;
     a.cand = cbuf_.p;
     a.cand_ub = cbuf_ub_.p;
-    a.cand_cnt = ccnt_.p;
+    a.cand_cnt = cnt;
     a.cap = cap;
     a.k = k;
     a.err = err_dev_.p;
     a.stages = stages;
-    a.wait_budget = wait_budget_;
+    a.wait_budget = budget;
     {
       Scope sc(this, "scan_bf16");
       launch_scan_bf16(tmap_, a, num_sms_, st_);
@@ -1602,7 +1678,7 @@ class IndexCore {
       // Second stage: the other lists, appended to the same buffers.
       {
         Scope sc(this, "kth_bound");
-        launch_kth_bound(cbuf_ub_.p, ccnt_.p, cap, nb, k, thr_.p, st_);
+        launch_kth_bound(cbuf_ub_.p, cnt, cap, nb, k, thr_.p, st_);
       }
       {
         Scope sc(this, "build_work");
@@ -1620,8 +1696,8 @@ class IndexCore {
     }
     {
       Scope sc(this, "rerank");
-      launch_rerank_bf16(cbuf_.p, cbuf_ub_.p, ccnt_.p, cap, nb, k, codes_.p, qpad_.p, static_cast<int>(dpad_), ids_.p, Dd,
-                         Id, cflag_.p, over_list_.p, over_n_.p, rr_m_.p, num_sms_, st_);
+      launch_rerank_bf16(cbuf_.p, cbuf_ub_.p, cnt, cap, nb, k, codes_.p, qpad_.p, static_cast<int>(dpad_), ids_.p, Dd,
+                         Id, cflag_.p, over_list_.p, over_n_.p, rr_m, num_sms_, st_);
     }
     // query prep, seed, scan, warp re-rank, and the three flat re-rank
     // kernels when the buffers can hold more than a warp's candidates.
@@ -1666,7 +1742,7 @@ class IndexCore {
         float ms = 1e30f;
         for (int rep = 0; rep < 2; ++rep) {
           HB_CUDA(cudaEventRecord(e0, st_));
-          filter_pipeline(nb, P, k, cap, c, S, Dd, Id);
+          filter_pipeline(nb, P, k, cap, c, S, ccnt_.p, rr_m_.p, wait_budget_, Dd, Id);
           HB_CUDA(cudaEventRecord(e1, st_));
           HB_CUDA(cudaEventSynchronize(e1));
           float t = 0.f;
@@ -1726,13 +1802,13 @@ class IndexCore {
   // Queries whose candidate buffer overflowed (listed by the re-rank, left
   // unwritten) are searched with the exact scan over their own probe rows,
   // and their result rows are written into Dd / Id.
-  void fix_overflow(int nb, int P, int k, float* Dd, int64_t* Id) {
+  // Returns their number.
+  int fix_overflow(int nb, int P, int k, float* Dd, int64_t* Id) {
     int n_over = 0;
     HB_CUDA(cudaMemcpyAsync(err_host_, over_n_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
     HB_CUDA(cudaStreamSynchronize(st_));
     n_over = *err_host_;
-    last_overflow_ = n_over;
-    if (n_over <= 0) return;
+    if (n_over <= 0) return n_over;
     HB_CHECK(n_over <= nb, HB_ERR_CUDA, "overflow list longer than the batch");
     Scope sc(this, "overflow_exact");
     const int dp = static_cast<int>(dpad_);
@@ -1750,6 +1826,7 @@ class IndexCore {
     launch_scatter_words(reinterpret_cast<const uint32_t*>(oi_.p), over_list_.p, n_over, 2 * k,
                          reinterpret_cast<uint32_t*>(Id), st_);
     launches_ += 4;
+    return n_over;
   }
 
   // Longest candidate row a query can have at nprobe P: the P largest lists,
@@ -2246,6 +2323,8 @@ class IndexCore {
   // bounded BF16 scan
   DevBuf<uint32_t> thr_;
   DevBuf<int> ccnt_, cflag_, over_list_, over_n_, rr_m_;
+  bool screen_ = false;              // this search's plain FP32 batches go through the bounded scan
+  DevBuf<int> scr_cnt_, scr_m_;      // its counts (bf16_stats reports BF16 searches only)
   int last_nb_ = 0;
   DevBuf<uint64_t> cbuf_;
   DevBuf<uint32_t> cbuf_ub_;  // each candidate's upper bound
