@@ -48,12 +48,12 @@ bool is_device_ptr(const void* p) {
 
 // Points x centroids x padded dimensions from which the tensor cores make the
 // assignment.  A training call (20 passes over the same points) gains from
-// about 5e8 on: 10k x 1000 x 128 6.4 -> 2.5 ms, 100k x 300 x 32 6.5 -> 4.8 ms,
-// but 10k x 100 x 128 2.1 -> 3.3 ms (five small launches a pass against one).
-// A single pass (add) has its scratch allocation to earn back: 200k x 1024 x
-// 128 8.1 -> 6.4 ms, 100k x 500 x 128 3.2 -> 3.7 ms.
+// about 5e8 on: 10k x 1000 x 128 6.4 -> 2.0 ms, 100k x 300 x 32 6.5 -> 4.3 ms,
+// but 10k x 100 x 128 1.4 -> 1.8 ms (five small launches a pass against one).
+// A single pass (add) has its first launches to earn back: 100k x 500 x 128
+// 2.7 -> 2.0 ms, 30k x 257 x 512 1.5 -> 2.2 ms.
 constexpr double kAssignTcTrain = 5.0e8;
-constexpr double kAssignTcAdd = 1.5e10;
+constexpr double kAssignTcAdd = 5.0e9;
 // (query, row) pairs from which a plain FP32 search takes the bounded scan
 // instead of the exact scan: below it the exact scan's fewer kernels win.
 // Lists of 600 and 1000 rows, k 10 and 20: 9.6e4 pairs 189 -> 204 us, 1.6e5
@@ -244,64 +244,85 @@ class IndexCore {
       HB_CUDA(cudaMemcpyAsync(tmp.p, x, n * d_ * sizeof(float), cudaMemcpyHostToDevice, st_));
       src = tmp.p;
     }
-    launch_pad_rows(src, n, static_cast<int>(d_), static_cast<int>(dpad_), dst.p, st_);
+    pad_rows(src, nullptr, n, dst.p);
+  }
+
+  // Rows of d floats on the device (all, or those idx names) to padded rows.
+  void pad_rows(const float* src, const int64_t* idx, size_t n, float* dst) {
+    launch_pad_rows(src, idx, n, static_cast<int>(d_), static_cast<int>(d_), static_cast<int>(dpad_), dst, st_);
     ++launches_;
+  }
+
+  // x as n padded device rows: x itself where it already is that (on the
+  // device, no padding, 16-byte aligned: build-time kernels only read it, and
+  // are done when the call returns), else a copy in `buf`.
+  const float* padded_rows(const float* x, size_t n, DevBuf<float>& buf) {
+    const bool dev = is_device_ptr(x);
+    if (dpad_ == d_ && dev && reinterpret_cast<uintptr_t>(x) % 16 == 0) return x;
+    buf.reserve(n * dpad_);
+    if (dpad_ == d_) {
+      HB_CUDA(cudaMemcpyAsync(buf.p, x, n * d_ * sizeof(float), cudaMemcpyDefault, st_));
+      return buf.p;
+    }
+    DevBuf<float> tmp;
+    const float* src = x;
+    if (!dev) {
+      tmp.reserve(n * d_);
+      HB_CUDA(cudaMemcpyAsync(tmp.p, x, n * d_ * sizeof(float), cudaMemcpyHostToDevice, st_));
+      src = tmp.p;
+    }
+    pad_rows(src, nullptr, n, buf.p);
+    if (tmp.p) HB_CUDA(cudaStreamSynchronize(st_));
+    return buf.p;
   }
 
   // ---- nearest-centroid assignment -----------------------------------------
 
-  // Buffers of one train or add call's assignments on the tensor cores (one
-  // allocation); `on` is false where the exact kernel does them (small
-  // problems, no memory for the buffers, or a wait that gave up).  One
-  // Assigner serves one set of points.
+  // One train or add call's assignments of one set of points on the tensor
+  // cores, in the caller's scratch; `on` is false where the exact kernel does
+  // them (small problems, no memory for the scratch, or a wait that gave up).
   struct Assigner {
-    bool on = false;
+    bool want = false, on = false;
     size_t chunk = 0;              // points per launch
     size_t split_at = ~size_t(0);  // first point of the chunk xsplit holds
-    DevBuf<unsigned char> mem;
     unsigned char *xsplit = nullptr, *csplit = nullptr;
     float *xnorm = nullptr, *cnorm = nullptr, *mu = nullptr;
     int2* pairs = nullptr;
     int *exact = nullptr, *ctl = nullptr, *err = nullptr;
   };
-
-  // For assignments of n points, at most `max_chunk` of them at a time, on the
-  // tensor cores from `min_work` on.
-  void assign_setup(Assigner& as, size_t n, size_t max_chunk, double min_work) {
-    if (static_cast<double>(n) * nlist_ * dpad_ < min_work) return;
-    const size_t kpad = static_cast<size_t>(assign_kpad(static_cast<int>(dpad_)));
-    as.chunk = std::min<size_t>(n, std::max<size_t>(128, max_chunk));
-    size_t total = 0;
-    for (int pass = 0; pass < 2; ++pass) {
-      size_t off = 0;
-      auto carve = [&](auto*& p, size_t count) {
-        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(as.mem.p + off);
-        off += (count * sizeof(*p) + 255) / 256 * 256;
-      };
-      carve(as.xsplit, as.chunk * 4 * kpad);
-      carve(as.csplit, nlist_ * 4 * kpad);
-      carve(as.xnorm, as.chunk);
-      carve(as.cnorm, (nlist_ + 127) / 128 * 128);
-      carve(as.mu, dpad_);
-      carve(as.pairs, as.chunk);
-      carve(as.exact, as.chunk);
-      carve(as.ctl, 4);
-      carve(as.err, 1);
-      total = off;
-      if (pass == 0) {
-        try {
-          as.mem.reserve(total);
-        } catch (const Error& e) {
-          if (e.code != HB_ERR_NOMEM) throw;
-          cudaGetLastError();
-          return;
-        }
-      }
+  // Consecutive 256-byte aligned pieces of one allocation (base null: sizes
+  // only).
+  struct Carver {
+    unsigned char* base;
+    size_t off = 0;
+    template <class T>
+    void take(T*& p, size_t count) {
+      p = base ? reinterpret_cast<T*>(base + off) : nullptr;
+      off += (count * sizeof(T) + 255) / 256 * 256;
     }
+  };
+
+  bool assign_wanted(size_t n, double min_work) const {
+    return static_cast<double>(n) * nlist_ * dpad_ >= min_work;
+  }
+  void carve_assigner(Assigner& as, Carver& c) {
+    const size_t kpad = static_cast<size_t>(assign_kpad(static_cast<int>(dpad_)));
+    c.take(as.xsplit, as.chunk * 4 * kpad);
+    c.take(as.csplit, nlist_ * 4 * kpad);
+    c.take(as.xnorm, as.chunk);
+    c.take(as.cnorm, (nlist_ + 127) / 128 * 128);
+    c.take(as.mu, dpad_);
+    c.take(as.pairs, as.chunk);
+    c.take(as.exact, as.chunk);
+    c.take(as.ctl, 4);
+    c.take(as.err, 1);
+  }
+  void assign_begin(Assigner& as) {
+    as.on = as.want;
+    if (!as.on) return;
     HB_CUDA(cudaMemsetAsync(as.err, 0, sizeof(int), st_));
     launch_column_mean(cent_.p, static_cast<int>(nlist_), static_cast<int>(dpad_), as.mu, st_);
     ++launches_;
-    as.on = true;
   }
 
   // arg[i] = the nearest centroid of x row i (the reference's strict '<' scan
@@ -369,32 +390,38 @@ class IndexCore {
     size_t m = n;
     std::vector<int64_t> sample;
     if (n > nlist_ * max_pts) {
-      std::vector<size_t> idx(n);
-      std::iota(idx.begin(), idx.end(), 0);
+      std::vector<uint32_t> idx(n);
+      std::iota(idx.begin(), idx.end(), 0u);
       std::shuffle(idx.begin(), idx.end(), std::default_random_engine(seed));
       m = nlist_ * max_pts;
       sample.assign(idx.begin(), idx.begin() + m);
     }
-    std::vector<size_t> iidx(m);
-    std::iota(iidx.begin(), iidx.end(), 0);
+    std::vector<uint32_t> iidx(m);
+    std::iota(iidx.begin(), iidx.end(), 0u);
     std::shuffle(iidx.begin(), iidx.end(), std::default_random_engine(seed));
     std::vector<int64_t> init(nlist_);
     for (size_t c = 0; c < nlist_; ++c) init[c] = static_cast<int64_t>(iidx[c]);
 
-    DevBuf<float> xall, tmp, xs;
-    stage_rows(x, n, xall, tmp);
-    tmp.release();
-    const float* pts = xall.p;
+    DevBuf<float> xs;
+    const float* pts = nullptr;
     if (!sample.empty()) {
+      // Only the sampled rows are kept (padded).
+      DevBuf<float> tmp;
+      const float* src = x;
+      if (!is_device_ptr(x)) {
+        tmp.reserve(n * d_);
+        HB_CUDA(cudaMemcpyAsync(tmp.p, x, n * d_ * sizeof(float), cudaMemcpyHostToDevice, st_));
+        src = tmp.p;
+      }
       DevBuf<int64_t> sidx;
       sidx.reserve(m);
       HB_CUDA(cudaMemcpyAsync(sidx.p, sample.data(), m * sizeof(int64_t), cudaMemcpyHostToDevice, st_));
       xs.reserve(m * dpad_);
-      launch_gather_rows(xall.p, sidx.p, m, static_cast<int>(dpad_), xs.p, st_);
-      ++launches_;
+      pad_rows(src, sidx.p, m, xs.p);
       HB_CUDA(cudaStreamSynchronize(st_));
-      xall.release();
       pts = xs.p;
+    } else {
+      pts = padded_rows(x, n, xs);
     }
     DevBuf<int64_t> cidx;
     cidx.reserve(nlist_);
@@ -403,28 +430,45 @@ class IndexCore {
       launch_gather_rows(pts, cidx.p, nlist_, static_cast<int>(dpad_), cent_.p, st_);
       ++launches_;
     };
-    DevBuf<int32_t> assign, counts;
-    DevBuf<double> sums;
-    assign.reserve(m);
-    counts.reserve(nlist_);
-    sums.reserve(nlist_ * dpad_);
+    // Scratch in one allocation.  The sample is split once for every iteration
+    // while its split rows fit 2 GiB.
+    int32_t *assign = nullptr, *counts = nullptr;
+    double* sums = nullptr;
     Assigner as;
+    as.want = assign_wanted(m, kAssignTcTrain);
+    as.chunk = std::min(m, (size_t(1) << 29) / static_cast<size_t>(assign_kpad(static_cast<int>(dpad_))));
+    DevBuf<unsigned char> scratch;
+    auto lay_out = [&](unsigned char* base) {
+      Carver c{base};
+      c.take(assign, m);
+      c.take(counts, nlist_);
+      c.take(sums, nlist_ * dpad_);
+      if (as.want) carve_assigner(as, c);
+      return c.off;
+    };
+    try {
+      scratch.reserve(lay_out(nullptr));
+    } catch (const Error& e) {
+      if (e.code != HB_ERR_NOMEM || !as.want) throw;
+      cudaGetLastError();
+      as.want = false;  // the exact kernel needs no scratch of its own
+      scratch.reserve(lay_out(nullptr));
+    }
+    lay_out(scratch.p);
     auto iterate = [&]() {
       for (int it = 0; it < niter; ++it) {
-        assign_rows(as, pts, m, assign.p, nullptr);
-        HB_CUDA(cudaMemsetAsync(sums.p, 0, nlist_ * dpad_ * sizeof(double), st_));
-        HB_CUDA(cudaMemsetAsync(counts.p, 0, nlist_ * sizeof(int32_t), st_));
-        launch_kmeans_accumulate(pts, assign.p, m, static_cast<int>(d_), static_cast<int>(dpad_), sums.p, counts.p,
+        assign_rows(as, pts, m, assign, nullptr);
+        HB_CUDA(cudaMemsetAsync(sums, 0, nlist_ * dpad_ * sizeof(double), st_));
+        HB_CUDA(cudaMemsetAsync(counts, 0, nlist_ * sizeof(int32_t), st_));
+        launch_kmeans_accumulate(pts, assign, m, static_cast<int>(d_), static_cast<int>(dpad_), sums, counts,
                                  st_);
-        launch_kmeans_update(sums.p, counts.p, static_cast<int>(nlist_), static_cast<int>(d_), static_cast<int>(dpad_),
+        launch_kmeans_update(sums, counts, static_cast<int>(nlist_), static_cast<int>(d_), static_cast<int>(dpad_),
                              cent_.p, st_);
         launches_ += 2;
       }
     };
     seed_centroids();
-    // The sample is split once for every iteration while its split rows fit
-    // 2 GiB.
-    assign_setup(as, m, (size_t(1) << 29) / static_cast<size_t>(assign_kpad(static_cast<int>(dpad_))), kAssignTcTrain);
+    assign_begin(as);
     iterate();
     if (assign_gave_up(as)) {
       seed_centroids();
@@ -443,43 +487,63 @@ class IndexCore {
     HB_CHECK(x, HB_ERR_INVALID, "null data");
     HB_CHECK(n < (1ull << 32) - 1, HB_ERR_INVALID, "add supports fewer than 2^32 - 1 vectors");
     HB_CUDA(cudaSetDevice(device_));
-    DevBuf<float> xpad, tmp;
-    stage_rows(x, n, xpad, tmp);
-    tmp.release();
-    DevBuf<int32_t> assign;
-    DevBuf<float> dist;
-    assign.reserve(n);
-    dist.reserve(n);
-    {
-      Assigner as;
-      assign_setup(as, n, size_t(1) << 17, kAssignTcAdd);
-      assign_rows(as, xpad.p, n, assign.p, dist.p);
-      if (assign_gave_up(as)) assign_rows(as, xpad.p, n, assign.p, dist.p);
-    }
-    DevBuf<uint64_t> k0, k1;
-    DevBuf<uint32_t> v0, v1;
-    k0.reserve(n);
-    k1.reserve(n);
-    v0.reserve(n);
-    v1.reserve(n);
-    launch_add_keys(assign.p, dist.p, n, k0.p, v0.p, st_);
+    DevBuf<float> xpad;
+    const float* xr = padded_rows(x, n, xpad);
+    // Scratch in one allocation: assignment and distances, then the sort's
+    // keys, values and scratch in the place of the assignment's.
     int list_bits = 1;
     while ((1ull << list_bits) < nlist_) ++list_bits;
     size_t sort_bytes = 0;
-    sort_pairs_u64(k0.p, k1.p, v0.p, v1.p, n, 32 + list_bits, nullptr, &sort_bytes, st_);
-    DevBuf<unsigned char> sort_tmp;
-    sort_tmp.reserve(sort_bytes);
-    sort_pairs_u64(k0.p, k1.p, v0.p, v1.p, n, 32 + list_bits, sort_tmp.p, &sort_bytes, st_);
+    sort_pairs_u64(nullptr, nullptr, nullptr, nullptr, n, 32 + list_bits, nullptr, &sort_bytes, st_);
+    const size_t ob = list_offsets_tmp_bytes(static_cast<int>(nlist_));
+    // Points per assignment launch: whole waves of 128-point tiles, about
+    // 64 MiB of split rows.
+    const size_t wave = static_cast<size_t>(num_sms_) * 128;
+    const size_t kpad = static_cast<size_t>(assign_kpad(static_cast<int>(dpad_)));
+    const size_t chunk = wave * std::max<size_t>(1, (size_t(64) << 20) / (wave * 4 * kpad));
+    DevBuf<unsigned char> scratch;
+    int32_t* assign = nullptr;
+    float* dist = nullptr;
+    uint64_t *k0 = nullptr, *k1 = nullptr;
+    uint32_t *v0 = nullptr, *v1 = nullptr;
+    unsigned char *sort_tmp = nullptr, *otmp = nullptr;
+    Assigner as;
+    auto lay_out = [&](unsigned char* base) {
+      Carver c{base};
+      c.take(assign, n);
+      c.take(dist, n);
+      Carver c2 = c;
+      c.take(k0, n);
+      c.take(k1, n);
+      c.take(v0, n);
+      c.take(v1, n);
+      c.take(sort_tmp, sort_bytes);
+      c.take(otmp, ob);
+      if (as.want) carve_assigner(as, c2);
+      return std::max(c.off, c2.off);
+    };
+    as.want = assign_wanted(n, kAssignTcAdd);
+    as.chunk = std::min(n, chunk);
+    try {
+      scratch.reserve(lay_out(nullptr));
+    } catch (const Error& e) {
+      if (e.code != HB_ERR_NOMEM || !as.want) throw;
+      cudaGetLastError();
+      as.want = false;  // the exact kernel needs no scratch of its own
+      scratch.reserve(lay_out(nullptr));
+    }
+    lay_out(scratch.p);
+    assign_begin(as);
+    assign_rows(as, xr, n, assign, dist);
+    if (assign_gave_up(as)) assign_rows(as, xr, n, assign, dist);
+    launch_add_keys(assign, dist, n, k0, v0, st_);
+    sort_pairs_u64(k0, k1, v0, v1, n, 32 + list_bits, sort_tmp, &sort_bytes, st_);
     codes_.reserve(n * dpad_);
     ids_.reserve(n);
     norms_.reserve(n);
-    launch_scatter_sorted(xpad.p, v1.p, n, static_cast<int>(d_), static_cast<int>(dpad_), codes_.p, ids_.p, st_);
-    const size_t ob = list_offsets_tmp_bytes(static_cast<int>(nlist_));
-    DevBuf<unsigned char> otmp;
-    otmp.reserve(ob);
-    launch_list_offsets(assign.p, n, static_cast<int>(nlist_), list_off_.p, otmp.p, ob, st_);
-    launch_row_norms(codes_.p, n, static_cast<int>(d_), static_cast<int>(dpad_), norms_.p, st_);
-    launches_ += 5;
+    launch_scatter_sorted(xr, v1, n, static_cast<int>(dpad_), codes_.p, ids_.p, norms_.p, st_);
+    launch_list_offsets(assign, n, static_cast<int>(nlist_), list_off_.p, otmp, ob, st_);
+    launches_ += 3;
     host_off_.resize(nlist_ + 1);
     HB_CUDA(cudaMemcpyAsync(host_off_.data(), list_off_.p, (nlist_ + 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
                             st_));
@@ -522,7 +586,7 @@ class IndexCore {
     codes_bf16_.reserve(ntotal_ * static_cast<size_t>(kpad_));
     rnorm_.reserve(ntotal_);
     rmax_.reserve(nlist_);
-    launch_residual_bf16(codes_.p, list_off_.p, cent_.p, static_cast<int>(nlist_), static_cast<int>(dpad_), kpad_,
+    launch_residual_bf16(codes_.p, list_off_.p, cent_.p, static_cast<int>(nlist_), ntotal_, static_cast<int>(dpad_), kpad_,
                          codes_bf16_.p, rnorm_.p, rmax_.p, st_);
     ++launches_;
     make_bf16_tensor_map(tmap_, codes_bf16_.p, ntotal_, kpad_);
@@ -892,8 +956,7 @@ class IndexCore {
                                 st_));
         qsrc = qtmp_.p;
       }
-      launch_pad_rows(qsrc, nb, static_cast<int>(d_), static_cast<int>(dpad_), qpad_.p, st_);
-      ++launches_;
+      pad_rows(qsrc, nullptr, nb, qpad_.p);
       if (P == 0 || ntotal_ == 0) {
         launch_fill_results(Dd, Id, static_cast<size_t>(nb) * k, st_);
         ++launches_;
@@ -937,8 +1000,7 @@ class IndexCore {
   }
 
   void run_batch_pipeline(int nb, int k, int P, int R, bool bf16) {
-    launch_pad_rows(qtmp_.p, nb, static_cast<int>(d_), static_cast<int>(dpad_), qpad_.p, st_);
-    ++launches_;
+    pad_rows(qtmp_.p, nullptr, nb, qpad_.p);
     if (P == 0 || ntotal_ == 0) {
       launch_fill_results(dout_.p, iout_.p, static_cast<size_t>(nb) * k, st_);
       ++launches_;
@@ -1260,7 +1322,7 @@ class IndexCore {
                     off, bytes);
       throw Error(HB_ERR_INVALID, msg);
     }
-    launch_pad_rows(q, nq, static_cast<int>(d_), static_cast<int>(dpad_), qpad, st_);
+    launch_pad_rows(q, nullptr, nq, static_cast<int>(d_), static_cast<int>(d_), static_cast<int>(dpad_), qpad, st_);
     launch_l2_matrix(qpad, nb, cent_.p, static_cast<int>(nlist_), static_cast<int>(dpad_), dmat,
                      static_cast<int>(nlist_), st_);
     launch_select_rows(dmat, nb, static_cast<int>(nlist_), static_cast<int>(nlist_), P, probes, nullptr, st_);

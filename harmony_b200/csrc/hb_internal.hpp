@@ -188,7 +188,9 @@ void launch_warmup_tops(const float* q, int nq, const int32_t* probes, int P, co
                         int warm_list_size, float* tops, cudaStream_t st);
 
 // k_build.cu
-void launch_pad_rows(const float* src, size_t n, int d, int dpad, float* dst, cudaStream_t st);
+// Rows of ld floats, in order or (idx) row idx[r], to rows of dpad (zero past d).
+void launch_pad_rows(const float* src, const int64_t* idx, size_t n, int ld, int d, int dpad, float* dst,
+                     cudaStream_t st);
 void launch_gather_rows(const float* src, const int64_t* idx, size_t n, int dpad, float* dst,
                         cudaStream_t st);
 void launch_kmeans_accumulate(const float* x, const int32_t* assign, size_t n, int d, int dpad,
@@ -200,8 +202,8 @@ void launch_add_keys(const int32_t* assign, const float* dist, size_t n, uint64_
                      uint32_t* vals, cudaStream_t st);
 void sort_pairs_u64(uint64_t* keys_in, uint64_t* keys_out, uint32_t* vals_in, uint32_t* vals_out,
                     size_t n, int end_bit, void* tmp, size_t* tmp_bytes, cudaStream_t st);
-void launch_scatter_sorted(const float* x, const uint32_t* order, size_t n, int d, int dpad,
-                           float* codes, int64_t* ids, cudaStream_t st);
+void launch_scatter_sorted(const float* x, const uint32_t* order, size_t n, int dpad, float* codes, int64_t* ids,
+                           float* norms, cudaStream_t st);
 void launch_list_offsets(const int32_t* assign, size_t n, int nlist, int64_t* list_off,
                          void* tmp, size_t tmp_bytes, cudaStream_t st);
 size_t list_offsets_tmp_bytes(int nlist);
@@ -261,8 +263,8 @@ void make_f32_store_map(void* tmap_out, const float* base, size_t rows, size_t c
 void launch_query_prep(int nq, uint32_t* thr, int* cnt, cudaStream_t st);
 // Residual BF16 codes BF16(x - c_l) (kpad columns), FP32 residual norms per row
 // and the largest residual norm per list.
-void launch_residual_bf16(const float* codes, const int64_t* list_off, const float* cent, int nlist, int dpad, int kpad,
-                          void* dst, float* rnorm, float* rmax, cudaStream_t st);
+void launch_residual_bf16(const float* codes, const int64_t* list_off, const float* cent, int nlist, size_t ntotal,
+                          int dpad, int kpad, void* dst, float* rnorm, float* rmax, cudaStream_t st);
 // Seed bound from the first S <= 256 rows of each query's nearest list (probe
 // rank 0 in the list-major work description; with probes given and a small
 // batch, one CTA per query).

@@ -11,13 +11,31 @@
 namespace hb {
 namespace {
 
-__global__ void pad_rows_kernel(const float* __restrict__ src, size_t n, int d, int dpad, float* __restrict__ dst) {
-  const size_t total = n * static_cast<size_t>(dpad);
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const size_t r = i / dpad;
-    const int c = static_cast<int>(i - r * dpad);
-    dst[i] = c < d ? src[r * d + c] : 0.0f;
+// Rows of ld floats (row r of src, or row idx[r]) -> rows of dpad, zero past
+// d.  A CTA takes kPadRows rows at a time, a thread four columns (16-byte
+// loads where V4: ld a multiple of 4 and src 16-byte aligned).
+constexpr int kPadRows = 32;
+
+template <bool V4>
+__global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ src, const int64_t* __restrict__ idx,
+                                                       int64_t n, int ld, int d, int dpad, float* __restrict__ dst) {
+  const int c4 = dpad / 4;
+  for (int64_t r0 = static_cast<int64_t>(blockIdx.x) * kPadRows; r0 < n; r0 += static_cast<int64_t>(gridDim.x) * kPadRows) {
+    const int rows = static_cast<int>(min(static_cast<int64_t>(kPadRows), n - r0));
+    for (int i = threadIdx.x; i < rows * c4; i += blockDim.x) {
+      const int r = i / c4, c = 4 * (i - r * c4);
+      const float* row = src + (idx ? idx[r0 + r] : r0 + r) * ld;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (V4) {
+        if (c < d) v = *reinterpret_cast<const float4*>(row + c);  // d = ld here: no partial piece
+      } else {
+        if (c + 0 < d) v.x = row[c + 0];
+        if (c + 1 < d) v.y = row[c + 1];
+        if (c + 2 < d) v.z = row[c + 2];
+        if (c + 3 < d) v.w = row[c + 3];
+      }
+      *reinterpret_cast<float4*>(dst + (r0 + r) * dpad + c) = v;
+    }
   }
 }
 
@@ -86,17 +104,55 @@ __global__ void add_keys_kernel(const int32_t* __restrict__ assign, const float*
   vals[i] = static_cast<uint32_t>(i);
 }
 
-__global__ void scatter_sorted_kernel(const float* __restrict__ x, const uint32_t* __restrict__ order, size_t n,
-                                      int dpad, float* __restrict__ codes, int64_t* __restrict__ ids) {
-  const int c4 = dpad / 4;
-  const size_t total = n * c4;
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const size_t p = i / c4;
-    const int c = static_cast<int>(i - p * c4);
-    const uint32_t src = order[p];
-    reinterpret_cast<float4*>(codes)[p * c4 + c] = reinterpret_cast<const float4*>(x)[static_cast<size_t>(src) * c4 + c];
-    if (c == 0) ids[p] = static_cast<int64_t>(src);
+// The lists' content in sorted order: codes[p] = x[order[p]], its id and its
+// norm <x, x> (the sequential loop of row_norms_kernel; the zero padding adds
+// exact zeros).  A warp takes 32 consecutive rows, staged in shared memory 64
+// columns at a time by coalesced copies, half a warp per row; each lane sums
+// its own row from there.  Bound by DRAM (each row read and written once).
+constexpr int kScatWarps = 4;
+
+__global__ void __launch_bounds__(kScatWarps * 32) scatter_sorted_kernel(const float* __restrict__ x,
+                                                                         const uint32_t* __restrict__ order, int64_t n,
+                                                                         int dpad, float* __restrict__ codes,
+                                                                         int64_t* __restrict__ ids,
+                                                                         float* __restrict__ norms) {
+  __shared__ __align__(16) float s_stage[kScatWarps][32 * kHalfStageStride];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int64_t p0 = (static_cast<int64_t>(blockIdx.x) * kScatWarps + wib) * 32;
+  if (p0 >= n) return;
+  const int nv = static_cast<int>(min(static_cast<int64_t>(32), n - p0));
+  const uint32_t src = lane < nv ? order[p0 + lane] : 0u;
+  float* stage = s_stage[wib];
+  const int h = lane >> 4, cl = 4 * (lane & 15);
+  float acc = 0.0f;
+  for (int c0 = 0; c0 < dpad; c0 += 64) {
+    const int nc = min(64, dpad - c0);
+    __syncwarp();
+    for (int r = h; r < 32; r += 2) {
+      const uint32_t row = __shfl_sync(0xffffffffu, src, r);
+      if (r < nv && cl < nc)
+        cp_async16(stage + r * kHalfStageStride + cl, x + static_cast<size_t>(row) * dpad + c0 + cl, true);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncwarp();
+    if (cl < nc)
+      for (int r = h; r < nv; r += 2)
+        *reinterpret_cast<float4*>(codes + (p0 + r) * dpad + c0 + cl) =
+            *reinterpret_cast<const float4*>(stage + r * kHalfStageStride + cl);
+    const float* row = stage + lane * kHalfStageStride;
+    if (lane < nv)
+      for (int c = 0; c < nc; c += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(row + c);
+        acc = __fadd_rn(acc, __fmul_rn(v.x, v.x));
+        acc = __fadd_rn(acc, __fmul_rn(v.y, v.y));
+        acc = __fadd_rn(acc, __fmul_rn(v.z, v.z));
+        acc = __fadd_rn(acc, __fmul_rn(v.w, v.w));
+      }
+  }
+  if (lane < nv) {
+    ids[p0 + lane] = static_cast<int64_t>(src);
+    norms[p0 + lane] = acc;
   }
 }
 
@@ -132,9 +188,14 @@ inline unsigned grid_exact(size_t n, int tb) {
 
 }  // namespace
 
-void launch_pad_rows(const float* src, size_t n, int d, int dpad, float* dst, cudaStream_t st) {
+void launch_pad_rows(const float* src, const int64_t* idx, size_t n, int ld, int d, int dpad, float* dst,
+                     cudaStream_t st) {
   if (!n) return;
-  pad_rows_kernel<<<grid_for(n * dpad, 256), 256, 0, st>>>(src, n, d, dpad, dst);
+  const unsigned g = grid_for(n, kPadRows, 148u * 16u);
+  if (ld == d && d % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0)
+    pad_rows_kernel<true><<<g, 256, 0, st>>>(src, idx, static_cast<int64_t>(n), ld, d, dpad, dst);
+  else
+    pad_rows_kernel<false><<<g, 256, 0, st>>>(src, idx, static_cast<int64_t>(n), ld, d, dpad, dst);
   HB_CUDA(cudaGetLastError());
 }
 
@@ -177,11 +238,11 @@ void sort_pairs_u64(uint64_t* keys_in, uint64_t* keys_out, uint32_t* vals_in, ui
                                           static_cast<int64_t>(n), 0, end_bit, st));
 }
 
-void launch_scatter_sorted(const float* x, const uint32_t* order, size_t n, int d, int dpad, float* codes,
-                           int64_t* ids, cudaStream_t st) {
-  (void)d;
+void launch_scatter_sorted(const float* x, const uint32_t* order, size_t n, int dpad, float* codes, int64_t* ids,
+                           float* norms, cudaStream_t st) {
   if (!n) return;
-  scatter_sorted_kernel<<<grid_for(n * dpad / 4, 256), 256, 0, st>>>(x, order, n, dpad, codes, ids);
+  scatter_sorted_kernel<<<grid_exact(n, 32 * kScatWarps), kScatWarps * 32, 0, st>>>(x, order, static_cast<int64_t>(n),
+                                                                                    dpad, codes, ids, norms);
   HB_CUDA(cudaGetLastError());
 }
 

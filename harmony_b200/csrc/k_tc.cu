@@ -692,41 +692,69 @@ __global__ void query_prep_kernel(int nq, uint32_t* __restrict__ thr, int* __res
   cnt[qi] = 0;
 }
 
-// BF16 residual codes for the tensor-core scans, one CTA per list: row r of
-// list l becomes BF16(x_r - c_l) (kpad columns, zero past dpad), its FP32
-// residual norm ||x_r - c_l||^2, and the list's largest residual norm
-// (slightly rounded up).
-__global__ void residual_bf16_kernel(const float* __restrict__ codes, const int64_t* __restrict__ list_off,
-                                     const float* __restrict__ cent, int dpad, int kpad,
-                                     __nv_bfloat16* __restrict__ dst, float* __restrict__ rnorm,
-                                     float* __restrict__ rmax) {
-  __shared__ float s_max[32];
-  const int l = blockIdx.x;
-  const int64_t r0 = list_off[l], r1 = list_off[l + 1];
-  const float* c = cent + static_cast<size_t>(l) * dpad;
-  for (int64_t i = threadIdx.x; i < (r1 - r0) * kpad; i += blockDim.x) {
-    const int64_t r = r0 + i / kpad;
-    const int col = static_cast<int>(i % kpad);
-    dst[r * kpad + col] = __float2bfloat16_rn(col < dpad ? codes[r * dpad + col] - c[col] : 0.0f);
-  }
+// BF16 residual codes for the tensor-core scans: row r of list l becomes
+// BF16(x_r - c_l) (kpad columns, zero past dpad), its FP32 residual norm
+// ||x_r - c_l||^2, and the list's largest residual norm (slightly rounded up;
+// rmax holds its square until residual_rmax_kernel).  A warp takes 32
+// consecutive rows, four at a time while they share a list, so the rows of
+// long lists spread over the GPU.  Bound by DRAM: 6.5 bytes a column.  (A CTA
+// per list with a 64-bit division per element took 6.5 ms for 1M x 128.)
+__global__ void __launch_bounds__(256) residual_bf16_kernel(const float* __restrict__ codes,
+                                                            const int64_t* __restrict__ list_off, int nlist,
+                                                            int64_t ntotal, const float* __restrict__ cent, int dpad,
+                                                            int kpad, __nv_bfloat16* __restrict__ dst,
+                                                            float* __restrict__ rnorm, float* __restrict__ rmax) {
   const int lane = threadIdx.x & 31;
+  const int64_t w = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
+  const int64_t r0 = w * 32, r1 = min(ntotal, r0 + 32);
+  if (r0 >= r1) return;
+  int lo = 0, hi = nlist;  // list_off[lo] <= r0 < list_off[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (list_off[mid] <= r0) lo = mid; else hi = mid;
+  }
+  int l = lo;
+  int64_t end = list_off[l + 1];
   float m = 0.0f;
-  for (int64_t r = r0 + (threadIdx.x >> 5); r < r1; r += blockDim.x >> 5) {
-    float sq = 0.0f;
-    for (int j = lane; j < dpad; j += 32) {
-      const float v = codes[r * dpad + j] - c[j];
-      sq = fmaf(v, v, sq);
+  for (int64_t r = r0; r < r1;) {
+    while (r >= end) {
+      if (lane == 0 && m > 0.0f) atomicMax(reinterpret_cast<int*>(rmax + l), __float_as_int(m));
+      m = 0.0f;
+      ++l;
+      end = list_off[l + 1];
     }
-    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if (lane == 0) rnorm[r] = sq;
-    m = fmaxf(m, sq);
+    const float* c = cent + static_cast<size_t>(l) * dpad;
+    const int nr = static_cast<int>(min(static_cast<int64_t>(4), min(end, r1) - r));
+    float sq[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int j = lane; j < kpad; j += 32) {
+      const float cj = j < dpad ? c[j] : 0.0f;
+      float x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = u < nr && j < dpad ? codes[(r + u) * dpad + j] : cj;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float v = x[u] - cj;
+        if (j < dpad) sq[u] = fmaf(v, v, sq[u]);
+        if (u < nr) dst[(r + u) * kpad + j] = __float2bfloat16_rn(j < dpad ? v : 0.0f);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      for (int o = 16; o > 0; o >>= 1) sq[u] += __shfl_xor_sync(0xffffffffu, sq[u], o);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (u < nr) {
+        if (lane == 0) rnorm[r + u] = sq[u];
+        m = fmaxf(m, sq[u]);
+      }
+    r += nr;
   }
-  if (lane == 0) s_max[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) m = fmaxf(m, s_max[w]);
-    rmax[l] = sqrtf(m) * 1.0001f;
-  }
+  if (lane == 0 && m > 0.0f) atomicMax(reinterpret_cast<int*>(rmax + l), __float_as_int(m));
+}
+
+__global__ void residual_rmax_kernel(float* __restrict__ rmax, int nlist) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l < nlist) rmax[l] = sqrtf(rmax[l]) * 1.0001f;
 }
 
 constexpr int kSmallKth = 32;  // largest k for warp_kth_small8
@@ -1285,11 +1313,15 @@ void launch_query_prep(int nq, uint32_t* thr, int* cnt, cudaStream_t st) {
   HB_CUDA(cudaGetLastError());
 }
 
-void launch_residual_bf16(const float* codes, const int64_t* list_off, const float* cent, int nlist, int dpad, int kpad,
-                          void* dst, float* rnorm, float* rmax, cudaStream_t st) {
+void launch_residual_bf16(const float* codes, const int64_t* list_off, const float* cent, int nlist, size_t ntotal,
+                          int dpad, int kpad, void* dst, float* rnorm, float* rmax, cudaStream_t st) {
   if (nlist <= 0) return;
-  residual_bf16_kernel<<<nlist, 256, 0, st>>>(codes, list_off, cent, dpad, kpad, static_cast<__nv_bfloat16*>(dst),
-                                              rnorm, rmax);
+  HB_CUDA(cudaMemsetAsync(rmax, 0, static_cast<size_t>(nlist) * sizeof(float), st));
+  if (ntotal)
+    residual_bf16_kernel<<<static_cast<unsigned>((ntotal + 255) / 256), 256, 0, st>>>(
+        codes, list_off, nlist, static_cast<int64_t>(ntotal), cent, dpad, kpad, static_cast<__nv_bfloat16*>(dst), rnorm,
+        rmax);
+  residual_rmax_kernel<<<(nlist + 255) / 256, 256, 0, st>>>(rmax, nlist);
   HB_CUDA(cudaGetLastError());
 }
 
