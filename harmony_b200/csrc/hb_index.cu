@@ -1931,14 +1931,13 @@ class IndexCore {
     list_qoff_.reserve(nlist_ + 1);
     item_off_.reserve(nlist_ + 1);
     list_q_.reserve(nqp);
-    slot_base_.reserve(nqp + 1);
     const size_t wtmp = std::max(build_work_tmp_bytes(nb, P, static_cast<int>(nlist_)), cand_segments_tmp_bytes(nb, P));
     work_tmp_.reserve(wtmp);
     {
       Scope sc(this, "build_work");
       launches_ += launch_build_work(probes_.p, nb, P, list_off_.p, static_cast<int>(nlist_), cr, 128, list_cnt_.p,
-                                     list_qoff_.p, list_cursor_.p, list_q_.p, item_off_.p, slot_base_.p, work_tmp_.p,
-                                     wtmp, st_);
+                                     list_qoff_.p, list_cursor_.p, list_q_.p, item_off_.p, nullptr, work_tmp_.p, wtmp,
+                                     st_);
     }
     seg_.reserve(nqp + 1);
     {
@@ -1946,6 +1945,8 @@ class IndexCore {
       launch_cand_segments(probes_.p, nb, P, list_off_.p, seg_.p, work_tmp_.p, wtmp, st_);
     }
     launches_ += 2;
+    pcd_.reserve(nqp);
+    cand_m_.reserve(static_cast<size_t>(nb));
     if (fp8_) {
       ensure_fp8();
       qscale8_.reserve(nqp);
@@ -1953,8 +1954,8 @@ class IndexCore {
       gq8_.reserve(nqp * static_cast<size_t>(kpad8_));
       Scope sc(this, "gather_queries");
       launch_gather_residual(qpad_.p, static_cast<int>(dpad_), kpad8_, true, list_q_.p, list_qoff_.p,
-                             static_cast<int>(nlist_), cent_.p, static_cast<int64_t>(nqp), qscale8_.p, qcd8_.p,
-                             gq8_.p, st_);
+                             static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), qscale8_.p, qcd8_.p,
+                             pcd_.p, gq8_.p, st_);
       make_u8_tensor_map(gqmap_, gq8_.p, nqp, kpad8_);
       ++launches_;
     } else {
@@ -1962,8 +1963,8 @@ class IndexCore {
       qcd8_.reserve(nqp);
       Scope sc(this, "gather_queries");
       launch_gather_residual(qpad_.p, static_cast<int>(dpad_), kpad_, false, list_q_.p, list_qoff_.p,
-                             static_cast<int>(nlist_), cent_.p, static_cast<int64_t>(nqp), nullptr, qcd8_.p, gq_.p,
-                             st_);
+                             static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), nullptr, qcd8_.p,
+                             pcd_.p, gq_.p, st_);
       make_bf16_tensor_map(gqmap_, gq_.p, nqp, kpad_);
       ++launches_;
     }
@@ -2000,11 +2001,12 @@ class IndexCore {
     ++launches_;
     {
       Scope sc(this, "cand_select");
-      launch_cand_select(cand_.p, seg_.p, probes_.p, nb, P, R, list_off_.p, cand_rows_.p, st_);
+      launch_cand_select(cand_.p, seg_.p, probes_.p, nb, P, R, k, list_off_.p, pcd_.p, rmax_.p, static_cast<int>(dpad_),
+                         a.kpad, fp8_, cand_rows_.p, cand_m_.p, st_);
     }
     {
       Scope sc(this, "cand_exact");
-      launch_cand_exact(cand_rows_.p, nb, R, k, codes_.p, qpad_.p, static_cast<int>(dpad_), ids_.p, Dd, Id, st_);
+      launch_cand_exact(cand_rows_.p, cand_m_.p, nb, R, k, codes_.p, qpad_.p, static_cast<int>(dpad_), ids_.p, Dd, Id, st_);
     }
     launches_ += 2;
     if (!capturing_) bf16_err_check();
@@ -2364,6 +2366,8 @@ class IndexCore {
   DevBuf<uint16_t> gq_;
   DevBuf<float> cand_;
   DevBuf<int64_t> cand_rows_;
+  DevBuf<float> pcd_;   // ||q - c_l||^2 per (query, probe rank)
+  DevBuf<int> cand_m_;  // rows re-ranked per query
   // tensor-core coarse quantizer
   bool coarse_ready_ = false;
   int coarse_kind_ = HB_COARSE_AUTO;

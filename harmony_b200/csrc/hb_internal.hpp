@@ -327,18 +327,22 @@ void launch_cand_scan(const void* tmap_q, const void* tmap_x, const CandArgs& a,
 // and ||q - c_l||^2.
 void launch_fp8_codes(const float* codes, const int64_t* list_off, const float* cent, int nlist, int dpad, int kpad8,
                       void* out, float* scale, float* rnorm, cudaStream_t st);
-// Per list-major entry e (query q, list l): row e of G = q - c_l in BF16, or
-// (fp8) E4M3 with its scale escale[e]; ecd[e] = ||q - c_l||^2.
+// Per list-major entry e (query q, probe rank j, list l): row e of G = q - c_l
+// in BF16, or (fp8) E4M3 with its scale escale[e]; ecd[e] = pcd[q * P + j] =
+// ||q - c_l||^2.
 void launch_gather_residual(const float* q, int dpad, int kpad, bool fp8, const int32_t* list_q,
-                            const int64_t* list_qoff, int nlist, const float* cent, int64_t max_rows, float* escale,
-                            float* ecd, void* G, cudaStream_t st);
+                            const int64_t* list_qoff, int nlist, int P, const float* cent, int64_t max_rows,
+                            float* escale, float* ecd, float* pcd, void* G, cudaStream_t st);
 void make_u8_tensor_map(void* tmap_out, const void* base, size_t rows, int row_bytes);
-// Selection of each query's R candidates (rows: nq x R stored rows, -1 past
-// the candidates), then their exact re-rank to the k best.
-void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* probes, int nq, int P, int R,
-                        const int64_t* list_off, int64_t* rows, cudaStream_t st);
-void launch_cand_exact(const int64_t* rows, int nq, int R, int k, const float* codes, const float* q, int dpad,
-                       const int64_t* ids, float* D, int64_t* I, cudaStream_t st);
+// Selection of each query's R best candidates, less those that cannot be among
+// the k best of them (rows: nq x R stored rows, m[q] of them), then their
+// exact re-rank to the k best.  pcd: nq x P ||q - c_l||^2, rmax: per list the
+// largest residual norm (the error bound's operands).
+void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* probes, int nq, int P, int R, int k,
+                        const int64_t* list_off, const float* pcd, const float* rmax, int dpad, int kpad, bool fp8,
+                        int64_t* rows, int* m, cudaStream_t st);
+void launch_cand_exact(const int64_t* rows, const int* m, int nq, int R, int k, const float* codes, const float* q,
+                       int dpad, const int64_t* ids, float* D, int64_t* I, cudaStream_t st);
 void launch_to_bf16(const float* src, size_t n, int dpad, int kpad, void* dst, cudaStream_t st);
 void launch_scan_bf16(const void* tmap, const TcArgs& a, int num_sms, cudaStream_t st);
 // One thread waits on an mbarrier nothing arrives on, with a budget of

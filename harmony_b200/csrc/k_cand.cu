@@ -36,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include <cub/cub.cuh>
 
@@ -58,9 +59,10 @@ constexpr int kAccN = 4;                    // TMEM accumulators of 128 columns 
 constexpr int kSelectThreads = 256;
 constexpr int kBins = 2048;                 // histogram bins of the candidate selection
 constexpr int kSelUnroll = 4;               // 32-value runs a warp loads at once
-constexpr int kExactThreads = 256;
+constexpr int kExactThreads = 128;
 constexpr int kExChunk = 32;                // dimensions per staged chunk of the exact re-rank
-constexpr int kExStride = kExChunk + 1;     // odd row stride: column reads hit distinct banks
+constexpr int kExStride = kExChunk + 4;     // row stride: 16-byte reads of eight rows hit distinct banks
+constexpr int kExStages = 3;
 
 struct CandShared {
   uint64_t full[kStg];
@@ -333,60 +335,71 @@ __global__ void list_fp8_kernel(const float* __restrict__ codes, const int64_t* 
   }
 }
 
-// One warp per list-major entry e (query q, list l): q' = q - c_l as row e of
-// the gathered matrix -- BF16, or (FP8) E4M3(q' / s_e) with the entry's scale
-// s_e = max |q'| / 448 -- and ||q'||^2 (the scan's value of a row is
-// ||q'||^2 + ||r||^2 - 2 q'.r with r = x - c_l).
-template <bool FP8>
-__global__ void gather_residual_kernel(const float* __restrict__ q, int dpad, int kpad,
-                                       const int32_t* __restrict__ list_q, const int64_t* __restrict__ list_qoff,
-                                       int nlist, const float* __restrict__ cent, int64_t max_rows,
-                                       float* __restrict__ escale, float* __restrict__ ecd, void* __restrict__ G) {
+// A warp per list-major entry e (query q, probe rank j, list l): q' = q - c_l
+// as row e of the gathered matrix -- BF16, or (FP8) E4M3(q' / s_e) with the
+// entry's scale s_e = max |q'| / 448 -- and ||q'||^2, also at probe slot
+// q * P + j (the scan's value of a row is ||q'||^2 + ||r||^2 - 2 q'.r with
+// r = x - c_l).  blockIdx.x is the list, whose centroid stays in registers
+// (4 consecutive columns per lane and 128-column block, NI blocks) while the
+// warps of its gridDim.y CTAs stride over its entries: no search for an
+// entry's list and one pass over its row.  Bound by the rows written.
+template <bool FP8, int NI>
+__global__ void __launch_bounds__(256) gather_residual_kernel(const float* __restrict__ q, int dpad, int kpad,
+                                                              const int32_t* __restrict__ list_q,
+                                                              const int64_t* __restrict__ list_qoff, int P,
+                                                              const float* __restrict__ cent, int64_t max_rows,
+                                                              float* __restrict__ escale, float* __restrict__ ecd,
+                                                              float* __restrict__ pcd, void* __restrict__ G) {
   const int lane = threadIdx.x & 31;
-  const int64_t rows = min(list_qoff[nlist], max_rows);
-  for (int64_t e = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5; e < rows;
-       e += (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5) {
-    int lo = 0, hi = nlist;  // list of entry e: largest l with list_qoff[l] <= e
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (list_qoff[mid] <= e) lo = mid; else hi = mid;
-    }
-    const int qi = static_cast<int>(static_cast<uint32_t>(list_q[e]) >> 16);
-    const float* src = q + static_cast<int64_t>(qi) * dpad;
-    const float* c = cent + static_cast<size_t>(lo) * dpad;
+  const int l = blockIdx.x;
+  const int64_t e1 = min(list_qoff[l + 1], max_rows);
+  int64_t e = list_qoff[l] + blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (e >= e1) return;
+  float4 c[NI];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int col = 128 * i + 4 * lane;
+    c[i] = col < dpad ? *reinterpret_cast<const float4*>(cent + static_cast<size_t>(l) * dpad + col)
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  for (; e < e1; e += static_cast<int64_t>(gridDim.y) * (blockDim.x >> 5)) {
+    const uint32_t ent = static_cast<uint32_t>(list_q[e]);
+    const float* src = q + static_cast<int64_t>(ent >> 16) * dpad;
+    float4 v[NI];
     float m = 0.0f, sq = 0.0f;
-    for (int j = lane; j < dpad; j += 32) {
-      const float v = src[j] - c[j];
-      m = fmaxf(m, fabsf(v));
-      sq = fmaf(v, v, sq);
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int col = 128 * i + 4 * lane;
+      v[i] = col < dpad ? __ldg(reinterpret_cast<const float4*>(src + col)) : c[i];
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      v[i] = make_float4(v[i].x - c[i].x, v[i].y - c[i].y, v[i].z - c[i].z, v[i].w - c[i].w);
+      sq = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, sq))));
+      if (FP8) m = fmaxf(m, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
     }
     for (int o = 16; o > 0; o >>= 1) {
-      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
       sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      if (FP8) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     }
-    if (lane == 0) ecd[e] = sq;
-    if (FP8) {
-      const float inv = m > 0.0f ? 448.0f / m : 1.0f;
-      if (lane == 0) escale[e] = 1.0f / inv;
-      uint8_t* row = static_cast<uint8_t*>(G) + e * kpad;
-      for (int cc = lane * 16; cc < kpad; cc += 32 * 16) {
-        float x[16];
+    if (lane == 0) {
+      ecd[e] = sq;
+      pcd[static_cast<int64_t>(ent >> 16) * P + (ent & 0xffffu)] = sq;
+    }
+    const float inv = FP8 && m > 0.0f ? 448.0f / m : 1.0f;
+    if (FP8 && lane == 0) escale[e] = 1.0f / inv;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = cc + j < dpad ? src[cc + j] - c[cc + j] : 0.0f;
-        *reinterpret_cast<uint4*>(row + cc) = to_e4m3x16(x, inv);
-      }
-    } else {
-      __nv_bfloat16* row = static_cast<__nv_bfloat16*>(G) + e * kpad;
-      for (int cc = lane * 8; cc < kpad; cc += 32 * 8) {
-        uint32_t w[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float a0 = cc + 2 * j < dpad ? src[cc + 2 * j] - c[cc + 2 * j] : 0.0f;
-          const float a1 = cc + 2 * j + 1 < dpad ? src[cc + 2 * j + 1] - c[cc + 2 * j + 1] : 0.0f;
-          __nv_bfloat162 p2 = __floats2bfloat162_rn(a0, a1);
-          w[j] = *reinterpret_cast<uint32_t*>(&p2);
-        }
-        *reinterpret_cast<uint4*>(row + cc) = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int i = 0; i < NI; ++i) {
+      const int col = 128 * i + 4 * lane;
+      if (col >= kpad) continue;
+      if (FP8) {
+        const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[i].x * inv, v[i].y * inv), __NV_SATFINITE, __NV_E4M3);
+        const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[i].z * inv, v[i].w * inv), __NV_SATFINITE, __NV_E4M3);
+        *reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(G) + e * kpad + col) = lo | (hi << 16);
+      } else {
+        const __nv_bfloat162 p0 = __floats2bfloat162_rn(v[i].x, v[i].y), p1 = __floats2bfloat162_rn(v[i].z, v[i].w);
+        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(G) + e * kpad + col) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
       }
     }
   }
@@ -414,6 +427,21 @@ __device__ __forceinline__ int value_bin(float v, float vmin, float scale) {
   return t < static_cast<float>(kBins) ? max(0, static_cast<int>(t)) : kBins - 1;
 }
 
+// |v - d| of a candidate row: v the scan's value, d the reference's sequential
+// FP32 distance, Q = ||q - c_l||, R = the list's largest residual norm.  BF16:
+// the terms of the bounded scan's error bound (k_tc.cu), the FP32 accumulation
+// scaled to kpad products.  E4M3: each operand within 2^-4 of its value (3
+// mantissa bits) plus 1e-4 of the norm (subnormals: half of 2^-9 of a scale of
+// max / 448, over at most 1024 columns), so the product within 2 * 0.0626 +
+// 0.0626^2 of Q R, and 2^-8 Q R per 128 products for the accumulation.
+__device__ __forceinline__ float cand_eps(float cd, float R, int d, int kpad, bool fp8) {
+  const float Q = sqrtf(cd) * 1.0001f + 1e-30f;
+  const float u = 5.9604645e-8f;  // 2^-24
+  const float blocks = static_cast<float>((kpad + 127) / 128);
+  const float c1 = fp8 ? 0.1292f + 0.00390625f * blocks : 0.00390625f + 0.0009765625f * blocks + 1.52587890625e-5f;
+  return 1.0625f * (2.0f * c1 * Q * R + (d + 3) * u * (R * R + Q * Q) + (d + 5) * u * (Q + R) * (Q + R)) + 1e-30f;
+}
+
 // One CTA per query: the R smallest keys (v, position) of the query's
 // candidate row -- unique, so the R chosen are the R smallest values with
 // ties to the earlier position -- mapped back to their stored rows, in
@@ -423,10 +451,15 @@ __device__ __forceinline__ int value_bin(float v, float vmin, float scale) {
 // the R-th value into shared memory, which a bitonic sort orders.  A row
 // whose compacted set would exceed the buffer (a dense bin) takes the
 // block radix selection instead.  Padding (+inf) is no candidate.
+// Of the R, those that the scan's error bound proves to be outside the k best
+// of the R are dropped: the first k candidates' largest upper bound U is at
+// least the k-th smallest distance, so a row with v - eps > U is not among the
+// k.  The others go out in ascending order, m_out[q] of them.
 __global__ void __launch_bounds__(kSelectThreads)
     cand_select_kernel(const float* __restrict__ cand, const int64_t* __restrict__ seg,
-                       const int32_t* __restrict__ probes, int P, int R, const int64_t* __restrict__ list_off,
-                       int cap, int64_t* __restrict__ out_rows) {
+                       const int32_t* __restrict__ probes, int P, int R, int k, const int64_t* __restrict__ list_off,
+                       const float* __restrict__ pcd, const float* __restrict__ rmax, int dpad, int kpad, int fp8,
+                       int cap, int64_t* __restrict__ out_rows, int* __restrict__ m_out) {
   extern __shared__ __align__(16) unsigned char smem_sel[];
   uint64_t* s_cand = reinterpret_cast<uint64_t*>(smem_sel);  // cap keys (a power of two >= 2 * pow2(R))
   __shared__ int s_hist[kBins];
@@ -558,88 +591,129 @@ __global__ void __launch_bounds__(kSelectThreads)
       block_topk_sorted(key_at, m, R, sh_sel, s_cand);
     }
   }
-  for (int i = tid; i < R; i += kSelectThreads) {
+  // Per candidate: its probe rank (the last whose segment starts at or before
+  // its position), stored row and eps; U over the first k.
+  __syncthreads();
+  if (tid == 0) {
+    s_cnt = 0;
+    s_hi = 0u;  // U, as ordered bits
+  }
+  __syncthreads();
+  auto locate = [&](int i, int& rank) -> int64_t {
+    const int64_t pos = r0 + key_tie(s_cand[i]);
+    int lo = 0, hi = P;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (sq[mid] <= pos) lo = mid; else hi = mid;
+    }
+    rank = lo;
+    return pos - sq[lo];
+  };
+  const int32_t* prow = probes + static_cast<int64_t>(qi) * P;
+  const float* cdrow = pcd + static_cast<int64_t>(qi) * P;
+  unsigned int ub = 0u;
+  for (int i = tid; i < min(k, need); i += kSelectThreads) {
+    int j;
+    locate(i, j);
+    const float v = ordered_to_float(static_cast<uint32_t>(s_cand[i] >> 32));
+    const float t = __fadd_ru(v, cand_eps(cdrow[j], rmax[prow[j]], dpad, kpad, fp8 != 0));
+    ub = max(ub, ordered_bits(t == t ? t : INFINITY));
+  }
+  for (int off = 16; off > 0; off >>= 1) ub = max(ub, __shfl_xor_sync(0xffffffffu, ub, off));
+  if (lane == 0 && ub) atomicMax(&s_hi, ub);
+  __syncthreads();
+  const float U = need < k ? INFINITY : ordered_to_float(s_hi);
+  // The kept rows in order: a CTA-wide running count, kSelectThreads at a time.
+  __shared__ int s_w[kSelectThreads / 32];
+  for (int b0 = 0; b0 < need; b0 += kSelectThreads) {
+    const int i = b0 + tid;
+    bool keep = false;
     int64_t row = -1;
     if (i < need) {
-      const int64_t pos = r0 + key_tie(s_cand[i]);
-      int lo = 0, hi = P;  // the last probe rank whose segment starts at or before pos
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (sq[mid] <= pos) lo = mid; else hi = mid;
-      }
-      row = list_off[probes[static_cast<int64_t>(qi) * P + lo]] + (pos - sq[lo]);
+      int j;
+      const int64_t off = locate(i, j);
+      const float v = ordered_to_float(static_cast<uint32_t>(s_cand[i] >> 32));
+      keep = !(__fsub_rd(v, cand_eps(cdrow[j], rmax[prow[j]], dpad, kpad, fp8 != 0)) > U);
+      row = list_off[prow[j]] + off;
     }
-    out_rows[static_cast<int64_t>(qi) * R + i] = row;
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    if (lane == 0) s_w[warp] = __popc(bal);
+    __syncthreads();
+    int base = s_cnt, tot = 0;
+    for (int w = 0; w < kSelectThreads / 32; ++w) {
+      if (w < warp) base += s_w[w];
+      tot += s_w[w];
+    }
+    if (keep) out_rows[static_cast<int64_t>(qi) * R + base + __popc(bal & ((1u << lane) - 1u))] = row;
+    __syncthreads();
+    if (tid == 0) s_cnt += tot;
+    __syncthreads();
   }
+  if (tid == 0) m_out[qi] = s_cnt;
 }
 
-// One CTA per query: exact distances of its R candidate rows with the
-// reference's sequential unfused FP32 loop (the same operations, in the same
-// order, as exact_l2_seq), then the k best (distance, row).  Thread t owns
-// candidate t of each batch of blockDim.x (R rounded up to a warp, 64 to
-// 256); the batch's rows and the query are staged 32 dimensions at a time
-// in shared memory by coalesced loads (four 128-byte rows per warp
-// instruction, all of a thread's loads in flight at once), and each thread
-// continues its own sum over the chunk from shared memory.
+// One CTA per query: exact distances of its m candidate rows (m[q] of the R
+// slots) with the reference's sequential unfused FP32 loop (the same
+// operations, in the same order, as exact_l2_seq), then the k best (distance,
+// row).  Thread t owns candidate t of each batch of kExactThreads rows; the
+// rows pass through shared memory kExChunk dimensions at a time, copied by
+// 16-byte cp.async in a ring of kExStages chunks so that the next chunks'
+// fetches overlap this one's sums, and each thread continues its own sum from
+// there.  Bound by the gathered rows (DRAM).
 __global__ void __launch_bounds__(kExactThreads)
-    cand_exact_kernel(const int64_t* __restrict__ rows, int R, int k, const float* __restrict__ codes,
-                      const float* __restrict__ q, int dpad, const int64_t* __restrict__ ids, float* __restrict__ D,
-                      int64_t* __restrict__ I) {
+    cand_exact_kernel(const int64_t* __restrict__ rows, const int* __restrict__ m_in, int R, int k,
+                      const float* __restrict__ codes, const float* __restrict__ q, int dpad,
+                      const int64_t* __restrict__ ids, float* __restrict__ D, int64_t* __restrict__ I) {
   extern __shared__ __align__(16) unsigned char smem_ex[];
   __shared__ int64_t s_rows[kExactThreads];
-  __shared__ __align__(16) float s_q[kExChunk];
-  const int qi = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
-  const int n2 = pow2_ceil(R < 2 ? 2 : R);
+  const int qi = blockIdx.x, tid = threadIdx.x;
+  const int m = m_in[qi];
+  const int n2 = pow2_ceil(max(2, max(m, k)));
   uint64_t* s_ex = reinterpret_cast<uint64_t*>(smem_ex);
-  float* s_tile = reinterpret_cast<float*>(s_ex + n2);  // nt x kExStride
+  float* s_q = reinterpret_cast<float*>(s_ex + pow2_ceil(R < 2 ? 2 : R));  // dpad
+  float* s_tile = s_q + dpad;                                             // [kExStages][kExactThreads][kExStride]
   const float* qrow = q + static_cast<size_t>(qi) * dpad;
-  for (int i = tid; i < n2; i += nt) s_ex[i] = kEmpty;
-  for (int b0 = 0; b0 < R; b0 += nt) {
-    const int i = b0 + tid;
-    const int64_t row = i < R ? rows[static_cast<int64_t>(qi) * R + i] : -1;
+  for (int c = 4 * tid; c < dpad; c += 4 * kExactThreads)
+    *reinterpret_cast<float4*>(s_q + c) = *reinterpret_cast<const float4*>(qrow + c);
+  for (int i = tid; i < n2; i += kExactThreads) s_ex[i] = kEmpty;
+  const int nch = (dpad + kExChunk - 1) / kExChunk;
+  for (int b0 = 0; b0 < m; b0 += kExactThreads) {
+    const int nb = min(kExactThreads, m - b0);
+    const int64_t row = tid < nb ? rows[static_cast<int64_t>(qi) * R + b0 + tid] : -1;
+    __syncthreads();  // the previous batch's readers are done
     s_rows[tid] = row;
-    float acc = 0.0f;
-    for (int c0 = 0; c0 < dpad; c0 += kExChunk) {
-      const int w4 = min(kExChunk, dpad - c0) / 4;  // dpad is a multiple of 4
-      __syncthreads();                              // rows published / previous chunk consumed
-      if (tid < w4) *reinterpret_cast<float4*>(s_q + 4 * tid) = *reinterpret_cast<const float4*>(qrow + c0 + 4 * tid);
-#pragma unroll
-      for (int j = 0; j < kExChunk / 4; ++j) {
-        const int u = tid + j * nt;
-        const int r = u / (kExChunk / 4), f = u % (kExChunk / 4);
-        const int64_t rr = s_rows[r];
-        if (rr >= 0 && f < w4) {
-          const float4 v = *reinterpret_cast<const float4*>(codes + rr * dpad + c0 + 4 * f);
-          float* dst = s_tile + r * kExStride + 4 * f;
-          dst[0] = v.x;
-          dst[1] = v.y;
-          dst[2] = v.z;
-          dst[3] = v.w;
+    __syncthreads();
+    // Four 16-byte pieces per row and chunk: eight rows per warp instruction.
+    auto fetch = [&](int ch) {
+      if (ch < nch) {
+        float* dst = s_tile + static_cast<size_t>(ch % kExStages) * kExactThreads * kExStride;
+        const int w4 = min(kExChunk, dpad - ch * kExChunk) / 4;
+        for (int u = tid; u < nb * (kExChunk / 4); u += kExactThreads) {
+          const int r = u / (kExChunk / 4), f = u % (kExChunk / 4);
+          if (f < w4) cp_async16(dst + r * kExStride + 4 * f, codes + s_rows[r] * dpad + ch * kExChunk + 4 * f, true);
         }
       }
-      __syncthreads();
-      if (row >= 0) {
-        const float* x = s_tile + tid * kExStride;
-        for (int c = 0; c < 4 * w4; c += 4) {
-          const float4 qq = *reinterpret_cast<const float4*>(s_q + c);
-          const float x0 = x[c], x1 = x[c + 1], x2 = x[c + 2], x3 = x[c + 3];
-          float t = __fsub_rn(qq.x, x0);
-          acc = __fadd_rn(acc, __fmul_rn(t, t));
-          t = __fsub_rn(qq.y, x1);
-          acc = __fadd_rn(acc, __fmul_rn(t, t));
-          t = __fsub_rn(qq.z, x2);
-          acc = __fadd_rn(acc, __fmul_rn(t, t));
-          t = __fsub_rn(qq.w, x3);
-          acc = __fadd_rn(acc, __fmul_rn(t, t));
-        }
+      cp_async_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < kExStages - 1; ++s) fetch(s);
+    float acc = 0.0f;
+    for (int ch = 0; ch < nch; ++ch) {
+      cp_async_wait<kExStages - 2>();
+      __syncthreads();  // chunk ch has landed for every thread; chunk ch - 1 is consumed
+      fetch(ch + kExStages - 1);
+      if (tid < nb) {
+        const float* x = s_tile + (static_cast<size_t>(ch % kExStages) * kExactThreads + tid) * kExStride;
+        acc = exact_l2_seq_from(acc, x, s_q + ch * kExChunk, min(kExChunk, dpad - ch * kExChunk));
       }
     }
-    if (row >= 0 && acc < FLT_MAX) s_ex[i] = make_key(acc, static_cast<uint32_t>(row));
+    cp_async_wait<0>();
+    if (tid < nb && acc < FLT_MAX) s_ex[b0 + tid] = make_key(acc, static_cast<uint32_t>(row));
   }
   __syncthreads();
   block_bitonic_sort(s_ex, n2);
-  for (int j = tid; j < k; j += nt) {
-    const uint64_t key = j < n2 ? s_ex[j] : kEmpty;
+  for (int j = tid; j < k; j += kExactThreads) {
+    const uint64_t key = s_ex[j];
     const size_t o = static_cast<size_t>(qi) * k + j;
     D[o] = key == kEmpty ? FLT_MAX : key_dist(key);
     I[o] = key == kEmpty ? -1 : ids[key_tie(key)];
@@ -702,18 +776,24 @@ void launch_fp8_codes(const float* codes, const int64_t* list_off, const float* 
 }
 
 void launch_gather_residual(const float* q, int dpad, int kpad, bool fp8, const int32_t* list_q,
-                            const int64_t* list_qoff, int nlist, const float* cent, int64_t max_rows, float* escale,
-                            float* ecd, void* G, cudaStream_t st) {
+                            const int64_t* list_qoff, int nlist, int P, const float* cent, int64_t max_rows,
+                            float* escale, float* ecd, float* pcd, void* G, cudaStream_t st) {
   if (max_rows <= 0) return;
-  HB_CHECK(kpad % (fp8 ? 128 : 64) == 0 && dpad <= kpad && kpad <= 2048, HB_ERR_INVALID, "bad residual padding");
-  int64_t g = (max_rows * 32 + 255) / 256;
-  if (g > 148 * 32) g = 148 * 32;
-  if (fp8)
-    gather_residual_kernel<true><<<static_cast<unsigned>(g), 256, 0, st>>>(q, dpad, kpad, list_q, list_qoff, nlist,
-                                                                           cent, max_rows, escale, ecd, G);
-  else
-    gather_residual_kernel<false><<<static_cast<unsigned>(g), 256, 0, st>>>(q, dpad, kpad, list_q, list_qoff, nlist,
-                                                                            cent, max_rows, escale, ecd, G);
+  HB_CHECK(kpad % (fp8 ? 128 : 64) == 0 && dpad <= kpad && kpad <= 1024, HB_ERR_INVALID, "bad residual padding");
+  // About 16 CTAs per SM over all lists.
+  const dim3 g(nlist, static_cast<unsigned>(std::max(1, std::min(64, 148 * 16 / nlist))));
+  auto go = [&](auto f, auto ni) {
+    gather_residual_kernel<decltype(f)::value, decltype(ni)::value>
+        <<<g, 256, 0, st>>>(q, dpad, kpad, list_q, list_qoff, P, cent, max_rows, escale, ecd, pcd, G);
+  };
+  auto width = [&](auto f) {
+    if (kpad <= 128) go(f, std::integral_constant<int, 1>{});
+    else if (kpad <= 256) go(f, std::integral_constant<int, 2>{});
+    else if (kpad <= 512) go(f, std::integral_constant<int, 4>{});
+    else go(f, std::integral_constant<int, 8>{});
+  };
+  if (fp8) width(std::true_type{});
+  else width(std::false_type{});
   HB_CUDA(cudaGetLastError());
 }
 
@@ -734,29 +814,31 @@ void make_u8_tensor_map(void* tmap_out, const void* base, size_t rows, int row_b
   HB_CHECK(r == CUDA_SUCCESS, HB_ERR_CUDA, "cuTensorMapEncodeTiled failed (FP8)");
 }
 
-void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* probes, int nq, int P, int R,
-                        const int64_t* list_off, int64_t* rows, cudaStream_t st) {
+void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* probes, int nq, int P, int R, int k,
+                        const int64_t* list_off, const float* pcd, const float* rmax, int dpad, int kpad, bool fp8,
+                        int64_t* rows, int* m_out, cudaStream_t st) {
   if (nq <= 0) return;
-  HB_CHECK(R >= 1 && R <= kCandMaxR, HB_ERR_INVALID, "candidate count out of range");
+  HB_CHECK(R >= 1 && R <= kCandMaxR && k >= 1 && k <= R, HB_ERR_INVALID, "candidate count out of range");
   // Compaction buffer: at least 2048 keys and four times the R kept.
   const int cap = std::max(2048, 4 * pow2_ceil(R < 2 ? 2 : R));
   const size_t smem_sel = static_cast<size_t>(cap) * sizeof(uint64_t);
   HB_CUDA(cudaFuncSetAttribute(cand_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem_sel)));
-  cand_select_kernel<<<nq, kSelectThreads, smem_sel, st>>>(cand, seg, probes, P, R, list_off, cap, rows);
+  cand_select_kernel<<<nq, kSelectThreads, smem_sel, st>>>(cand, seg, probes, P, R, k, list_off, pcd, rmax, dpad, kpad,
+                                                           fp8 ? 1 : 0, cap, rows, m_out);
   HB_CUDA(cudaGetLastError());
 }
 
-void launch_cand_exact(const int64_t* rows, int nq, int R, int k, const float* codes, const float* q, int dpad,
-                       const int64_t* ids, float* D, int64_t* I, cudaStream_t st) {
+void launch_cand_exact(const int64_t* rows, const int* m, int nq, int R, int k, const float* codes, const float* q,
+                       int dpad, const int64_t* ids, float* D, int64_t* I, cudaStream_t st) {
   if (nq <= 0) return;
   HB_CHECK(R >= 1 && R <= kCandMaxR && k <= R, HB_ERR_INVALID, "candidate count out of range");
-  const size_t keys = static_cast<size_t>(pow2_ceil(R < 2 ? 2 : R)) * sizeof(uint64_t);
-  const int nt = std::min(kExactThreads, std::max(64, (R + 31) / 32 * 32));
-  const size_t smem_ex = keys + static_cast<size_t>(nt) * kExStride * sizeof(float);
+  const size_t smem_ex = static_cast<size_t>(pow2_ceil(R < 2 ? 2 : R)) * sizeof(uint64_t) +
+                         (static_cast<size_t>(dpad) + static_cast<size_t>(kExStages) * kExactThreads * kExStride) *
+                             sizeof(float);
   HB_CUDA(cudaFuncSetAttribute(cand_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem_ex)));
-  cand_exact_kernel<<<nq, nt, smem_ex, st>>>(rows, R, k, codes, q, dpad, ids, D, I);
+  cand_exact_kernel<<<nq, kExactThreads, smem_ex, st>>>(rows, m, R, k, codes, q, dpad, ids, D, I);
   HB_CUDA(cudaGetLastError());
 }
 
