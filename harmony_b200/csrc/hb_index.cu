@@ -62,6 +62,11 @@ constexpr double kAssignTcAdd = 5.0e9;
 // 2.6e5 pairs 148 -> 181 us, 1.0e6 254 -> 194.
 constexpr double kScreenPairs = 2.0e5, kScreenPairsShort = 8.0e5;
 constexpr double kScreenShortRows = 256.0;
+// d > 128, pairs x padded dimensions: 270k x 500 (527 rows a list) 2.1e4 pairs
+// 193 -> 180 us, 8.4e4 313 -> 183, 1.4e6 797 -> 231; 100k x 200 5.1e4 pairs 145 ->
+// 141 us, 1.3e4 117 -> 134; 100-row lists 2.6e5 pairs 113 -> 137, 1.0e6 200 -> 159.
+constexpr double kScreenWideWork = 1.2e7, kScreenWideWorkShort = 1.0e8;
+constexpr int kScreenWideRows = 2048;  // rows re-ranked per query of a wide FP32 search; more go to the exact scan
 
 int pow2_floor(long long x) {
   int p = 1;
@@ -852,6 +857,7 @@ class IndexCore {
     // FP32 plain scans take the bounded tensor-core scan too where it serves
     // (screen_batch); the result is the exact scan's either way.
     screen_ = !bf16 && exact_k && screen_possible(static_cast<int>(k));
+    screen_wide_ = screen_ && kpad_ > 128;  // through the candidate matrix
     int mode = SCAN_PLAIN;
     size_t P = nprobe_;
     int W = 1, B = 1;
@@ -913,7 +919,13 @@ class IndexCore {
     const bool dev_in = is_device_ptr(q);
     size_t bs = std::min<size_t>(nq, batch_limit(P, k));
     if (cand_path_ && P > 0) bs = std::min(bs, cand_batch_limit(P));
-    const size_t bounded_bs = std::max<size_t>(1, (size_t(1) << 30) / (static_cast<size_t>(filter_cap(k)) * 8));
+    size_t bounded_bs = std::max<size_t>(1, (size_t(1) << 30) / (static_cast<size_t>(filter_cap(k)) * 8));
+    if (screen_wide_ && mode == SCAN_PLAIN && P > 0) {
+      // A query's candidate row has to fit.
+      const int64_t L = cand_row_bound(static_cast<int>(P));
+      screen_ = L <= (int64_t(1) << 30);
+      if (screen_) bounded_bs = cand_batch_limit(P);
+    }
     if (bf16 && !cand_path_) bs = std::min(bs, bounded_bs);
     screen_ = screen_ && mode == SCAN_PLAIN && P > 0 &&
               screen_pays(static_cast<int>(std::min(bs, bounded_bs)), static_cast<int>(P)) &&
@@ -1024,7 +1036,7 @@ class IndexCore {
       cut_src_ = npqin_.p;
     }
     cut_b0_ = 0;
-    if (screen_) screen_ = screen_reserve(nb, k);
+    if (screen_) screen_ = screen_reserve(nb, P, k);
     char key[256];
     std::snprintf(key, sizeof(key), "%d/%d/%d/%d/%d/%d/%d/%08x/%d/%d/%d/%d/%d/%d", nb, k, P, R, p.precision, p.mode,
                   cut_mode_, cut_mode_ == 1 ? *reinterpret_cast<const uint32_t*>(&cut_thr_) : 0u, cut_cap_,
@@ -1500,37 +1512,49 @@ class IndexCore {
   // The bounded scan decides which rows can be among the k nearest and
   // recomputes those with the exact FP32 loop; every distance returned is that
   // loop's, and so is the order (see k_tc.cu).  It serves plain FP32 searches
-  // of d <= 128 and k <= 256 as well, as the tensor-core coarse quantizer
-  // serves the probes.  Queries outside its error bound's range or with too
+  // of k <= 256 as well, as the tensor-core coarse quantizer serves the
+  // probes; for d > 128 the candidate matrix takes its place, with every row
+  // that the bound allows among the k nearest re-ranked (k_cand.cu).  Queries outside its error bound's range or with too
   // many candidates are searched with the exact scan, and so is the whole
   // batch when its buffers cannot be had or a device wait gave up.
   bool screen_possible(int k) const {
-    return bf16_ready_ && kpad_ <= 128 && k <= kFilterMaxK && ntotal_ < (size_t(1) << 31) - 8192;
+    return bf16_ready_ && k <= kFilterMaxK && ntotal_ < (size_t(1) << 31) - 8192;
   }
   bool screen_pays(int nb, int P) const {
     const double avg = static_cast<double>(ntotal_) / static_cast<double>(std::max<size_t>(nlist_, 1));
-    return static_cast<double>(nb) * P * avg >= (avg < kScreenShortRows ? kScreenPairsShort : kScreenPairs);
+    const double pairs = static_cast<double>(nb) * P * avg;
+    const bool short_lists = avg < kScreenShortRows;
+    if (kpad_ > 128) return pairs * dpad_ >= (short_lists ? kScreenWideWorkShort : kScreenWideWork);
+    return pairs >= (short_lists ? kScreenPairsShort : kScreenPairs);
   }
 
-  bool screen_reserve(int nb, int k) {
+  bool screen_reserve(int nb, int P, int k) {
     try {
-      bounded_reserve(nb, filter_cap(k), scr_cnt_, scr_m_);
+      if (screen_wide_)
+        cand_reserve(nb, P, kScreenWideRows, false);
+      else
+        bounded_reserve(nb, filter_cap(k), scr_cnt_, scr_m_);
       return true;
     } catch (const Error& e) {
       if (e.code != HB_ERR_NOMEM) throw;
       cudaGetLastError();
       cbuf_.release();  // the exact scan's buffers need the memory
       cbuf_ub_.release();
+      cand_.release();
+      gq_.release();
       return false;
     }
   }
 
   bool screen_batch(int nb, int P, int k, float* Dd, int64_t* Id) {
-    screen_ = screen_reserve(nb, k);
+    screen_ = screen_reserve(nb, P, k);
     if (!screen_) return false;
     const int cap = filter_cap(k);
     const int cr = std::max(128, chunk_rows_for(nb, P, 128));
-    filter_pipeline(nb, P, k, cap, cr, scan_bf16_stages(kpad_), scr_cnt_.p, scr_m_.p, kDefaultWaitBudget, Dd, Id);
+    if (screen_wide_)
+      cand_pipeline(nb, P, k, kScreenWideRows, false, true, Dd, Id);
+    else
+      filter_pipeline(nb, P, k, cap, cr, scan_bf16_stages(kpad_), scr_cnt_.p, scr_m_.p, kDefaultWaitBudget, Dd, Id);
     if (!capturing_) screen_finish(nb, P, k, Dd, Id);
     return true;
   }
@@ -1913,64 +1937,79 @@ class IndexCore {
     return std::max<size_t>(1, std::min(by_cand, by_q));
   }
 
-  // BF16 search of one batch through the candidate matrix: exact coarse
+  // BF16 / FP8 search of one batch through the candidate matrix: exact coarse
   // probes, the list-major work description, every probed row's
   // approximate value on the tensor cores, then per query the R smallest
   // re-ranked exactly.
   void search_batch_cand(int nb, int P, int k, int R, float* Dd, int64_t* Id) {
     probes_.reserve(static_cast<size_t>(nb) * P);
     coarse_and_cut(nb, P);
+    if (fp8_) ensure_fp8();
+    cand_reserve(nb, P, R, fp8_);
+    cand_pipeline(nb, P, k, R, fp8_, false, Dd, Id);
+    if (!capturing_) bf16_err_check();
+  }
+
+  // The batch's buffers, and the error flag cleared.
+  void cand_reserve(int nb, int P, int R, bool fp8) {
     err_dev_.reserve(1);
     HB_CUDA(cudaMemsetAsync(err_dev_.p, 0, sizeof(int), st_));
-    // One 128-row tile per work item: the queries' tile is fetched per row
-    // tile anyway, and small items balance the persistent CTAs.
-    const int cr = 128;
     const size_t nqp = static_cast<size_t>(nb) * P;
     list_cnt_.reserve(nlist_);
     list_cursor_.reserve(nlist_);
     list_qoff_.reserve(nlist_ + 1);
     item_off_.reserve(nlist_ + 1);
     list_q_.reserve(nqp);
-    const size_t wtmp = std::max(build_work_tmp_bytes(nb, P, static_cast<int>(nlist_)), cand_segments_tmp_bytes(nb, P));
-    work_tmp_.reserve(wtmp);
+    work_tmp_.reserve(std::max(build_work_tmp_bytes(nb, P, static_cast<int>(nlist_)), cand_segments_tmp_bytes(nb, P)));
+    seg_.reserve(nqp + 1);
+    pcd_.reserve(nqp);
+    cand_m_.reserve(static_cast<size_t>(nb));
+    qcd8_.reserve(nqp);
+    if (fp8) {
+      qscale8_.reserve(nqp);
+      gq8_.reserve(nqp * static_cast<size_t>(kpad8_));
+    } else {
+      gq_.reserve(nqp * static_cast<size_t>(kpad_));
+    }
+    cand_.reserve(std::max<size_t>(static_cast<size_t>(nb) * cand_row_bound(P), 1));
+    cand_rows_.reserve(static_cast<size_t>(nb) * R);
+    over_list_.reserve(2 * static_cast<size_t>(nb));
+    over_n_.reserve(2);
+  }
+
+  // After the coarse probes (buffers reserved).  `exact`: every row that can
+  // be among the k nearest is re-ranked (at most R), the queries with more
+  // are listed for the exact scan.
+  void cand_pipeline(int nb, int P, int k, int R, bool fp8, bool exact, float* Dd, int64_t* Id) {
+    // One 128-row tile per work item: the queries' tile is fetched per row
+    // tile anyway, and small items balance the persistent CTAs.
+    const int cr = 128;
+    const size_t nqp = static_cast<size_t>(nb) * P;
+    if (exact) HB_CUDA(cudaMemsetAsync(over_n_.p, 0, 2 * sizeof(int), st_));
     {
       Scope sc(this, "build_work");
       launches_ += launch_build_work(probes_.p, nb, P, list_off_.p, static_cast<int>(nlist_), cr, 128, list_cnt_.p,
-                                     list_qoff_.p, list_cursor_.p, list_q_.p, item_off_.p, nullptr, work_tmp_.p, wtmp,
-                                     st_);
+                                     list_qoff_.p, list_cursor_.p, list_q_.p, item_off_.p, nullptr, work_tmp_.p,
+                                     work_tmp_.n, st_);
     }
-    seg_.reserve(nqp + 1);
     {
       Scope sc(this, "cand_segments");
-      launch_cand_segments(probes_.p, nb, P, list_off_.p, seg_.p, work_tmp_.p, wtmp, st_);
+      launch_cand_segments(probes_.p, nb, P, list_off_.p, seg_.p, work_tmp_.p, work_tmp_.n, st_);
     }
-    launches_ += 2;
-    pcd_.reserve(nqp);
-    cand_m_.reserve(static_cast<size_t>(nb));
-    if (fp8_) {
-      ensure_fp8();
-      qscale8_.reserve(nqp);
-      qcd8_.reserve(nqp);
-      gq8_.reserve(nqp * static_cast<size_t>(kpad8_));
+    {
       Scope sc(this, "gather_queries");
-      launch_gather_residual(qpad_.p, static_cast<int>(dpad_), kpad8_, true, list_q_.p, list_qoff_.p,
-                             static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), qscale8_.p, qcd8_.p,
-                             pcd_.p, gq8_.p, st_);
-      make_u8_tensor_map(gqmap_, gq8_.p, nqp, kpad8_);
-      ++launches_;
-    } else {
-      gq_.reserve(nqp * static_cast<size_t>(kpad_));
-      qcd8_.reserve(nqp);
-      Scope sc(this, "gather_queries");
-      launch_gather_residual(qpad_.p, static_cast<int>(dpad_), kpad_, false, list_q_.p, list_qoff_.p,
-                             static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), nullptr, qcd8_.p,
-                             pcd_.p, gq_.p, st_);
-      make_bf16_tensor_map(gqmap_, gq_.p, nqp, kpad_);
-      ++launches_;
+      if (fp8) {
+        launch_gather_residual(qpad_.p, static_cast<int>(dpad_), kpad8_, true, list_q_.p, list_qoff_.p,
+                               static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), qscale8_.p, qcd8_.p,
+                               pcd_.p, gq8_.p, st_);
+        make_u8_tensor_map(gqmap_, gq8_.p, nqp, kpad8_);
+      } else {
+        launch_gather_residual(qpad_.p, static_cast<int>(dpad_), kpad_, false, list_q_.p, list_qoff_.p,
+                               static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), nullptr, qcd8_.p,
+                               pcd_.p, gq_.p, st_);
+        make_bf16_tensor_map(gqmap_, gq_.p, nqp, kpad_);
+      }
     }
-    const int64_t row_bound = cand_row_bound(P);
-    cand_.reserve(std::max<size_t>(static_cast<size_t>(nb) * row_bound, 1));
-    cand_rows_.reserve(static_cast<size_t>(nb) * R);
     CandArgs a{};
     a.list_off = list_off_.p;
     a.nlist = static_cast<int>(nlist_);
@@ -1987,7 +2026,7 @@ class IndexCore {
     a.cand = cand_.p;
     a.err = err_dev_.p;
     a.qcd = qcd8_.p;
-    if (fp8_) {
+    if (fp8) {
       a.fp8 = 1;
       a.kpad = kpad8_;
       a.qscale = qscale8_.p;
@@ -1996,20 +2035,19 @@ class IndexCore {
     }
     {
       Scope sc(this, "cand_scan");
-      launch_cand_scan(gqmap_, fp8_ ? tmap8_ : tmap_, a, num_sms_, st_);
+      launch_cand_scan(gqmap_, fp8 ? tmap8_ : tmap_, a, num_sms_, st_);
     }
-    ++launches_;
     {
       Scope sc(this, "cand_select");
       launch_cand_select(cand_.p, seg_.p, probes_.p, nb, P, R, k, list_off_.p, pcd_.p, rmax_.p, static_cast<int>(dpad_),
-                         a.kpad, fp8_, cand_rows_.p, cand_m_.p, st_);
+                         a.kpad, fp8, cand_rows_.p, cand_m_.p, exact ? over_list_.p : nullptr, over_n_.p, st_);
     }
     {
       Scope sc(this, "cand_exact");
-      launch_cand_exact(cand_rows_.p, cand_m_.p, nb, R, k, codes_.p, qpad_.p, static_cast<int>(dpad_), ids_.p, Dd, Id, st_);
+      launch_cand_exact(cand_rows_.p, cand_m_.p, nb, R, k, codes_.p, qpad_.p, static_cast<int>(dpad_), ids_.p, Dd, Id,
+                        st_);
     }
-    launches_ += 2;
-    if (!capturing_) bf16_err_check();
+    launches_ += 6;  // segment lengths, their sum (a library kernel), gather, scan, selection, re-rank
   }
 
   void bf16_err_check() {
@@ -2390,6 +2428,7 @@ class IndexCore {
   DevBuf<uint32_t> thr_;
   DevBuf<int> ccnt_, cflag_, over_list_, over_n_, rr_m_;
   bool screen_ = false;              // this search's plain FP32 batches go through the bounded scan
+  bool screen_wide_ = false;         // d > 128: through the candidate matrix
   DevBuf<int> scr_cnt_, scr_m_;      // its counts (bf16_stats reports BF16 searches only)
   int last_nb_ = 0;
   DevBuf<uint64_t> cbuf_;

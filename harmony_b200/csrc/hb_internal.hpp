@@ -337,10 +337,13 @@ void make_u8_tensor_map(void* tmap_out, const void* base, size_t rows, int row_b
 // Selection of each query's R best candidates, less those that cannot be among
 // the k best of them (rows: nq x R stored rows, m[q] of them), then their
 // exact re-rank to the k best.  pcd: nq x P ||q - c_l||^2, rmax: per list the
-// largest residual norm (the error bound's operands).
+// largest residual norm (the error bound's operands).  over_list non-null: not
+// the R best but every row that can be among the k nearest, at most R of them;
+// over_list[0 .. over_n[0]) gets the queries with more, or outside the bound's
+// range (m = 0; over_n zeroed by the caller).
 void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* probes, int nq, int P, int R, int k,
                         const int64_t* list_off, const float* pcd, const float* rmax, int dpad, int kpad, bool fp8,
-                        int64_t* rows, int* m, cudaStream_t st);
+                        int64_t* rows, int* m, int* over_list, int* over_n, cudaStream_t st);
 void launch_cand_exact(const int64_t* rows, const int* m, int nq, int R, int k, const float* codes, const float* q,
                        int dpad, const int64_t* ids, float* D, int64_t* I, cudaStream_t st);
 void launch_to_bf16(const float* src, size_t n, int dpad, int kpad, void* dst, cudaStream_t st);

@@ -455,11 +455,18 @@ __device__ __forceinline__ float cand_eps(float cd, float R, int d, int kpad, bo
 // of the R are dropped: the first k candidates' largest upper bound U is at
 // least the k-th smallest distance, so a row with v - eps > U is not among the
 // k.  The others go out in ascending order, m_out[q] of them.
+// EXACT (FP32 searches): instead of the R smallest, every row that the bound
+// allows among the k nearest: with e the largest eps over the query's lists,
+// the k-th smallest distance is at most v_k + e, so all of them have
+// v <= v_k + 2 e.  A query with more than R of those, or outside the bound's
+// range, is listed in over_list for the exact scan.
+template <bool EXACT>
 __global__ void __launch_bounds__(kSelectThreads)
     cand_select_kernel(const float* __restrict__ cand, const int64_t* __restrict__ seg,
                        const int32_t* __restrict__ probes, int P, int R, int k, const int64_t* __restrict__ list_off,
                        const float* __restrict__ pcd, const float* __restrict__ rmax, int dpad, int kpad, int fp8,
-                       int cap, int64_t* __restrict__ out_rows, int* __restrict__ m_out) {
+                       int cap, int64_t* __restrict__ out_rows, int* __restrict__ m_out,
+                       int* __restrict__ over_list, int* __restrict__ over_n) {
   extern __shared__ __align__(16) unsigned char smem_sel[];
   uint64_t* s_cand = reinterpret_cast<uint64_t*>(smem_sel);  // cap keys (a power of two >= 2 * pow2(R))
   __shared__ int s_hist[kBins];
@@ -510,8 +517,20 @@ __global__ void __launch_bounds__(kSelectThreads)
   }
   __syncthreads();
   const int real = s_real;
-  const int need = min(R, real);
+  int need = min(EXACT ? k : R, real);
   int C = 0;
+  const int32_t* prow = probes + static_cast<int64_t>(qi) * P;
+  const float* cdrow = pcd + static_cast<int64_t>(qi) * P;
+  float emax = 0.0f;
+  if (EXACT) {
+    // Every thread needs the largest eps: all warps form it alike.
+    for (int j = lane; j < P; j += 32)
+      if (prow[j] >= 0) {
+        const float e = cand_eps(cdrow[j], rmax[prow[j]], dpad, kpad, fp8 != 0);
+        emax = e < 1e23f ? fmaxf(emax, e) : INFINITY;
+      }
+    for (int off = 16; off > 0; off >>= 1) emax = fmaxf(emax, __shfl_xor_sync(0xffffffffu, emax, off));
+  }
   if (real > 0) {
     const float vmin = ordered_to_float(s_lo), vmax = ordered_to_float(s_hi);
     const float range = vmax - vmin;
@@ -555,8 +574,15 @@ __global__ void __launch_bounds__(kSelectThreads)
     }
     __syncthreads();
     C = s_C;
-    if (C <= cap) {
-      // Pass 3: every key in bins <= s_bin, in any order (the keys are unique).
+    // EXACT: the bound on v, from the upper edge of the k-th value's bin.
+    float lim = vmax;
+    if (EXACT && need == k && scale > 0.0f && s_bin < kBins - 1) {
+      const float edge = vmin + static_cast<float>(s_bin + 1) / scale;
+      lim = __fadd_ru(__fadd_ru(edge, 1e-5f * (fabsf(edge) + fabsf(vmin))), 2.0f * emax);
+    }
+    if (EXACT || C <= cap) {
+      // Pass 3: every key in bins <= s_bin (EXACT: at most lim), in any order
+      // (the keys are unique).
       const int bsel = s_bin;
       for (int base = tid & ~31; base < m; base += kSelUnroll * kSelectThreads) {
         float vv[kSelUnroll];
@@ -568,15 +594,26 @@ __global__ void __launch_bounds__(kSelectThreads)
 #pragma unroll
         for (int u = 0; u < kSelUnroll; ++u) {
           const int i = base + u * kSelectThreads + lane;
-          const bool take = vv[u] < INFINITY && value_bin(vv[u], vmin, scale) <= bsel;
+          const bool take = vv[u] < INFINITY && (EXACT ? vv[u] <= lim : value_bin(vv[u], vmin, scale) <= bsel);
           const unsigned tm = __ballot_sync(0xffffffffu, take);
           int pos0 = 0;
           if (lane == 0 && tm) pos0 = atomicAdd(&s_cnt, __popc(tm));
           pos0 = __shfl_sync(0xffffffffu, pos0, 0);
-          if (take)
-            s_cand[pos0 + __popc(tm & ((1u << lane) - 1u))] =
-                (static_cast<uint64_t>(ordered_bits(vv[u])) << 32) | static_cast<uint32_t>(i);
+          const int at = pos0 + __popc(tm & ((1u << lane) - 1u));
+          if (take && at < cap)
+            s_cand[at] = (static_cast<uint64_t>(ordered_bits(vv[u])) << 32) | static_cast<uint32_t>(i);
         }
+      }
+      if (EXACT) {
+        __syncthreads();
+        C = need = s_cnt;
+      }
+      if (EXACT && (C > R || !(emax < 1e23f))) {
+        if (tid == 0) {
+          over_list[atomicAdd(over_n, 1)] = qi;
+          m_out[qi] = 0;
+        }
+        return;
       }
       const int c2 = pow2_ceil(C < 2 ? 2 : C);
       for (int i = C + tid; i < c2; i += kSelectThreads) s_cand[i] = kEmpty;
@@ -609,8 +646,6 @@ __global__ void __launch_bounds__(kSelectThreads)
     rank = lo;
     return pos - sq[lo];
   };
-  const int32_t* prow = probes + static_cast<int64_t>(qi) * P;
-  const float* cdrow = pcd + static_cast<int64_t>(qi) * P;
   unsigned int ub = 0u;
   for (int i = tid; i < min(k, need); i += kSelectThreads) {
     int j;
@@ -816,16 +851,21 @@ void make_u8_tensor_map(void* tmap_out, const void* base, size_t rows, int row_b
 
 void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* probes, int nq, int P, int R, int k,
                         const int64_t* list_off, const float* pcd, const float* rmax, int dpad, int kpad, bool fp8,
-                        int64_t* rows, int* m_out, cudaStream_t st) {
+                        int64_t* rows, int* m_out, int* over_list, int* over_n, cudaStream_t st) {
   if (nq <= 0) return;
   HB_CHECK(R >= 1 && R <= kCandMaxR && k >= 1 && k <= R, HB_ERR_INVALID, "candidate count out of range");
-  // Compaction buffer: at least 2048 keys and four times the R kept.
-  const int cap = std::max(2048, 4 * pow2_ceil(R < 2 ? 2 : R));
+  // Compaction buffer: at least 2048 keys and four times the R kept; an exact
+  // selection keeps at most R.
+  const bool exact = over_list != nullptr;
+  const int cap = exact ? pow2_ceil(R < 2 ? 2 : R) : std::max(2048, 4 * pow2_ceil(R < 2 ? 2 : R));
   const size_t smem_sel = static_cast<size_t>(cap) * sizeof(uint64_t);
-  HB_CUDA(cudaFuncSetAttribute(cand_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem_sel)));
-  cand_select_kernel<<<nq, kSelectThreads, smem_sel, st>>>(cand, seg, probes, P, R, k, list_off, pcd, rmax, dpad, kpad,
-                                                           fp8 ? 1 : 0, cap, rows, m_out);
+  auto go = [&](auto kernel) {
+    HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_sel)));
+    kernel<<<nq, kSelectThreads, smem_sel, st>>>(cand, seg, probes, P, R, k, list_off, pcd, rmax, dpad, kpad,
+                                                 fp8 ? 1 : 0, cap, rows, m_out, over_list, over_n);
+  };
+  if (exact) go(cand_select_kernel<true>);
+  else go(cand_select_kernel<false>);
   HB_CUDA(cudaGetLastError());
 }
 

@@ -55,7 +55,7 @@ enum {
 };
 
 /* Arithmetic of the list scan. FP32 reproduces the reference's distances
- * bit for bit (plain searches with d <= 128 and k <= 256 let the bounded
+ * bit for bit (plain searches with k <= 256 let the bounded
  * tensor-core scan pick the rows whose FP32 distances are formed, from a
  * batch size on; the result is the full FP32 scan's); BF16 / FP8 scan on
  * tensor cores and re-rank a widened candidate set in exact FP32.  BF16 with d <= 128 and k <= 256 re-ranks every

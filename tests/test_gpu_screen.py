@@ -32,7 +32,7 @@ def screened(ix, q, k, mode=SearchMode.ORIGINAL, graph=False, npq=None):
     names = set(ix.profile_read())
     ix.profile(False)
     sp.use_graph, sp.nprobe_per_query, sp.max_nprobe = False, None, 0
-    assert graph or "scan_bf16" in names, names  # the route under test ran
+    assert graph or names & {"scan_bf16", "cand_scan"}, names  # the route under test ran
     return D, I
 
 
@@ -67,10 +67,26 @@ def test_equals_exact_scan(d, k):
     assert ix.bf16_stats()["queries"] == 0 and ix.bf16_fallbacks() == 0  # those report BF16 searches
 
 
+@pytest.mark.parametrize("d,k", [(129, 1), (256, 20), (500, 100), (1000, 30)])
+def test_wide_equals_exact_scan(d, k):
+    """d > 128: the candidate matrix, every row the bound allows re-ranked."""
+    nq = 40
+    base, q = datasets.config3(seed=d + k, nb=NB, nq=nq, d=d, ncomp=60)
+    ix = build(d, base)
+    ref = exact(ix, q, k)
+    same(screened(ix, q, k), ref)
+    for _ in range(2):
+        same(screened(ix, q, k, graph=True), ref)
+    npq = (np.arange(nq) % (P + 1)).astype(np.int32)
+    D, I = screened(ix, q, k, npq=npq)
+    same((D[npq == P], I[npq == P]), (ref[0][npq == P], ref[1][npq == P]))
+    assert (I[npq == 0] == -1).all()
+
+
+@pytest.mark.parametrize("d", [64, 200])
 @pytest.mark.parametrize("kind", ["nonfinite", "huge", "tiny", "ties", "far", "outlier"])
-def test_values_outside_the_bound(kind):
+def test_values_outside_the_bound(kind, d):
     rng = np.random.default_rng(3)
-    d = 64
     cent = (rng.standard_normal((NLIST, d)) * 3).astype(np.float32)
     base = (cent[rng.integers(0, NLIST, NB)] + rng.standard_normal((NB, d))).astype(np.float32)
     q = base[::311][:120] + np.float32(0.01)
