@@ -127,7 +127,10 @@ class IndexCore {
     HB_CUDA(cudaSetDevice(device));
     HB_CUDA(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device));
     HB_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
-    HB_CUDA(cudaMallocHost(&err_host_, sizeof(int)));
+    HB_CUDA(cudaMallocHost(&pin_, kPinnedBytes));
+    err_host_ = reinterpret_cast<int*>(pin_);
+    status_.reserve(kStatusWords);
+    HB_CUDA(cudaMemsetAsync(status_.p, 0, kStatusWords * sizeof(int), st_));
     reshape(d, nlist);
   }
   ~IndexCore() {
@@ -137,7 +140,7 @@ class IndexCore {
       cudaStreamSynchronize(st_);
       cudaStreamDestroy(st_);
     }
-    if (err_host_) cudaFreeHost(err_host_);
+    if (pin_) cudaFreeHost(pin_);
   }
 
   // Index ctor state: zero centroids, empty lists (src/Index.cpp:24-43).
@@ -152,6 +155,7 @@ class IndexCore {
     list_off_.reserve(nlist_ + 1);
     HB_CUDA(cudaMemsetAsync(list_off_.p, 0, (nlist_ + 1) * sizeof(int64_t), st_));
     host_off_.assign(nlist_ + 1, 0);
+    sizes_desc_.clear();
     ntotal_ = 0;
     coarse_ready_ = false;
     coarse_last_nq_ = 0;
@@ -554,7 +558,7 @@ class IndexCore {
                             st_));
     HB_CUDA(cudaStreamSynchronize(st_));
     ntotal_ = n;
-    plan_rows_ = 0;
+    sizes_desc_.clear();
     build_bf16();
     drop_graphs();
   }
@@ -648,7 +652,7 @@ class IndexCore {
     {
       Scope sc(this, "coarse_tc");
       launch_coarse_tc(ctmap_, qpad, nq, static_cast<int>(dpad_), ckpad_, cnorm_.p, static_cast<int>(nlist_), dmat_.p,
-                       qsplit_.p, qsnorm_.p, cmins_.p, cerr_dev_.p, num_sms_, st_);
+                       qsplit_.p, qsnorm_.p, cmins_.p, (status_.p + kStCoarseErr), num_sms_, st_);
     }
     {
       Scope sc(this, "coarse_select");
@@ -701,7 +705,7 @@ class IndexCore {
     {
       Scope sc(this, "coarse_tc");
       launch_coarse_tc(ctmap_, qpad, nq, static_cast<int>(dpad_), ckpad_, cnorm_.p, nl, dmat_.p, qsplit_.p, qsnorm_.p,
-                       cmins_.p, cerr_dev_.p, num_sms_, st_);
+                       cmins_.p, (status_.p + kStCoarseErr), num_sms_, st_);
     }
     {
       Scope sc(this, "coarse_select");
@@ -753,8 +757,6 @@ class IndexCore {
     launch_row_norms(cent_.p, nlist_, static_cast<int>(d_), static_cast<int>(dpad_), cnorm_.p, st_);
     cmaxnorm_.reserve(1);
     launch_max_norm(cnorm_.p, nlist_, cmaxnorm_.p, st_);
-    cerr_dev_.reserve(1);
-    HB_CUDA(cudaMemsetAsync(cerr_dev_.p, 0, sizeof(int), st_));
     launches_ += 3;
     coarse_ready_ = true;
   }
@@ -762,14 +764,15 @@ class IndexCore {
   // Raises when a bounded wait of the tensor-core quantizer gave up since the
   // last check (the flag is sticky until read here).
   void coarse_err_check() {
-    if (!cerr_dev_.p) return;
-    HB_CUDA(cudaMemcpyAsync(err_host_, cerr_dev_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    HB_CUDA(cudaMemcpyAsync(err_host_, status_.p, kStatusWords * sizeof(int), cudaMemcpyDeviceToHost, st_));
     HB_CUDA(cudaStreamSynchronize(st_));
-    if (*err_host_ != 0) {
-      const int code = *err_host_;
-      HB_CUDA(cudaMemsetAsync(cerr_dev_.p, 0, sizeof(int), st_));
-      throw Error(HB_ERR_CUDA, "tensor-core coarse quantizer gave up waiting (code " + std::to_string(code) + ")");
-    }
+    coarse_err_raise();
+  }
+  void coarse_err_raise() {
+    const int code = err_host_[kStCoarseErr];
+    if (code == 0) return;
+    HB_CUDA(cudaMemsetAsync(status_.p + kStCoarseErr, 0, sizeof(int), st_));
+    throw Error(HB_ERR_CUDA, "tensor-core coarse quantizer gave up waiting (code " + std::to_string(code) + ")");
   }
 
   void set_wait_budget(long long cycles) { wait_budget_ = cycles > 0 ? cycles : kDefaultWaitBudget; }
@@ -951,24 +954,18 @@ class IndexCore {
     for (size_t b0 = 0; b0 < nq; b0 += bs) {
       const int nb = static_cast<int>(std::min(bs, nq - b0));
       cut_b0_ = b0;
-      float* Dd = dev_out ? D + b0 * k : nullptr;
-      int64_t* Id = dev_out ? I + b0 * k : nullptr;
-      if (!dev_out) {
-        dout_.reserve(static_cast<size_t>(nb) * k);
-        iout_.reserve(static_cast<size_t>(nb) * k);
-        Dd = dout_.p;
-        Id = iout_.p;
-      }
+      float* Dd = D + b0 * k;
+      int64_t* Id = I + b0 * k;
+      if (!dev_out) out_rows(nb, static_cast<int>(k), Dd, Id);
       // Queries.
-      qpad_.reserve(static_cast<size_t>(nb) * dpad_);
       const float* qsrc = q + b0 * d_;
-      if (!dev_in) {
-        qtmp_.reserve(static_cast<size_t>(nb) * d_);
-        HB_CUDA(cudaMemcpyAsync(qtmp_.p, qsrc, static_cast<size_t>(nb) * d_ * sizeof(float), cudaMemcpyHostToDevice,
-                                st_));
-        qsrc = qtmp_.p;
+      if (dev_in && d_ == dpad_ && reinterpret_cast<uintptr_t>(qsrc) % 16 == 0) {
+        qp_ = qsrc;  // already padded rows, read only during this call
+      } else {
+        qpad_.reserve(static_cast<size_t>(nb) * dpad_);
+        stage_queries(qsrc, nb, dev_in);
       }
-      pad_rows(qsrc, nullptr, nb, qpad_.p);
+      begin_batch();
       if (P == 0 || ntotal_ == 0) {
         launch_fill_results(Dd, Id, static_cast<size_t>(nb) * k, st_);
         ++launches_;
@@ -979,15 +976,88 @@ class IndexCore {
           search_batch(nb, static_cast<int>(P), static_cast<int>(k), mode, p.pruning != 0, need_tops, warm_lists,
                        warm_size, W, B, qblock, Dd, Id);
       }
-      if (!dev_out) {
-        HB_CUDA(cudaMemcpyAsync(D + b0 * k, Dd, static_cast<size_t>(nb) * k * sizeof(float), cudaMemcpyDeviceToHost,
-                                st_));
-        HB_CUDA(cudaMemcpyAsync(I + b0 * k, Id, static_cast<size_t>(nb) * k * sizeof(int64_t),
-                                cudaMemcpyDeviceToHost, st_));
-      }
+      finish_batch(nb, static_cast<int>(P), static_cast<int>(k), bf16, Dd, Id, D + b0 * k, I + b0 * k,
+                   !dev_out && !is_device_ptr(D) && !is_device_ptr(I));
     }
+  }
+
+  // Result rows of a batch on the device: ids, then distances, in one buffer.
+  void out_rows(int nb, int k, float*& Dd, int64_t*& Id) {
+    const size_t n = static_cast<size_t>(nb) * k;
+    out_.reserve(n * (sizeof(int64_t) + sizeof(float)));
+    Id = reinterpret_cast<int64_t*>(out_.p);
+    Dd = reinterpret_cast<float*>(out_.p + n * sizeof(int64_t));
+  }
+
+  // Queries of a batch to padded device rows (qpad_).
+  void stage_queries(const float* q, int nb, bool dev) {
+    const size_t bytes = static_cast<size_t>(nb) * d_ * sizeof(float);
+    const float* src = q;
+    if (!dev) {
+      if (bytes <= kPinnedQueries) {
+        unsigned char* h = pin_ + 256 + kPinnedResults;
+        std::memcpy(h, q, bytes);
+        src = reinterpret_cast<const float*>(h);
+      }
+      float* dst = qpad_.p;
+      if (d_ != dpad_) dst = qtmp_.reserve(static_cast<size_t>(nb) * d_);
+      HB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st_));
+      src = dst;
+    }
+    if (src != qpad_.p) pad_rows(src, nullptr, nb, qpad_.p);
+    qp_ = qpad_.p;
+  }
+
+  void begin_batch() {
+    HB_CUDA(cudaMemsetAsync(status_.p, 0, kStPerBatch * sizeof(int), st_));
+  }
+
+  // Ends a batch: its results to the caller's arrays, its status words back,
+  // one wait for both; then what they ask for (queries to search again
+  // exactly, errors).
+  void finish_batch(int nb, int P, int k, bool bf16, float* Dd, int64_t* Id, float* D, int64_t* I, bool host_out) {
+    const size_t n = static_cast<size_t>(nb) * k;
+    const size_t bytes = n * (sizeof(int64_t) + sizeof(float));
+    const bool pinned = host_out && bytes <= kPinnedResults;
+    unsigned char* h = pin_ + 256;
+    auto copy_out = [&]() {
+      if (Dd == D) return;
+      if (pinned) {
+        HB_CUDA(cudaMemcpyAsync(h, Id, bytes, cudaMemcpyDeviceToHost, st_));
+        return;
+      }
+      HB_CUDA(cudaMemcpyAsync(D, Dd, n * sizeof(float), host_out ? cudaMemcpyDeviceToHost : cudaMemcpyDefault, st_));
+      HB_CUDA(cudaMemcpyAsync(I, Id, n * sizeof(int64_t), host_out ? cudaMemcpyDeviceToHost : cudaMemcpyDefault, st_));
+    };
+    if (!host_out || pinned) copy_out();
+    HB_CUDA(cudaMemcpyAsync(err_host_, status_.p, kStatusWords * sizeof(int), cudaMemcpyDeviceToHost, st_));
     HB_CUDA(cudaStreamSynchronize(st_));
-    coarse_err_check();
+    const int err = err_host_[kStErr], over = err_host_[kStOver];
+    coarse_err_raise();
+    const bool searched = P > 0 && ntotal_ > 0;
+    const bool bounded = searched && ((bf16 && !cand_path_) || screen_);
+    if (bf16 && err != 0)
+      throw Error(HB_ERR_CUDA, "tensor-core scan gave up waiting (code " + std::to_string(err) + ")");
+    if (bf16 && bounded) last_overflow_ = over;
+    bool again = host_out && !pinned;
+    if (bounded && err != 0) {
+      // A wait of a screened FP32 batch gave up: the exact scan for all of it.
+      begin_batch();
+      scan_exact_from(nb, P, k, qp_, probes_.p, SCAN_PLAIN, false, nullptr, 1, 1, 0, Dd, Id);
+      again = true;
+    } else if (bounded && over > 0) {
+      begin_batch();
+      fix_overflow(nb, P, k, over, Dd, Id);
+      again = true;
+    }
+    if (again) {
+      copy_out();
+      HB_CUDA(cudaStreamSynchronize(st_));
+    }
+    if (pinned && Dd != D) {
+      std::memcpy(I, h, n * sizeof(int64_t));
+      std::memcpy(D, h + n * sizeof(int64_t), n * sizeof(float));
+    }
   }
 
   // ---- one batch as a CUDA graph --------------------------------------------
@@ -1011,25 +1081,39 @@ class IndexCore {
     graphs_.clear();
   }
 
-  void run_batch_pipeline(int nb, int k, int P, int R, bool bf16) {
-    pad_rows(qtmp_.p, nullptr, nb, qpad_.p);
+  void run_batch_pipeline(int nb, int k, int P, int R, bool bf16, float* Dd, int64_t* Id) {
+    if (d_ != dpad_) pad_rows(qtmp_.p, nullptr, nb, qpad_.p);
+    begin_batch();
     if (P == 0 || ntotal_ == 0) {
-      launch_fill_results(dout_.p, iout_.p, static_cast<size_t>(nb) * k, st_);
+      launch_fill_results(Dd, Id, static_cast<size_t>(nb) * k, st_);
       ++launches_;
     } else if (bf16) {
-      search_batch_bf16(nb, P, k, R, dout_.p, iout_.p);
+      search_batch_bf16(nb, P, k, R, Dd, Id);
     } else {
-      search_batch(nb, P, k, SCAN_PLAIN, false, false, 0, k, 1, 1, 0, dout_.p, iout_.p);
+      search_batch(nb, P, k, SCAN_PLAIN, false, false, 0, k, 1, 1, 0, Dd, Id);
     }
   }
 
   void search_graph(int nb, const float* q, int k, int P, int R, bool bf16, const hb_search_params& p, float* D,
                     int64_t* I) {
-    qtmp_.reserve(static_cast<size_t>(nb) * d_);
     qpad_.reserve(static_cast<size_t>(nb) * dpad_);
-    dout_.reserve(static_cast<size_t>(nb) * k);
-    iout_.reserve(static_cast<size_t>(nb) * k);
-    HB_CUDA(cudaMemcpyAsync(qtmp_.p, q, static_cast<size_t>(nb) * d_ * sizeof(float), cudaMemcpyDefault, st_));
+    qp_ = qpad_.p;
+    float* Dd = nullptr;
+    int64_t* Id = nullptr;
+    out_rows(nb, k, Dd, Id);
+    // The queries into the graph's fixed buffer (the padded rows themselves
+    // where nothing is padded).
+    {
+      const size_t bytes = static_cast<size_t>(nb) * d_ * sizeof(float);
+      float* dst = d_ == dpad_ ? qpad_.p : qtmp_.reserve(static_cast<size_t>(nb) * d_);
+      const float* src = q;
+      if (bytes <= kPinnedQueries && !is_device_ptr(q)) {
+        unsigned char* h = pin_ + 256 + kPinnedResults;
+        std::memcpy(h, q, bytes);
+        src = reinterpret_cast<const float*>(h);
+      }
+      HB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, st_));
+    }
     if (cut_mode_ == 2) {
       npqin_.reserve(static_cast<size_t>(nb));
       HB_CUDA(cudaMemcpyAsync(npqin_.p, cut_src_, static_cast<size_t>(nb) * sizeof(int32_t), cudaMemcpyDefault, st_));
@@ -1048,13 +1132,12 @@ class IndexCore {
       it = graphs_.end();
     }
     if (it != graphs_.end()) {
-      if (bf16 || screen_) HB_CUDA(cudaMemsetAsync(err_dev_.p, 0, sizeof(int), st_));
       HB_CUDA(cudaGraphLaunch(it->second.exec, st_));
       launches_ += it->second.launches;
     } else {
       // An ordinary run sizes every buffer (and gives this call's results),
       // then the same sequence is captured.
-      run_batch_pipeline(nb, k, P, R, bf16);
+      run_batch_pipeline(nb, k, P, R, bf16, Dd, Id);
       HB_CUDA(cudaStreamSynchronize(st_));
       const uint64_t gen = devbuf_generation().load();
       const uint64_t l0 = launches_;
@@ -1062,7 +1145,7 @@ class IndexCore {
       capturing_ = true;
       cudaGraph_t graph = nullptr;
       try {
-        run_batch_pipeline(nb, k, P, R, bf16);
+        run_batch_pipeline(nb, k, P, R, bf16, Dd, Id);
       } catch (...) {
         capturing_ = false;
         cudaStreamEndCapture(st_, &graph);
@@ -1086,17 +1169,7 @@ class IndexCore {
       cudaGraphDestroy(graph);
       launches_ = l0;
     }
-    if (bf16 && !cand_path_) {
-      bf16_err_check();
-      last_overflow_ = fix_overflow(nb, P, k, dout_.p, iout_.p);
-    } else if (screen_) {
-      screen_finish(nb, P, k, dout_.p, iout_.p);
-    }
-    HB_CUDA(cudaMemcpyAsync(D, dout_.p, static_cast<size_t>(nb) * k * sizeof(float), cudaMemcpyDefault, st_));
-    HB_CUDA(cudaMemcpyAsync(I, iout_.p, static_cast<size_t>(nb) * k * sizeof(int64_t), cudaMemcpyDefault, st_));
-    HB_CUDA(cudaStreamSynchronize(st_));
-    if (bf16) bf16_err_check();
-    coarse_err_check();
+    finish_batch(nb, P, k, bf16, Dd, Id, D, I, !is_device_ptr(D) && !is_device_ptr(I));
   }
 
   void probe_lists(size_t nq, const float* q, size_t P, int64_t* probes, float* cdist) {
@@ -1269,7 +1342,7 @@ class IndexCore {
     HB_CUDA(cudaStreamSynchronize(st_));
     ntotal_ = nt;
     trained_ = true;
-    plan_rows_ = 0;
+    sizes_desc_.clear();
     build_bf16();
     drop_graphs();
   }
@@ -1378,9 +1451,8 @@ class IndexCore {
     HB_CUDA(cudaSetDevice(device_));
     DevBuf<long long> w;
     w.reserve(1);
-    err_dev_.reserve(1);
-    HB_CUDA(cudaMemsetAsync(err_dev_.p, 0, sizeof(int), st_));
-    launch_wait_selftest(budget, 99, err_dev_.p, w.p, st_);
+    HB_CUDA(cudaMemsetAsync(status_.p + kStErr, 0, sizeof(int), st_));
+    launch_wait_selftest(budget, 99, (status_.p + kStErr), w.p, st_);
     ++launches_;
     long long wh = 0;
     HB_CUDA(cudaMemcpyAsync(&wh, w.p, sizeof(long long), cudaMemcpyDeviceToHost, st_));
@@ -1429,7 +1501,7 @@ class IndexCore {
                             st_));
     HB_CUDA(cudaStreamSynchronize(st_));
     ntotal_ = kept;
-    plan_rows_ = 0;
+    sizes_desc_.clear();
     build_bf16();
     drop_graphs();
   }
@@ -1475,13 +1547,18 @@ class IndexCore {
   // Upper bound of the output slots of a batch: nq x (sum of the P largest
   // per-list chunk counts).
   size_t max_slots(int nq, int P, int cr) {
-    std::vector<int64_t> ch(nlist_);
-    for (size_t l = 0; l < nlist_; ++l) ch[l] = (host_off_[l + 1] - host_off_[l] + cr - 1) / cr;
-    const size_t take = std::min<size_t>(P, nlist_);
-    std::partial_sort(ch.begin(), ch.begin() + take, ch.end(), std::greater<int64_t>());
     int64_t s = 0;
-    for (size_t i = 0; i < take; ++i) s += ch[i];
+    for (size_t i = 0; i < std::min<size_t>(P, nlist_); ++i) s += (sizes_desc()[i] + cr - 1) / cr;
     return static_cast<size_t>(nq) * static_cast<size_t>(std::max<int64_t>(s, 1));
+  }
+  // List lengths, longest first (formed once per set of lists).
+  const std::vector<int64_t>& sizes_desc() {
+    if (sizes_desc_.empty()) {
+      sizes_desc_.resize(nlist_);
+      for (size_t l = 0; l < nlist_; ++l) sizes_desc_[l] = host_off_[l + 1] - host_off_[l];
+      std::sort(sizes_desc_.begin(), sizes_desc_.end(), std::greater<int64_t>());
+    }
+    return sizes_desc_;
   }
 
   void search_batch(int nb, int P, int k, int mode, bool cut, bool need_tops, int warm_lists, int warm_size, int W,
@@ -1499,13 +1576,13 @@ class IndexCore {
                                 cudaMemcpyDefault, st_));
       } else {
         Scope sc(this, "warmup_tops");
-        launch_warmup_tops(qpad_.p, nb, probes_.p, P, codes_.p, list_off_.p, static_cast<int>(dpad_), k, warm_lists,
+        launch_warmup_tops(qp_, nb, probes_.p, P, codes_.p, list_off_.p, static_cast<int>(dpad_), k, warm_lists,
                            warm_size, tops_.p, st_);
         ++launches_;
       }
     }
     if (screen_ && screen_batch(nb, P, k, Dd, Id)) return;
-    scan_exact_from(nb, P, k, qpad_.p, probes_.p, mode, cut, need_tops ? tops_.p : nullptr, W, B, qblock, Dd, Id);
+    scan_exact_from(nb, P, k, qp_, probes_.p, mode, cut, need_tops ? tops_.p : nullptr, W, B, qblock, Dd, Id);
   }
 
   // ---- FP32 searches on the bounded scan ------------------------------------
@@ -1555,32 +1632,17 @@ class IndexCore {
       cand_pipeline(nb, P, k, kScreenWideRows, false, true, Dd, Id);
     else
       filter_pipeline(nb, P, k, cap, cr, scan_bf16_stages(kpad_), scr_cnt_.p, scr_m_.p, kDefaultWaitBudget, Dd, Id);
-    if (!capturing_) screen_finish(nb, P, k, Dd, Id);
     return true;
   }
 
-  // After a screened batch: queries left to the exact scan, or all of them
-  // when a wait gave up.
-  void screen_finish(int nb, int P, int k, float* Dd, int64_t* Id) {
-    HB_CUDA(cudaMemcpyAsync(err_host_, err_dev_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
-    HB_CUDA(cudaStreamSynchronize(st_));
-    if (*err_host_ != 0)
-      scan_exact_from(nb, P, k, qpad_.p, probes_.p, SCAN_PLAIN, false, nullptr, 1, 1, 0, Dd, Id);
-    else
-      fix_overflow(nb, P, k, Dd, Id);
-  }
-
   // Per-batch buffers of the bounded scan (counts and re-ranked rows in the
-  // caller's own), and its error flag cleared.
+  // caller's own).
   void bounded_reserve(int nb, int cap, DevBuf<int>& cnt, DevBuf<int>& m) {
-    err_dev_.reserve(1);
-    HB_CUDA(cudaMemsetAsync(err_dev_.p, 0, sizeof(int), st_));
     thr_.reserve(nb);
     cnt.reserve(nb);
     m.reserve(nb);
     cflag_.reserve(nb);
     over_list_.reserve(2 * static_cast<size_t>(nb));
-    over_n_.reserve(2);
     cbuf_.reserve(static_cast<size_t>(nb) * cap);
     cbuf_ub_.reserve(static_cast<size_t>(nb) * cap);
   }
@@ -1608,8 +1670,6 @@ class IndexCore {
                                      wtmp, st_);
     }
     part_.reserve(max_slots(nb, P, cr) * static_cast<size_t>(k));
-    counter_.reserve(1);
-    HB_CUDA(cudaMemsetAsync(counter_.p, 0, sizeof(unsigned int), st_));
     ScanArgs a{};
     a.codes = codes_.p;
     a.list_off = list_off_.p;
@@ -1627,7 +1687,7 @@ class IndexCore {
     a.slot_base = slot_base_.p;
     a.chunk_rows = cr;
     a.qgroup = qg;
-    a.work_counter = counter_.p;
+    a.work_counter = counter(0);
     a.part = part_.p;
     a.mode = mode;
     a.tops = tops;
@@ -1679,10 +1739,6 @@ class IndexCore {
     const int cr = it != tune_.end() ? it->second.chunk_rows : cr0;
     const int stages = it != tune_.end() ? it->second.stages : s0;
     filter_pipeline(nb, P, k, cap, cr, stages, ccnt_.p, rr_m_.p, wait_budget_, Dd, Id);
-    if (!capturing_) {
-      bf16_err_check();
-      last_overflow_ = fix_overflow(nb, P, k, Dd, Id);
-    }
   }
 
   // The bounded scan of one batch after the coarse probes: per-query prep,
@@ -1693,7 +1749,6 @@ class IndexCore {
   // (cr, stages) gives the same result.
   void filter_pipeline(int nb, int P, int k, int cap, int cr, int stages, int* cnt, int* rr_m, long long budget,
                        float* Dd, int64_t* Id) {
-    HB_CUDA(cudaMemsetAsync(over_n_.p, 0, 2 * sizeof(int), st_));
     {
       Scope sc(this, "query_prep");
       launch_query_prep(nb, thr_.p, cnt, st_);
@@ -1725,17 +1780,15 @@ class IndexCore {
     }
     {
       Scope sc(this, "seed");
-      launch_seed_bound(qpad_.p, static_cast<int>(d_), static_cast<int>(dpad_), cent_.p, nb, kpad_, codes_bf16_.p,
+      launch_seed_bound(qp_, static_cast<int>(d_), static_cast<int>(dpad_), cent_.p, nb, kpad_, codes_bf16_.p,
                         list_off_.p, static_cast<int>(nlist_), list_qoff_.p, list_q_.p, rnorm_.p, rmax_.p,
                         std::max(seed_rows_, k), k, thr_.p, st_, probes_a, P_a);
     }
-    counter_.reserve(1);
-    HB_CUDA(cudaMemsetAsync(counter_.p, 0, sizeof(unsigned int), st_));
     TcArgs a{};
     a.list_off = list_off_.p;
     a.nlist = static_cast<int>(nlist_);
     a.kpad = kpad_;
-    a.q = qpad_.p;
+    a.q = qp_;
     a.dpad = static_cast<int>(dpad_);
     a.cent = cent_.p;
     a.tile_norm = tile_norm_.p;
@@ -1745,7 +1798,7 @@ class IndexCore {
     a.list_q = list_q_.p;
     a.item_off = item_off_.p;
     a.chunk_rows = cr_a;
-    a.work_counter = counter_.p;
+    a.work_counter = counter(0);
     a.thr = thr_.p;
     a.rmax = rmax_.p;
     a.cand = cbuf_.p;
@@ -1753,7 +1806,7 @@ class IndexCore {
     a.cand_cnt = cnt;
     a.cap = cap;
     a.k = k;
-    a.err = err_dev_.p;
+    a.err = (status_.p + kStErr);
     a.stages = stages;
     a.wait_budget = budget;
     {
@@ -1772,7 +1825,7 @@ class IndexCore {
                                        list_cnt_.p, list_qoff_.p, list_cursor_.p, list_q_.p, item_off_.p, nullptr,
                                        work_tmp_.p, wtmp, st_);
       }
-      HB_CUDA(cudaMemsetAsync(counter_.p, 0, sizeof(unsigned int), st_));
+      a.work_counter = counter(1);
       a.chunk_rows = cr;
       {
         Scope sc(this, "scan_bf16");
@@ -1782,8 +1835,8 @@ class IndexCore {
     }
     {
       Scope sc(this, "rerank");
-      launch_rerank_bf16(cbuf_.p, cbuf_ub_.p, cnt, cap, nb, k, codes_.p, qpad_.p, static_cast<int>(dpad_), ids_.p, Dd,
-                         Id, cflag_.p, over_list_.p, over_n_.p, rr_m, num_sms_, st_);
+      launch_rerank_bf16(cbuf_.p, cbuf_ub_.p, cnt, cap, nb, k, codes_.p, qp_, static_cast<int>(dpad_), ids_.p, Dd,
+                         Id, cflag_.p, over_list_.p, (status_.p + kStOver), rr_m, num_sms_, st_);
     }
     // query prep, seed, scan, warp re-rank, and the three flat re-rank
     // kernels when the buffers can hold more than a warp's candidates.
@@ -1827,6 +1880,7 @@ class IndexCore {
       for (int c : crs) {
         float ms = 1e30f;
         for (int rep = 0; rep < 2; ++rep) {
+          begin_batch();
           HB_CUDA(cudaEventRecord(e0, st_));
           filter_pipeline(nb, P, k, cap, c, S, ccnt_.p, rr_m_.p, wait_budget_, Dd, Id);
           HB_CUDA(cudaEventRecord(e1, st_));
@@ -1846,6 +1900,7 @@ class IndexCore {
     ev_pool_.push_back(e0);
     ev_pool_.push_back(e1);
     bf16_err_check();
+    begin_batch();
     tune_[key] = best;
   }
 
@@ -1888,13 +1943,7 @@ class IndexCore {
   // Queries whose candidate buffer overflowed (listed by the re-rank, left
   // unwritten) are searched with the exact scan over their own probe rows,
   // and their result rows are written into Dd / Id.
-  // Returns their number.
-  int fix_overflow(int nb, int P, int k, float* Dd, int64_t* Id) {
-    int n_over = 0;
-    HB_CUDA(cudaMemcpyAsync(err_host_, over_n_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
-    HB_CUDA(cudaStreamSynchronize(st_));
-    n_over = *err_host_;
-    if (n_over <= 0) return n_over;
+  void fix_overflow(int nb, int P, int k, int n_over, float* Dd, int64_t* Id) {
     HB_CHECK(n_over <= nb, HB_ERR_CUDA, "overflow list longer than the batch");
     Scope sc(this, "overflow_exact");
     const int dp = static_cast<int>(dpad_);
@@ -1902,7 +1951,7 @@ class IndexCore {
     op_.reserve(static_cast<size_t>(n_over) * P);
     od_.reserve(static_cast<size_t>(n_over) * k);
     oi_.reserve(static_cast<size_t>(n_over) * k);
-    launch_gather_words(reinterpret_cast<const uint32_t*>(qpad_.p), over_list_.p, n_over, dp,
+    launch_gather_words(reinterpret_cast<const uint32_t*>(qp_), over_list_.p, n_over, dp,
                         reinterpret_cast<uint32_t*>(oq_.p), st_);
     launch_gather_words(reinterpret_cast<const uint32_t*>(probes_.p), over_list_.p, n_over, P,
                         reinterpret_cast<uint32_t*>(op_.p), st_);
@@ -1912,18 +1961,14 @@ class IndexCore {
     launch_scatter_words(reinterpret_cast<const uint32_t*>(oi_.p), over_list_.p, n_over, 2 * k,
                          reinterpret_cast<uint32_t*>(Id), st_);
     launches_ += 4;
-    return n_over;
   }
 
   // Longest candidate row a query can have at nprobe P: the P largest lists,
   // each rounded up to 4 entries.
   int64_t cand_row_bound(int P) {
-    std::vector<int64_t> n(nlist_);
-    for (size_t l = 0; l < nlist_; ++l) n[l] = (host_off_[l + 1] - host_off_[l] + 3) & ~int64_t(3);
-    const size_t take = std::min<size_t>(static_cast<size_t>(P), nlist_);
-    std::partial_sort(n.begin(), n.begin() + take, n.end(), std::greater<int64_t>());
     int64_t s = 0;
-    for (size_t i = 0; i < take; ++i) s += n[i];
+    for (size_t i = 0; i < std::min<size_t>(static_cast<size_t>(P), nlist_); ++i)
+      s += (sizes_desc()[i] + 3) & ~int64_t(3);
     return s;
   }
 
@@ -1947,13 +1992,10 @@ class IndexCore {
     if (fp8_) ensure_fp8();
     cand_reserve(nb, P, R, fp8_);
     cand_pipeline(nb, P, k, R, fp8_, false, Dd, Id);
-    if (!capturing_) bf16_err_check();
   }
 
-  // The batch's buffers, and the error flag cleared.
+  // The batch's buffers.
   void cand_reserve(int nb, int P, int R, bool fp8) {
-    err_dev_.reserve(1);
-    HB_CUDA(cudaMemsetAsync(err_dev_.p, 0, sizeof(int), st_));
     const size_t nqp = static_cast<size_t>(nb) * P;
     list_cnt_.reserve(nlist_);
     list_cursor_.reserve(nlist_);
@@ -1974,7 +2016,6 @@ class IndexCore {
     cand_.reserve(std::max<size_t>(static_cast<size_t>(nb) * cand_row_bound(P), 1));
     cand_rows_.reserve(static_cast<size_t>(nb) * R);
     over_list_.reserve(2 * static_cast<size_t>(nb));
-    over_n_.reserve(2);
   }
 
   // After the coarse probes (buffers reserved).  `exact`: every row that can
@@ -1985,7 +2026,6 @@ class IndexCore {
     // tile anyway, and small items balance the persistent CTAs.
     const int cr = 128;
     const size_t nqp = static_cast<size_t>(nb) * P;
-    if (exact) HB_CUDA(cudaMemsetAsync(over_n_.p, 0, 2 * sizeof(int), st_));
     {
       Scope sc(this, "build_work");
       launches_ += launch_build_work(probes_.p, nb, P, list_off_.p, static_cast<int>(nlist_), cr, 128, list_cnt_.p,
@@ -1999,12 +2039,12 @@ class IndexCore {
     {
       Scope sc(this, "gather_queries");
       if (fp8) {
-        launch_gather_residual(qpad_.p, static_cast<int>(dpad_), kpad8_, true, list_q_.p, list_qoff_.p,
+        launch_gather_residual(qp_, static_cast<int>(dpad_), kpad8_, true, list_q_.p, list_qoff_.p,
                                static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), qscale8_.p, qcd8_.p,
                                pcd_.p, gq8_.p, st_);
         make_u8_tensor_map(gqmap_, gq8_.p, nqp, kpad8_);
       } else {
-        launch_gather_residual(qpad_.p, static_cast<int>(dpad_), kpad_, false, list_q_.p, list_qoff_.p,
+        launch_gather_residual(qp_, static_cast<int>(dpad_), kpad_, false, list_q_.p, list_qoff_.p,
                                static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), nullptr, qcd8_.p,
                                pcd_.p, gq_.p, st_);
         make_bf16_tensor_map(gqmap_, gq_.p, nqp, kpad_);
@@ -2024,7 +2064,7 @@ class IndexCore {
     a.P = P;
     a.seg = seg_.p;
     a.cand = cand_.p;
-    a.err = err_dev_.p;
+    a.err = (status_.p + kStErr);
     a.qcd = qcd8_.p;
     if (fp8) {
       a.fp8 = 1;
@@ -2040,18 +2080,18 @@ class IndexCore {
     {
       Scope sc(this, "cand_select");
       launch_cand_select(cand_.p, seg_.p, probes_.p, nb, P, R, k, list_off_.p, pcd_.p, rmax_.p, static_cast<int>(dpad_),
-                         a.kpad, fp8, cand_rows_.p, cand_m_.p, exact ? over_list_.p : nullptr, over_n_.p, st_);
+                         a.kpad, fp8, cand_rows_.p, cand_m_.p, exact ? over_list_.p : nullptr, (status_.p + kStOver), st_);
     }
     {
       Scope sc(this, "cand_exact");
-      launch_cand_exact(cand_rows_.p, cand_m_.p, nb, R, k, codes_.p, qpad_.p, static_cast<int>(dpad_), ids_.p, Dd, Id,
+      launch_cand_exact(cand_rows_.p, cand_m_.p, nb, R, k, codes_.p, qp_, static_cast<int>(dpad_), ids_.p, Dd, Id,
                         st_);
     }
     launches_ += 6;  // segment lengths, their sum (a library kernel), gather, scan, selection, re-rank
   }
 
   void bf16_err_check() {
-    HB_CUDA(cudaMemcpyAsync(err_host_, err_dev_.p, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    HB_CUDA(cudaMemcpyAsync(err_host_, (status_.p + kStErr), sizeof(int), cudaMemcpyDeviceToHost, st_));
     HB_CUDA(cudaStreamSynchronize(st_));
     if (*err_host_ != 0)
       throw Error(HB_ERR_CUDA, "tensor-core scan gave up waiting (code " + std::to_string(*err_host_) + ")");
@@ -2060,14 +2100,14 @@ class IndexCore {
   // Coarse probes of the batch in qpad_, then the per-query cut.
   void coarse_and_cut(int nb, int P) {
     if (cut_mode_ == 1 && coarse_tc_route(P) && probe_.C <= P) {
-      coarse_learned(qpad_.p, nb, P, probes_.p, cut_thr_, cut_cap_);
+      coarse_learned(qp_, nb, P, probes_.p, cut_thr_, cut_cap_);
     } else if (cut_mode_ == 1) {
       cdist_.reserve(static_cast<size_t>(nb) * P);
-      coarse(qpad_.p, nb, P, probes_.p, cdist_.p);
+      coarse(qp_, nb, P, probes_.p, cdist_.p);
       Scope sc(this, "probe_mlp");
-      probe_infer(nb, qpad_.p, cdist_.p, P, probes_.p, cut_thr_, cut_cap_, nullptr);
+      probe_infer(nb, qp_, cdist_.p, P, probes_.p, cut_thr_, cut_cap_, nullptr);
     } else {
-      coarse(qpad_.p, nb, P, probes_.p, nullptr);
+      coarse(qp_, nb, P, probes_.p, nullptr);
       if (cut_mode_ == 2) {
         npq_.reserve(static_cast<size_t>(nb));
         HB_CUDA(cudaMemcpyAsync(npq_.p, cut_src_ + cut_b0_, static_cast<size_t>(nb) * sizeof(int32_t), cudaMemcpyDefault,
@@ -2111,10 +2151,6 @@ class IndexCore {
                    int32_t* nprobe_out) {
     ProbeModel& m = probe_;
     if (m.tc) {
-      if (!cerr_dev_.p) {
-        cerr_dev_.reserve(1);
-        HB_CUDA(cudaMemsetAsync(cerr_dev_.p, 0, sizeof(int), st_));
-      }
       int32_t* np = nprobe_out;
       if (!np) {
         npq_.reserve(static_cast<size_t>(nb));
@@ -2122,7 +2158,7 @@ class IndexCore {
       }
       mlp_infer_tc(qpad, nb, static_cast<int>(d_), static_cast<int>(dpad_), cdist, P, m.C, m.mean.p, m.inv_std.p, m.K1,
                    m.W1b.p, m.B1.p, m.W2b.p, m.B2.p, m.W3b.p, m.B3.p, m.NB, m.bucket_val.p, thr, cap, np,
-                   cerr_dev_.p, st_);
+                   (status_.p + kStCoarseErr), st_);
       ++launches_;
       if (probes) {
         launch_cut_probes(np, nb, P, probes, st_);
@@ -2420,13 +2456,13 @@ class IndexCore {
   DevBuf<uint32_t> cmins_;   // per 16-column chunk of dmat_ and query: the chunk's smallest value
   DevBuf<float> cnorm_, cmaxnorm_, cval_;
   DevBuf<int32_t> ccand_;
-  DevBuf<int> cflags_, cerr_dev_;
+  DevBuf<int> cflags_;
   bool capturing_ = false;
   std::map<std::string, GraphEntry> graphs_;
   DevBuf<int32_t> npqin_;
   // bounded BF16 scan
   DevBuf<uint32_t> thr_;
-  DevBuf<int> ccnt_, cflag_, over_list_, over_n_, rr_m_;
+  DevBuf<int> ccnt_, cflag_, over_list_, rr_m_;
   bool screen_ = false;              // this search's plain FP32 batches go through the bounded scan
   bool screen_wide_ = false;         // d > 128: through the candidate matrix
   DevBuf<int> scr_cnt_, scr_m_;      // its counts (bf16_stats reports BF16 searches only)
@@ -2446,7 +2482,19 @@ class IndexCore {
   DevBuf<int64_t> tile_off_;
   DevBuf<int32_t> probes1_;
   DevBuf<int32_t> probe0_, probes_rest_;  // the two stages' probe tables (k > kFilterTightK)
-  DevBuf<int> err_dev_;
+  // Status words of the searches on the device, read back in one copy: the
+  // scans' error flag, queries to search again exactly, queries with many
+  // candidates, the work counters of a batch's (at most two) scans -- these
+  // are cleared per batch -- and the coarse quantizer's (sticky) error flag.
+  enum { kStErr = 0, kStOver = 1, kStBig = 2, kStCounter = 3, kStPerBatch = 5, kStCoarseErr = 7, kStatusWords = 8 };
+  DevBuf<int> status_;
+  unsigned int* counter(int i) { return reinterpret_cast<unsigned int*>(status_.p + kStCounter + i); }
+  // Pinned host block: the status words, then small batches' results and
+  // queries on their way (a copy to or from pageable memory is two to three
+  // times slower, and each waits for the stream).
+  static constexpr size_t kPinnedResults = 48 << 10, kPinnedQueries = 64 << 10;
+  static constexpr size_t kPinnedBytes = 256 + kPinnedResults + kPinnedQueries;
+  unsigned char* pin_ = nullptr;
   int* err_host_ = nullptr;
   bool prof_ = false;
   std::vector<ProfRecord> prof_log_;
@@ -2457,18 +2505,19 @@ class IndexCore {
   cudaStream_t st_ = nullptr;
   bool trained_ = false;
   size_t ntotal_ = 0;
-  size_t plan_rows_ = 0;
+  std::vector<int64_t> sizes_desc_;
   uint64_t launches_ = 0;
   std::vector<int64_t> host_off_;
 
   DevBuf<float> cent_, codes_, norms_;
   DevBuf<int64_t> list_off_, ids_;
   // search workspace
-  DevBuf<float> qpad_, qtmp_, dmat_, tops_, dout_;
-  DevBuf<int64_t> iout_, list_qoff_, item_off_, slot_base_;
+  const float* qp_ = nullptr;  // this batch's padded queries: qpad_, or the caller's rows where nothing is padded
+  DevBuf<unsigned char> out_;  // a batch's ids and distances on their way to the host
+  DevBuf<float> qpad_, qtmp_, dmat_, tops_;
+  DevBuf<int64_t> list_qoff_, item_off_, slot_base_;
   DevBuf<int32_t> probes_, list_cnt_, list_cursor_, list_q_, order_dev_;
   DevBuf<uint64_t> part_;
-  DevBuf<unsigned int> counter_;
   DevBuf<unsigned char> work_tmp_;
 };
 
