@@ -257,6 +257,86 @@ __device__ uint32_t warp_kth_smallest(Get get, int n, int k, int* h, int lane) {
   return prefix;
 }
 
+// The same by a whole block of NT threads (keys v[0 .. n-1], 1 <= k <= n);
+// every thread returns it.
+template <int NT>
+__device__ uint32_t block_kth_smallest(const uint32_t* __restrict__ v, int n, int k, int* h) {
+  __shared__ uint32_t s_lo, s_hi, s_prefix;
+  __shared__ int s_need;
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) {
+    s_lo = 0xFFFFFFFFu;
+    s_hi = 0u;
+  }
+  __syncthreads();
+  uint32_t lo = 0xFFFFFFFFu, hi = 0u;
+#pragma unroll 4
+  for (int i = tid; i < n; i += NT) {
+    lo = min(lo, v[i]);
+    hi = max(hi, v[i]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (lane == 0) {
+    atomicMin(&s_lo, lo);
+    atomicMax(&s_hi, hi);
+  }
+  __syncthreads();
+  lo = s_lo;
+  hi = s_hi;
+  uint32_t prefix = 0u, pmask = 0u;
+  int need = k;
+  for (int shift = 24; shift >= 0; shift -= 8) {
+    if ((lo >> shift) == (hi >> shift)) {
+      prefix |= lo & (255u << shift);
+      pmask |= 255u << shift;
+      continue;
+    }
+    for (int i = tid; i < 256; i += NT) h[i] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (int i = tid; i < n; i += NT) {
+      const uint32_t x = v[i];
+      if ((x & pmask) == prefix) atomicAdd(&h[(x >> shift) & 255u], 1);
+    }
+    __syncthreads();
+    if (tid < 32) {
+      int loc[8], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        loc[j] = h[8 * lane + j];
+        sum += loc[j];
+      }
+      int incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+      }
+      int before = incl - sum;
+      if (before < need && need <= incl) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (before + loc[j] >= need) {
+            s_prefix = prefix | (static_cast<uint32_t>(8 * lane + j) << shift);
+            s_need = need - before;
+            break;
+          }
+          before += loc[j];
+        }
+      }
+    }
+    __syncthreads();
+    prefix = s_prefix;
+    need = s_need;
+    pmask |= 255u << shift;
+  }
+  return prefix;
+}
+
 __host__ __device__ __forceinline__ int pow2_ceil(int x) {
   int p = 1;
   while (p < x) p <<= 1;

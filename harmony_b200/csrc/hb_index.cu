@@ -1641,8 +1641,7 @@ class IndexCore {
     thr_.reserve(nb);
     cnt.reserve(nb);
     m.reserve(nb);
-    cflag_.reserve(nb);
-    over_list_.reserve(2 * static_cast<size_t>(nb));
+    over_list_.reserve(static_cast<size_t>(nb));
     cbuf_.reserve(static_cast<size_t>(nb) * cap);
     cbuf_ub_.reserve(static_cast<size_t>(nb) * cap);
   }
@@ -1836,11 +1835,9 @@ class IndexCore {
     {
       Scope sc(this, "rerank");
       launch_rerank_bf16(cbuf_.p, cbuf_ub_.p, cnt, cap, nb, k, codes_.p, qp_, static_cast<int>(dpad_), ids_.p, Dd,
-                         Id, cflag_.p, over_list_.p, (status_.p + kStOver), rr_m, num_sms_, st_);
+                         Id, over_list_.p, status_.p + kStOver, rr_m, st_);
     }
-    // query prep, seed, scan, warp re-rank, and the three flat re-rank
-    // kernels when the buffers can hold more than a warp's candidates.
-    launches_ += 4 + (cap > 256 ? 3 : 0);
+    launches_ += 4;  // query prep, seed, scan, re-rank
   }
 
   // ---- autotuner of the bounded scan ----------------------------------------
@@ -2015,7 +2012,7 @@ class IndexCore {
     }
     cand_.reserve(std::max<size_t>(static_cast<size_t>(nb) * cand_row_bound(P), 1));
     cand_rows_.reserve(static_cast<size_t>(nb) * R);
-    over_list_.reserve(2 * static_cast<size_t>(nb));
+    over_list_.reserve(static_cast<size_t>(nb));
   }
 
   // After the coarse probes (buffers reserved).  `exact`: every row that can
@@ -2462,7 +2459,7 @@ class IndexCore {
   DevBuf<int32_t> npqin_;
   // bounded BF16 scan
   DevBuf<uint32_t> thr_;
-  DevBuf<int> ccnt_, cflag_, over_list_, rr_m_;
+  DevBuf<int> ccnt_, over_list_, rr_m_;
   bool screen_ = false;              // this search's plain FP32 batches go through the bounded scan
   bool screen_wide_ = false;         // d > 128: through the candidate matrix
   DevBuf<int> scr_cnt_, scr_m_;      // its counts (bf16_stats reports BF16 searches only)
@@ -2486,7 +2483,7 @@ class IndexCore {
   // scans' error flag, queries to search again exactly, queries with many
   // candidates, the work counters of a batch's (at most two) scans -- these
   // are cleared per batch -- and the coarse quantizer's (sticky) error flag.
-  enum { kStErr = 0, kStOver = 1, kStBig = 2, kStCounter = 3, kStPerBatch = 5, kStCoarseErr = 7, kStatusWords = 8 };
+  enum { kStErr = 0, kStOver = 1, kStCounter = 2, kStPerBatch = 4, kStCoarseErr = 4, kStatusWords = 8 };
   DevBuf<int> status_;
   unsigned int* counter(int i) { return reinterpret_cast<unsigned int*>(status_.p + kStCounter + i); }
   // Pinned host block: the status words, then small batches' results and

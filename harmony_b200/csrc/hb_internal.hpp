@@ -273,15 +273,13 @@ void launch_seed_bound(const float* q, int d, int dpad, const float* cent, int n
                        const float* rnorm, const float* rmax, int S, int k, uint32_t* thr, cudaStream_t st,
                        const int32_t* probes = nullptr, int P = 0);
 // Exact re-rank of the admitted rows whose lower bound is at most U, the k-th
-// smallest admitted upper bound (cand_ub); flag[q] = 2 and
-// over_list[0 .. over_n[0]) for queries whose buffer overflowed (left
-// unwritten); over_list[nq ..] / over_n[1] list the queries with more than
-// 256 candidates, re-ranked by the flat kernels, which overwrite their
-// buffers (over_list holds 2 nq ints, over_n 2, zeroed by the caller);
-// m_out[q] = rows re-ranked.
+// smallest admitted upper bound (cand_ub); over_list[0 .. over_n[0]) gets the
+// queries whose buffer overflowed (left unwritten; over_n zeroed by the
+// caller); m_out[q] = rows re-ranked.  Buffers of queries with many candidates
+// are overwritten.
 void launch_rerank_bf16(uint64_t* cand, const uint32_t* cand_ub, const int* cnt, int cap, int nq, int k,
                         const float* codes, const float* q, int dpad, const int64_t* ids, float* D, int64_t* I,
-                        int* flag, int* over_list, int* over_n, int* m_out, int num_sms, cudaStream_t st);
+                        int* over_list, int* over_n, int* m_out, cudaStream_t st);
 
 // Largest k whose bound tightens inside the BF16 scan; a larger k takes two
 // stages (the nearest list of every query first, then the rest under the

@@ -760,102 +760,141 @@ __global__ void residual_rmax_kernel(float* __restrict__ rmax, int nlist) {
 constexpr int kSmallKth = 32;  // largest k for warp_kth_small8
 
 
-// Re-rank, one warp per query with at most kRrWarpCap candidates: U = the
-// k-th smallest upper bound among them (radix selection), the candidates
-// whose lower bound is at most U recomputed with the reference's sequential
-// FP32 loop, sorted by (distance, position) and cut at k.  A query with more
-// candidates goes to the flat kernels below (flag 1); one whose buffer
-// overflowed to the host's exact search (flag 2, and listed).
-constexpr int kRrWarpCap = 256;
-constexpr int kRrWarps = 8;
+// Re-rank, one CTA per query: U = the k-th smallest upper bound among its
+// candidates, the candidates whose lower bound is at most U recomputed with
+// the reference's sequential FP32 loop, sorted by (distance, position) and cut
+// at k.  A query whose buffer overflowed goes to the host's exact search (flag
+// 2, and listed).  The rows to recompute come into shared memory kRrRows at a
+// time by 16-byte cp.async, coalesced and all in flight together, and a thread
+// sums each from there; keys live in shared memory, or, for more than kRrKeys
+// of them, in the query's buffer.  Bound by DRAM in large batches (the
+// recomputed rows), by the chain of its phases in small ones.  k <= 16 takes
+// two warps and 16 rows, so that fifteen CTAs fit an SM (a query re-ranks about
+// 15 rows there), a larger k four warps and 32 rows.  A warp per query walking
+// its rows from global memory, with three flat kernels for the queries with
+// more than 256 candidates, took 477 us for 10k queries on 1M x 128 with k 100
+// (124 rows each) and 85 us on 10M x 128 with k 10: now 192 and 62; one query
+// 21 -> 11 us.  (Other splits, threads x rows, for k 100: 128 x 64 242 us, 64 x
+// 32 219, 128 x 16 226, 64 x 16 227.)
+constexpr int kRrKeys = 512;
+constexpr int kRerankMaxDim = 128;  // dpad of the BF16 scan's rows (d <= 128)
+constexpr int kRrStride = kRerankMaxDim + 4;
 
-__global__ void __launch_bounds__(kRrWarps * 32) rerank_warp_kernel(
-    const uint64_t* __restrict__ cand, const uint32_t* __restrict__ cand_ub, const int* __restrict__ cnt, int cap,
-    int nq, int k, const float* __restrict__ codes, const float* __restrict__ q, int dpad,
-    const int64_t* __restrict__ ids, float* __restrict__ D, int64_t* __restrict__ I, int* __restrict__ flag,
-    int* __restrict__ over_list, int* __restrict__ over_n, int* __restrict__ m_out, int* __restrict__ big_list) {
-  __shared__ uint64_t s_c[kRrWarps][kRrWarpCap];
-  __shared__ uint64_t s_x[kRrWarps][kRrWarpCap];
-  __shared__ int s_h[kRrWarps][256];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int qi = blockIdx.x * kRrWarps + wib;
-  if (qi >= nq) return;
+template <int kRrThreads, int kRrRows>
+__global__ void __launch_bounds__(kRrThreads) rerank_kernel(
+    uint64_t* __restrict__ cand, const uint32_t* __restrict__ cand_ub, const int* __restrict__ cnt, int cap, int k,
+    const float* __restrict__ codes, const float* __restrict__ q, int dpad, const int64_t* __restrict__ ids,
+    float* __restrict__ D, int64_t* __restrict__ I, int* __restrict__ over_list, int* __restrict__ over_n,
+    int* __restrict__ m_out) {
+  extern __shared__ uint64_t s_top[];  // pow2_ceil(k), for queries with more than kRrKeys rows to recompute
+  __shared__ uint64_t s_key[kRrKeys];
+  __shared__ __align__(16) float s_row[kRrRows * kRrStride];
+  __shared__ __align__(16) float s_q[kRerankMaxDim];
+  __shared__ int s_h[256];
+  __shared__ uint32_t s_u;
+  __shared__ int s_m;
+  __shared__ SelectShared sh_sel;
+  const int qi = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int c = cnt[qi];
   if (c > cap) {
-    if (lane == 0) {
-      flag[qi] = 2;
+    if (tid == 0) {
       m_out[qi] = 0;
       over_list[atomicAdd(over_n, 1)] = qi;
     }
     return;
   }
-  if (c > kRrWarpCap) {
-    if (lane == 0) {
-      flag[qi] = 1;
-      big_list[atomicAdd(over_n + 1, 1)] = qi;
+  uint64_t* buf = cand + static_cast<size_t>(qi) * cap;
+  const uint32_t* ubs = cand_ub + static_cast<size_t>(qi) * cap;
+  if (tid < dpad / 4)
+    *reinterpret_cast<float4*>(s_q + 4 * tid) =
+        *reinterpret_cast<const float4*>(q + static_cast<size_t>(qi) * dpad + 4 * tid);
+  if (tid == 0) s_m = 0;
+  // The first keys are on their way while U is formed.
+  uint64_t key[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) key[u] = u * kRrThreads + tid < c ? buf[u * kRrThreads + tid] : kEmpty;
+  // U (every candidate when there are fewer than k).
+  if (c < k) {
+    if (tid == 0) s_u = 0xFFFFFFFFu;
+  } else if (c <= 256 && k <= kSmallKth) {
+    if (wid == 0) {
+      uint32_t v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < c ? ubs[32 * i + lane] : 0xFFFFFFFFu;
+      const uint32_t u = warp_kth_small8(v, k, lane);
+      if (lane == 0) s_u = u;
     }
-    return;
+  } else {
+    const uint32_t u = block_kth_smallest<kRrThreads>(ubs, c, k, s_h);
+    if (tid == 0) s_u = u;
   }
-  if (lane == 0) flag[qi] = 0;
-  uint64_t* buf = s_c[wib];
-  uint64_t* ex = s_x[wib];
-  const uint64_t* src = cand + static_cast<size_t>(qi) * cap;
-  const uint32_t* usrc = cand_ub + static_cast<size_t>(qi) * cap;
-  // U (every candidate when there are fewer than k): for small k from the
-  // upper bounds held eight per lane, else by radix from the upper bounds
-  // staged in ex (free until the exact phase) so its passes read shared
-  // memory.
-  uint32_t u_bits = 0xFFFFFFFFu;
-  if (c >= k && k <= kSmallKth) {
-    static_assert(kRrWarpCap == 256, "eight upper bounds per lane");
-    uint32_t v[8];
+  __syncthreads();
+  const uint32_t u_bits = s_u;
+  // The candidates with lower bound <= U: into s_key, or, past kRrKeys of
+  // them, compacted at the front of the buffer.  A block of 8 * kRrThreads keys
+  // is read before any of it is written, and writes land at or below the read
+  // position.
+  for (int base = 0; base < c; base += 8 * kRrThreads) {
+    if (base > 0) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < c ? usrc[32 * i + lane] : 0xFFFFFFFFu;
-    u_bits = warp_kth_small8(v, k, lane);
-  } else if (c >= k) {
-    uint32_t* ubs = reinterpret_cast<uint32_t*>(ex);
-    for (int i = lane; i < c; i += 32) ubs[i] = usrc[i];
-    __syncwarp();
-    u_bits = warp_kth_smallest([&](int i) { return ubs[i]; }, c, k, s_h[wib], lane);
-  }
-  // The candidates with lower bound <= U, compacted into buf (c <= 256:
-  // eight keys per lane, their loads in flight together).
-  int m = 0;
-  {
-    uint64_t key[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) key[u] = 32 * u + lane < c ? src[32 * u + lane] : kEmpty;
+      for (int u = 0; u < 8; ++u) {
+        const int i = base + u * kRrThreads + tid;
+        key[u] = i < c ? buf[i] : kEmpty;
+      }
+    }
+    __syncthreads();
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const bool in = 32 * u + lane < c && static_cast<uint32_t>(key[u] >> 32) <= u_bits;
+      const bool in = base + u * kRrThreads + tid < c && static_cast<uint32_t>(key[u] >> 32) <= u_bits;
       const unsigned bal = __ballot_sync(0xffffffffu, in);
-      if (in) buf[m + __popc(bal & ((1u << lane) - 1u))] = key[u];
-      m += __popc(bal);
+      int at = 0;
+      if (lane == 0 && bal) at = atomicAdd(&s_m, __popc(bal));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
+      if (in) {
+        if (at < kRrKeys) s_key[at] = key[u];
+        if (c > kRrKeys) buf[at] = key[u];
+      }
     }
   }
-  __syncwarp();
-  if (lane == 0) m_out[qi] = m;
-  // Every line of the rows to recompute requested at once (the lane loops
-  // below then wait for one DRAM round trip, not one per batch of loads).
-  for (int j = lane; j < m; j += 32) {
-    const char* rp = reinterpret_cast<const char*>(codes + static_cast<size_t>(key_tie(buf[j])) * dpad);
-    for (int o = 0; o < dpad * 4; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(rp + o));
-  }
-  const float* qrow = q + static_cast<size_t>(qi) * dpad;
-  const int e2n = pow2_ceil(m < 2 ? 2 : m);
-  for (int j = lane; j < e2n; j += 32) {
-    uint64_t key = kEmpty;
-    if (j < m) {
-      const uint32_t pos = key_tie(buf[j]);
-      const float acc = exact_l2_seq(codes + static_cast<size_t>(pos) * dpad, qrow, dpad);
-      if (acc < FLT_MAX) key = make_key(acc, pos);
+  __syncthreads();
+  const int m = s_m;
+  if (tid == 0) m_out[qi] = m;
+  const bool small = m <= kRrKeys;
+  const int cpr = dpad >> 2;
+  for (int b0 = 0; b0 < m; b0 += kRrRows) {
+    const int nb = min(kRrRows, m - b0);
+    for (int i = tid; i < nb * cpr; i += kRrThreads) {
+      const int r = i / cpr, f = i - r * cpr;
+      const uint32_t pos = key_tie(small ? s_key[b0 + r] : buf[b0 + r]);
+      cp_async16(s_row + r * kRrStride + 4 * f, codes + static_cast<size_t>(pos) * dpad + 4 * f, true);
     }
-    ex[j] = key;
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    if (tid < nb) {
+      const uint32_t pos = key_tie(small ? s_key[b0 + tid] : buf[b0 + tid]);
+      const float d = exact_l2_seq_from(0.0f, s_row + tid * kRrStride, s_q, dpad);
+      const uint64_t key = d < FLT_MAX ? make_key(d, pos) : kEmpty;
+      if (small) s_key[b0 + tid] = key;
+      else buf[b0 + tid] = key;
+    }
+    __syncthreads();
   }
-  __syncwarp();
-  warp_bitonic_sort(ex, e2n, lane);
-  for (int j = lane; j < k; j += 32) {
-    const uint64_t key = j < m ? ex[j] : kEmpty;
+  const uint64_t* top = s_key;
+  int n2;
+  if (small) {
+    n2 = pow2_ceil(m < 2 ? 2 : m);
+    for (int i = m + tid; i < n2; i += kRrThreads) s_key[i] = kEmpty;
+    __syncthreads();
+    block_bitonic_sort(s_key, n2);
+  } else {
+    auto key_at = [&](int i) -> uint64_t { return buf[i]; };
+    block_topk_sorted(key_at, m, k, sh_sel, s_top);
+    top = s_top;
+    n2 = k;
+  }
+  for (int j = tid; j < k; j += kRrThreads) {
+    const uint64_t key = j < n2 ? top[j] : kEmpty;
     const size_t o = static_cast<size_t>(qi) * k + j;
     D[o] = key == kEmpty ? FLT_MAX : key_dist(key);
     I[o] = key == kEmpty ? -1 : ids[key_tie(key)];
@@ -893,134 +932,6 @@ __global__ void split_first_probe_kernel(const int32_t* __restrict__ probes, int
   const int32_t v = probes[i];
   rest[i] = j == 0 ? -1 : v;
   if (j == 0) first[i / P] = v;
-}
-
-// The queries the warp kernel listed in big_list (more than kRrWarpCap
-// candidates, at most cap; *big_n of them) in three flat kernels, so the
-// exact distances -- the bulk of the work -- run with every SM's threads
-// loading rows rather than behind per-query sorts:
-//   rerank_big_bound_kernel  a warp per query: U, the k-th smallest upper
-//                            bound, by radix selection, then the candidates
-//                            whose lower bound is at most U compacted in
-//                            place at the front of the query's buffer (m of
-//                            them);
-//   rerank_big_exact_kernel  a CTA per query: the exact distance of each of
-//                            the m rows (two rows per thread in flight),
-//                            written back in place as (distance, position)
-//                            keys;
-//   rerank_big_topk_kernel   a CTA per query: the k smallest keys, sorted.
-constexpr int kBigWarps = 8;
-constexpr int kRerankMaxDim = 128;  // dpad of the BF16 scan's rows (d <= 128)
-
-__global__ void __launch_bounds__(kBigWarps * 32) rerank_big_bound_kernel(
-    uint64_t* __restrict__ cand, const uint32_t* __restrict__ cand_ub, const int* __restrict__ cnt, int cap, int k,
-    const int* __restrict__ big_list, const int* __restrict__ big_n, int* __restrict__ m_out) {
-  __shared__ int s_h[kBigWarps][256];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int nbig = *big_n;
-  for (int w = blockIdx.x * kBigWarps + wib; w < nbig; w += gridDim.x * kBigWarps) {
-    const int qi = big_list[w];
-    const int c = cnt[qi];
-    uint64_t* buf = cand + static_cast<size_t>(qi) * cap;
-    const uint32_t* ubs = cand_ub + static_cast<size_t>(qi) * cap;
-    const uint32_t lim_bits = warp_kth_smallest([&](int i) { return ubs[i]; }, c, k, s_h[wib], lane);
-    // In-place compaction: a block of 256 keys (eight per lane, their loads
-    // in flight together) is read before any of it is written, and writes
-    // land at or below the read position.
-    int m = 0;
-    for (int base = 0; base < c; base += 256) {
-      uint64_t key[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) key[u] = base + 32 * u + lane < c ? buf[base + 32 * u + lane] : kEmpty;
-      __syncwarp();
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const bool in = base + 32 * u + lane < c && static_cast<uint32_t>(key[u] >> 32) <= lim_bits;
-        const unsigned bal = __ballot_sync(0xffffffffu, in);
-        if (in) buf[m + __popc(bal & ((1u << lane) - 1u))] = key[u];
-        m += __popc(bal);
-      }
-    }
-    if (lane == 0) m_out[qi] = m;
-    __syncwarp();
-  }
-}
-
-__global__ void __launch_bounds__(256) rerank_big_exact_kernel(uint64_t* __restrict__ cand, int cap,
-                                                               const float* __restrict__ codes,
-                                                               const float* __restrict__ q, int dpad,
-                                                               const int* __restrict__ big_list,
-                                                               const int* __restrict__ big_n,
-                                                               const int* __restrict__ m_in) {
-  __shared__ __align__(16) float s_q[kRerankMaxDim];
-  const int nbig = *big_n;
-  for (int w = blockIdx.x; w < nbig; w += gridDim.x) {
-    const int qi = big_list[w];
-    const int m = m_in[qi];
-    uint64_t* buf = cand + static_cast<size_t>(qi) * cap;
-    __syncthreads();  // the previous query's readers of s_q are done
-    for (int c = threadIdx.x; c < dpad; c += blockDim.x) s_q[c] = q[static_cast<size_t>(qi) * dpad + c];
-    __syncthreads();
-    // Rows j and j + blockDim.x together: two independent chains, each the
-    // reference's sequential loop (many small CTAs per SM keep the loads in
-    // flight).
-    for (int j0 = threadIdx.x; j0 < m; j0 += 2 * blockDim.x) {
-      const int j1 = j0 + blockDim.x;
-      const uint32_t p0 = key_tie(buf[j0]);
-      const uint32_t p1 = j1 < m ? key_tie(buf[j1]) : p0;
-      const float4* x0 = reinterpret_cast<const float4*>(codes + static_cast<size_t>(p0) * dpad);
-      const float4* x1 = reinterpret_cast<const float4*>(codes + static_cast<size_t>(p1) * dpad);
-      float a0 = 0.0f, a1 = 0.0f;
-#pragma unroll 4
-      for (int i = 0; i < dpad / 4; ++i) {
-        const float4 u = __ldg(x0 + i), v = __ldg(x1 + i);
-        const float4 g = *reinterpret_cast<const float4*>(s_q + 4 * i);
-        float t;
-        t = __fsub_rn(g.x, u.x);
-        a0 = __fadd_rn(a0, __fmul_rn(t, t));
-        t = __fsub_rn(g.x, v.x);
-        a1 = __fadd_rn(a1, __fmul_rn(t, t));
-        t = __fsub_rn(g.y, u.y);
-        a0 = __fadd_rn(a0, __fmul_rn(t, t));
-        t = __fsub_rn(g.y, v.y);
-        a1 = __fadd_rn(a1, __fmul_rn(t, t));
-        t = __fsub_rn(g.z, u.z);
-        a0 = __fadd_rn(a0, __fmul_rn(t, t));
-        t = __fsub_rn(g.z, v.z);
-        a1 = __fadd_rn(a1, __fmul_rn(t, t));
-        t = __fsub_rn(g.w, u.w);
-        a0 = __fadd_rn(a0, __fmul_rn(t, t));
-        t = __fsub_rn(g.w, v.w);
-        a1 = __fadd_rn(a1, __fmul_rn(t, t));
-      }
-      buf[j0] = a0 < FLT_MAX ? make_key(a0, p0) : kEmpty;
-      if (j1 < m) buf[j1] = a1 < FLT_MAX ? make_key(a1, p1) : kEmpty;
-    }
-  }
-}
-
-__global__ void __launch_bounds__(256) rerank_big_topk_kernel(const uint64_t* __restrict__ cand, int cap, int k,
-                                                              const int64_t* __restrict__ ids, float* __restrict__ D,
-                                                              int64_t* __restrict__ I, const int* __restrict__ big_list,
-                                                              const int* __restrict__ big_n,
-                                                              const int* __restrict__ m_in) {
-  extern __shared__ uint64_t s_top[];  // pow2_ceil(k)
-  __shared__ SelectShared sh_sel;
-  const int nbig = *big_n;
-  for (int w = blockIdx.x; w < nbig; w += gridDim.x) {
-    const int qi = big_list[w];
-    const int m = m_in[qi];
-    const uint64_t* buf = cand + static_cast<size_t>(qi) * cap;
-    auto key_at = [&](int i) -> uint64_t { return buf[i]; };
-    __syncthreads();  // the previous query's readers of s_top are done
-    block_topk_sorted(key_at, m, k, sh_sel, s_top);
-    for (int j = threadIdx.x; j < k; j += blockDim.x) {
-      const uint64_t key = s_top[j];
-      const size_t o = static_cast<size_t>(qi) * k + j;
-      D[o] = key == kEmpty ? FLT_MAX : key_dist(key);
-      I[o] = key == kEmpty ? -1 : ids[key_tie(key)];
-    }
-  }
 }
 
 // Seed bound per query before the scan: U = the k-th smallest w over the
@@ -1342,27 +1253,18 @@ void launch_seed_bound(const float* q, int d, int dpad, const float* cent, int n
 
 void launch_rerank_bf16(uint64_t* cand, const uint32_t* cand_ub, const int* cnt, int cap, int nq, int k,
                         const float* codes, const float* q, int dpad, const int64_t* ids, float* D, int64_t* I,
-                        int* flag, int* over_list, int* over_n, int* m_out, int num_sms, cudaStream_t st) {
+                        int* over_list, int* over_n, int* m_out, cudaStream_t st) {
   if (nq <= 0) return;
-  HB_CHECK(k >= 1 && cap >= k && cap <= kRerankMaxCap && (cap & (cap - 1)) == 0, HB_ERR_INVALID,
+  HB_CHECK(k >= 1 && k <= kFilterMaxK && cap >= k && cap <= kRerankMaxCap && (cap & (cap - 1)) == 0, HB_ERR_INVALID,
            "candidate buffer size out of range");
   HB_CHECK(dpad % 4 == 0 && dpad <= kRerankMaxDim, HB_ERR_INVALID, "re-rank rows wider than 128 floats");
-  rerank_warp_kernel<<<(nq + kRrWarps - 1) / kRrWarps, kRrWarps * 32, 0, st>>>(
-      cand, cand_ub, cnt, cap, nq, k, codes, q, dpad, ids, D, I, flag, over_list, over_n, m_out, over_list + nq);
+  const size_t smem = static_cast<size_t>(pow2_ceil(k < 2 ? 2 : k)) * sizeof(uint64_t);
+  auto go = [&](auto kernel, int threads) {
+    kernel<<<nq, threads, smem, st>>>(cand, cand_ub, cnt, cap, k, codes, q, dpad, ids, D, I, over_list, over_n, m_out);
+  };
+  if (k <= kFilterTightK) go(rerank_kernel<64, 16>, 64);
+  else go(rerank_kernel<128, 32>, 128);
   HB_CUDA(cudaGetLastError());
-  if (cap > kRrWarpCap) {
-    // At most nq queries are big (*big_n of them, known on the device
-    // only): grids of at most eight CTAs per SM stride over the list.
-    const int* big_list = over_list + nq;
-    const int* big_n = over_n + 1;
-    const int gmax = 8 * std::max(1, num_sms);
-    rerank_big_bound_kernel<<<std::min((nq + kBigWarps - 1) / kBigWarps, gmax), kBigWarps * 32, 0, st>>>(
-        cand, cand_ub, cnt, cap, k, big_list, big_n, m_out);
-    rerank_big_exact_kernel<<<std::min(nq, gmax), 256, 0, st>>>(cand, cap, codes, q, dpad, big_list, big_n, m_out);
-    const size_t smem = static_cast<size_t>(pow2_ceil(k < 2 ? 2 : k)) * sizeof(uint64_t);
-    rerank_big_topk_kernel<<<std::min(nq, gmax), 256, smem, st>>>(cand, cap, k, ids, D, I, big_list, big_n, m_out);
-    HB_CUDA(cudaGetLastError());
-  }
 }
 
 void launch_kth_bound(const uint32_t* cand_ub, const int* cnt, int cap, int nq, int k, uint32_t* thr,
