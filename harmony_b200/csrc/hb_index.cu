@@ -55,17 +55,22 @@ bool is_device_ptr(const void* p) {
 constexpr double kAssignTcTrain = 5.0e8;
 constexpr double kAssignTcAdd = 5.0e9;
 // (query, row) pairs from which a plain FP32 search takes the bounded scan
-// instead of the exact scan: below it the exact scan's fewer kernels win.
-// Lists of 600 and 1000 rows, k 10 and 20: 9.6e4 pairs 189 -> 204 us, 1.6e5
-// 229 -> 171, 3.8e5 282 -> 218; k 100: 1.5e5 205 -> 242 us, 2.5e5 338 -> 324,
-// 3.8e5 296 -> 230.  Short lists (100 rows) keep the exact scan's items small:
-// 2.6e5 pairs 148 -> 181 us, 1.0e6 254 -> 194.
-constexpr double kScreenPairs = 2.0e5, kScreenPairsShort = 8.0e5;
+// instead of the exact scan; below it the exact scan's fewer kernels win.
+// k <= 32, lists of 300 to 1800 rows: 9.6e3 pairs 97 -> 96 us, 2.0e4 110 -> 91,
+// 6.2e4 158 -> 97; lists of 100 rows: 2.6e4 pairs 90 -> 99 us, 6.4e4 107 -> 92.
+// k 100: 2.4e4 pairs 119 -> 125 us, 3.9e4 140 -> 141 and 267 -> 137 (one query),
+// 9.6e4 169 -> 134.
+constexpr double kScreenPairs = 1.2e4, kScreenPairsShort = 4.0e4, kScreenPairsLargeK = 4.0e4;
+constexpr double kScreenPairsShortLargeK = 1.0e5;
+constexpr int kScreenLargeK = 32;
 constexpr double kScreenShortRows = 256.0;
-// d > 128, pairs x padded dimensions: 270k x 500 (527 rows a list) 2.1e4 pairs
-// 193 -> 180 us, 8.4e4 313 -> 183, 1.4e6 797 -> 231; 100k x 200 5.1e4 pairs 145 ->
-// 141 us, 1.3e4 117 -> 134; 100-row lists 2.6e5 pairs 113 -> 137, 1.0e6 200 -> 159.
-constexpr double kScreenWideWork = 1.2e7, kScreenWideWorkShort = 1.0e8;
+// d > 128, pairs x padded dimensions: 270k x 500 (527 rows a list) 5.3e3 pairs
+// 124 -> 127 us, 2.1e4 162 -> 128 (k 100: 169 -> 145, 224 -> 147); 100k x 200
+// 5.1e3 pairs 95 -> 104 us, 2.0e4 124 -> 111; lists of 100 rows, d 200: 1.6e4 pairs
+// 94 -> 107, 6.4e4 110 -> 110.
+constexpr double kScreenWideWork = 4.0e6, kScreenWideWorkShort = 1.3e7;
+constexpr int kOneStageQueries = 256;
+constexpr double kSeedSample = 256.0;
 constexpr int kScreenWideRows = 2048;  // rows re-ranked per query of a wide FP32 search; more go to the exact scan
 
 int pow2_floor(long long x) {
@@ -625,7 +630,8 @@ class IndexCore {
   void coarse(const float* qpad, int nq, int P, int32_t* probes_out, float* cdist_out) {
     dmat_.reserve(static_cast<size_t>(nq) * nlist_);
     const int Pm = std::min<int>(static_cast<int>(nlist_), P + coarse_extra(P));
-    const bool tc = coarse_kind_ != HB_COARSE_EXACT && d_ <= 128 && Pm <= kCoarseMaxPm && nq > 0;
+    const bool tc = coarse_kind_ != HB_COARSE_EXACT && d_ <= 128 && Pm <= kCoarseMaxPm && nq > 0 &&
+                    (coarse_kind_ == HB_COARSE_TENSOR || coarse_tc_pays(nq, Pm));
     HB_CHECK(tc || coarse_kind_ != HB_COARSE_TENSOR, HB_ERR_INVALID,
              "the tensor-core coarse quantizer needs d <= 128 and nprobe + margin <= 1024");
     if (!tc) {
@@ -668,6 +674,18 @@ class IndexCore {
     }
     launches_ += 6;
     coarse_last_nq_ = nq;
+  }
+
+  // Both routes give the same rows; the FP32 matrix costs its nq * nlist
+  // distances, the tensor-core one four more launches (about 25 us) and the
+  // re-ranking of nq * Pm candidates.  Seconds per element-pair of each,
+  // measured (matrix 6.4e12 per second, re-ranking 1e12): 777 queries, 4096
+  // lists of 96 dimensions, nprobe 256 126 -> 110 us by the matrix, nprobe 10 59
+  // against 90; 10k queries, 1024 lists of 128, nprobe 256 644 -> 403, nprobe 64
+  // 198 against 273; one query, 4096 lists 53 -> 36.
+  bool coarse_tc_pays(int nq, int Pm) const {
+    const double pair = static_cast<double>(nq) * dpad_;
+    return pair * nlist_ * 1.55e-13 > 25e-6 + pair * Pm * 1e-12;
   }
 
   int coarse_extra(int P) const { return coarse_margin_ >= 0 ? coarse_margin_ : std::max(16, P / 4); }
@@ -931,7 +949,7 @@ class IndexCore {
     }
     if (bf16 && !cand_path_) bs = std::min(bs, bounded_bs);
     screen_ = screen_ && mode == SCAN_PLAIN && P > 0 &&
-              screen_pays(static_cast<int>(std::min(bs, bounded_bs)), static_cast<int>(P)) &&
+              screen_pays(static_cast<int>(std::min(bs, bounded_bs)), static_cast<int>(P), static_cast<int>(k)) &&
               !(p.use_graph && nq <= bs && nq > bounded_bs);  // a graph is one batch
     if (screen_) bs = std::min(bs, bounded_bs);
     const int warm_lists = p.warmup_lists;
@@ -1597,11 +1615,12 @@ class IndexCore {
   bool screen_possible(int k) const {
     return bf16_ready_ && k <= kFilterMaxK && ntotal_ < (size_t(1) << 31) - 8192;
   }
-  bool screen_pays(int nb, int P) const {
+  bool screen_pays(int nb, int P, int k) const {
     const double avg = static_cast<double>(ntotal_) / static_cast<double>(std::max<size_t>(nlist_, 1));
     const double pairs = static_cast<double>(nb) * P * avg;
     const bool short_lists = avg < kScreenShortRows;
     if (kpad_ > 128) return pairs * dpad_ >= (short_lists ? kScreenWideWorkShort : kScreenWideWork);
+    if (k > kScreenLargeK) return pairs >= (short_lists ? kScreenPairsShortLargeK : kScreenPairsLargeK);
     return pairs >= (short_lists ? kScreenPairsShort : kScreenPairs);
   }
 
@@ -1748,10 +1767,6 @@ class IndexCore {
   // (cr, stages) gives the same result.
   void filter_pipeline(int nb, int P, int k, int cap, int cr, int stages, int* cnt, int* rr_m, long long budget,
                        float* Dd, int64_t* Id) {
-    {
-      Scope sc(this, "query_prep");
-      launch_query_prep(nb, thr_.p, cnt, st_);
-    }
     list_cnt_.reserve(nlist_);
     list_cursor_.reserve(nlist_);
     list_qoff_.reserve(nlist_ + 1);
@@ -1759,7 +1774,13 @@ class IndexCore {
     list_q_.reserve(static_cast<size_t>(nb) * P);
     const size_t wtmp = build_work_tmp_bytes(nb, P, static_cast<int>(nlist_));
     work_tmp_.reserve(wtmp);
-    const bool two_stage = k > kFilterTightK && P > 1;
+    // One stage where the seed's bound alone cannot fill the buffers (it lets
+    // about k of its kSeedSample rows pass, and fewer in the other lists) and
+    // the batch is small: the second stage's four launches then cost more than
+    // the rows it saves (33 queries, 17 lists of 600 rows, k 20: 145 -> 126 us).
+    const double probed = static_cast<double>(P) * static_cast<double>(ntotal_) / static_cast<double>(nlist_);
+    const bool two_stage = k > kFilterTightK && P > 1 &&
+                           (nb > kOneStageQueries || probed * k / kSeedSample > 0.5 * cap);
     const int32_t* probes_a = probes_.p;
     int P_a = P, cr_a = cr;
     if (two_stage) {
@@ -1779,9 +1800,9 @@ class IndexCore {
     }
     {
       Scope sc(this, "seed");
-      launch_seed_bound(qp_, static_cast<int>(d_), static_cast<int>(dpad_), cent_.p, nb, kpad_, codes_bf16_.p,
-                        list_off_.p, static_cast<int>(nlist_), list_qoff_.p, list_q_.p, rnorm_.p, rmax_.p,
-                        std::max(seed_rows_, k), k, thr_.p, st_, probes_a, P_a);
+      launches_ += launch_seed_bound(qp_, static_cast<int>(dpad_), cent_.p, nb, kpad_, codes_bf16_.p, list_off_.p,
+                                     static_cast<int>(nlist_), list_qoff_.p, list_q_.p, rnorm_.p, rmax_.p,
+                                     std::max(seed_rows_, k), k, thr_.p, cnt, st_, probes_a, P_a);
     }
     TcArgs a{};
     a.list_off = list_off_.p;
@@ -1837,7 +1858,7 @@ class IndexCore {
       launch_rerank_bf16(cbuf_.p, cbuf_ub_.p, cnt, cap, nb, k, codes_.p, qp_, static_cast<int>(dpad_), ids_.p, Dd,
                          Id, over_list_.p, status_.p + kStOver, rr_m, st_);
     }
-    launches_ += 4;  // query prep, seed, scan, re-rank
+    launches_ += 2;  // scan, re-rank
   }
 
   // ---- autotuner of the bounded scan ----------------------------------------

@@ -259,19 +259,18 @@ void make_bf16_tensor_map(void* tmap_out, const void* codes_bf16, size_t rows, i
 // Tensor map of a row-major FP32 matrix (rows x cols, cols a multiple of 4)
 // for TMA stores of 32 x 32 boxes with the 128-byte swizzle.
 void make_f32_store_map(void* tmap_out, const float* base, size_t rows, size_t cols);
-// Per query: bound reset to FLT_MAX (none yet), candidate count 0.
-void launch_query_prep(int nq, uint32_t* thr, int* cnt, cudaStream_t st);
 // Residual BF16 codes BF16(x - c_l) (kpad columns), FP32 residual norms per row
 // and the largest residual norm per list.
 void launch_residual_bf16(const float* codes, const int64_t* list_off, const float* cent, int nlist, size_t ntotal,
                           int dpad, int kpad, void* dst, float* rnorm, float* rmax, cudaStream_t st);
-// Seed bound from the first S <= 256 rows of each query's nearest list (probe
-// rank 0 in the list-major work description; with probes given and a small
-// batch, one CTA per query).
-void launch_seed_bound(const float* q, int d, int dpad, const float* cent, int nq, int kpad, const void* codes_bf16,
-                       const int64_t* list_off, int nlist, const int64_t* list_qoff, const int32_t* list_q,
-                       const float* rnorm, const float* rmax, int S, int k, uint32_t* thr, cudaStream_t st,
-                       const int32_t* probes = nullptr, int P = 0);
+// Per query: candidate count 0 and the seed bound from the first S <= 256 rows
+// of its nearest list (probe rank 0 in the list-major work description; with
+// probes given and a small batch, one CTA per query), FLT_MAX where that holds
+// fewer than k.  Returns the kernels launched.
+int launch_seed_bound(const float* q, int dpad, const float* cent, int nq, int kpad, const void* codes_bf16,
+                      const int64_t* list_off, int nlist, const int64_t* list_qoff, const int32_t* list_q,
+                      const float* rnorm, const float* rmax, int S, int k, uint32_t* thr, int* cnt, cudaStream_t st,
+                      const int32_t* probes = nullptr, int P = 0);
 // Exact re-rank of the admitted rows whose lower bound is at most U, the k-th
 // smallest admitted upper bound (cand_ub); over_list[0 .. over_n[0]) gets the
 // queries whose buffer overflowed (left unwritten; over_n zeroed by the

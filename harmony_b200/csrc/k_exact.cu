@@ -716,7 +716,10 @@ void launch_l2_matrix(const float* q, int nq, const float* rows, int nrows, int 
   if (nq <= 0 || nrows <= 0) return;
   HB_CHECK(dpad <= 1024, HB_ERR_INVALID, "dimension above 1024 is not supported");
   const Shape s = matrix_shape(dpad);
-  if (s.tv == 128) matrix_launch<128, 8>(q, nq, rows, nrows, dpad, D, ldD, st);
+  // A few queries: no more than that many sums per thread.
+  if (s.tv == 128 && nq <= 2) matrix_launch<128, 1>(q, nq, rows, nrows, dpad, D, ldD, st);
+  else if (s.tv == 128 && nq <= 4) matrix_launch<128, 2>(q, nq, rows, nrows, dpad, D, ldD, st);
+  else if (s.tv == 128) matrix_launch<128, 8>(q, nq, rows, nrows, dpad, D, ldD, st);
   else if (s.tv == 64) matrix_launch<64, 8>(q, nq, rows, nrows, dpad, D, ldD, st);
   else if (s.tv == 32) matrix_launch<32, 4>(q, nq, rows, nrows, dpad, D, ldD, st);
   else matrix_launch<32, 2>(q, nq, rows, nrows, dpad, D, ldD, st);

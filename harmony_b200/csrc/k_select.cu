@@ -59,6 +59,10 @@ __global__ void __launch_bounds__(kSelThreads) select_rows_kernel(const float* _
 // select_rows_kernel's: the k smallest (value bits, column) keys, ascending.
 constexpr int kBins = 1024;
 constexpr int kCandCap = 2048;
+// Rows up to which each gets a CTA (six per SM) rather than a warp: one row of
+// 4096 columns, the 256 smallest, 42 -> 18 us, 777 rows 52 -> 32; 2500 rows of
+// 1024 columns, 10 smallest, 22 us by warps, 23 by CTAs.
+constexpr int kCtaRows = 888;
 constexpr int kFlaggedGrid = 296;  // CTAs striding over the rows flagged by the warp kernel
 
 template <int VPT>
@@ -596,44 +600,85 @@ __device__ void block_exclusive_scan(Get get, int n, int64_t* __restrict__ out, 
 // The whole work description of a small batch in one CTA (the multi-kernel
 // path's count, prefix sums and scatter, with the counters in shared
 // memory): list_cnt, list_qoff, item_off, slot_base and list_q as
-// launch_build_work defines them.
+// launch_build_work defines them.  Both per-list sums run as one 64-bit scan
+// (queries in the low word, items in the high one) over lists dealt out so that
+// neighbouring threads read neighbouring offsets, and chunk counts are 32-bit
+// divisions: 64 pairs over 4096 lists took 13.5 us with two scans and 64-bit
+// divisions, 9 now.
 __global__ void __launch_bounds__(kWorkThreads) build_work_small_kernel(
     const int32_t* __restrict__ probes, int nqp, int P, const int64_t* __restrict__ list_off, int nlist,
     int chunk_rows, int qgroup, int32_t* __restrict__ list_cnt, int64_t* __restrict__ list_qoff,
     int32_t* __restrict__ list_q, int64_t* __restrict__ item_off, int64_t* __restrict__ slot_base) {
-  extern __shared__ int32_t s_work[];  // [nlist] counts, then [nlist] cursors
+  extern __shared__ int32_t s_work[];  // [nlist] counts, then [nlist] cursors (a list's first entry, then the next)
   __shared__ int64_t s_warp[64];
+  __shared__ unsigned long long s_tot[kWorkThreads / 32];
   int32_t* cnt = s_work;
   int32_t* cur = s_work + nlist;
-  for (int l = threadIdx.x; l < nlist; l += blockDim.x) {
-    cnt[l] = 0;
-    cur[l] = 0;
-  }
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  for (int l = tid; l < nlist; l += kWorkThreads) cnt[l] = 0;
   __syncthreads();
+  // Chunks of a list's rows (list lengths fit 32 bits: the builders hold to
+  // fewer than 2^32 rows in all).
+  auto chunks = [&](int l) -> uint32_t {
+    const uint32_t n = static_cast<uint32_t>(list_off[l + 1] - list_off[l]);
+    return n / static_cast<uint32_t>(chunk_rows) + (n % static_cast<uint32_t>(chunk_rows) != 0u ? 1u : 0u);
+  };
   auto nch_of = [&](int idx) -> int64_t {
     const int l = probes[idx];
-    if (l < 0) return 0;
-    const int64_t n = list_off[l + 1] - list_off[l];
-    return n > 0 ? (n + chunk_rows - 1) / chunk_rows : 0;
+    return l < 0 ? 0 : static_cast<int64_t>(chunks(l));
   };
-  for (int idx = threadIdx.x; idx < nqp; idx += blockDim.x)
-    if (nch_of(idx) > 0) atomicAdd(&cnt[probes[idx]], 1);
-  __syncthreads();
-  for (int l = threadIdx.x; l < nlist; l += blockDim.x) list_cnt[l] = cnt[l];
-  block_exclusive_scan([&](int l) -> int64_t { return cnt[l]; }, nlist, list_qoff, s_warp);
-  block_exclusive_scan(
-      [&](int l) -> int64_t {
-        const int64_t n = list_off[l + 1] - list_off[l];
-        return ((n + chunk_rows - 1) / chunk_rows) * ((cnt[l] + qgroup - 1) / qgroup);
-      },
-      nlist, item_off, s_warp);
-  if (slot_base) block_exclusive_scan(nch_of, nqp, slot_base, s_warp);
-  for (int idx = threadIdx.x; idx < nqp; idx += blockDim.x) {
-    if (nch_of(idx) == 0) continue;
+  for (int idx = tid; idx < nqp; idx += kWorkThreads) {
     const int l = probes[idx];
-    const int pos = atomicAdd(&cur[l], 1);
+    if (l >= 0 && list_off[l + 1] > list_off[l]) atomicAdd(&cnt[l], 1);
+  }
+  __syncthreads();
+  // Scan in blocks of kWorkThreads lists.
+  unsigned long long run = 0;
+  for (int l0 = 0; l0 < nlist; l0 += kWorkThreads) {
+    const int l = l0 + tid;
+    const uint32_t c = l < nlist ? static_cast<uint32_t>(cnt[l]) : 0u;
+    unsigned long long v = 0;
+    if (c) {
+      const uint32_t groups = (c + static_cast<uint32_t>(qgroup) - 1u) / static_cast<uint32_t>(qgroup);
+      v = (static_cast<unsigned long long>(chunks(l) * groups) << 32) | c;
+    }
+    unsigned long long incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    if (lane == 31) s_tot[wid] = incl;
+    __syncthreads();
+    unsigned long long t = s_tot[lane];  // kWorkThreads / 32 = 32 warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long x = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += x;
+    }
+    const unsigned long long before = __shfl_sync(0xffffffffu, t, wid > 0 ? wid - 1 : 0);
+    const unsigned long long total = __shfl_sync(0xffffffffu, t, 31);
+    const unsigned long long excl = run + (wid > 0 ? before : 0ull) + incl - v;
+    if (l < nlist) {
+      list_cnt[l] = static_cast<int32_t>(c);
+      cur[l] = static_cast<int32_t>(excl & 0xffffffffull);
+      list_qoff[l] = static_cast<int64_t>(excl & 0xffffffffull);
+      item_off[l] = static_cast<int64_t>(excl >> 32);
+    }
+    run += total;
+    __syncthreads();  // s_tot is reused
+  }
+  if (tid == 0) {
+    list_qoff[nlist] = static_cast<int64_t>(run & 0xffffffffull);
+    item_off[nlist] = static_cast<int64_t>(run >> 32);
+  }
+  if (slot_base) block_exclusive_scan(nch_of, nqp, slot_base, s_warp);
+  for (int idx = tid; idx < nqp; idx += kWorkThreads) {
+    const int l = probes[idx];
+    if (l < 0 || list_off[l + 1] <= list_off[l]) continue;
     const int q = idx / P, j = idx - q * P;
-    list_q[list_qoff[l] + pos] = static_cast<int32_t>((static_cast<uint32_t>(q) << 16) | static_cast<uint32_t>(j));
+    list_q[atomicAdd(&cur[l], 1)] =
+        static_cast<int32_t>((static_cast<uint32_t>(q) << 16) | static_cast<uint32_t>(j));
   }
 }
 
@@ -743,7 +788,7 @@ void launch_select_rows(const float* D, int nrows, int ncols, int ldD, int k, in
         D, nrows, ncols, ldD, k, out_idx, out_val, k_row, row_flags, cmins);
     HB_CUDA(cudaGetLastError());
     only = row_flags;
-  } else if (row_flags && k <= 256 && ncols <= 8192 && ncols % 4 == 0 && ldD % 4 == 0) {
+  } else if (row_flags && k <= 256 && ncols <= 8192 && ncols % 4 == 0 && ldD % 4 == 0 && nrows > kCtaRows) {
     // Warp per row; rows it flags go through the CTA kernel below.
     select_rows_warp_kernel<<<(nrows + kSelWarps - 1) / kSelWarps, kSelWarps * 32, 0, st>>>(
         D, nrows, ncols, ldD, k, out_idx, out_val, k_row, row_flags);

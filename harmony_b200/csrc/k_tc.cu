@@ -960,7 +960,7 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
     const __nv_bfloat16* __restrict__ codes,
     const int64_t* __restrict__ list_off, const int64_t* __restrict__ list_qoff, const int32_t* __restrict__ list_q,
     const float* __restrict__ xnorm, const float* __restrict__ rmax, int S, int k, uint32_t* __restrict__ thr,
-    const int32_t* __restrict__ probes, int P) {
+    int* __restrict__ cnt, const int32_t* __restrict__ probes, int P) {
   __shared__ __align__(16) float s_q[kSeedQ][kRerankMaxDim];
   __shared__ int s_qs[kSeedWarps * 32];
   __shared__ int s_nq;
@@ -972,6 +972,12 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
   int l;
   int64_t e0, e1;
   if (by_query) {
+    // The query's bound and candidate count start here (query_prep_kernel's
+    // work, one launch less).
+    if (tid == 0) {
+      thr[blockIdx.x] = ordered_bits(FLT_MAX);
+      cnt[blockIdx.x] = 0;
+    }
     l = probes[static_cast<size_t>(blockIdx.x) * P];
     if (l < 0) return;
     e0 = 0;
@@ -1083,7 +1089,7 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
         }
         // U = the k-th smallest w + eps(q, l): every one of those k rows has
         // an upper bound at most that.
-        if (lane == 0)
+        if (lane == 0)  // (by_query: the same CTA's initial store is ordered before by the barriers above)
           thr[qi] = ordered_bits(
               fminf(__fadd_ru(ordered_to_float(kth), pair_eps(s_cd[wib], rmax[l], dpad)), FLT_MAX));
       }
@@ -1218,12 +1224,6 @@ void launch_scan_bf16(const void* tmap, const TcArgs& a, int num_sms, cudaStream
   HB_CUDA(cudaGetLastError());
 }
 
-void launch_query_prep(int nq, uint32_t* thr, int* cnt, cudaStream_t st) {
-  if (nq <= 0) return;
-  query_prep_kernel<<<(nq + 255) / 256, 256, 0, st>>>(nq, thr, cnt);
-  HB_CUDA(cudaGetLastError());
-}
-
 void launch_residual_bf16(const float* codes, const int64_t* list_off, const float* cent, int nlist, size_t ntotal,
                           int dpad, int kpad, void* dst, float* rnorm, float* rmax, cudaStream_t st) {
   if (nlist <= 0) return;
@@ -1236,19 +1236,26 @@ void launch_residual_bf16(const float* codes, const int64_t* list_off, const flo
   HB_CUDA(cudaGetLastError());
 }
 
-void launch_seed_bound(const float* q, int d, int dpad, const float* cent, int nq, int kpad, const void* codes_bf16,
-                       const int64_t* list_off, int nlist, const int64_t* list_qoff, const int32_t* list_q,
-                       const float* rnorm, const float* rmax, int S, int k, uint32_t* thr, cudaStream_t st,
-                       const int32_t* probes, int P) {
-  if (nq <= 0) return;
+int launch_seed_bound(const float* q, int dpad, const float* cent, int nq, int kpad, const void* codes_bf16,
+                      const int64_t* list_off, int nlist, const int64_t* list_qoff, const int32_t* list_q,
+                      const float* rnorm, const float* rmax, int S, int k, uint32_t* thr, int* cnt, cudaStream_t st,
+                      const int32_t* probes, int P) {
+  if (nq <= 0) return 0;
   HB_CHECK(kpad == 64 || kpad == 128, HB_ERR_INVALID, "the BF16 scan supports d <= 128");
   HB_CHECK(S >= 1 && S <= kSeedRows && k >= 1, HB_ERR_INVALID, "seed sample out of range");
-  if (k > S) return;  // no sample holds k rows: every bound stays FLT_MAX
-  const bool by_query = probes && static_cast<long long>(nq) * 4 < nlist;
+  // A CTA per query sets its query's bound and count up itself; else a
+  // launch before does.
+  const bool by_query = probes && static_cast<long long>(nq) * 4 < nlist && k <= S;
+  if (!by_query) {
+    query_prep_kernel<<<(nq + 255) / 256, 256, 0, st>>>(nq, thr, cnt);
+    HB_CUDA(cudaGetLastError());
+    if (k > S) return 1;  // no sample holds k rows: every bound stays FLT_MAX
+  }
   seed_bound_kernel<<<by_query ? nq : nlist, kSeedWarps * 32, 0, st>>>(
       q, dpad, cent, kpad, static_cast<const __nv_bfloat16*>(codes_bf16), list_off, list_qoff, list_q, rnorm, rmax, S, k,
-      thr, by_query ? probes : nullptr, P);
+      thr, cnt, by_query ? probes : nullptr, P);
   HB_CUDA(cudaGetLastError());
+  return by_query ? 1 : 2;
 }
 
 void launch_rerank_bf16(uint64_t* cand, const uint32_t* cand_ub, const int* cnt, int cap, int nq, int k,
