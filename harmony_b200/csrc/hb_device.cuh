@@ -7,6 +7,16 @@
 
 namespace hb {
 
+// Kernels of a search's chain are launched so that the next one's CTAs may be
+// set up while this one drains (programmatic stream serialization; see
+// launch_chain).  Each calls this before it touches global memory: it returns
+// once every kernel before it in the stream has completed and its writes are
+// visible, and lets the next kernel be set up.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 // 16-byte asynchronous global->shared copy; src_valid = false zero-fills.
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool src_valid) {
   unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));

@@ -33,6 +33,27 @@ struct Error : std::runtime_error {
     if (!(cond)) throw ::hb::Error((code), (msg));    \
   } while (0)
 
+#ifdef __CUDACC__
+// Launches a kernel that calls chain_wait() in every thread before it reads or
+// writes global memory: its CTAs may be set up while the kernel before it in
+// the stream drains, which takes about 2 us off each step of a chain of short
+// kernels.
+template <class... P, class... A>
+void launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  HB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+#endif
+
 // Bumped on every device allocation of a DevBuf: CUDA graphs that captured
 // buffer addresses are valid only while it is unchanged.
 inline std::atomic<uint64_t>& devbuf_generation() {

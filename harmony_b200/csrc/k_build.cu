@@ -19,6 +19,7 @@ constexpr int kPadRows = 32;
 template <bool V4>
 __global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ src, const int64_t* __restrict__ idx,
                                                        int64_t n, int ld, int d, int dpad, float* __restrict__ dst) {
+  chain_wait();
   const int c4 = dpad / 4;
   for (int64_t r0 = static_cast<int64_t>(blockIdx.x) * kPadRows; r0 < n; r0 += static_cast<int64_t>(gridDim.x) * kPadRows) {
     const int rows = static_cast<int>(min(static_cast<int64_t>(kPadRows), n - r0));
@@ -193,9 +194,9 @@ void launch_pad_rows(const float* src, const int64_t* idx, size_t n, int ld, int
   if (!n) return;
   const unsigned g = grid_for(n, kPadRows, 148u * 16u);
   if (ld == d && d % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0)
-    pad_rows_kernel<true><<<g, 256, 0, st>>>(src, idx, static_cast<int64_t>(n), ld, d, dpad, dst);
+    launch_chain(pad_rows_kernel<true>, g, 256, 0, st, src, idx, static_cast<int64_t>(n), ld, d, dpad, dst);
   else
-    pad_rows_kernel<false><<<g, 256, 0, st>>>(src, idx, static_cast<int64_t>(n), ld, d, dpad, dst);
+    launch_chain(pad_rows_kernel<false>, g, 256, 0, st, src, idx, static_cast<int64_t>(n), ld, d, dpad, dst);
   HB_CUDA(cudaGetLastError());
 }
 

@@ -111,6 +111,7 @@ template <bool FP8>
 __global__ void __launch_bounds__(kThreads, 1)
     cand_scan_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_x,
                      CandArgs a) {
+  chain_wait();
   extern __shared__ uint8_t smem_raw[];
   __shared__ CandShared sh;
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -350,6 +351,7 @@ __global__ void __launch_bounds__(256) gather_residual_kernel(const float* __res
                                                               const float* __restrict__ cent, int64_t max_rows,
                                                               float* __restrict__ escale, float* __restrict__ ecd,
                                                               float* __restrict__ pcd, void* __restrict__ G) {
+  chain_wait();
   const int lane = threadIdx.x & 31;
   const int l = blockIdx.x;
   const int64_t e1 = min(list_qoff[l + 1], max_rows);
@@ -409,6 +411,7 @@ __global__ void __launch_bounds__(256) gather_residual_kernel(const float* __res
 // probe), in (query, probe rank) order; the exclusive sum gives the starts.
 __global__ void seg_len_kernel(const int32_t* __restrict__ probes, int nqp, const int64_t* __restrict__ list_off,
                                int64_t* __restrict__ len) {
+  chain_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx > nqp) return;
   int64_t n = 0;
@@ -467,6 +470,7 @@ __global__ void __launch_bounds__(kSelectThreads)
                        const float* __restrict__ pcd, const float* __restrict__ rmax, int dpad, int kpad, int fp8,
                        int cap, int64_t* __restrict__ out_rows, int* __restrict__ m_out,
                        int* __restrict__ over_list, int* __restrict__ over_n) {
+  chain_wait();
   extern __shared__ __align__(16) unsigned char smem_sel[];
   uint64_t* s_cand = reinterpret_cast<uint64_t*>(smem_sel);  // cap keys (a power of two >= 2 * pow2(R))
   __shared__ int s_hist[kBins];
@@ -699,6 +703,7 @@ __global__ void __launch_bounds__(kExactThreads)
     cand_exact_kernel(const int64_t* __restrict__ rows, const int* __restrict__ m_in, int R, int k,
                       const float* __restrict__ codes, const float* __restrict__ q, int dpad,
                       const int64_t* __restrict__ ids, float* __restrict__ D, int64_t* __restrict__ I) {
+  chain_wait();
   extern __shared__ __align__(16) unsigned char smem_ex[];
   __shared__ int64_t s_rows[kExactThreads];
   const int qi = blockIdx.x, tid = threadIdx.x;
@@ -776,7 +781,7 @@ void launch_cand_segments(const int32_t* probes, int nq, int P, const int64_t* l
   const size_t cub_pad = (cub_bytes + 255) / 256 * 256;
   HB_CHECK(tmp_bytes >= cub_pad + n * sizeof(int64_t), HB_ERR_INVALID, "segment scratch too small");
   int64_t* len = reinterpret_cast<int64_t*>(static_cast<unsigned char*>(tmp) + cub_pad);
-  seg_len_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(probes, nqp, list_off, len);
+  launch_chain(seg_len_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0, st, probes, nqp, list_off, len);
   HB_CUDA(cudaGetLastError());
   size_t bytes = cub_bytes;
   HB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, bytes, len, seg, static_cast<int64_t>(n), st));
@@ -793,11 +798,11 @@ void launch_cand_scan(const void* tmap_q, const void* tmap_x, const CandArgs& a,
   if (a.fp8) {
     HB_CUDA(cudaFuncSetAttribute(cand_scan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
-    cand_scan_kernel<true><<<num_sms, kThreads, smem, st>>>(*mq, *mx, a);
+    launch_chain(cand_scan_kernel<true>, num_sms, kThreads, smem, st, *mq, *mx, a);
   } else {
     HB_CUDA(cudaFuncSetAttribute(cand_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
-    cand_scan_kernel<false><<<num_sms, kThreads, smem, st>>>(*mq, *mx, a);
+    launch_chain(cand_scan_kernel<false>, num_sms, kThreads, smem, st, *mq, *mx, a);
   }
   HB_CUDA(cudaGetLastError());
 }
@@ -818,8 +823,8 @@ void launch_gather_residual(const float* q, int dpad, int kpad, bool fp8, const 
   // About 16 CTAs per SM over all lists.
   const dim3 g(nlist, static_cast<unsigned>(std::max(1, std::min(64, 148 * 16 / nlist))));
   auto go = [&](auto f, auto ni) {
-    gather_residual_kernel<decltype(f)::value, decltype(ni)::value>
-        <<<g, 256, 0, st>>>(q, dpad, kpad, list_q, list_qoff, P, cent, max_rows, escale, ecd, pcd, G);
+    launch_chain(gather_residual_kernel<decltype(f)::value, decltype(ni)::value>, g, 256, 0, st, q, dpad, kpad,
+                 list_q, list_qoff, P, cent, max_rows, escale, ecd, pcd, G);
   };
   auto width = [&](auto f) {
     if (kpad <= 128) go(f, std::integral_constant<int, 1>{});
@@ -861,7 +866,8 @@ void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* pr
   const size_t smem_sel = static_cast<size_t>(cap) * sizeof(uint64_t);
   auto go = [&](auto kernel) {
     HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_sel)));
-    kernel<<<nq, kSelectThreads, smem_sel, st>>>(cand, seg, probes, P, R, k, list_off, pcd, rmax, dpad, kpad,
+    launch_chain(kernel, nq, kSelectThreads, smem_sel, st, cand, seg, probes, P, R, k, list_off, pcd, rmax, dpad,
+                 kpad,
                                                  fp8 ? 1 : 0, cap, rows, m_out, over_list, over_n);
   };
   if (exact) go(cand_select_kernel<true>);
@@ -878,7 +884,7 @@ void launch_cand_exact(const int64_t* rows, const int* m, int nq, int R, int k, 
                              sizeof(float);
   HB_CUDA(cudaFuncSetAttribute(cand_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem_ex)));
-  cand_exact_kernel<<<nq, kExactThreads, smem_ex, st>>>(rows, m, R, k, codes, q, dpad, ids, D, I);
+  launch_chain(cand_exact_kernel, nq, kExactThreads, smem_ex, st, rows, m, R, k, codes, q, dpad, ids, D, I);
   HB_CUDA(cudaGetLastError());
 }
 

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh.tmem;
+  chain_wait();
 
   if (warp == kCTmaWarp) {
     if (lane == 0) {
@@ -317,6 +318,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
 // and, when norm is given, each row's ||x||^2; a warp per row.
 __global__ void split_rows_kernel(const float* __restrict__ x, int n, int dpad, int kpad,
                                   __nv_bfloat16* __restrict__ out, float* __restrict__ norm) {
+  chain_wait();
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
@@ -346,6 +348,7 @@ __global__ void __launch_bounds__(256) coarse_refine_kernel(const float* __restr
                                                             int Pm, int P, int nlist, const float* __restrict__ cmaxnorm,
                                                             int32_t* __restrict__ probes, float* __restrict__ cdist,
                                                             int* __restrict__ flags, CoarseRows rows) {
+  chain_wait();
   // [warps][pow2(Pm)] keys, then a stage of 32 rows x 64 columns per warp.
   extern __shared__ __align__(16) uint8_t s_ref_raw[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -429,6 +432,7 @@ __global__ void __launch_bounds__(256) coarse_refine_block_kernel(
     const float* __restrict__ q, int nq, int dpad, const float* __restrict__ cent, const int32_t* __restrict__ cand,
     const float* __restrict__ cval, int Pm, int P, int nlist, const float* __restrict__ cmaxnorm,
     int32_t* __restrict__ probes, float* __restrict__ cdist, int* __restrict__ flags, CoarseRows rows) {
+  chain_wait();
   extern __shared__ uint64_t s_blk[];  // pow2(Pm)
   __shared__ float s_qn[8];
   const int qi = blockIdx.x;
@@ -496,6 +500,7 @@ __global__ void __launch_bounds__(256) coarse_fallback_kernel(const float* __res
                                                               int32_t* __restrict__ probes, float* __restrict__ cdist,
                                                               const int32_t* __restrict__ width,
                                                               uint32_t* __restrict__ cmins) {
+  chain_wait();
   extern __shared__ uint64_t s_fb[];
   __shared__ SelectShared sh_sel;
   __shared__ unsigned s_mask;
@@ -553,6 +558,7 @@ __global__ void __launch_bounds__(256) coarse_fallback_kernel(const float* __res
 // already holds the row's width, else width + margin (at most nlist).
 __global__ void coarse_widths_kernel(const int32_t* __restrict__ width, int nq, int wmax, int pre_w, int margin,
                                      int nlist, int32_t* __restrict__ kq) {
+  chain_wait();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nq) return;
   const int w = min(width[r], wmax);
@@ -564,7 +570,7 @@ __global__ void coarse_widths_kernel(const int32_t* __restrict__ width, int nq, 
 void launch_coarse_widths(const int32_t* width, int nq, int wmax, int pre_w, int margin, int nlist, int32_t* kq,
                           cudaStream_t st) {
   if (nq <= 0) return;
-  coarse_widths_kernel<<<(nq + 255) / 256, 256, 0, st>>>(width, nq, wmax, pre_w, margin, nlist, kq);
+  launch_chain(coarse_widths_kernel, (nq + 255) / 256, 256, 0, st, width, nq, wmax, pre_w, margin, nlist, kq);
   HB_CUDA(cudaGetLastError());
 }
 
@@ -576,7 +582,8 @@ void make_centroid_split(const float* cent, int nlist, int dpad, int kpad, void*
   HB_CHECK(kpad == 64 || kpad == 128, HB_ERR_INVALID, "the tensor-core coarse quantizer supports d <= 128");
   if (nlist > 0) {
     const unsigned g = static_cast<unsigned>(std::min<int>((nlist + 7) / 8, 148 * 16));
-    split_rows_kernel<<<g, 256, 0, st>>>(cent, nlist, dpad, kpad, static_cast<__nv_bfloat16*>(out), nullptr);
+    launch_chain(split_rows_kernel, g, 256, 0, st, cent, nlist, dpad, kpad, static_cast<__nv_bfloat16*>(out),
+                 nullptr);
   }
   HB_CUDA(cudaGetLastError());
   make_bf16_tensor_map(tmap_out, out, static_cast<size_t>(nlist), 2 * kpad);
@@ -589,7 +596,7 @@ void launch_coarse_tc(const void* tmap, const float* q, int nq, int dpad, int kp
   HB_CHECK(kpad == 64 || kpad == 128, HB_ERR_INVALID, "the tensor-core coarse quantizer supports d <= 128");
   // Query rows -> [hi | lo] BF16 and ||q||^2, then their tensor map.
   const unsigned g = static_cast<unsigned>(std::min<int>((nq + 7) / 8, 148 * 16));
-  split_rows_kernel<<<g, 256, 0, st>>>(q, nq, dpad, kpad, static_cast<__nv_bfloat16*>(qsplit), qnorm);
+  launch_chain(split_rows_kernel, g, 256, 0, st, q, nq, dpad, kpad, static_cast<__nv_bfloat16*>(qsplit), qnorm);
   HB_CUDA(cudaGetLastError());
   alignas(64) unsigned char tmap_q[128];
   make_bf16_tensor_map(tmap_q, qsplit, static_cast<size_t>(nq), 2 * kpad);
@@ -604,7 +611,7 @@ void launch_coarse_tc(const void* tmap, const float* q, int nq, int dpad, int kp
   const int G = std::max(1, std::min(pairs, num_sms));
   const size_t smem = coarse_tc_smem_bytes(kpad);
   HB_CUDA(cudaFuncSetAttribute(coarse_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  coarse_tc_kernel<<<G, kCThreads, smem, st>>>(*static_cast<const CUtensorMap*>(tmap),
+  launch_chain(coarse_tc_kernel, G, kCThreads, smem, st, *static_cast<const CUtensorMap*>(tmap),
                                                 *reinterpret_cast<const CUtensorMap*>(tmap_q),
                                                 *reinterpret_cast<const CUtensorMap*>(tmap_v), tma_v, qnorm, nq, kpad,
                                                 cnorm, nlist, qt, pairs, V, cmins, err);
@@ -626,7 +633,8 @@ void launch_coarse_refine(const float* q, int nq, int dpad, const float* cent, c
     const size_t smem = static_cast<size_t>(n2) * 8;
     HB_CUDA(cudaFuncSetAttribute(coarse_refine_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
-    coarse_refine_block_kernel<<<nq, 256, smem, st>>>(q, nq, dpad, cent, cand, cval, Pm, P, nlist, cmaxnorm, probes,
+    launch_chain(coarse_refine_block_kernel, nq, 256, smem, st, q, nq, dpad, cent, cand, cval, Pm, P, nlist,
+                 cmaxnorm, probes,
                                                       cdist, flags, rows);
     HB_CUDA(cudaGetLastError());
     return;
@@ -636,7 +644,8 @@ void launch_coarse_refine(const float* q, int nq, int dpad, const float* cent, c
   const int warps = 4;
   const size_t smem = static_cast<size_t>(warps) * (n2 * 8 + stage);
   HB_CUDA(cudaFuncSetAttribute(coarse_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  coarse_refine_kernel<<<(nq + warps - 1) / warps, warps * 32, smem, st>>>(q, nq, dpad, cent, cand, cval, Pm, P, nlist,
+  launch_chain(coarse_refine_kernel, (nq + warps - 1) / warps, warps * 32, smem, st, q, nq, dpad, cent, cand, cval,
+               Pm, P, nlist,
                                                                           cmaxnorm, probes, cdist, flags, rows);
   HB_CUDA(cudaGetLastError());
 }
@@ -647,7 +656,8 @@ void launch_coarse_fallback(const float* q, int nq, int dpad, const float* cent,
   if (nq <= 0) return;
   const size_t smem = static_cast<size_t>(pow2_ceil(P < 2 ? 2 : P)) * 8;
   HB_CUDA(cudaFuncSetAttribute(coarse_fallback_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  coarse_fallback_kernel<<<std::min((nq + 31) / 32, 296), 256, smem, st>>>(q, nq, dpad, cent, nlist, P, flags, V,
+  launch_chain(coarse_fallback_kernel, std::min((nq + 31) / 32, 296), 256, smem, st, q, nq, dpad, cent, nlist, P,
+               flags, V,
                                                                            probes, cdist, width, cmins);
   HB_CUDA(cudaGetLastError());
 }

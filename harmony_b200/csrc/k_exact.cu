@@ -181,6 +181,7 @@ template <int TV, int QT>
 __global__ void __launch_bounds__(kThreads) l2_matrix_kernel(const float* __restrict__ q, int nq,
                                                              const float* __restrict__ rows, int nrows,
                                                              int dpad, float* __restrict__ D, int ldD) {
+  chain_wait();
   constexpr int G = kThreads / TV;
   constexpr int QG = G * QT;
   extern __shared__ __align__(16) float smem[];
@@ -300,6 +301,7 @@ struct ItemShared {
 
 template <int TV, int QT, int MODE>
 __global__ void __launch_bounds__(kThreads, 1) scan_exact_kernel(ScanArgs a, int cap) {
+  chain_wait();
   constexpr int G = kThreads / TV;
   constexpr int QG = G * QT;
   constexpr int MAXSEG = (MODE == SCAN_DIMBLOCK) ? 8 : 4;
@@ -516,6 +518,7 @@ constexpr bool kPackedExact = true;
 
 template <int TV, int QT, bool PK>
 __global__ void __launch_bounds__(kPackThreads, 1) scan_plain_x2_kernel(ScanArgs a, int cap) {
+  chain_wait();
   constexpr int NT = kPackThreads;
   constexpr int G = NT / TV;
   constexpr int QG = G * QT;
@@ -683,7 +686,7 @@ void matrix_launch(const float* q, int nq, const float* rows, int nrows, int dpa
   HB_CUDA(cudaFuncSetAttribute(l2_matrix_kernel<TV, QT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem)));
   dim3 grid((nrows + TV - 1) / TV, (nq + QG - 1) / QG);
-  l2_matrix_kernel<TV, QT><<<grid, kThreads, smem, st>>>(q, nq, rows, nrows, dpad, D, ldD);
+  launch_chain(l2_matrix_kernel<TV, QT>, grid, kThreads, smem, st, q, nq, rows, nrows, dpad, D, ldD);
   HB_CUDA(cudaGetLastError());
 }
 
@@ -802,7 +805,7 @@ template <int TV, int QT, int MODE>
 void scan_launch(const ScanArgs& a, int cap, size_t smem, int num_sms, cudaStream_t st) {
   HB_CUDA(cudaFuncSetAttribute(scan_exact_kernel<TV, QT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem)));
-  scan_exact_kernel<TV, QT, MODE><<<num_sms, kThreads, smem, st>>>(a, cap);
+  launch_chain(scan_exact_kernel<TV, QT, MODE>, num_sms, kThreads, smem, st, a, cap);
   HB_CUDA(cudaGetLastError());
 }
 
@@ -824,7 +827,7 @@ template <int TV, int QT>
 void x2_launch(const ScanArgs& a, int cap, size_t smem, int num_sms, cudaStream_t st) {
   HB_CUDA(cudaFuncSetAttribute(scan_plain_x2_kernel<TV, QT, kPackedExact>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  scan_plain_x2_kernel<TV, QT, kPackedExact><<<num_sms, kPackThreads, smem, st>>>(a, cap);
+  launch_chain(scan_plain_x2_kernel<TV, QT, kPackedExact>, num_sms, kPackThreads, smem, st, a, cap);
   HB_CUDA(cudaGetLastError());
 }
 }  // namespace

@@ -34,6 +34,7 @@ constexpr int kMaxSelect = 8192;  // largest k a single selection returns
 __global__ void __launch_bounds__(kSelThreads) select_rows_kernel(const float* __restrict__ D, int ncols,
                                                                   int ldD, int k, int32_t* __restrict__ out_idx,
                                                                   float* __restrict__ out_val) {
+  chain_wait();
   extern __shared__ uint64_t s_out[];
   __shared__ SelectShared sh;
   const float* row = D + static_cast<size_t>(blockIdx.x) * ldD;
@@ -72,6 +73,7 @@ __global__ void __launch_bounds__(kSelThreads, 6) select_rows_reg_kernel(const f
                                                                       float* __restrict__ out_val,
                                                                       const int32_t* __restrict__ k_row,
                                                                       const int* __restrict__ only) {
+  chain_wait();
   __shared__ int hist[kBins];
   __shared__ uint64_t s_keys[kCandCap];
   __shared__ SelectShared sh;
@@ -232,6 +234,7 @@ constexpr int kWarpCand = 512;
 __global__ void __launch_bounds__(kSelWarps * 32) select_rows_warp_kernel(
     const float* __restrict__ D, int nrows, int ncols, int ldD, int kmax, int32_t* __restrict__ out_idx,
     float* __restrict__ out_val, const int32_t* __restrict__ k_row, int* __restrict__ overflow) {
+  chain_wait();
   __shared__ int s_hist[kSelWarps][kBins];
   __shared__ uint64_t s_cand[kSelWarps][kWarpCand];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -357,6 +360,7 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_rows_chunk_kernel(
     const float* __restrict__ D, int nrows, int ncols, int ldD, int kmax, int32_t* __restrict__ out_idx,
     float* __restrict__ out_val, const int32_t* __restrict__ k_row, int* __restrict__ overflow,
     const uint32_t* __restrict__ cmins) {
+  chain_wait();
   __shared__ uint64_t s_cand[kSelWarps][kWarpCand];
   __shared__ int s_chk[kSelWarps][kChunkMax];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -434,6 +438,7 @@ __global__ void __launch_bounds__(kSelThreads) merge_kernel(const uint64_t* __re
                                                             const int64_t* __restrict__ slot_base, int P, int k,
                                                             const int64_t* __restrict__ ids, float* __restrict__ D,
                                                             int64_t* __restrict__ I) {
+  chain_wait();
   extern __shared__ uint64_t s_out[];
   __shared__ SelectShared sh;
   const int q = blockIdx.x;
@@ -456,6 +461,7 @@ __global__ void __launch_bounds__(kSelThreads) warmup_tops_kernel(const float* _
                                                                   const float* __restrict__ codes,
                                                                   const int64_t* __restrict__ list_off, int dpad,
                                                                   int k, int wl, int wls, float* __restrict__ tops) {
+  chain_wait();
   extern __shared__ __align__(16) unsigned char wsm[];
   __shared__ SelectShared sh;
   __shared__ int64_t sbeg[64];
@@ -526,6 +532,7 @@ __global__ void __launch_bounds__(kSelThreads) warmup_tops_kernel(const float* _
 __global__ void count_probes_kernel(const int32_t* __restrict__ probes, int nqp, int P,
                                     const int64_t* __restrict__ list_off, int chunk_rows,
                                     int32_t* __restrict__ list_cnt, int64_t* __restrict__ slot_cnt) {
+  chain_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= nqp) return;
   const int l = probes[idx];
@@ -609,6 +616,7 @@ __global__ void __launch_bounds__(kWorkThreads) build_work_small_kernel(
     const int32_t* __restrict__ probes, int nqp, int P, const int64_t* __restrict__ list_off, int nlist,
     int chunk_rows, int qgroup, int32_t* __restrict__ list_cnt, int64_t* __restrict__ list_qoff,
     int32_t* __restrict__ list_q, int64_t* __restrict__ item_off, int64_t* __restrict__ slot_base) {
+  chain_wait();
   extern __shared__ int32_t s_work[];  // [nlist] counts, then [nlist] cursors (a list's first entry, then the next)
   __shared__ int64_t s_warp[64];
   __shared__ unsigned long long s_tot[kWorkThreads / 32];
@@ -689,6 +697,7 @@ __global__ void __launch_bounds__(kWorkThreads) list_scan_kernel(const int32_t* 
                                                                  int chunk_rows, int qgroup,
                                                                  int64_t* __restrict__ list_qoff,
                                                                  int64_t* __restrict__ item_off) {
+  chain_wait();
   __shared__ int64_t s_warp[64];
   block_exclusive_scan([&](int l) -> int64_t { return list_cnt[l]; }, nlist, list_qoff, s_warp);
   block_exclusive_scan(
@@ -702,6 +711,7 @@ __global__ void __launch_bounds__(kWorkThreads) list_scan_kernel(const int32_t* 
 __global__ void scatter_probes_kernel(const int32_t* __restrict__ probes, int nqp, int P,
                                       const int64_t* __restrict__ list_off, const int64_t* __restrict__ list_qoff,
                                       int32_t* __restrict__ cursor, int32_t* __restrict__ list_q) {
+  chain_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= nqp) return;
   const int l = probes[idx];
@@ -784,13 +794,13 @@ void launch_select_rows(const float* D, int nrows, int ncols, int ldD, int k, in
     // Chunk minima given and k small against the chunk count (else T would
     // sit near the largest minima): a warp per row reads the chunks that can
     // hold the k smallest; rows it flags go through the CTA kernel below.
-    select_rows_chunk_kernel<<<(nrows + kSelWarps - 1) / kSelWarps, kSelWarps * 32, 0, st>>>(
+    launch_chain(select_rows_chunk_kernel, (nrows + kSelWarps - 1) / kSelWarps, kSelWarps * 32, 0, st, 
         D, nrows, ncols, ldD, k, out_idx, out_val, k_row, row_flags, cmins);
     HB_CUDA(cudaGetLastError());
     only = row_flags;
   } else if (row_flags && k <= 256 && ncols <= 8192 && ncols % 4 == 0 && ldD % 4 == 0 && nrows > kCtaRows) {
     // Warp per row; rows it flags go through the CTA kernel below.
-    select_rows_warp_kernel<<<(nrows + kSelWarps - 1) / kSelWarps, kSelWarps * 32, 0, st>>>(
+    launch_chain(select_rows_warp_kernel, (nrows + kSelWarps - 1) / kSelWarps, kSelWarps * 32, 0, st, 
         D, nrows, ncols, ldD, k, out_idx, out_val, k_row, row_flags);
     HB_CUDA(cudaGetLastError());
     only = row_flags;
@@ -804,20 +814,24 @@ void launch_select_rows(const float* D, int nrows, int ncols, int ldD, int k, in
     // grid strides over the flags instead of a CTA per row.
     const int g = only ? std::min((nrows + 31) / 32, kFlaggedGrid) : nrows;
     if (vpt <= 4)
-      select_rows_reg_kernel<4><<<g, kSelThreads, 0, st>>>(D, nrows, ncols, ldD, k, out_idx, out_val, k_row, only);
+      launch_chain(select_rows_reg_kernel<4>, g, kSelThreads, 0, st, D, nrows, ncols, ldD, k, out_idx, out_val,
+                   k_row, only);
     else if (vpt <= 8)
-      select_rows_reg_kernel<8><<<g, kSelThreads, 0, st>>>(D, nrows, ncols, ldD, k, out_idx, out_val, k_row, only);
+      launch_chain(select_rows_reg_kernel<8>, g, kSelThreads, 0, st, D, nrows, ncols, ldD, k, out_idx, out_val,
+                   k_row, only);
     else if (vpt <= 16)
-      select_rows_reg_kernel<16><<<g, kSelThreads, 0, st>>>(D, nrows, ncols, ldD, k, out_idx, out_val, k_row, only);
+      launch_chain(select_rows_reg_kernel<16>, g, kSelThreads, 0, st, D, nrows, ncols, ldD, k, out_idx, out_val,
+                   k_row, only);
     else
-      select_rows_reg_kernel<32><<<g, kSelThreads, 0, st>>>(D, nrows, ncols, ldD, k, out_idx, out_val, k_row, only);
+      launch_chain(select_rows_reg_kernel<32>, g, kSelThreads, 0, st, D, nrows, ncols, ldD, k, out_idx, out_val,
+                   k_row, only);
     HB_CUDA(cudaGetLastError());
     return;
   }
   const size_t smem = static_cast<size_t>(pow2_ceil(k < 2 ? 2 : k)) * 8;
   HB_CUDA(cudaFuncSetAttribute(select_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem)));
-  select_rows_kernel<<<nrows, kSelThreads, smem, st>>>(D, ncols, ldD, k, out_idx, out_val);
+  launch_chain(select_rows_kernel, nrows, kSelThreads, smem, st, D, ncols, ldD, k, out_idx, out_val);
   HB_CUDA(cudaGetLastError());
 }
 
@@ -858,7 +872,8 @@ int launch_build_work(const int32_t* probes, int nq, int P, const int64_t* list_
     const size_t smem = static_cast<size_t>(2) * nlist * sizeof(int32_t);
     HB_CUDA(cudaFuncSetAttribute(build_work_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
-    build_work_small_kernel<<<1, kWorkThreads, smem, st>>>(probes, nqp, P, list_off, nlist, chunk_rows, qgroup,
+    launch_chain(build_work_small_kernel, 1, kWorkThreads, smem, st, probes, nqp, P, list_off, nlist, chunk_rows,
+                 qgroup,
                                                            list_cnt, list_qoff, list_q, item_off, slot_base);
     HB_CUDA(cudaGetLastError());
     return 1;
@@ -867,11 +882,12 @@ int launch_build_work(const int32_t* probes, int nq, int P, const int64_t* list_
   HB_CUDA(cudaMemsetAsync(list_cursor, 0, sizeof(int32_t) * nlist, st));
   if (slot_base) HB_CUDA(cudaMemsetAsync(slot_cnt + nqp, 0, sizeof(int64_t), st));
   const int tb = 256;
-  count_probes_kernel<<<(nqp + tb - 1) / tb, tb, 0, st>>>(probes, nqp, P, list_off, chunk_rows, list_cnt,
+  launch_chain(count_probes_kernel, (nqp + tb - 1) / tb, tb, 0, st, probes, nqp, P, list_off, chunk_rows, list_cnt,
                                                           slot_base ? slot_cnt : nullptr);
   if (nlist <= kScanListsOneCta) {
     // One CTA scans both per-list counts (a few thousand lists).
-    list_scan_kernel<<<1, kWorkThreads, 0, st>>>(list_cnt, list_off, nlist, chunk_rows, qgroup, list_qoff, item_off);
+    launch_chain(list_scan_kernel, 1, kWorkThreads, 0, st, list_cnt, list_off, nlist, chunk_rows, qgroup, list_qoff,
+                 item_off);
   } else {
     list_items_kernel<<<(nlist + 1 + tb - 1) / tb, tb, 0, st>>>(list_cnt, list_off, nlist, chunk_rows, qgroup, cnt64,
                                                                 items64);
@@ -883,7 +899,8 @@ int launch_build_work(const int32_t* probes, int nq, int P, const int64_t* list_
   // The per-(query, probe) output slots: only the exact scan's partial
   // results use them.
   if (slot_base) exclusive_sum(slot_cnt, slot_base, n2, cub_tmp, cub_bytes, st);
-  scatter_probes_kernel<<<(nqp + tb - 1) / tb, tb, 0, st>>>(probes, nqp, P, list_off, list_qoff, list_cursor,
+  launch_chain(scatter_probes_kernel, (nqp + tb - 1) / tb, tb, 0, st, probes, nqp, P, list_off, list_qoff,
+               list_cursor,
                                                             list_q);
   HB_CUDA(cudaGetLastError());
   return 3;  // count, the per-list sums, scatter (the CUB scans are library kernels)
@@ -895,7 +912,7 @@ void launch_merge(const uint64_t* part, const int64_t* slot_base, int nq, int P,
   HB_CHECK(k <= kMaxSelect, HB_ERR_INVALID, "k above 8192 is not supported");
   const size_t smem = static_cast<size_t>(pow2_ceil(k < 2 ? 2 : k)) * 8;
   HB_CUDA(cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  merge_kernel<<<nq, kSelThreads, smem, st>>>(part, slot_base, P, k, ids, D, I);
+  launch_chain(merge_kernel, nq, kSelThreads, smem, st, part, slot_base, P, k, ids, D, I);
   HB_CUDA(cudaGetLastError());
 }
 
@@ -912,7 +929,8 @@ void launch_warmup_tops(const float* q, int nq, const int32_t* probes, int P, co
                       static_cast<size_t>(k) * 8 + 16;
   HB_CUDA(cudaFuncSetAttribute(warmup_tops_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem)));
-  warmup_tops_kernel<<<nq, kSelThreads, smem, st>>>(q, probes, P, codes, list_off, dpad, k, wl, warm_list_size,
+  launch_chain(warmup_tops_kernel, nq, kSelThreads, smem, st, q, probes, P, codes, list_off, dpad, k, wl,
+               warm_list_size,
                                                     tops);
   HB_CUDA(cudaGetLastError());
 }

@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh.tmem;
+  chain_wait();
   const int64_t total_items = a.item_off[a.nlist];
 
   if (warp == kFetchWarp) {
@@ -686,6 +687,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // Per query, before the scan: the bound U reset to FLT_MAX (none yet; +inf
 // padding rows never pass) and the candidate counter reset.
 __global__ void query_prep_kernel(int nq, uint32_t* __restrict__ thr, int* __restrict__ cnt) {
+  chain_wait();
   const int qi = blockIdx.x * blockDim.x + threadIdx.x;
   if (qi >= nq) return;
   thr[qi] = ordered_bits(FLT_MAX);
@@ -786,6 +788,7 @@ __global__ void __launch_bounds__(kRrThreads) rerank_kernel(
     const float* __restrict__ codes, const float* __restrict__ q, int dpad, const int64_t* __restrict__ ids,
     float* __restrict__ D, int64_t* __restrict__ I, int* __restrict__ over_list, int* __restrict__ over_n,
     int* __restrict__ m_out) {
+  chain_wait();
   extern __shared__ uint64_t s_top[];  // pow2_ceil(k), for queries with more than kRrKeys rows to recompute
   __shared__ uint64_t s_key[kRrKeys];
   __shared__ __align__(16) float s_row[kRrRows * kRrStride];
@@ -911,6 +914,7 @@ constexpr int kKthWarps = 8;
 __global__ void __launch_bounds__(kKthWarps * 32) kth_bound_kernel(const uint32_t* __restrict__ cand_ub,
                                                                   const int* __restrict__ cnt, int cap, int nq, int k,
                                                                   uint32_t* __restrict__ thr) {
+  chain_wait();
   __shared__ int s_h[kKthWarps][256];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int qi = blockIdx.x * kKthWarps + wib;
@@ -926,6 +930,7 @@ __global__ void __launch_bounds__(kKthWarps * 32) kth_bound_kernel(const uint32_
 // rest = the table with that column set to -1.
 __global__ void split_first_probe_kernel(const int32_t* __restrict__ probes, int nq, int P,
                                          int32_t* __restrict__ first, int32_t* __restrict__ rest) {
+  chain_wait();
   const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
   if (i >= static_cast<int64_t>(nq) * P) return;
   const int j = static_cast<int>(i % P);
@@ -961,6 +966,7 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
     const int64_t* __restrict__ list_off, const int64_t* __restrict__ list_qoff, const int32_t* __restrict__ list_q,
     const float* __restrict__ xnorm, const float* __restrict__ rmax, int S, int k, uint32_t* __restrict__ thr,
     int* __restrict__ cnt, const int32_t* __restrict__ probes, int P) {
+  chain_wait();
   __shared__ __align__(16) float s_q[kSeedQ][kRerankMaxDim];
   __shared__ int s_qs[kSeedWarps * 32];
   __shared__ int s_nq;
@@ -1215,11 +1221,11 @@ void launch_scan_bf16(const void* tmap, const TcArgs& a, int num_sms, cudaStream
   if (a.k <= kTightK) {
     HB_CUDA(cudaFuncSetAttribute(scan_bf16_kernel<kTightK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
-    scan_bf16_kernel<kTightK><<<num_sms, kTcThreads, smem, st>>>(*static_cast<const CUtensorMap*>(tmap), a);
+    launch_chain(scan_bf16_kernel<kTightK>, num_sms, kTcThreads, smem, st, *static_cast<const CUtensorMap*>(tmap), a);
   } else {
     HB_CUDA(cudaFuncSetAttribute(scan_bf16_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
-    scan_bf16_kernel<0><<<num_sms, kTcThreads, smem, st>>>(*static_cast<const CUtensorMap*>(tmap), a);
+    launch_chain(scan_bf16_kernel<0>, num_sms, kTcThreads, smem, st, *static_cast<const CUtensorMap*>(tmap), a);
   }
   HB_CUDA(cudaGetLastError());
 }
@@ -1247,11 +1253,11 @@ int launch_seed_bound(const float* q, int dpad, const float* cent, int nq, int k
   // launch before does.
   const bool by_query = probes && static_cast<long long>(nq) * 4 < nlist && k <= S;
   if (!by_query) {
-    query_prep_kernel<<<(nq + 255) / 256, 256, 0, st>>>(nq, thr, cnt);
+    launch_chain(query_prep_kernel, (nq + 255) / 256, 256, 0, st, nq, thr, cnt);
     HB_CUDA(cudaGetLastError());
     if (k > S) return 1;  // no sample holds k rows: every bound stays FLT_MAX
   }
-  seed_bound_kernel<<<by_query ? nq : nlist, kSeedWarps * 32, 0, st>>>(
+  launch_chain(seed_bound_kernel, by_query ? nq : nlist, kSeedWarps * 32, 0, st, 
       q, dpad, cent, kpad, static_cast<const __nv_bfloat16*>(codes_bf16), list_off, list_qoff, list_q, rnorm, rmax, S, k,
       thr, cnt, by_query ? probes : nullptr, P);
   HB_CUDA(cudaGetLastError());
@@ -1267,7 +1273,8 @@ void launch_rerank_bf16(uint64_t* cand, const uint32_t* cand_ub, const int* cnt,
   HB_CHECK(dpad % 4 == 0 && dpad <= kRerankMaxDim, HB_ERR_INVALID, "re-rank rows wider than 128 floats");
   const size_t smem = static_cast<size_t>(pow2_ceil(k < 2 ? 2 : k)) * sizeof(uint64_t);
   auto go = [&](auto kernel, int threads) {
-    kernel<<<nq, threads, smem, st>>>(cand, cand_ub, cnt, cap, k, codes, q, dpad, ids, D, I, over_list, over_n, m_out);
+    launch_chain(kernel, nq, threads, smem, st, cand, cand_ub, cnt, cap, k, codes, q, dpad, ids, D, I, over_list,
+                 over_n, m_out);
   };
   if (k <= kFilterTightK) go(rerank_kernel<64, 16>, 64);
   else go(rerank_kernel<128, 32>, 128);
@@ -1277,14 +1284,16 @@ void launch_rerank_bf16(uint64_t* cand, const uint32_t* cand_ub, const int* cnt,
 void launch_kth_bound(const uint32_t* cand_ub, const int* cnt, int cap, int nq, int k, uint32_t* thr,
                       cudaStream_t st) {
   if (nq <= 0) return;
-  kth_bound_kernel<<<(nq + kKthWarps - 1) / kKthWarps, kKthWarps * 32, 0, st>>>(cand_ub, cnt, cap, nq, k, thr);
+  launch_chain(kth_bound_kernel, (nq + kKthWarps - 1) / kKthWarps, kKthWarps * 32, 0, st, cand_ub, cnt, cap, nq, k,
+               thr);
   HB_CUDA(cudaGetLastError());
 }
 
 void launch_split_first_probe(const int32_t* probes, int nq, int P, int32_t* first, int32_t* rest, cudaStream_t st) {
   const int64_t n = static_cast<int64_t>(nq) * P;
   if (n <= 0) return;
-  split_first_probe_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(probes, nq, P, first, rest);
+  launch_chain(split_first_probe_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0, st, probes, nq, P, first,
+               rest);
   HB_CUDA(cudaGetLastError());
 }
 
