@@ -267,10 +267,10 @@ __device__ uint32_t warp_kth_smallest(Get get, int n, int k, int* h, int lane) {
   return prefix;
 }
 
-// The same by a whole block of NT threads (keys v[0 .. n-1], 1 <= k <= n);
-// every thread returns it.
-template <int NT>
-__device__ uint32_t block_kth_smallest(const uint32_t* __restrict__ v, int n, int k, int* h) {
+// The same by a whole block of NT threads (1 <= k <= n); every thread returns
+// it.
+template <int NT, class Get>
+__device__ uint32_t block_kth_smallest(Get get, int n, int k, int* h) {
   __shared__ uint32_t s_lo, s_hi, s_prefix;
   __shared__ int s_need;
   const int tid = threadIdx.x, lane = tid & 31;
@@ -282,8 +282,9 @@ __device__ uint32_t block_kth_smallest(const uint32_t* __restrict__ v, int n, in
   uint32_t lo = 0xFFFFFFFFu, hi = 0u;
 #pragma unroll 4
   for (int i = tid; i < n; i += NT) {
-    lo = min(lo, v[i]);
-    hi = max(hi, v[i]);
+    const uint32_t x = get(i);
+    lo = min(lo, x);
+    hi = max(hi, x);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -309,7 +310,7 @@ __device__ uint32_t block_kth_smallest(const uint32_t* __restrict__ v, int n, in
     __syncthreads();
 #pragma unroll 4
     for (int i = tid; i < n; i += NT) {
-      const uint32_t x = v[i];
+      const uint32_t x = get(i);
       if ((x & pmask) == prefix) atomicAdd(&h[(x >> shift) & 255u], 1);
     }
     __syncthreads();

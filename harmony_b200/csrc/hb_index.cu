@@ -1982,11 +1982,11 @@ class IndexCore {
   }
 
   // Longest candidate row a query can have at nprobe P: the P largest lists,
-  // each rounded up to 4 entries.
+  // each rounded up to 8 entries.
   int64_t cand_row_bound(int P) {
     int64_t s = 0;
     for (size_t i = 0; i < std::min<size_t>(static_cast<size_t>(P), nlist_); ++i)
-      s += (sizes_desc()[i] + 3) & ~int64_t(3);
+      s += (sizes_desc()[i] + 7) & ~int64_t(7);
     return s;
   }
 
@@ -2040,9 +2040,9 @@ class IndexCore {
   // be among the k nearest is re-ranked (at most R), the queries with more
   // are listed for the exact scan.
   void cand_pipeline(int nb, int P, int k, int R, bool fp8, bool exact, float* Dd, int64_t* Id) {
-    // One 128-row tile per work item: the queries' tile is fetched per row
-    // tile anyway, and small items balance the persistent CTAs.
-    const int cr = 128;
+    // Up to eight row tiles per item: the group's queries stay in shared
+    // memory over them, and items stay short enough to balance the CTAs.
+    const int cr = std::min(1024, std::max(128, chunk_rows_for(nb, P, 128)));
     const size_t nqp = static_cast<size_t>(nb) * P;
     {
       Scope sc(this, "build_work");

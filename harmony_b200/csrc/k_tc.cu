@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(kRrThreads) rerank_kernel(
       if (lane == 0) s_u = u;
     }
   } else {
-    const uint32_t u = block_kth_smallest<kRrThreads>(ubs, c, k, s_h);
+    const uint32_t u = block_kth_smallest<kRrThreads>([&](int i) { return ubs[i]; }, c, k, s_h);
     if (tid == 0) s_u = u;
   }
   __syncthreads();
