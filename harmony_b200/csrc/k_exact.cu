@@ -30,6 +30,7 @@ namespace hb {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kMatrixFew = 8;  // queries up to which a CTA sweeps whole rows for them
 
 // ----------------------------------------------------------------------------
 // Distance micro-kernels.
@@ -205,6 +206,113 @@ __global__ void __launch_bounds__(kThreads) l2_matrix_kernel(const float* __rest
       const int qi = q0 + g * QT + i;
       if (qi < nq) D[static_cast<size_t>(qi) * ldD + r0 + r] = acc[i];
     }
+  }
+}
+
+// The same for more than a few queries: a CTA takes 64 rows x 32 queries, a
+// thread 4 rows x 2 query pairs in packed f32x2 arithmetic, 32 dimensions at a
+// time through double-buffered shared memory (rows by cp.async, queries pair-
+// interleaved by way of registers).  Per four dimensions a thread issues eight
+// 16-byte shared loads for 128 FP32 instructions, so the FP32 pipe is what
+// bounds it; the form above holds whole rows in shared memory (one CTA per SM
+// past 256 dimensions) and reloads a query per row.
+// 5000 x 256 rows of 512 floats 247 -> 147 us, 2000 x 256 105 -> 72, 777 x 4096
+// of 96 57 -> 40.
+constexpr int kMtRows = 64, kMtQ = 32, kMtThreads = 128, kMtChunk = 32;
+constexpr int kMtStride = kMtChunk + 4;
+
+__global__ void __launch_bounds__(kMtThreads) l2_matrix_tile_kernel(const float* __restrict__ q, int nq,
+                                                                    const float* __restrict__ rows, int nrows,
+                                                                    int dpad, float* __restrict__ D, int ldD) {
+  chain_wait();
+  __shared__ __align__(16) float s_r[2][kMtRows * kMtStride];
+  __shared__ __align__(16) float s_q[2][kMtQ * kMtChunk];  // [pair][dimension][2]
+  const int tid = threadIdx.x;
+  const int tr = tid & 15, tq = tid >> 4;  // rows tr + 16 i, query pairs 2 tq and 2 tq + 1
+  const int r0 = blockIdx.x * kMtRows, q0 = blockIdx.y * kMtQ;
+  const int nch = (dpad + kMtChunk - 1) / kMtChunk;
+  auto fetch_rows = [&](int ch, int buf) {
+#pragma unroll
+    for (int u = 0; u < kMtRows * kMtChunk / 4 / kMtThreads; ++u) {
+      const int i = tid + u * kMtThreads;
+      const int r = i / (kMtChunk / 4), c = ch * kMtChunk + 4 * (i % (kMtChunk / 4));
+      const bool ok = r0 + r < nrows && c < dpad;
+      cp_async16(s_r[buf] + r * kMtStride + 4 * (i % (kMtChunk / 4)),
+                 ok ? rows + static_cast<size_t>(r0 + r) * dpad + c : rows, ok);
+    }
+    cp_async_commit();
+  };
+  // Two 16-byte pieces of the queries' chunk per thread.
+  float4 qv[2];
+  auto load_q = [&](int ch) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = tid + u * kMtThreads;
+      const int e = i / (kMtChunk / 4), c = ch * kMtChunk + 4 * (i % (kMtChunk / 4));
+      qv[u] = q0 + e < nq && c < dpad
+                  ? __ldg(reinterpret_cast<const float4*>(q + static_cast<size_t>(q0 + e) * dpad + c))
+                  : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  auto store_q = [&](int buf) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = tid + u * kMtThreads;
+      const int e = i / (kMtChunk / 4), c = 4 * (i % (kMtChunk / 4));
+      float* dst = s_q[buf] + ((e >> 1) * kMtChunk + c) * 2 + (e & 1);
+      dst[0] = qv[u].x;
+      dst[2] = qv[u].y;
+      dst[4] = qv[u].z;
+      dst[6] = qv[u].w;
+    }
+  };
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+  fetch_rows(0, 0);
+  load_q(0);
+  store_q(0);
+  for (int ch = 0; ch < nch; ++ch) {
+    const int buf = ch & 1;
+    cp_async_wait<0>();
+    __syncthreads();  // chunk ch is in; the other buffers' readers are done
+    if (ch + 1 < nch) {
+      fetch_rows(ch + 1, buf ^ 1);
+      load_q(ch + 1);
+    }
+    const float* xr = s_r[buf] + tr * kMtStride;
+    const float* qp = s_q[buf] + 2 * tq * kMtChunk * 2;
+#pragma unroll 2
+    for (int c = 0; c < kMtChunk; c += 4) {
+      float4 x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(xr + 16 * i * kMtStride + c);
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const ulonglong2 qa = *reinterpret_cast<const ulonglong2*>(qp + (p * kMtChunk + c) * 2);
+        const ulonglong2 qb = *reinterpret_cast<const ulonglong2*>(qp + (p * kMtChunk + c) * 2 + 4);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          f2_sq_acc(acc[i][2 * p], acc[i][2 * p + 1], qa.x, f2_pack(x[i].x, x[i].x));
+          f2_sq_acc(acc[i][2 * p], acc[i][2 * p + 1], qa.y, f2_pack(x[i].y, x[i].y));
+          f2_sq_acc(acc[i][2 * p], acc[i][2 * p + 1], qb.x, f2_pack(x[i].z, x[i].z));
+          f2_sq_acc(acc[i][2 * p], acc[i][2 * p + 1], qb.y, f2_pack(x[i].w, x[i].w));
+        }
+      }
+    }
+    if (ch + 1 < nch) store_q(buf ^ 1);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int qi = q0 + 4 * tq + j;
+    if (qi < nq)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + tr + 16 * i;
+        if (r < nrows) D[static_cast<size_t>(qi) * ldD + r] = acc[i][j];
+      }
   }
 }
 
@@ -718,8 +826,14 @@ void launch_l2_matrix(const float* q, int nq, const float* rows, int nrows, int 
                       cudaStream_t st) {
   if (nq <= 0 || nrows <= 0) return;
   HB_CHECK(dpad <= 1024, HB_ERR_INVALID, "dimension above 1024 is not supported");
-  const Shape s = matrix_shape(dpad);
+  if (nq > kMatrixFew) {
+    const dim3 grid((nrows + kMtRows - 1) / kMtRows, (nq + kMtQ - 1) / kMtQ);
+    launch_chain(l2_matrix_tile_kernel, grid, kMtThreads, 0, st, q, nq, rows, nrows, dpad, D, ldD);
+    HB_CUDA(cudaGetLastError());
+    return;
+  }
   // A few queries: no more than that many sums per thread.
+  const Shape s = matrix_shape(dpad);
   if (s.tv == 128 && nq <= 2) matrix_launch<128, 1>(q, nq, rows, nrows, dpad, D, ldD, st);
   else if (s.tv == 128 && nq <= 4) matrix_launch<128, 2>(q, nq, rows, nrows, dpad, D, ldD, st);
   else if (s.tv == 128) matrix_launch<128, 8>(q, nq, rows, nrows, dpad, D, ldD, st);
