@@ -202,6 +202,19 @@ __device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[32]) {
       : "memory");
 }
 
+// Eight columns, and the wait over them.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+               :
+               : "memory");
+}
+
 // Shared-memory matrix descriptor for a K-major operand stored with the
 // 128-byte swizzle in 1024-byte atoms (8 rows x 128 bytes): start address,
 // stride between 8-row groups 1024 bytes, descriptor version 1, layout

@@ -72,16 +72,21 @@
 //   warp 18     item fetcher: takes items from the global work counter and
 //               finds their list and queries two items ahead of the builders.
 // What bounds it: cycle counters in an instrumented copy (10M x 128, 10k
-// queries, nprobe 40, k 10) put the epilogue first (a group is busy 65 % of
-// the time, about 290 cycles per 32-column chunk and 2000 per chunk with an
-// admission, whose code is out of the instruction cache), then the tensor
-// pipe (34 %).  With two builder warps that also fetched the items, builders
-// were busy all the time on short lists, and a loop of one lane over the MMAs
-// took 97 cycles per instruction; splitting the builders' work over four
-// warps and a fetcher, nine shuffles for eight row sums, the converged issue
-// loop and two-column arithmetic took this search from 1404 to 1164 us, a
-// batch of 10k queries on 1M x 128 (nprobe 64, k 100) from 2224 to 1630 us and
-// 777 queries with their own nprobe on 4M x 96 from 804 to 611 us.
+// queries, nprobe 40, k 10) show the epilogue groups busy 60 % of the time and
+// the tensor pipe 36 %; the rest they wait on each other, because a warp with
+// an admission holds its accumulator for another 1000 cycles per eight columns
+// (380 per 32-column chunk without one).  A single warp there runs about five
+// cycles per instruction and thirty per branch, so the admission is branch-free
+// code over eight columns read again from TMEM: with a loop over the set bits
+// of each lane's mask and divergent writes it took 2000 to 7000 cycles per
+// chunk, and this search 640 us, 10k queries on 1M x 128 (nprobe 64, k 100)
+// 600 us and 777 queries with their own nprobe on 4M x 96 283 us; now 605, 385
+// and 273.  (Straight-line code over all 32 columns in registers: 823, 409,
+// 361, and it spilled.)  With two builder warps that also fetched the items,
+// builders were busy all the time on short lists, and a loop of one lane over
+// the MMAs took 97 cycles per instruction: four builder warps, a fetcher, nine
+// shuffles for eight row sums, the converged issue loop and two-column
+// arithmetic took 1404 us to 1164, 2224 to 1630 and 804 to 611 (whole batches).
 // More than 16 warps hold the kernel to 96 registers per thread (five warps
 // on one SM sub-partition); a spill there costs more than the warps give, so
 // the builders keep one batch of rows in flight.
@@ -119,7 +124,7 @@ constexpr int kAcc = 4;                            // TMEM accumulators of 128 c
 constexpr int kNormSlots = 8;                      // tiles whose row norms sit in shared memory
 constexpr size_t kSmemCap = 226 * 1024;            // dynamic shared memory budget
 constexpr int kTightK = kFilterTightK;             // largest k whose bound tightens during the scan
-constexpr int kStage = 8;                          // admitted keys staged per epilogue thread before a flush
+constexpr int kFifo = 192;                         // admitted values an epilogue warp collects (a multiple of 32)
 
 // The error bound of one (query, list) pair (see the top of this file):
 // Q = ||q - c_l|| from its FP32 square cd, R = the list's largest residual
@@ -137,6 +142,12 @@ __device__ __forceinline__ void fma2_m2(uint32_t& a, uint32_t& b, uint64_t n) {
       " mov.b64 {%0, %1}, t;\n}\n"
       : "+r"(a), "+r"(b)
       : "l"(n), "r"(0xC0000000u));
+}
+// (lo, v) to the shared-memory address `to` where v <= bound, without a branch.
+__device__ __forceinline__ void st_if_le(uint32_t to, uint32_t lo, uint32_t v, float bound) {
+  asm volatile("{\n .reg .pred p;\n setp.le.f32 p, %2, %3;\n @p st.shared.v2.b32 [%0], {%1, %4};\n}\n" ::"r"(to),
+               "r"(lo), "f"(__uint_as_float(v)), "f"(bound), "r"(v)
+               : "memory");
 }
 __device__ __forceinline__ float min3(float a, float b, float c) {
   float d;
@@ -228,7 +239,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   float* meta_eps = meta_thr + 2 * kTile;                                   // [2][128] eps(q, l)
   float* meta_cd = meta_eps + 2 * kTile;                                    // [2][128] ||q - c_l||^2
   int* fetch_q = reinterpret_cast<int*>(meta_cd + 2 * kTile);               // [2][128] queries fetched ahead
-  uint64_t* staging = reinterpret_cast<uint64_t*>(fetch_q + 2 * kTile);     // [kGroups][kStage][128]
+  uint64_t* staging = reinterpret_cast<uint64_t*>(fetch_q + 2 * kTile);     // [kGroups * 4][kFifo]
+  uint4* pending = reinterpret_cast<uint4*>(staging + kGroups * 4 * kFifo);  // [kGroups * 4][32]
 
   const int tid = threadIdx.x;
   const int warp = warp_uniform(tid >> 5), lane = tid & 31;
@@ -520,118 +532,138 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const float te = t < FLT_MAX ? __fadd_ru(t, eps) : FLT_MAX;
         return fminf(__fadd_ru(__fsub_ru(te, cd), 1e-6f * (fminf(fabsf(te), 1e30f) + cd)), FLT_MAX);
       };
-      float thr_s = shifted(thr);
+      // Lanes without a query admit nothing (no value is <= NaN).
+      float thr_s = my_q >= 0 ? shifted(thr) : __int_as_float(0x7fffffff);
       // The k smallest upper bounds this thread knows for the query,
       // ascending, in the last k of KT places (the others hold -inf, which no
       // insertion moves), so the k-th is the last place whatever k is (KT = 0:
-      // no tightening).  A published U says that k rows have upper bounds
-      // <= U, so U may stand in for k of them: the k-th of a mix of stand-ins
-      // and real values is the k-th of k distinct rows or U itself.  Only a
-      // value under the current k-th changes the set.
+      // no tightening).  The item's first U says that k rows have upper bounds
+      // <= U, so it stands in for k of them: the k-th of a mix of stand-ins and
+      // real values is the k-th of k distinct rows or U itself.  A U published
+      // later only lowers thr.
       float best[KB];
       const float top0 = thr < FLT_MAX ? thr : INFINITY;
 #pragma unroll
       for (int i = 0; i < KB; ++i) best[i] = i >= KB - a.k ? top0 : -INFINITY;
-      uint64_t* cbuf = a.cand + static_cast<size_t>(my_q < 0 ? 0 : my_q) * a.cap;
-      uint32_t* ubuf = a.cand_ub + static_cast<size_t>(my_q < 0 ? 0 : my_q) * a.cap;
-      // Admitted keys (lower bound, position) wait here (stride kEpiThreads:
-      // conflict-free) in two halves of kHalf.  A full half takes its slots in
-      // the query's buffer with one atomicAdd and is written out only when
-      // the other half fills (or at the item's end), so the atomic's round
-      // trip overlaps the scan instead of stalling the warp once per lane.
-      // Staged entries hold (w, position); every entry of an item shares eps,
-      // so the written key (w - eps rounded down, position) and upper bound
-      // (w + eps rounded up) are formed at write time.
-      constexpr int kHalf = kStage / 2;
-      uint64_t* stg = staging + static_cast<size_t>(grp) * kStage * kEpiThreads + etid;
-      int ns = 0, half = 0, pend_base = 0;
-      bool pend = false;
-      auto write_half = [&](int h, int base, int n) {
-        for (int i = 0; i < n; ++i) {
-          if (base + i < a.cap) {
-            const uint64_t e = stg[(h * kHalf + i) * kEpiThreads];
-            const float wv = ordered_to_float(static_cast<uint32_t>(e >> 32));
-            cbuf[base + i] = (static_cast<uint64_t>(ordered_bits(__fsub_rd(wv, eps))) << 32) | (e & 0xffffffffull);
-            ubuf[base + i] = ordered_bits(__fadd_ru(wv, eps));
+      // Admitted values (w', column and lane) collect in the warp's FIFO in
+      // shared memory; 32 at a time, a lane each, they take a slot in their
+      // query's buffer and are formed (w - eps rounded down, position; w + eps
+      // rounded up).  A lane writes its entry out at the next drain (or after
+      // the item), so the atomics' round trip overlaps the scan.
+      uint64_t* fifo = staging + warp * kFifo;
+      int fill = 0;          // entries in the FIFO, the same in every lane
+      int p_n = 0, p_base;   // entries in flight, the lane's slot
+      const uint32_t row0 = static_cast<uint32_t>(d.row0), lanes_below = (1u << lane) - 1u;
+      uint4* pend = pending + warp * 32 + lane;  // the lane's entry in flight: key, upper bound, query
+      auto write_out = [&]() {
+        if (lane < p_n && p_base < a.cap) {
+          const uint4 e = *pend;
+          const size_t at = static_cast<size_t>(e.w) * a.cap + p_base;
+          a.cand[at] = (static_cast<uint64_t>(e.y) << 32) | e.x;
+          a.cand_ub[at] = e.z;
+        }
+      };
+      // The FIFO's last n <= 32 entries.
+      auto drain = [&](int n) {
+        write_out();
+        const uint64_t e = fifo[fill - n + min(lane, n - 1)];
+        fill -= n;
+        p_n = n;
+        const int src = static_cast<int>(e & 31);
+        const int q = __shfl_sync(0xffffffffu, my_q, src);
+        const float e_eps = __shfl_sync(0xffffffffu, eps, src);
+        const float w = __shfl_sync(0xffffffffu, cd, src) + __uint_as_float(static_cast<uint32_t>(e >> 32));
+        if (lane < n) {
+          *pend = make_uint4(row0 + (static_cast<uint32_t>(e) >> 5), ordered_bits(__fsub_rd(w, e_eps)),
+                             ordered_bits(__fadd_ru(w, e_eps)), static_cast<uint32_t>(q));
+          p_base = atomicAdd(a.cand_cnt + q, 1);
+        }
+      };
+      // Eight columns of the tile, read again from TMEM at a column known only
+      // at run time, so that this code is small and needs no register array:
+      // those at or under the lanes' bounds go to the FIFO (a window of it at a
+      // time, should they not fit) and tighten the bounds.
+      auto admit = [&](uint32_t tcol, const float* nb, uint32_t col, uint32_t row_t) {
+        uint32_t v[8];
+        tmem_ld8(tcol + col, v);
+        const ulonglong2* n2 = reinterpret_cast<const ulonglong2*>(nb + col);
+        const ulonglong2 na = n2[0], nc = n2[1];
+        tmem_ld_wait(v);
+        fma2_m2(v[0], v[1], na.x);
+        fma2_m2(v[2], v[3], na.y);
+        fma2_m2(v[4], v[5], nc.x);
+        fma2_m2(v[6], v[7], nc.y);
+        int cnt = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cnt += __uint_as_float(v[j]) <= thr_s ? 1 : 0;
+        // Places by ballots over the bits of the lanes' counts.
+        const uint32_t b0 = __ballot_sync(0xffffffffu, (cnt & 1) != 0);
+        int at = fill + __popc(b0 & lanes_below), n_all = fill + __popc(b0);
+        if (__any_sync(0xffffffffu, cnt > 1)) {
+#pragma unroll
+          for (int u = 1; u < 4; ++u) {
+            const uint32_t bu = __ballot_sync(0xffffffffu, ((cnt >> u) & 1) != 0);
+            at += __popc(bu & lanes_below) << u;
+            n_all += __popc(bu) << u;
           }
         }
-      };
-      auto stage = [&](uint64_t key) {
-        stg[(half * kHalf + ns) * kEpiThreads] = key;
-        if (++ns == kHalf) {
-          if (pend) write_half(half ^ 1, pend_base, kHalf);
-          pend_base = atomicAdd(a.cand_cnt + my_q, kHalf);
-          pend = true;
-          half ^= 1;
-          ns = 0;
-        }
-      };
-      auto flush = [&]() {
-        if (pend) write_half(half ^ 1, pend_base, kHalf);
-        if (ns > 0) write_half(half, atomicAdd(a.cand_cnt + my_q, ns), ns);
-        pend = false;
-        ns = 0;
-      };
-      // Admission of one column value under the bound.
-      auto admit = [&](float wv, uint32_t pos) {
-        stage((static_cast<uint64_t>(ordered_bits(wv)) << 32) | pos);
-        const float ub = __fadd_ru(wv, eps);
-        if (KT > 0 && ub < best[KB - 1]) {
-          float v = ub;
+        const uint32_t low = ((row_t + col) << 5) | lane;
+        if (n_all <= kFifo) {
+          uint32_t to = smem_u32(fifo + at);
 #pragma unroll
-          for (int i = 0; i < KB; ++i) {
-            const float o = best[i];
-            best[i] = fminf(o, v);
-            v = fmaxf(o, v);
+          for (int j = 0; j < 8; ++j) {
+            st_if_le(to, low + 32u * j, v[j], thr_s);
+            to += __uint_as_float(v[j]) <= thr_s ? 8u : 0u;
           }
-          if (best[KB - 1] < thr) {
-            thr = best[KB - 1];
-            thr_s = shifted(thr);
-            atomicMin(a.thr + my_q, ordered_bits(thr));  // shared at once (no return value used)
+          __syncwarp();
+        } else {
+#pragma unroll 1
+          for (;;) {
+            int i = at;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              if (__uint_as_float(v[j]) <= thr_s) {
+                if (static_cast<unsigned>(i) < static_cast<unsigned>(kFifo))
+                  fifo[i] = (static_cast<uint64_t>(v[j]) << 32) | (low + 32u * j);
+                ++i;
+              }
+            __syncwarp();
+            if (n_all <= kFifo) break;
+            fill = kFifo;
+            while (fill > 0) drain(32);
+            __syncwarp();
+            n_all -= kFifo;
+            at -= kFifo;
           }
         }
-      };
-      // One 32-column chunk of the accumulator in r: w' = ||r||^2 - 2 q'.r
-      // (rows past the list carry an infinite norm) two columns per
-      // instruction, their minimum (three-input minima) against the bound, and
-      // the admission of the columns under it.
-      auto chunk = [&](uint32_t(&r)[32], const float* nb, uint32_t pos0) {
-        const ulonglong2* n2 = reinterpret_cast<const ulonglong2*>(nb);
-        float mn = INFINITY;
+        fill = n_all;
+        if (KT > 0) {
+          // The lane's values in the window, into the k smallest (each place
+          // from its old value and its neighbour's: no chain of 16; +inf moves
+          // nothing).
+          for (int i = 0; __any_sync(0xffffffffu, i < cnt); ++i) {
+            const bool on = i < cnt && at + i >= 0;
+            const uint32_t x = static_cast<uint32_t>(fifo[on ? at + i : 0] >> 32);
+            const float ub = on ? __fadd_ru(cd + __uint_as_float(x), eps) : INFINITY;
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          uint32_t* v = r + 4 * g;
-          const ulonglong2 nv = n2[g];
-          fma2_m2(v[0], v[1], nv.x);
-          fma2_m2(v[2], v[3], nv.y);
-          mn = min3(mn, __uint_as_float(v[0]), __uint_as_float(v[1]));
-          mn = min3(mn, __uint_as_float(v[2]), __uint_as_float(v[3]));
-        }
-        if (my_q >= 0 && mn <= thr_s) {
-          uint32_t mq[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-          for (int j = 0; j < 32; ++j) mq[j & 3] |= (__uint_as_float(r[j]) <= thr_s ? 1u : 0u) << j;
-          uint32_t mask = (mq[0] | mq[1]) | (mq[2] | mq[3]);
-          while (mask) {
-            const int j = __ffs(mask) - 1;
-            mask &= mask - 1;
-            // r[j] by a 5-level select tree (no register indexing).
-            uint32_t t16[16], t8[8], t4[4], t2[2];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) t16[i] = (j & 1) ? r[2 * i + 1] : r[2 * i];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) t8[i] = (j & 2) ? t16[2 * i + 1] : t16[2 * i];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) t4[i] = (j & 4) ? t8[2 * i + 1] : t8[2 * i];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) t2[i] = (j & 8) ? t4[2 * i + 1] : t4[2 * i];
-            admit(cd + __uint_as_float((j & 16) ? t2[1] : t2[0]), pos0 + static_cast<uint32_t>(j));
+            for (int u = KB - 1; u > 0; --u) best[u] = fminf(best[u], fmaxf(best[u - 1], ub));
+            best[0] = fminf(best[0], ub);
           }
+          const bool lower = best[KB - 1] < thr;
+          if (__any_sync(0xffffffffu, lower)) {
+            thr = fminf(thr, best[KB - 1]);
+            thr_s = my_q >= 0 ? shifted(thr) : thr_s;
+            if (lower) atomicMin(a.thr + my_q, ordered_bits(thr));  // shared at once (no return value used)
+          }
+          __syncwarp();
+        }
+        if (fill >= 32) {
+          while (fill >= 32) drain(32);
+          __syncwarp();
         }
       };
-      // The query's bound as other threads have lowered it, read one tile
-      // ahead (the load is in flight while a tile is processed).
-      uint32_t g_thr = my_q >= 0 ? *reinterpret_cast<volatile uint32_t*>(a.thr + my_q) : 0u;
+      const volatile uint32_t* g_src = a.thr + (my_q >= 0 ? my_q : 0);
+      uint32_t g_thr = ordered_bits(thr);
       constexpr uint32_t kG = kGroups;
       for (int t = static_cast<int>((static_cast<uint32_t>(grp) + kG - G % kG) % kG); t < d.ntiles; t += kGroups) {
         const uint32_t gt = G + static_cast<uint32_t>(t);  // the CTA's global tile index
@@ -642,34 +674,59 @@ __global__ void __launch_bounds__(kTcThreads, 1)
              mbar_wait(&sh.normf[nslot], (gt / kNormSlots) & 1u, err, 15, budget);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
-        if (my_q >= 0 && ordered_to_float(g_thr) < thr) {
-          thr = ordered_to_float(g_thr);
-          thr_s = shifted(thr);
-          if (KT > 0) {
-#pragma unroll
-            for (int i = 0; i < KB; ++i) best[i] = fminf(best[i], thr);
-          }
+        if (KT > 0) {
+          // The query's bound as other threads have lowered it, read one tile
+          // ahead (the load is in flight while a tile is processed).
+          thr = fminf(thr, ordered_to_float(g_thr));
+          thr_s = my_q >= 0 ? shifted(thr) : thr_s;
+          g_thr = *g_src;
         }
-        g_thr = my_q >= 0 ? *reinterpret_cast<volatile uint32_t*>(a.thr + my_q) : 0u;
         if (ok && warp_on) {
+          // Each 32-column chunk: w' = ||r||^2 - 2 q'.r (rows past the list
+          // carry an infinite norm) two columns per instruction, and for each
+          // eight columns whether their minimum (three-input minima) is at or
+          // under the bound.  The admission follows once per tile.
           const float* nb = nrm + nslot * kTile;
           const uint32_t col = tmem + lane_base + static_cast<uint32_t>(b * kTile);
-          const uint32_t pos_t = static_cast<uint32_t>(d.row0 + t * kTile);
-          // One register set (a second one, to load the next chunk while this
-          // one is processed, measured slower: it held the kernel to two
-          // epilogue warpgroups within the register file).
-          uint32_t ra[32];
+          uint32_t hit = 0u;  // bit 4 (3 - chunk) + eighth
 #pragma unroll 1
           for (int c = 0; c < kTile / 32; ++c) {
-            tmem_ld32(col + static_cast<uint32_t>(32 * c), ra);
-            tmem_ld_wait(ra);
-            chunk(ra, nb + 32 * c, pos_t + static_cast<uint32_t>(32 * c));
+            // One register set (a second one, to load the next chunk while this
+            // one is processed, measured slower: it held the kernel to two
+            // epilogue warpgroups within the register file).
+            uint32_t r[32];
+            tmem_ld32(col + static_cast<uint32_t>(32 * c), r);
+            tmem_ld_wait(r);
+            const ulonglong2* n2 = reinterpret_cast<const ulonglong2*>(nb + 32 * c);
+            hit <<= 4;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              uint32_t* v = r + 8 * g;
+              const ulonglong2 na = n2[2 * g], nc = n2[2 * g + 1];
+              fma2_m2(v[0], v[1], na.x);
+              fma2_m2(v[2], v[3], na.y);
+              fma2_m2(v[4], v[5], nc.x);
+              fma2_m2(v[6], v[7], nc.y);
+              float mn = min3(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]));
+              mn = min3(mn, __uint_as_float(v[3]), __uint_as_float(v[4]));
+              mn = min3(mn, __uint_as_float(v[5]), __uint_as_float(v[6]));
+              hit |= fminf(mn, __uint_as_float(v[7])) <= thr_s ? 1u << g : 0u;
+            }
+          }
+          uint32_t hits = __reduce_or_sync(0xffffffffu, hit);
+          const uint32_t row_t = static_cast<uint32_t>(t * kTile);
+          while (hits) {
+            const uint32_t g = 31 - __clz(hits);
+            hits ^= 1u << g;
+            const uint32_t c8 = 32 * (3 - (g >> 2)) + 8 * (g & 3);
+            admit(col, nb, c8, row_t);
           }
         }
         tc_fence_before();
         mbar_arrive(&sh.acce[b]);
       }
-      if (my_q >= 0) flush();
+      if (fill > 0) drain(fill);
+      write_out();
       if (!ok) break;
       G += static_cast<uint32_t>(d.ntiles);
     }
@@ -1168,7 +1225,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 size_t scan_bf16_smem_bytes(int kpad, int stages) {
   const size_t tile = static_cast<size_t>(kpad / 64) * kTile * 128;
   return 1024 + tile * (2 + stages) + static_cast<size_t>(kNormSlots) * kTile * 4 + 2 * kTile * (4 + 4 + 4 + 4 + 4) +
-         static_cast<size_t>(kGroups) * kStage * kEpiThreads * 8;
+         static_cast<size_t>(kGroups) * 4 * (kFifo * 8 + 32 * 16);
 }
 
 int scan_bf16_stages(int kpad) {
