@@ -1408,7 +1408,6 @@ class IndexCore {
     float* dmat = reinterpret_cast<float*>(carve(nq * nlist_ * sizeof(float)));
     int32_t* probes = reinterpret_cast<int32_t*>(carve(nq * P * sizeof(int32_t)));
     int32_t* list_cnt = reinterpret_cast<int32_t*>(carve(nlist_ * sizeof(int32_t)));
-    int32_t* cursor = reinterpret_cast<int32_t*>(carve(nlist_ * sizeof(int32_t)));
     int64_t* list_qoff = reinterpret_cast<int64_t*>(carve((nlist_ + 1) * sizeof(int64_t)));
     int64_t* item_off = reinterpret_cast<int64_t*>(carve((nlist_ + 1) * sizeof(int64_t)));
     int32_t* list_q = reinterpret_cast<int32_t*>(carve(nq * P * sizeof(int32_t)));
@@ -1430,7 +1429,7 @@ class IndexCore {
                      static_cast<int>(nlist_), st_);
     launch_select_rows(dmat, nb, static_cast<int>(nlist_), static_cast<int>(nlist_), P, probes, nullptr, st_);
     const int nbw = launch_build_work(probes, nb, P, list_off_.p, static_cast<int>(nlist_), cr, qg, list_cnt, list_qoff,
-                                      cursor, list_q, item_off, slot_base, work_tmp, wtmp, st_);
+                                      list_q, item_off, slot_base, work_tmp, wtmp, st_);
     HB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned int), st_));
     ScanArgs a{};
     a.codes = codes_.p;
@@ -1674,7 +1673,6 @@ class IndexCore {
     HB_CHECK(smem > 0, HB_ERR_INVALID, "k too large for the fused scan at this dimension");
     const int cr = chunk_rows_for(nb, P, tv);
     list_cnt_.reserve(nlist_);
-    list_cursor_.reserve(nlist_);
     list_qoff_.reserve(nlist_ + 1);
     item_off_.reserve(nlist_ + 1);
     list_q_.reserve(static_cast<size_t>(nb) * P);
@@ -1684,7 +1682,7 @@ class IndexCore {
     {
       Scope sc(this, "build_work");
       launches_ += launch_build_work(probes, nb, P, list_off_.p, static_cast<int>(nlist_), cr, qg, list_cnt_.p,
-                                     list_qoff_.p, list_cursor_.p, list_q_.p, item_off_.p, slot_base_.p, work_tmp_.p,
+                                     list_qoff_.p, list_q_.p, item_off_.p, slot_base_.p, work_tmp_.p,
                                      wtmp, st_);
     }
     part_.reserve(max_slots(nb, P, cr) * static_cast<size_t>(k));
@@ -1768,7 +1766,6 @@ class IndexCore {
   void filter_pipeline(int nb, int P, int k, int cap, int cr, int stages, int* cnt, int* rr_m, long long budget,
                        float* Dd, int64_t* Id) {
     list_cnt_.reserve(nlist_);
-    list_cursor_.reserve(nlist_);
     list_qoff_.reserve(nlist_ + 1);
     item_off_.reserve(nlist_ + 1);
     list_q_.reserve(static_cast<size_t>(nb) * P);
@@ -1795,7 +1792,7 @@ class IndexCore {
     {
       Scope sc(this, "build_work");
       launches_ += launch_build_work(probes_a, nb, P_a, list_off_.p, static_cast<int>(nlist_), cr_a, 128, list_cnt_.p,
-                                     list_qoff_.p, list_cursor_.p, list_q_.p, item_off_.p, nullptr, work_tmp_.p, wtmp,
+                                     list_qoff_.p, list_q_.p, item_off_.p, nullptr, work_tmp_.p, wtmp,
                                      st_);
     }
     {
@@ -1842,7 +1839,7 @@ class IndexCore {
       {
         Scope sc(this, "build_work");
         launches_ += launch_build_work(probes_rest_.p, nb, P, list_off_.p, static_cast<int>(nlist_), cr, 128,
-                                       list_cnt_.p, list_qoff_.p, list_cursor_.p, list_q_.p, item_off_.p, nullptr,
+                                       list_cnt_.p, list_qoff_.p, list_q_.p, item_off_.p, nullptr,
                                        work_tmp_.p, wtmp, st_);
       }
       a.work_counter = counter(1);
@@ -2016,7 +2013,6 @@ class IndexCore {
   void cand_reserve(int nb, int P, int R, bool fp8) {
     const size_t nqp = static_cast<size_t>(nb) * P;
     list_cnt_.reserve(nlist_);
-    list_cursor_.reserve(nlist_);
     list_qoff_.reserve(nlist_ + 1);
     item_off_.reserve(nlist_ + 1);
     list_q_.reserve(nqp);
@@ -2047,7 +2043,7 @@ class IndexCore {
     {
       Scope sc(this, "build_work");
       launches_ += launch_build_work(probes_.p, nb, P, list_off_.p, static_cast<int>(nlist_), cr, 128, list_cnt_.p,
-                                     list_qoff_.p, list_cursor_.p, list_q_.p, item_off_.p, nullptr, work_tmp_.p,
+                                     list_qoff_.p, list_q_.p, item_off_.p, nullptr, work_tmp_.p,
                                      work_tmp_.n, st_);
     }
     {
@@ -2534,7 +2530,7 @@ class IndexCore {
   DevBuf<unsigned char> out_;  // a batch's ids and distances on their way to the host
   DevBuf<float> qpad_, qtmp_, dmat_, tops_;
   DevBuf<int64_t> list_qoff_, item_off_, slot_base_;
-  DevBuf<int32_t> probes_, list_cnt_, list_cursor_, list_q_, order_dev_;
+  DevBuf<int32_t> probes_, list_cnt_, list_q_, order_dev_;
   DevBuf<uint64_t> part_;
   DevBuf<unsigned char> work_tmp_;
 };

@@ -193,7 +193,7 @@ void launch_select_rows(const float* D, int nrows, int ncols, int ldD, int k, in
 // launched.
 int launch_build_work(const int32_t* probes, int nq, int P, const int64_t* list_off, int nlist,
                        int chunk_rows, int qgroup, int32_t* list_cnt, int64_t* list_qoff,
-                       int32_t* list_cursor, int32_t* list_q, int64_t* item_off, int64_t* slot_base,
+                       int32_t* list_q, int64_t* item_off, int64_t* slot_base,
                        void* scan_tmp, size_t scan_tmp_bytes, cudaStream_t st);
 size_t build_work_tmp_bytes(int nq, int P, int nlist);
 // The reference master's heap merge of nparts result rows per query

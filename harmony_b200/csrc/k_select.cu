@@ -529,22 +529,58 @@ __global__ void __launch_bounds__(kSelThreads) warmup_tops_kernel(const float* _
 // ---------------------------------------------------------------------------
 // Work description.
 
-__global__ void count_probes_kernel(const int32_t* __restrict__ probes, int nqp, int P,
-                                    const int64_t* __restrict__ list_off, int chunk_rows,
-                                    int32_t* __restrict__ list_cnt, int64_t* __restrict__ slot_cnt) {
+// Queries per list, and each (query, probe) pair's place among its list's, so
+// that scatter_probes_kernel needs no second pass of atomics.  Bound by the
+// atomics on the few lists' counters: a CTA first counts its kCountPairs pairs
+// in shared memory and takes its share of every list with one global atomic
+// (AGG, while the lists are not many more than those pairs; past that a global
+// atomic per pair).  The whole description of 640k pairs over 1024
+// lists took 140 us with an atomic per pair in both kernels, 44 now; 160k over
+// 512 62 -> 17, 400k over 4096 46 -> 30.
+constexpr int kCountThreads = 512;
+constexpr int kCountEach = 8;  // pairs per thread
+constexpr int kCountPairs = kCountThreads * kCountEach;
+
+template <bool AGG>
+__global__ void __launch_bounds__(kCountThreads) count_probes_kernel(const int32_t* __restrict__ probes, int nqp,
+                                                                     int nlist,
+                                                                     const int64_t* __restrict__ list_off,
+                                                                     int chunk_rows, int32_t* __restrict__ list_cnt,
+                                                                     int32_t* __restrict__ rank,
+                                                                     int64_t* __restrict__ slot_cnt) {
   chain_wait();
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= nqp) return;
-  const int l = probes[idx];
-  int64_t nch = 0;
-  if (l >= 0) {
-    const int64_t n = list_off[l + 1] - list_off[l];
-    if (n > 0) {
-      nch = (n + chunk_rows - 1) / chunk_rows;
-      atomicAdd(&list_cnt[l], 1);
-    }
+  extern __shared__ int32_t s_cnt[];  // [nlist] (AGG)
+  const int tid = threadIdx.x;
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kCountPairs;
+  if (AGG) {
+    for (int l = tid; l < nlist; l += kCountThreads) s_cnt[l] = 0;
+    __syncthreads();
   }
-  if (slot_cnt) slot_cnt[idx] = nch;
+  int l[kCountEach], r[kCountEach];
+#pragma unroll
+  for (int u = 0; u < kCountEach; ++u) {
+    const int64_t idx = base + u * kCountThreads + tid;
+    l[u] = idx < nqp ? probes[idx] : -1;
+  }
+#pragma unroll
+  for (int u = 0; u < kCountEach; ++u) {
+    const int64_t idx = base + u * kCountThreads + tid;
+    const int64_t n = l[u] >= 0 ? list_off[l[u] + 1] - list_off[l[u]] : 0;
+    if (slot_cnt && idx < nqp) slot_cnt[idx] = (n + chunk_rows - 1) / chunk_rows;
+    if (n <= 0) l[u] = -1;
+    if (l[u] >= 0) r[u] = atomicAdd(AGG ? &s_cnt[l[u]] : &list_cnt[l[u]], 1);
+  }
+  if (AGG) {
+    __syncthreads();
+    for (int i = tid; i < nlist; i += kCountThreads) {
+      const int c = s_cnt[i];
+      if (c) s_cnt[i] = atomicAdd(&list_cnt[i], c);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < kCountEach; ++u)
+    if (l[u] >= 0) rank[base + u * kCountThreads + tid] = r[u] + (AGG ? s_cnt[l[u]] : 0);
 }
 
 __global__ void list_items_kernel(const int32_t* __restrict__ list_cnt, const int64_t* __restrict__ list_off,
@@ -691,34 +727,76 @@ __global__ void __launch_bounds__(kWorkThreads) build_work_small_kernel(
 }
 
 // Per list: queries (list_cnt) and work items (chunks x query groups), and
-// their exclusive sums list_qoff and item_off (nlist + 1 each), by one CTA.
+// their exclusive sums list_qoff and item_off (nlist + 1 each), by one CTA, a
+// list per thread and 1024 lists at a time (32-bit divisions: list lengths fit,
+// the builders hold to fewer than 2^32 rows in all).
 __global__ void __launch_bounds__(kWorkThreads) list_scan_kernel(const int32_t* __restrict__ list_cnt,
                                                                  const int64_t* __restrict__ list_off, int nlist,
                                                                  int chunk_rows, int qgroup,
                                                                  int64_t* __restrict__ list_qoff,
                                                                  int64_t* __restrict__ item_off) {
   chain_wait();
-  __shared__ int64_t s_warp[64];
-  block_exclusive_scan([&](int l) -> int64_t { return list_cnt[l]; }, nlist, list_qoff, s_warp);
-  block_exclusive_scan(
-      [&](int l) -> int64_t {
-        const int64_t n = list_off[l + 1] - list_off[l];
-        return ((n + chunk_rows - 1) / chunk_rows) * ((list_cnt[l] + qgroup - 1) / qgroup);
-      },
-      nlist, item_off, s_warp);
+  __shared__ long long s_c[kWorkThreads / 32], s_i[kWorkThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  long long run_c = 0, run_i = 0;
+  for (int l0 = 0; l0 < nlist; l0 += kWorkThreads) {
+    const int l = l0 + tid;
+    const uint32_t c = l < nlist ? static_cast<uint32_t>(list_cnt[l]) : 0u;
+    long long it = 0;
+    if (c) {
+      const uint32_t n = static_cast<uint32_t>(list_off[l + 1] - list_off[l]), cr = static_cast<uint32_t>(chunk_rows);
+      const uint32_t qg = static_cast<uint32_t>(qgroup);
+      it = static_cast<long long>(n / cr + (n % cr ? 1u : 0u)) * (c / qg + (c % qg ? 1u : 0u));
+    }
+    long long ic = c, ii = it;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long xc = __shfl_up_sync(0xffffffffu, ic, o), xi = __shfl_up_sync(0xffffffffu, ii, o);
+      if (lane >= o) {
+        ic += xc;
+        ii += xi;
+      }
+    }
+    if (lane == 31) {
+      s_c[wid] = ic;
+      s_i[wid] = ii;
+    }
+    __syncthreads();
+    long long tc = s_c[lane], ti = s_i[lane];  // kWorkThreads / 32 = 32 warps
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long xc = __shfl_up_sync(0xffffffffu, tc, o), xi = __shfl_up_sync(0xffffffffu, ti, o);
+      if (lane >= o) {
+        tc += xc;
+        ti += xi;
+      }
+    }
+    const int before = wid > 0 ? wid - 1 : 0;
+    const long long bc = __shfl_sync(0xffffffffu, tc, before), bi = __shfl_sync(0xffffffffu, ti, before);
+    if (l < nlist) {
+      list_qoff[l] = run_c + (wid > 0 ? bc : 0) + ic - c;
+      item_off[l] = run_i + (wid > 0 ? bi : 0) + ii - it;
+    }
+    run_c += __shfl_sync(0xffffffffu, tc, 31);
+    run_i += __shfl_sync(0xffffffffu, ti, 31);
+    __syncthreads();  // the sums are reused
+  }
+  if (tid == 0) {
+    list_qoff[nlist] = run_c;
+    item_off[nlist] = run_i;
+  }
 }
 
 __global__ void scatter_probes_kernel(const int32_t* __restrict__ probes, int nqp, int P,
                                       const int64_t* __restrict__ list_off, const int64_t* __restrict__ list_qoff,
-                                      int32_t* __restrict__ cursor, int32_t* __restrict__ list_q) {
+                                      const int32_t* __restrict__ rank, int32_t* __restrict__ list_q) {
   chain_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= nqp) return;
   const int l = probes[idx];
   if (l < 0 || list_off[l + 1] == list_off[l]) return;
-  const int pos = atomicAdd(&cursor[l], 1);
   const int q = idx / P, j = idx - q * P;
-  list_q[list_qoff[l] + pos] = static_cast<int32_t>((static_cast<uint32_t>(q) << 16) | static_cast<uint32_t>(j));
+  list_q[list_qoff[l] + rank[idx]] = static_cast<int32_t>((static_cast<uint32_t>(q) << 16) | static_cast<uint32_t>(j));
 }
 
 // Binary max-heap of (value, id) rows in place, restating the reference's
@@ -852,7 +930,7 @@ size_t build_work_tmp_bytes(int nq, int P, int nlist) {
 }
 
 int launch_build_work(const int32_t* probes, int nq, int P, const int64_t* list_off, int nlist, int chunk_rows,
-                       int qgroup, int32_t* list_cnt, int64_t* list_qoff, int32_t* list_cursor, int32_t* list_q,
+                       int qgroup, int32_t* list_cnt, int64_t* list_qoff, int32_t* list_q,
                        int64_t* item_off, int64_t* slot_base, void* scan_tmp, size_t scan_tmp_bytes,
                        cudaStream_t st) {
   const size_t n1 = static_cast<size_t>(nlist) + 1;
@@ -879,11 +957,19 @@ int launch_build_work(const int32_t* probes, int nq, int P, const int64_t* list_
     return 1;
   }
   HB_CUDA(cudaMemsetAsync(list_cnt, 0, sizeof(int32_t) * nlist, st));
-  HB_CUDA(cudaMemsetAsync(list_cursor, 0, sizeof(int32_t) * nlist, st));
   if (slot_base) HB_CUDA(cudaMemsetAsync(slot_cnt + nqp, 0, sizeof(int64_t), st));
+  // The pairs' places wait in the 8 bytes per pair that are not needed yet
+  // (slot_base is written last) or not at all (slot_cnt without it).
+  int32_t* rank = reinterpret_cast<int32_t*>(slot_base ? slot_base : slot_cnt);
   const int tb = 256;
-  launch_chain(count_probes_kernel, (nqp + tb - 1) / tb, tb, 0, st, probes, nqp, P, list_off, chunk_rows, list_cnt,
-                                                          slot_base ? slot_cnt : nullptr);
+  const int ncta = (nqp + kCountPairs - 1) / kCountPairs;
+  int64_t* slots = slot_base ? slot_cnt : nullptr;
+  if (nlist <= 2 * kCountPairs)
+    launch_chain(count_probes_kernel<true>, ncta, kCountThreads, static_cast<size_t>(nlist) * sizeof(int32_t), st,
+                 probes, nqp, nlist, list_off, chunk_rows, list_cnt, rank, slots);
+  else
+    launch_chain(count_probes_kernel<false>, ncta, kCountThreads, 0, st, probes, nqp, nlist, list_off, chunk_rows,
+                 list_cnt, rank, slots);
   if (nlist <= kScanListsOneCta) {
     // One CTA scans both per-list counts (a few thousand lists).
     launch_chain(list_scan_kernel, 1, kWorkThreads, 0, st, list_cnt, list_off, nlist, chunk_rows, qgroup, list_qoff,
@@ -896,12 +982,11 @@ int launch_build_work(const int32_t* probes, int nq, int P, const int64_t* list_
     exclusive_sum(items64, item_off, n1, cub_tmp, cub_bytes, st);
   }
   HB_CUDA(cudaGetLastError());
+  launch_chain(scatter_probes_kernel, (nqp + tb - 1) / tb, tb, 0, st, probes, nqp, P, list_off, list_qoff, rank,
+               list_q);
   // The per-(query, probe) output slots: only the exact scan's partial
   // results use them.
   if (slot_base) exclusive_sum(slot_cnt, slot_base, n2, cub_tmp, cub_bytes, st);
-  launch_chain(scatter_probes_kernel, (nqp + tb - 1) / tb, tb, 0, st, probes, nqp, P, list_off, list_qoff,
-               list_cursor,
-                                                            list_q);
   HB_CUDA(cudaGetLastError());
   return 3;  // count, the per-list sums, scatter (the CUB scans are library kernels)
 }
