@@ -172,9 +172,7 @@ __device__ __forceinline__ uint32_t warp_kth_small8(uint32_t (&v)[8], int k, int
   cx(1, 2), cx(3, 4), cx(5, 6);
   uint32_t m = 0;
   for (int r = 0; r < k; ++r) {
-    m = v[0];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
+    m = __reduce_min_sync(0xffffffffu, v[0]);
     const unsigned who = __ballot_sync(0xffffffffu, v[0] == m);
     if (lane == __ffs(who) - 1) {
 #pragma unroll

@@ -1002,35 +1002,52 @@ __global__ void split_first_probe_kernel(const int32_t* __restrict__ probes, int
 // of the probe set have upper bounds at most that.  Queries whose nearest
 // list holds fewer than k rows keep FLT_MAX.
 //
-// List-major: one CTA per list; the queries whose nearest list it is (probe
-// rank 0 in the list-major work description) go kSeedQ at a time: warp j
-// forms query j's BF16 residual row in shared memory, thread t streams row t
-// of the list's first S rows from global memory once (16-byte loads) and
-// forms its value for each of those queries (their rows broadcast from
-// shared memory), then a warp per query selects its k-th smallest by radix
-// (four 8-bit passes).  Nothing is staged in shared memory, so several CTAs
-// share an SM and keep their row loads in flight.  Small batches (probes
-// given): one CTA per query.
+// List-major: a CTA per list (and part of its queries: gridDim.y); the queries
+// whose nearest list it is (probe rank 0 in the list-major work description) go
+// kSeedQ at a time: warp j forms query j's BF16 residual row in shared memory,
+// the warps multiply the list's first S rows with them, 32 rows each in two
+// mma.sync tiles read straight from global memory (thread t of a row's four
+// takes 16 bytes of each 32 columns, and of the queries the same 16 bytes: the
+// order of the columns in a sum is free), and a warp per query selects its k-th
+// smallest value.  At these sizes (256 rows, a handful of queries) a list's
+// time is its chain of loads and barriers, so four CTAs share an SM.  10k
+// queries on 1M x 128 with 1024 lists, k 100: 117 us with the sums on the FP32
+// pipe, operands read from shared memory; 87 with the rows of both tiles kept
+// in registers and two CTAs per SM; 52 now.  10M with 4096 lists, k 10 (268 MB
+// of rows): 117, 90, 70; 777 queries on 4M x 96 30 -> 19.  Small batches
+// (probes given): one CTA per query.
 constexpr int kSeedRows = 256;
 constexpr int kSeedWarps = 8;
-constexpr int kSeedQ = 4;  // queries per pass
-static_assert(kSeedWarps * 32 >= kSeedRows, "the seed forms a row per thread");
-static_assert(kSeedQ <= kSeedWarps, "a warp per query of a pass");
+constexpr int kSeedQ = 8;  // queries per pass: the N of an mma, a warp each
+constexpr int kSeedKeyStride = kSeedRows + 4;
+static_assert(kSeedWarps * 32 == kSeedRows && kSeedQ == kSeedWarps, "32 rows and a query per warp");
 
+__device__ __forceinline__ void mma_bf16_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                 uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// KB = kpad / 32.
+template <int KB>
 __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
-    const float* __restrict__ q, int dpad, const float* __restrict__ cent, int kpad,
+    const float* __restrict__ q, int dpad, const float* __restrict__ cent,
     const __nv_bfloat16* __restrict__ codes,
     const int64_t* __restrict__ list_off, const int64_t* __restrict__ list_qoff, const int32_t* __restrict__ list_q,
     const float* __restrict__ xnorm, const float* __restrict__ rmax, int S, int k, uint32_t* __restrict__ thr,
     int* __restrict__ cnt, const int32_t* __restrict__ probes, int P) {
   chain_wait();
-  __shared__ __align__(16) float s_q[kSeedQ][kRerankMaxDim];
+  constexpr int kpad = 32 * KB;
+  constexpr int kQStride = kpad + 32;  // 16-byte reads of eight queries hit distinct banks
+  __shared__ __align__(16) __nv_bfloat16 s_q[kSeedQ * kQStride];
   __shared__ int s_qs[kSeedWarps * 32];
   __shared__ int s_nq;
   __shared__ float s_cd[kSeedQ];
-  __shared__ uint32_t s_keys[kSeedQ][kSeedRows];
+  __shared__ uint32_t s_keys[kSeedQ * kSeedKeyStride];
   __shared__ int s_hist[kSeedQ][256];
-  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5, g = lane >> 2, t = lane & 3;
   const bool by_query = probes != nullptr;
   int l;
   int64_t e0, e1;
@@ -1052,22 +1069,22 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
   }
   const int64_t b = list_off[l];
   const int n = static_cast<int>(min(static_cast<int64_t>(S), list_off[l + 1] - b));
-  if (n < k) return;  // no seed: the bound stays FLT_MAX
-  const bool row_ok = tid < n;
-  if (row_ok) {
+  if (n < k || e0 == e1) return;  // no seed: the bound stays FLT_MAX
+  if (tid < n) {
     // Row tid's fetch from DRAM overlaps the query gathering below.
     const char* rp = reinterpret_cast<const char*>(codes + static_cast<size_t>(b + tid) * kpad);
+#pragma unroll
     for (int o = 0; o < kpad * 2; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(rp + o));
   }
-  const uint4* xrow = reinterpret_cast<const uint4*>(codes + static_cast<size_t>(b + (row_ok ? tid : 0)) * kpad);
-  const float xn = row_ok ? xnorm[b + tid] : 0.0f;
   for (int64_t r0 = e0; r0 < e1; r0 += blockDim.x) {
     if (tid == 0) s_nq = 0;
     __syncthreads();
     if (r0 + tid < e1) {
       const uint32_t ent =
           by_query ? (static_cast<uint32_t>(blockIdx.x) << 16) : static_cast<uint32_t>(list_q[r0 + tid]);
-      if ((ent & 0xffff) == 0) s_qs[atomicAdd(&s_nq, 1)] = static_cast<int>(ent >> 16);
+      // (Parts of a list's queries by query number.)
+      if ((ent & 0xffff) == 0 && (ent >> 16) % gridDim.y == blockIdx.y)
+        s_qs[atomicAdd(&s_nq, 1)] = static_cast<int>(ent >> 16);
     }
     __syncthreads();
     const int nqr = s_nq;  // 0 for a list that is no query's nearest: nothing to do
@@ -1078,77 +1095,64 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
         const float* qrow = q + static_cast<size_t>(qi) * dpad;
         const float* crow = cent + static_cast<size_t>(l) * dpad;
         float cd = 0.0f;
-        float qv[kRerankMaxDim / 32], cv[kRerankMaxDim / 32];
+        float qv[KB], cv[KB];
 #pragma unroll
-        for (int i = 0; i < kRerankMaxDim / 32; ++i) {
+        for (int i = 0; i < KB; ++i) {
           const int c = lane + 32 * i;
           qv[i] = c < dpad ? qrow[c] : 0.0f;
           cv[i] = c < dpad ? crow[c] : 0.0f;
         }
 #pragma unroll
-        for (int i = 0; i < kRerankMaxDim / 32; ++i) {
-          const int c = lane + 32 * i;
-          if (c < kpad) {
-            const float v = qv[i] - cv[i];
-            cd = fmaf(v, v, cd);
-            s_q[wib][c] = __bfloat162float(__float2bfloat16_rn(v));
-          }
+        for (int i = 0; i < KB; ++i) {
+          const float v = qv[i] - cv[i];
+          cd = fmaf(v, v, cd);
+          s_q[wib * kQStride + lane + 32 * i] = __float2bfloat16_rn(v);
         }
         for (int o = 16; o > 0; o >>= 1) cd += __shfl_xor_sync(0xffffffffu, cd, o);
         if (lane == 0) s_cd[wib] = cd;
       }
       __syncthreads();
-      if (row_ok) {
-        // Four partial sums per query (any order is within eps).
-        float d[kSeedQ][4];
+      // (Queries past nb multiply what an earlier pass left, and are not read.)
+#pragma unroll 1
+      for (int i = 0; i < 2; ++i) {
+        // Rows r and r + 8 of a 16-row tile.
+        const int r = 32 * wib + 16 * i + g;
+        const uint4* xa = reinterpret_cast<const uint4*>(codes + static_cast<size_t>(b + (r < n ? r : 0)) * kpad);
+        const uint4* xb = reinterpret_cast<const uint4*>(codes + static_cast<size_t>(b + (r + 8 < n ? r + 8 : 0)) * kpad);
+        uint4 ra[KB], rb[KB];
 #pragma unroll
-        for (int j = 0; j < kSeedQ; ++j) d[j][0] = d[j][1] = d[j][2] = d[j][3] = 0.0f;
-        // 64-byte pieces of the row: four loads in flight, then their values.
-        for (int c0 = 0; c0 < kpad; c0 += 32) {
-          uint4 xq[4];
+        for (int c = 0; c < KB; ++c) {
+          ra[c] = __ldg(xa + 4 * c + t);
+          rb[c] = __ldg(xb + 4 * c + t);
+        }
+        const float na = r < n ? xnorm[b + r] : 0.0f, nc = r + 8 < n ? xnorm[b + r + 8] : 0.0f;
+        float d[4] = {};
 #pragma unroll
-          for (int u = 0; u < 4; ++u) xq[u] = __ldg(xrow + c0 / 8 + u);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int c = c0 + 8 * u;
-            const uint4 xv = xq[u];
-            const float x0 = __uint_as_float(xv.x << 16), x1 = __uint_as_float(xv.x & 0xffff0000u);
-            const float x2 = __uint_as_float(xv.y << 16), x3 = __uint_as_float(xv.y & 0xffff0000u);
-            const float x4 = __uint_as_float(xv.z << 16), x5 = __uint_as_float(xv.z & 0xffff0000u);
-            const float x6 = __uint_as_float(xv.w << 16), x7 = __uint_as_float(xv.w & 0xffff0000u);
-#pragma unroll
-            for (int j = 0; j < kSeedQ; ++j) {
-              if (j < nb) {
-                const float4 qa = *reinterpret_cast<const float4*>(&s_q[j][c]);
-                const float4 qc = *reinterpret_cast<const float4*>(&s_q[j][c + 4]);
-                d[j][0] = fmaf(qa.x, x0, d[j][0]);
-                d[j][1] = fmaf(qa.y, x1, d[j][1]);
-                d[j][2] = fmaf(qa.z, x2, d[j][2]);
-                d[j][3] = fmaf(qa.w, x3, d[j][3]);
-                d[j][0] = fmaf(qc.x, x4, d[j][0]);
-                d[j][1] = fmaf(qc.y, x5, d[j][1]);
-                d[j][2] = fmaf(qc.z, x6, d[j][2]);
-                d[j][3] = fmaf(qc.w, x7, d[j][3]);
-              }
-            }
-          }
+        for (int c = 0; c < KB; ++c) {
+          const uint4 qf = *reinterpret_cast<const uint4*>(s_q + g * kQStride + 32 * c + 8 * t);
+          mma_bf16_16x8x16(d, ra[c].x, rb[c].x, ra[c].y, rb[c].y, qf.x, qf.y);
+          mma_bf16_16x8x16(d, ra[c].z, rb[c].z, ra[c].w, rb[c].w, qf.z, qf.w);
         }
 #pragma unroll
-        for (int j = 0; j < kSeedQ; ++j)
+        for (int u = 0; u < 4; ++u) {  // row r + 8 (u / 2), query 2 t + u % 2
+          const int j = 2 * t + (u & 1);
           if (j < nb)
-            s_keys[j][tid] = ordered_bits(s_cd[j] + fmaf(-2.0f, (d[j][0] + d[j][1]) + (d[j][2] + d[j][3]), xn));
+            s_keys[j * kSeedKeyStride + r + 8 * (u >> 1)] =
+                ordered_bits(s_cd[j] + fmaf(-2.0f, d[u], (u >> 1) ? nc : na));
+        }
       }
       __syncthreads();
       if (wib < nb) {
         const int qi = s_qs[t0 + wib];
+        const uint32_t* keys = s_keys + wib * kSeedKeyStride;
         uint32_t kth;
         if (k <= kSmallKth) {
           uint32_t v[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < n ? s_keys[wib][32 * i + lane] : 0xFFFFFFFFu;
+          for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < n ? keys[32 * i + lane] : 0xFFFFFFFFu;
           kth = warp_kth_small8(v, k, lane);
         } else {
-          kth = warp_kth_smallest([&](int i) { return s_keys[wib][i]; }, n, k, s_hist[wib], lane);
+          kth = warp_kth_smallest([&](int i) { return keys[i]; }, n, k, s_hist[wib], lane);
         }
         // U = the k-th smallest w + eps(q, l): every one of those k rows has
         // an upper bound at most that.
@@ -1314,9 +1318,14 @@ int launch_seed_bound(const float* q, int dpad, const float* cent, int nq, int k
     HB_CUDA(cudaGetLastError());
     if (k > S) return 1;  // no sample holds k rows: every bound stays FLT_MAX
   }
-  launch_chain(seed_bound_kernel, by_query ? nq : nlist, kSeedWarps * 32, 0, st, 
-      q, dpad, cent, kpad, static_cast<const __nv_bfloat16*>(codes_bf16), list_off, list_qoff, list_q, rnorm, rmax, S, k,
-      thr, cnt, by_query ? probes : nullptr, P);
+  // Several CTAs for the lists that many queries are nearest to.
+  const dim3 grid(by_query ? nq : nlist, by_query ? 1 : std::min(8, 1 + nq / (16 * nlist)));
+  auto go = [&](auto kernel) {
+    launch_chain(kernel, grid, kSeedWarps * 32, 0, st, q, dpad, cent, static_cast<const __nv_bfloat16*>(codes_bf16),
+                 list_off, list_qoff, list_q, rnorm, rmax, S, k, thr, cnt, by_query ? probes : nullptr, P);
+  };
+  if (kpad == 128) go(seed_bound_kernel<4>);
+  else go(seed_bound_kernel<2>);
   HB_CUDA(cudaGetLastError());
   return by_query ? 1 : 2;
 }
