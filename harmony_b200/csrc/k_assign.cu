@@ -30,7 +30,9 @@
 // cycle and SM, from L2).  Wider rows stream both operands, 64 columns of
 // each per stage (85 bytes per cycle and SM).  Measured: train on 1M x 128 (20
 // passes over 262,144 points, 1024 centroids) 130 -> 22 ms against the FP32
-// kernel, train on 270k x 500 (131,072 points, 512 centroids) 137 -> 20 ms.
+// kernel, train on 270k x 500 (131,072 points, 512 centroids) 137 -> 20 ms.  The
+// 21 launches of a 1M x 128 build (1024 centroids) took 6.0 ms with one lane
+// looping over the MMAs, 4.0 with the issuing warp converged.
 #include <cudaTypedefs.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -105,7 +107,7 @@ __global__ void __launch_bounds__(kAThreads, 1)
   const int nh = kpad / 64;
   const uint32_t a_bytes = RES ? static_cast<uint32_t>(2 * nh) * kABlk : 0u;
   uint8_t* ring = smem + 2 * a_bytes;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int ptiles = (n + kAT - 1) / kAT;
   const int ctiles = (nlist + kAT - 1) / kAT;
 
@@ -175,38 +177,39 @@ __global__ void __launch_bounds__(kAThreads, 1)
           mbar_wait(&sh.afull[j & 1u], (j >> 1) & 1u, nullptr, 0, 200000000LL);
     }
   } else if (warp == kAMmaWarp) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_bf16_f32(kAT, kAT);
-      const uint32_t abase = smem_u32(smem), rbase = smem_u32(ring);
-      uint32_t it = 0, ia = 0, tile = 0;
-      bool ok = true;
-      auto chain = [&](uint32_t d, uint64_t ad, uint64_t bd, bool first) {
+    // The warp converged, one lane issuing (a loop of one lane over the MMAs
+    // takes about a hundred cycles per instruction).
+    const uint32_t idesc = idesc_bf16_f32(kAT, kAT);
+    const uint32_t tm = static_cast<uint32_t>(warp_uniform(static_cast<int>(tmem)));
+    const uint32_t abase = static_cast<uint32_t>(warp_uniform(static_cast<int>(smem_u32(smem))));
+    const uint32_t rbase = static_cast<uint32_t>(warp_uniform(static_cast<int>(smem_u32(ring))));
+    uint32_t it = 0, ia = 0, tile = 0;
+    bool ok = true;
+    auto chain = [&](uint32_t d, uint64_t ad, uint64_t bd, bool first) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) mma_bf16(d, ad + 2 * kk, bd + 2 * kk, idesc, (first && kk == 0) ? 0u : 1u);
-      };
-      for (int p = blockIdx.x; ok && p < ptiles; p += gridDim.x, ++ia) {
-        const uint32_t ab = ia & 1u;
-        if (RES) {
-          if (!mbar_wait(&sh.afull[ab], (ia >> 1) & 1u, err, 43)) break;
+      for (int kk = 0; kk < 4; ++kk) mma_bf16(d, ad + 2 * kk, bd + 2 * kk, idesc, (first && kk == 0) ? 0u : 1u);
+    };
+    for (int p = blockIdx.x; ok && p < ptiles; p += gridDim.x, ++ia) {
+      const uint32_t ab = ia & 1u;
+      if (RES) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.afull[ab], (ia >> 1) & 1u, err, 43));
+        if (!ok) break;
+        tc_fence_after();
+      }
+      for (int c = 0; c < ctiles; ++c, ++tile) {
+        const uint32_t b = tile % kAAcc;
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.acce[b], ((tile / kAAcc) & 1u) ^ 1u, err, 44));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = tm + b * kAT;
+        const int steps = RES ? 2 * nh : nh;
+        for (int kb = 0; kb < steps; ++kb, ++it) {
+          const uint32_t s = it % ST;
+          ok = __all_sync(0xffffffffu, mbar_wait(&sh.full[s], (it / ST) & 1u, err, 45));
+          if (!ok) break;
           tc_fence_after();
-        }
-        for (int c = 0; c < ctiles; ++c, ++tile) {
-          const uint32_t b = tile % kAAcc;
-          if (!mbar_wait(&sh.acce[b], ((tile / kAAcc) & 1u) ^ 1u, err, 44)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t d = tmem + b * kAT;
-          const int steps = RES ? 2 * nh : nh;
-          for (int kb = 0; kb < steps; ++kb, ++it) {
-            const uint32_t s = it % ST;
-            if (!mbar_wait(&sh.full[s], (it / ST) & 1u, err, 45)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t sb = rbase + s * kStageBytes;
+          const uint32_t sb = rbase + s * kStageBytes;
+          if (elect_one()) {
             if (RES) {
               // Centroid block kb < nh: c_hi meets x_hi and x_lo; else c_lo
               // meets x_hi.
@@ -223,15 +226,21 @@ __global__ void __launch_bounds__(kAThreads, 1)
             }
             mma_commit(&sh.empty[s]);
           }
-          if (!ok) break;
-          mma_commit(&sh.accf[b]);
+          __syncwarp();
         }
-        if (RES) mma_commit(&sh.aempty[ab]);  // the point buffer is free once these MMAs are done
+        if (!ok) break;
+        if (elect_one()) mma_commit(&sh.accf[b]);
+        __syncwarp();
       }
-      // Every MMA is done before TMEM is released.
-      mma_commit(&sh.drain);
-      mbar_wait(&sh.drain, 0u, nullptr, 0, 200000000LL);
+      if (RES) {  // the point buffer is free once these MMAs are done
+        if (elect_one()) mma_commit(&sh.aempty[ab]);
+        __syncwarp();
+      }
     }
+    // Every MMA is done before TMEM is released.
+    if (elect_one()) mma_commit(&sh.drain);
+    __syncwarp();
+    mbar_wait(&sh.drain, 0u, nullptr, 0, 200000000LL);
   } else {
     const uint32_t lane_base = (32u * static_cast<uint32_t>(warp & 3)) << 16;
     const int half = warp >> 2;

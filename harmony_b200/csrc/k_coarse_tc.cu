@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kCThreads, 1)
   // Per epilogue warp, two 32 x 32 FP32 boxes (128-byte swizzle) for the
   // TMA stores of its two chunks of a tile.
   uint8_t* stg = ring + static_cast<size_t>(kCStages) * kBlk;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   int p0, p1;
   coarse_range(blockIdx.x, gridDim.x, pairs, p0, p1);
 
@@ -141,55 +141,62 @@ __global__ void __launch_bounds__(kCThreads, 1)
       }
     }
   } else if (warp == kCMmaWarp) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_bf16_f32(kCT, kCT);
-      const uint32_t bbase = smem_u32(Bt), rbase = smem_u32(ring);
-      int it = 0, nb = 0, cur = -1, issued = 0;
-      bool ok = true;
-      for (int p = p0; p < p1 && ok; ++p) {
-        const int c = p / qt;
-        if (c != cur) {
-          if (!mbar_wait(&sh.bfull, nb & 1u, err, 26)) break;
-          tc_fence_after();
-          cur = c;
-          ++nb;
-        }
-        const int i = p - p0, b = i & 1;
-        if (!mbar_wait(&sh.acce[b], ((i >> 1) & 1u) ^ 1u, err, 23)) break;
+    // The warp converged, one lane issuing.
+    const uint32_t idesc = idesc_bf16_f32(kCT, kCT);
+    const uint32_t tm = static_cast<uint32_t>(warp_uniform(static_cast<int>(tmem)));
+    const uint32_t bbase = static_cast<uint32_t>(warp_uniform(static_cast<int>(smem_u32(Bt))));
+    const uint32_t rbase = static_cast<uint32_t>(warp_uniform(static_cast<int>(smem_u32(ring))));
+    int it = 0, nb = 0, cur = -1, issued = 0;
+    bool ok = true;
+    for (int p = p0; p < p1 && ok; ++p) {
+      const int c = p / qt;
+      if (c != cur) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.bfull, nb & 1u, err, 26));
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t d = tmem + static_cast<uint32_t>(b * kCT);
-        // A block kb: q_hi block kb (kb < nh) meets c_hi and c_lo block kb;
-        // q_lo block kb - nh meets c_hi block kb - nh.
-        for (int kb = 0; kb < 2 * nh; ++kb, ++it) {
-          const int s = it % kCStages;
-          if (!mbar_wait(&sh.full[s], (it / kCStages) & 1u, err, 22)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t ad = desc_sw128(rbase + static_cast<uint32_t>(s) * kBlk);
-          const int j = kb < nh ? kb : kb - nh;
-          const uint64_t bh = desc_sw128(bbase + static_cast<uint32_t>(j) * kBlk);
+        cur = c;
+        ++nb;
+      }
+      const int i = p - p0, b = i & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&sh.acce[b], ((i >> 1) & 1u) ^ 1u, err, 23));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d = tm + static_cast<uint32_t>(b * kCT);
+      // A block kb: q_hi block kb (kb < nh) meets c_hi and c_lo block kb;
+      // q_lo block kb - nh meets c_hi block kb - nh.
+      for (int kb = 0; kb < 2 * nh; ++kb, ++it) {
+        const int s = it % kCStages;
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.full[s], (it / kCStages) & 1u, err, 22));
+        if (!ok) break;
+        tc_fence_after();
+        const uint64_t ad = desc_sw128(rbase + static_cast<uint32_t>(s) * kBlk);
+        const int j = kb < nh ? kb : kb - nh;
+        const uint64_t bh = desc_sw128(bbase + static_cast<uint32_t>(j) * kBlk);
+        const uint64_t bl = desc_sw128(bbase + static_cast<uint32_t>(nh + j) * kBlk);
+        if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) mma_bf16(d, ad + 2 * kk, bh + 2 * kk, idesc, (kb | kk) != 0 ? 1u : 0u);
           if (kb < nh) {
-            const uint64_t bl = desc_sw128(bbase + static_cast<uint32_t>(nh + j) * kBlk);
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) mma_bf16(d, ad + 2 * kk, bl + 2 * kk, idesc, 1u);
           }
           mma_commit(&sh.empty[s]);
         }
-        if (!ok) break;
+        __syncwarp();
+      }
+      if (!ok) break;
+      // The last tile against this centroid tile: its MMAs free B.
+      if (elect_one()) {
         mma_commit(&sh.accf[b]);
-        ++issued;
-        // The last tile against this centroid tile: its MMAs free B.
         if (p + 1 == p1 || (p + 1) / qt != c) mma_commit(&sh.bempty);
       }
-      // Drain: the tensor cores must be done before TMEM is released.
-      if (issued > 0) {
-        const int l = issued - 1;
-        mbar_wait(&sh.accf[l & 1], (l >> 1) & 1u, nullptr, 0, 200000000LL);
-      }
+      __syncwarp();
+      ++issued;
+    }
+    // Drain: the tensor cores must be done before TMEM is released.
+    if (issued > 0) {
+      const int l = issued - 1;
+      mbar_wait(&sh.accf[l & 1], (l >> 1) & 1u, nullptr, 0, 200000000LL);
     }
   } else {
     // Warp w: TMEM lanes (queries) 32 (w % 4) .. + 31, columns 64 (w / 4)
