@@ -183,6 +183,35 @@ __device__ __forceinline__ uint32_t warp_kth_small8(uint32_t (&v)[8], int k, int
   return m;
 }
 
+// A value at or a little above the k-th smallest (1 <= k) of the 32 N keys a
+// warp holds, N per lane (pad with 0xFFFFFFFF; k of them at least are no
+// padding): `bits` bits of it from the first one in which the keys differ, a
+// warp-wide count of the keys up to the middle of what is left per bit, and ones
+// below.  No shared memory and no branches over the lanes; whatever k.
+template <int N>
+__device__ __forceinline__ uint32_t warp_kth_above(const uint32_t (&v)[N], int k, int bits) {
+  uint32_t lo = v[0], hi = 0u;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    lo = min(lo, v[i]);
+    hi = max(hi, v[i] == 0xFFFFFFFFu ? 0u : v[i]);
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lo >= hi) return lo;
+  const int top = 31 - __clz(lo ^ hi);
+  uint32_t res = top == 31 ? 0u : hi >> (top + 1) << (top + 1);
+  int b = top;
+  for (; b >= 0 && b > top - bits; --b) {
+    const uint32_t mid = res | ((1u << b) - 1u);
+    int c = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) c += v[i] <= mid ? 1 : 0;
+    if (static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<unsigned>(c))) < k) res |= 1u << b;
+  }
+  return b < 0 ? res : res | ((2u << b) - 1u);
+}
+
 // The k-th smallest (k >= 1) of n 32-bit keys get(0 .. n-1), by one warp:
 // radix selection over four 8-bit digits with a 256-bin histogram h in
 // shared memory.  n >= k.  A digit that the smallest and the largest key

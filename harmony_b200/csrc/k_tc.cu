@@ -817,29 +817,33 @@ __global__ void residual_rmax_kernel(float* __restrict__ rmax, int nlist) {
 }
 
 constexpr int kSmallKth = 32;  // largest k for warp_kth_small8
+constexpr int kBoundBits = 9;  // bits of a k-th value that is only a bound (U may be any value above)
 
 
 // Re-rank, one CTA per query: U = the k-th smallest upper bound among its
-// candidates, the candidates whose lower bound is at most U recomputed with
-// the reference's sequential FP32 loop, sorted by (distance, position) and cut
-// at k.  A query whose buffer overflowed goes to the host's exact search (flag
-// 2, and listed).  The rows to recompute come into shared memory kRrRows at a
-// time by 16-byte cp.async, coalesced and all in flight together, and a thread
-// sums each from there; keys live in shared memory, or, for more than kRrKeys
-// of them, in the query's buffer.  Bound by DRAM in large batches (the
-// recomputed rows), by the chain of its phases in small ones.  k <= 16 takes
-// two warps and 16 rows, so that fifteen CTAs fit an SM (a query re-ranks about
-// 15 rows there), a larger k four warps and 32 rows.  A warp per query walking
-// its rows from global memory, with three flat kernels for the queries with
-// more than 256 candidates, took 477 us for 10k queries on 1M x 128 with k 100
-// (124 rows each) and 85 us on 10M x 128 with k 10: now 192 and 62; one query
-// 21 -> 11 us.  (Other splits, threads x rows, for k 100: 128 x 64 242 us, 64 x
-// 32 219, 128 x 16 226, 64 x 16 227.)
+// candidates (or a value just above it), the candidates whose lower bound is at
+// most U recomputed with the reference's sequential FP32 loop, ordered by
+// (distance, position) and cut at k.  A query whose buffer overflowed goes to
+// the host's exact search (flag 2, and listed).  The rows to recompute come into
+// shared memory kRrRows at a time, kRrCols columns of each, by 16-byte cp.async,
+// coalesced and all in flight together, and a thread sums each from there; keys
+// live in shared memory, or, for more than kRrKeys of them, in the query's
+// buffer.  Up to kRrRank rows are placed by counting the smaller keys, more are
+// sorted.  Bound by DRAM in large batches (512-byte rows at random places, 3.6
+// TB/s), by the chain of its phases in small ones.  k <= 16 takes two warps and
+// 16 whole rows, so that fifteen CTAs fit an SM (a query re-ranks about 15 rows
+// there), a larger k four warps and 128 rows, 32 columns at a time, so that all
+// its threads sum.  10k queries on 1M x 128 with k 100 (125 rows each): 477 us
+// with a warp per query walking its rows from global memory, 192 with 32 whole
+// rows, a radix selection of U and a bitonic sort, 176 now (64 x 32 on two
+// warps 181, 64 x 64 191); 10M x 128 with k 10: 85, 60, 55; one query 21, 11,
+// 10.  (In the order of the queries' nearest lists 210: the rows that
+// neighbours share do not stay in L2.)
 constexpr int kRrKeys = 512;
 constexpr int kRerankMaxDim = 128;  // dpad of the BF16 scan's rows (d <= 128)
-constexpr int kRrStride = kRerankMaxDim + 4;
+constexpr int kRrRank = 256;  // rows up to which they are ranked by counting
 
-template <int kRrThreads, int kRrRows>
+template <int kRrThreads, int kRrRows, int kRrCols>
 __global__ void __launch_bounds__(kRrThreads) rerank_kernel(
     uint64_t* __restrict__ cand, const uint32_t* __restrict__ cand_ub, const int* __restrict__ cnt, int cap, int k,
     const float* __restrict__ codes, const float* __restrict__ q, int dpad, const int64_t* __restrict__ ids,
@@ -848,14 +852,32 @@ __global__ void __launch_bounds__(kRrThreads) rerank_kernel(
   chain_wait();
   extern __shared__ uint64_t s_top[];  // pow2_ceil(k), for queries with more than kRrKeys rows to recompute
   __shared__ uint64_t s_key[kRrKeys];
+  constexpr int kRrStride = kRrCols + 4;
   __shared__ __align__(16) float s_row[kRrRows * kRrStride];
   __shared__ __align__(16) float s_q[kRerankMaxDim];
+  __shared__ int s_n;
   __shared__ int s_h[256];
   __shared__ uint32_t s_u;
   __shared__ int s_m;
   __shared__ SelectShared sh_sel;
   const int qi = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  // The first keys and upper bounds are on their way before their number is
+  // known (what is read past it is not used).
+  uint64_t* buf = cand + static_cast<size_t>(qi) * cap;
+  const uint32_t* ubs = cand_ub + static_cast<size_t>(qi) * cap;
   const int c = cnt[qi];
+  uint64_t key[8];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) key[u] = u * kRrThreads + tid < cap ? buf[u * kRrThreads + tid] : kEmpty;
+  uint32_t ub[8];
+  if (wid == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ub[i] = 32 * i + lane < cap ? ubs[32 * i + lane] : 0xFFFFFFFFu;
+  }
+  if (tid < dpad / 4)
+    *reinterpret_cast<float4*>(s_q + 4 * tid) =
+        *reinterpret_cast<const float4*>(q + static_cast<size_t>(qi) * dpad + 4 * tid);
+  if (tid == 0) s_m = s_n = 0;
   if (c > cap) {
     if (tid == 0) {
       m_out[qi] = 0;
@@ -863,25 +885,17 @@ __global__ void __launch_bounds__(kRrThreads) rerank_kernel(
     }
     return;
   }
-  uint64_t* buf = cand + static_cast<size_t>(qi) * cap;
-  const uint32_t* ubs = cand_ub + static_cast<size_t>(qi) * cap;
-  if (tid < dpad / 4)
-    *reinterpret_cast<float4*>(s_q + 4 * tid) =
-        *reinterpret_cast<const float4*>(q + static_cast<size_t>(qi) * dpad + 4 * tid);
-  if (tid == 0) s_m = 0;
-  // The first keys are on their way while U is formed.
-  uint64_t key[8];
 #pragma unroll
-  for (int u = 0; u < 8; ++u) key[u] = u * kRrThreads + tid < c ? buf[u * kRrThreads + tid] : kEmpty;
-  // U (every candidate when there are fewer than k).
+  for (int u = 2; u < 8; ++u) key[u] = u * kRrThreads + tid < c ? buf[u * kRrThreads + tid] : kEmpty;
+  // U (every candidate when there are fewer than k), or for few candidates a
+  // value within 2^-kBoundBits of their range above it.
   if (c < k) {
     if (tid == 0) s_u = 0xFFFFFFFFu;
-  } else if (c <= 256 && k <= kSmallKth) {
+  } else if (c <= 256) {
     if (wid == 0) {
-      uint32_t v[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < c ? ubs[32 * i + lane] : 0xFFFFFFFFu;
-      const uint32_t u = warp_kth_small8(v, k, lane);
+      for (int i = 0; i < 8; ++i) ub[i] = 32 * i + lane < c ? ub[i] : 0xFFFFFFFFu;
+      const uint32_t u = warp_kth_above(ub, k, kBoundBits);
       if (lane == 0) s_u = u;
     }
   } else {
@@ -920,25 +934,54 @@ __global__ void __launch_bounds__(kRrThreads) rerank_kernel(
   const int m = s_m;
   if (tid == 0) m_out[qi] = m;
   const bool small = m <= kRrKeys;
-  const int cpr = dpad >> 2;
   for (int b0 = 0; b0 < m; b0 += kRrRows) {
     const int nb = min(kRrRows, m - b0);
-    for (int i = tid; i < nb * cpr; i += kRrThreads) {
-      const int r = i / cpr, f = i - r * cpr;
-      const uint32_t pos = key_tie(small ? s_key[b0 + r] : buf[b0 + r]);
-      cp_async16(s_row + r * kRrStride + 4 * f, codes + static_cast<size_t>(pos) * dpad + 4 * f, true);
+    const bool mine = tid < nb;
+    const uint32_t pos = mine ? key_tie(small ? s_key[b0 + tid] : buf[b0 + tid]) : 0u;
+    float acc = 0.0f;
+    for (int c0 = 0; c0 < dpad; c0 += kRrCols) {
+      const int w = min(kRrCols, dpad - c0), cpr = w >> 2;
+      if (c0 > 0) __syncthreads();  // the chunk before is consumed
+      for (int i = tid; i < nb * cpr; i += kRrThreads) {
+        const int r = i / cpr, f = i - r * cpr;
+        const uint32_t p = key_tie(small ? s_key[b0 + r] : buf[b0 + r]);
+        cp_async16(s_row + r * kRrStride + 4 * f, codes + static_cast<size_t>(p) * dpad + c0 + 4 * f, true);
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
+      __syncthreads();
+      if (mine) acc = exact_l2_seq_from(acc, s_row + tid * kRrStride, s_q + c0, w);
     }
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-    if (tid < nb) {
-      const uint32_t pos = key_tie(small ? s_key[b0 + tid] : buf[b0 + tid]);
-      const float d = exact_l2_seq_from(0.0f, s_row + tid * kRrStride, s_q, dpad);
-      const uint64_t key = d < FLT_MAX ? make_key(d, pos) : kEmpty;
+    if (mine) {
+      const uint64_t key = acc < FLT_MAX ? make_key(acc, pos) : kEmpty;
       if (small) s_key[b0 + tid] = key;
       else buf[b0 + tid] = key;
     }
     __syncthreads();
+  }
+  if (m <= kRrRank) {
+    // Few rows: each thread counts the keys before its own, which is its place
+    // in the result (equal keys are all kEmpty, which has none).
+    for (int i = tid; i < m; i += kRrThreads) {
+      const uint64_t key = s_key[i];
+      if (key == kEmpty) continue;
+      int rank = 0;
+#pragma unroll 8
+      for (int j = 0; j < m; ++j) rank += s_key[j] < key ? 1 : 0;
+      atomicAdd(&s_n, 1);
+      if (rank < k) {
+        const size_t o = static_cast<size_t>(qi) * k + rank;
+        D[o] = key_dist(key);
+        I[o] = ids[key_tie(key)];
+      }
+    }
+    __syncthreads();
+    for (int j = s_n + tid; j < k; j += kRrThreads) {
+      const size_t o = static_cast<size_t>(qi) * k + j;
+      D[o] = FLT_MAX;
+      I[o] = -1;
+    }
+    return;
   }
   const uint64_t* top = s_key;
   int n2;
@@ -963,8 +1006,8 @@ __global__ void __launch_bounds__(kRrThreads) rerank_kernel(
 
 // The bound of the second stage of a batch with k > kTightK: the first stage
 // scanned only each query's nearest list, so the k-th smallest upper bound
-// admitted there (a radix selection, 8 bits per pass) is a U for the whole
-// probe set.  One warp per query; a query with fewer than k admitted rows, or
+// admitted there (or a value just above it; past 256 rows by radix selection)
+// is a U for the whole probe set.  One warp per query; a query with fewer than k admitted rows, or
 // an overflowed buffer, keeps its bound.
 constexpr int kKthWarps = 8;
 
@@ -979,7 +1022,15 @@ __global__ void __launch_bounds__(kKthWarps * 32) kth_bound_kernel(const uint32_
   const int c = cnt[qi];
   if (c < k || c > cap) return;
   const uint32_t* src = cand_ub + static_cast<size_t>(qi) * cap;
-  const uint32_t u = warp_kth_smallest([&](int i) { return src[i]; }, c, k, s_h[wib], lane);
+  uint32_t u;
+  if (c <= 256) {
+    uint32_t v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < c ? src[32 * i + lane] : 0xFFFFFFFFu;
+    u = warp_kth_above(v, k, kBoundBits);
+  } else {
+    u = warp_kth_smallest([&](int i) { return src[i]; }, c, k, s_h[wib], lane);
+  }
   if (lane == 0 && u < thr[qi]) thr[qi] = u;
 }
 
@@ -1013,8 +1064,9 @@ __global__ void split_first_probe_kernel(const int32_t* __restrict__ probes, int
 // time is its chain of loads and barriers, so four CTAs share an SM.  10k
 // queries on 1M x 128 with 1024 lists, k 100: 117 us with the sums on the FP32
 // pipe, operands read from shared memory; 87 with the rows of both tiles kept
-// in registers and two CTAs per SM; 52 now.  10M with 4096 lists, k 10 (268 MB
-// of rows): 117, 90, 70; 777 queries on 4M x 96 30 -> 19.  Small batches
+// in registers and two CTAs per SM; 52 with four CTAs; 37 with the k-th value
+// found bit by bit, without a histogram.  10M with 4096 lists, k 10 (268 MB of
+// rows): 117, 90, 70; 777 queries on 4M x 96 30 -> 19.  Small batches
 // (probes given): one CTA per query.
 constexpr int kSeedRows = 256;
 constexpr int kSeedWarps = 8;
@@ -1046,7 +1098,6 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
   __shared__ int s_nq;
   __shared__ float s_cd[kSeedQ];
   __shared__ uint32_t s_keys[kSeedQ * kSeedKeyStride];
-  __shared__ int s_hist[kSeedQ][256];
   const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5, g = lane >> 2, t = lane & 3;
   const bool by_query = probes != nullptr;
   int l;
@@ -1146,14 +1197,11 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
         const int qi = s_qs[t0 + wib];
         const uint32_t* keys = s_keys + wib * kSeedKeyStride;
         uint32_t kth;
-        if (k <= kSmallKth) {
-          uint32_t v[8];
+        uint32_t v[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < n ? keys[32 * i + lane] : 0xFFFFFFFFu;
-          kth = warp_kth_small8(v, k, lane);
-        } else {
-          kth = warp_kth_smallest([&](int i) { return keys[i]; }, n, k, s_hist[wib], lane);
-        }
+        for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < n ? keys[32 * i + lane] : 0xFFFFFFFFu;
+        if (k <= kSmallKth) kth = warp_kth_small8(v, k, lane);
+        else kth = warp_kth_above(v, k, kBoundBits);
         // U = the k-th smallest w + eps(q, l): every one of those k rows has
         // an upper bound at most that.
         if (lane == 0)  // (by_query: the same CTA's initial store is ordered before by the barriers above)
@@ -1342,8 +1390,8 @@ void launch_rerank_bf16(uint64_t* cand, const uint32_t* cand_ub, const int* cnt,
     launch_chain(kernel, nq, threads, smem, st, cand, cand_ub, cnt, cap, k, codes, q, dpad, ids, D, I, over_list,
                  over_n, m_out);
   };
-  if (k <= kFilterTightK) go(rerank_kernel<64, 16>, 64);
-  else go(rerank_kernel<128, 32>, 128);
+  if (k <= kFilterTightK) go(rerank_kernel<64, 16, 128>, 64);
+  else go(rerank_kernel<128, 128, 32>, 128);
   HB_CUDA(cudaGetLastError());
 }
 
