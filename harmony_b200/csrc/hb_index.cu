@@ -11,9 +11,11 @@
 //   norms      float [ntotal]                <x, x> (the reference stores them too)
 //
 // Search runs per batch of queries, all on the index's stream:
-//   pad queries -> exact coarse distance matrix -> per-query top-nprobe
-//   -> [warm-up heap tops] -> list-major work description -> persistent
-//   exact list scan -> per-query merge of the partial top-k slots.
+//   pad queries -> exact coarse distance matrix (or its tensor-core form) ->
+//   per-query top-nprobe -> [warm-up heap tops] -> list-major work description
+//   -> persistent exact list scan -> per-query merge of the partial top-k slots;
+//   BF16 and larger plain FP32 searches: -> tensor-core scan under an error
+//   bound, or candidate matrix -> exact re-rank, the same results.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -977,8 +977,7 @@ void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* pr
   auto go = [&](auto kernel) {
     HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_sel)));
     launch_chain(kernel, nq, kSelectThreads, smem_sel, st, cand, seg, probes, P, R, k, list_off, pcd, rmax, dpad,
-                 kpad,
-                                                 fp8 ? 1 : 0, cap, rows, m_out, over_list, over_n);
+                 kpad, fp8 ? 1 : 0, cap, rows, m_out, over_list, over_n);
   };
   if (exact) go(cand_select_kernel<true>);
   else go(cand_select_kernel<false>);

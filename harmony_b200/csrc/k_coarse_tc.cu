@@ -619,9 +619,8 @@ void launch_coarse_tc(const void* tmap, const float* q, int nq, int dpad, int kp
   const size_t smem = coarse_tc_smem_bytes(kpad);
   HB_CUDA(cudaFuncSetAttribute(coarse_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   launch_chain(coarse_tc_kernel, G, kCThreads, smem, st, *static_cast<const CUtensorMap*>(tmap),
-                                                *reinterpret_cast<const CUtensorMap*>(tmap_q),
-                                                *reinterpret_cast<const CUtensorMap*>(tmap_v), tma_v, qnorm, nq, kpad,
-                                                cnorm, nlist, qt, pairs, V, cmins, err);
+               *reinterpret_cast<const CUtensorMap*>(tmap_q), *reinterpret_cast<const CUtensorMap*>(tmap_v), tma_v,
+               qnorm, nq, kpad, cnorm, nlist, qt, pairs, V, cmins, err);
   HB_CUDA(cudaGetLastError());
 }
 
@@ -640,9 +639,8 @@ void launch_coarse_refine(const float* q, int nq, int dpad, const float* cent, c
     const size_t smem = static_cast<size_t>(n2) * 8;
     HB_CUDA(cudaFuncSetAttribute(coarse_refine_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
-    launch_chain(coarse_refine_block_kernel, nq, 256, smem, st, q, nq, dpad, cent, cand, cval, Pm, P, nlist,
-                 cmaxnorm, probes,
-                                                      cdist, flags, rows);
+    launch_chain(coarse_refine_block_kernel, nq, 256, smem, st, q, nq, dpad, cent, cand, cval, Pm, P, nlist, cmaxnorm,
+                 probes, cdist, flags, rows);
     HB_CUDA(cudaGetLastError());
     return;
   }
@@ -652,8 +650,7 @@ void launch_coarse_refine(const float* q, int nq, int dpad, const float* cent, c
   const size_t smem = static_cast<size_t>(warps) * (n2 * 8 + stage);
   HB_CUDA(cudaFuncSetAttribute(coarse_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   launch_chain(coarse_refine_kernel, (nq + warps - 1) / warps, warps * 32, smem, st, q, nq, dpad, cent, cand, cval,
-               Pm, P, nlist,
-                                                                          cmaxnorm, probes, cdist, flags, rows);
+               Pm, P, nlist, cmaxnorm, probes, cdist, flags, rows);
   HB_CUDA(cudaGetLastError());
 }
 
@@ -664,8 +661,7 @@ void launch_coarse_fallback(const float* q, int nq, int dpad, const float* cent,
   const size_t smem = static_cast<size_t>(pow2_ceil(P < 2 ? 2 : P)) * 8;
   HB_CUDA(cudaFuncSetAttribute(coarse_fallback_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   launch_chain(coarse_fallback_kernel, std::min((nq + 31) / 32, 296), 256, smem, st, q, nq, dpad, cent, nlist, P,
-               flags, V,
-                                                                           probes, cdist, width, cmins);
+               flags, V, probes, cdist, width, cmins);
   HB_CUDA(cudaGetLastError());
 }
 

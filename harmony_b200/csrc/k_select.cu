@@ -872,14 +872,14 @@ void launch_select_rows(const float* D, int nrows, int ncols, int ldD, int k, in
     // Chunk minima given and k small against the chunk count (else T would
     // sit near the largest minima): a warp per row reads the chunks that can
     // hold the k smallest; rows it flags go through the CTA kernel below.
-    launch_chain(select_rows_chunk_kernel, (nrows + kSelWarps - 1) / kSelWarps, kSelWarps * 32, 0, st, 
-        D, nrows, ncols, ldD, k, out_idx, out_val, k_row, row_flags, cmins);
+    launch_chain(select_rows_chunk_kernel, (nrows + kSelWarps - 1) / kSelWarps, kSelWarps * 32, 0, st, D, nrows,
+                 ncols, ldD, k, out_idx, out_val, k_row, row_flags, cmins);
     HB_CUDA(cudaGetLastError());
     only = row_flags;
   } else if (row_flags && k <= 256 && ncols <= 8192 && ncols % 4 == 0 && ldD % 4 == 0 && nrows > kCtaRows) {
     // Warp per row; rows it flags go through the CTA kernel below.
-    launch_chain(select_rows_warp_kernel, (nrows + kSelWarps - 1) / kSelWarps, kSelWarps * 32, 0, st, 
-        D, nrows, ncols, ldD, k, out_idx, out_val, k_row, row_flags);
+    launch_chain(select_rows_warp_kernel, (nrows + kSelWarps - 1) / kSelWarps, kSelWarps * 32, 0, st, D, nrows, ncols,
+                 ldD, k, out_idx, out_val, k_row, row_flags);
     HB_CUDA(cudaGetLastError());
     only = row_flags;
   }
@@ -951,8 +951,7 @@ int launch_build_work(const int32_t* probes, int nq, int P, const int64_t* list_
     HB_CUDA(cudaFuncSetAttribute(build_work_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
     launch_chain(build_work_small_kernel, 1, kWorkThreads, smem, st, probes, nqp, P, list_off, nlist, chunk_rows,
-                 qgroup,
-                                                           list_cnt, list_qoff, list_q, item_off, slot_base);
+                 qgroup, list_cnt, list_qoff, list_q, item_off, slot_base);
     HB_CUDA(cudaGetLastError());
     return 1;
   }
@@ -1015,8 +1014,7 @@ void launch_warmup_tops(const float* q, int nq, const int32_t* probes, int P, co
   HB_CUDA(cudaFuncSetAttribute(warmup_tops_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem)));
   launch_chain(warmup_tops_kernel, nq, kSelThreads, smem, st, q, probes, P, codes, list_off, dpad, k, wl,
-               warm_list_size,
-                                                    tops);
+               warm_list_size, tops);
   HB_CUDA(cudaGetLastError());
 }
 

@@ -122,6 +122,9 @@ constexpr int kTile = 128;     // rows per B tile, queries per item (M)
 constexpr int kMaxStages = 4;
 constexpr int kAcc = 4;                            // TMEM accumulators of 128 columns, tile t -> t % 4
 constexpr int kNormSlots = 8;                      // tiles whose row norms sit in shared memory
+// A group's tile before t is t - kGroups at the latest: with no more groups than
+// accumulators the phase its wait asks for is the next one of that accumulator.
+static_assert(kGroups <= kAcc, "an accumulator's phases are waited for in order");
 constexpr size_t kSmemCap = 226 * 1024;            // dynamic shared memory budget
 constexpr int kTightK = kFilterTightK;             // largest k whose bound tightens during the scan
 constexpr int kFifo = 192;                         // admitted values an epilogue warp collects (a multiple of 32)

@@ -180,10 +180,11 @@ int hb_probe_lists(hb_index* ix, size_t nq, const float* q, size_t nprobe, int64
                    float* cdist);
 
 /* Coarse quantizer route (no reference counterpart; the probe rows are the
- * same on every route).  AUTO: tensor cores for d <= 128 (a 3-term BF16
- * split picks nprobe + margin candidates, re-ranked in exact FP32; queries
- * whose candidates cannot be proven to hold the exact top nprobe are
- * recomputed exactly), else the FP32 distance matrix.  EXACT: always the
+ * same on every route).  AUTO: tensor cores for d <= 128 where the FP32
+ * distance matrix would cost more (a 3-term BF16 split picks nprobe + margin
+ * candidates, re-ranked in exact FP32; queries whose candidates cannot be
+ * proven to hold the exact top nprobe are recomputed exactly), else the FP32
+ * distance matrix.  EXACT: always the
  * FP32 matrix.  TENSOR: tensor cores or HB_ERR_INVALID.  margin -1 picks
  * max(16, nprobe / 4). */
 enum { HB_COARSE_AUTO = 0, HB_COARSE_EXACT = 1, HB_COARSE_TENSOR = 2 };
