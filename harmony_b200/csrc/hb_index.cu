@@ -580,10 +580,10 @@ class IndexCore {
     if (fp8_ready_) return;
     kpad8_ = static_cast<int>((d_ + 127) / 128 * 128);
     codes8_.reserve(std::max<size_t>(ntotal_ * static_cast<size_t>(kpad8_), 1));
-    list_scale8_.reserve(nlist_);
+    list_scale8_.reserve(2 * nlist_);
     rnorm8_.reserve(std::max<size_t>(ntotal_, 1));
     launch_fp8_codes(codes_.p, list_off_.p, cent_.p, static_cast<int>(nlist_), static_cast<int>(dpad_), kpad8_,
-                     codes8_.p, list_scale8_.p, rnorm8_.p, st_);
+                     codes8_.p, list_scale8_.p, rnorm8_.p, list_scale8_.p + nlist_, st_);
     tile_rnorm8_.reserve(std::max<size_t>(tile_norm_.n, 1));
     launch_tile_norms(rnorm8_.p, list_off_.p, static_cast<int>(nlist_), tile_off_.p, tile_rnorm8_.p, st_);
     launches_ += 2;
@@ -2020,8 +2020,8 @@ class IndexCore {
     list_q_.reserve(nqp);
     work_tmp_.reserve(std::max(build_work_tmp_bytes(nb, P, static_cast<int>(nlist_)), cand_segments_tmp_bytes(nb, P)));
     seg_.reserve(nqp + 1);
-    pcd_.reserve(nqp);
-    cand_m_.reserve(static_cast<size_t>(nb));
+    pcd_.reserve((fp8 ? 2 : 1) * nqp);
+    cand_m_.reserve(2 * static_cast<size_t>(nb));
     qcd8_.reserve(nqp);
     if (fp8) {
       qscale8_.reserve(nqp);
@@ -2030,7 +2030,7 @@ class IndexCore {
       gq_.reserve(nqp * static_cast<size_t>(kpad_));
     }
     cand_.reserve(std::max<size_t>(static_cast<size_t>(nb) * cand_row_bound(P), 1));
-    cand_rows_.reserve(static_cast<size_t>(nb) * R);
+    cand_rows_.reserve((3 * static_cast<size_t>(nb) * R + 1) / 2);
     over_list_.reserve(static_cast<size_t>(nb));
   }
 
@@ -2042,6 +2042,7 @@ class IndexCore {
     // memory over them, and items stay short enough to balance the CTAs.
     const int cr = std::min(1024, std::max(128, chunk_rows_for(nb, P, 128)));
     const size_t nqp = static_cast<size_t>(nb) * P;
+    float* lb = reinterpret_cast<float*>(cand_rows_.p + static_cast<size_t>(nb) * R);  // after the rows
     {
       Scope sc(this, "build_work");
       launches_ += launch_build_work(probes_.p, nb, P, list_off_.p, static_cast<int>(nlist_), cr, 128, list_cnt_.p,
@@ -2057,12 +2058,12 @@ class IndexCore {
       if (fp8) {
         launch_gather_residual(qp_, static_cast<int>(dpad_), kpad8_, true, list_q_.p, list_qoff_.p,
                                static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), qscale8_.p, qcd8_.p,
-                               pcd_.p, gq8_.p, st_);
+                               pcd_.p, pcd_.p + nqp, gq8_.p, st_);
         make_u8_tensor_map(gqmap_, gq8_.p, nqp, kpad8_);
       } else {
         launch_gather_residual(qp_, static_cast<int>(dpad_), kpad_, false, list_q_.p, list_qoff_.p,
                                static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), nullptr, qcd8_.p,
-                               pcd_.p, gq_.p, st_);
+                               pcd_.p, nullptr, gq_.p, st_);
         make_bf16_tensor_map(gqmap_, gq_.p, nqp, kpad_);
       }
     }
@@ -2095,13 +2096,15 @@ class IndexCore {
     }
     {
       Scope sc(this, "cand_select");
-      launch_cand_select(cand_.p, seg_.p, probes_.p, nb, P, R, k, list_off_.p, pcd_.p, rmax_.p, static_cast<int>(dpad_),
-                         a.kpad, fp8, cand_rows_.p, cand_m_.p, exact ? over_list_.p : nullptr, (status_.p + kStOver), st_);
+      launch_cand_select(cand_.p, seg_.p, probes_.p, nb, P, R, k, list_off_.p, pcd_.p, rmax_.p,
+                         fp8 ? pcd_.p + nqp : nullptr, fp8 ? list_scale8_.p + nlist_ : nullptr,
+                         static_cast<int>(dpad_), a.kpad, cand_rows_.p, lb, cand_m_.p, cand_m_.p + nb,
+                         exact ? over_list_.p : nullptr, (status_.p + kStOver), st_);
     }
     {
       Scope sc(this, "cand_exact");
-      launch_cand_exact(cand_rows_.p, cand_m_.p, nb, R, k, codes_.p, qp_, static_cast<int>(dpad_), ids_.p, Dd, Id,
-                        st_);
+      launch_cand_exact(cand_rows_.p, fp8 ? lb : nullptr, cand_m_.p, cand_m_.p + nb, nb, R, k, codes_.p, qp_,
+                        static_cast<int>(dpad_), ids_.p, Dd, Id, st_);
     }
     launches_ += 6;  // segment lengths, their sum (a library kernel), gather, scan, selection, re-rank
   }
@@ -2456,8 +2459,8 @@ class IndexCore {
   DevBuf<uint16_t> gq_;
   DevBuf<float> cand_;
   DevBuf<int64_t> cand_rows_;
-  DevBuf<float> pcd_;   // ||q - c_l||^2 per (query, probe rank)
-  DevBuf<int> cand_m_;  // rows re-ranked per query
+  DevBuf<float> pcd_;   // ||q - c_l||^2 per (query, probe rank); FP8: then the entries' rounding errors
+  DevBuf<int> cand_m_;  // rows re-ranked per query, then how many of them come first
   // tensor-core coarse quantizer
   bool coarse_ready_ = false;
   int coarse_kind_ = HB_COARSE_AUTO;

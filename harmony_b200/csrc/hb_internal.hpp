@@ -341,29 +341,33 @@ void launch_cand_segments(const int32_t* probes, int nq, int P, const int64_t* l
 void launch_cand_scan(const void* tmap_q, const void* tmap_x, const CandArgs& a, int num_sms, cudaStream_t st);
 // FP8 E4M3 copies for the candidate scan, as residuals to the list centroid:
 // codes per list with s_l = max |x - c_l| / 448 (and the rows' FP32 residual
-// norms), and per list-major entry (q, l) the row q - c_l with its own scale
+// norms and each list's largest ||x - c_l - s_l code||), and per list-major entry (q, l) the row q - c_l with its own scale
 // and ||q - c_l||^2.
 void launch_fp8_codes(const float* codes, const int64_t* list_off, const float* cent, int nlist, int dpad, int kpad8,
-                      void* out, float* scale, float* rnorm, cudaStream_t st);
+                      void* out, float* scale, float* rnorm, float* emax, cudaStream_t st);
 // Per list-major entry e (query q, probe rank j, list l): row e of G = q - c_l
 // in BF16, or (fp8) E4M3 with its scale escale[e]; ecd[e] = pcd[q * P + j] =
-// ||q - c_l||^2.
+// ||q - c_l||^2, (fp8) pdq[q * P + j] the norm of the entry's rounding error.
 void launch_gather_residual(const float* q, int dpad, int kpad, bool fp8, const int32_t* list_q,
                             const int64_t* list_qoff, int nlist, int P, const float* cent, int64_t max_rows,
-                            float* escale, float* ecd, float* pcd, void* G, cudaStream_t st);
+                            float* escale, float* ecd, float* pcd, float* pdq, void* G, cudaStream_t st);
 void make_u8_tensor_map(void* tmap_out, const void* base, size_t rows, int row_bytes);
 // Selection of each query's R best candidates, less those that cannot be among
 // the k best of them (rows: nq x R stored rows, m[q] of them), then their
 // exact re-rank to the k best.  pcd: nq x P ||q - c_l||^2, rmax: per list the
-// largest residual norm (the error bound's operands).  over_list non-null: not
+// largest residual norm, and for an FP8 scan (else null) pdq and emax8 the
+// rounding errors' norms (the error bound's operands).  FP8 only: lb, the rows'
+// lower bounds, and first[q], the number of rows with the k smallest values,
+// which come first.  over_list non-null: not
 // the R best but every row that can be among the k nearest, at most R of them;
 // over_list[0 .. over_n[0]) gets the queries with more, or outside the bound's
 // range (m = 0; over_n zeroed by the caller).
 void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* probes, int nq, int P, int R, int k,
-                        const int64_t* list_off, const float* pcd, const float* rmax, int dpad, int kpad, bool fp8,
-                        int64_t* rows, int* m, int* over_list, int* over_n, cudaStream_t st);
-void launch_cand_exact(const int64_t* rows, const int* m, int nq, int R, int k, const float* codes, const float* q,
-                       int dpad, const int64_t* ids, float* D, int64_t* I, cudaStream_t st);
+                        const int64_t* list_off, const float* pcd, const float* rmax, const float* pdq,
+                        const float* emax8, int dpad, int kpad, int64_t* rows, float* lb, int* m, int* first,
+                        int* over_list, int* over_n, cudaStream_t st);
+void launch_cand_exact(const int64_t* rows, const float* lb, const int* m, const int* first, int nq, int R, int k,
+                       const float* codes, const float* q, int dpad, const int64_t* ids, float* D, int64_t* I, cudaStream_t st);
 void launch_to_bf16(const float* src, size_t n, int dpad, int kpad, void* dst, cudaStream_t st);
 void launch_scan_bf16(const void* tmap, const TcArgs& a, int num_sms, cudaStream_t st);
 // One thread waits on an mbarrier nothing arrives on, with a budget of

@@ -329,14 +329,24 @@ __device__ __forceinline__ uint4 to_e4m3x16(const float* x, float inv) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+__device__ __forceinline__ float from_e4m3(__nv_fp8_storage_t v) {
+  return __half2float(__half(__nv_cvt_fp8_to_halfraw(v, __NV_E4M3)));
+}
+
+__device__ __forceinline__ float2 from_e4m3x2(uint32_t v) {
+  return __half22float2(__half2(__nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(v), __NV_E4M3)));
+}
+
 // FP8 copy of the codes as residuals, one CTA per list: r = x - c_l (FP32),
 // the list's scale s_l = max |r| / 448 (E4M3's largest finite value), every
 // row as E4M3(r / s_l) in kpad8 bytes (columns past dpad zero), and the
-// row's FP32 residual norm ||r||^2.
+// row's FP32 residual norm ||r||^2; emax[l] = the largest ||r - s_l code|| of
+// its rows (slightly rounded up; infinite when it cannot be formed).
 __global__ void list_fp8_kernel(const float* __restrict__ codes, const int64_t* __restrict__ list_off,
                                 const float* __restrict__ cent, int dpad, int kpad8, uint8_t* __restrict__ out,
-                                float* __restrict__ scale, float* __restrict__ rnorm) {
+                                float* __restrict__ scale, float* __restrict__ rnorm, float* __restrict__ emax) {
   __shared__ float s_max[32];
+  __shared__ unsigned int s_e;
   const int l = blockIdx.x;
   const int64_t r0 = list_off[l], r1 = list_off[l + 1];
   const float* c = cent + static_cast<size_t>(l) * dpad;
@@ -366,21 +376,33 @@ __global__ void list_fp8_kernel(const float* __restrict__ codes, const int64_t* 
   }
   // Residual norms, one warp per row.
   const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) s_e = 0u;
+  __syncthreads();
+  float e = 0.0f;
   for (int64_t r = r0 + (threadIdx.x >> 5); r < r1; r += blockDim.x >> 5) {
-    float sq = 0.0f;
+    float sq = 0.0f, er = 0.0f;
     for (int j = lane; j < dpad; j += 32) {
       const float v = codes[r * dpad + j] - c[j];
       sq = fmaf(v, v, sq);
+      const float t = v - from_e4m3(__nv_cvt_float_to_fp8(v * inv, __NV_SATFINITE, __NV_E4M3)) * (1.0f / inv);
+      er = fmaf(t, t, er);
     }
-    for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+    for (int o = 16; o > 0; o >>= 1) {
+      sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      er += __shfl_xor_sync(0xffffffffu, er, o);
+    }
     if (lane == 0) rnorm[r] = sq;
+    e = fmaxf(e, er < 1e30f ? sqrtf(er) * 1.0001f : INFINITY);
   }
+  if (lane == 0) atomicMax(&s_e, __float_as_uint(e));
+  __syncthreads();
+  if (threadIdx.x == 0) emax[l] = __uint_as_float(s_e);
 }
 
 // A warp per list-major entry e (query q, probe rank j, list l): q' = q - c_l
 // as row e of the gathered matrix -- BF16, or (FP8) E4M3(q' / s_e) with the
 // entry's scale s_e = max |q'| / 448 -- and ||q'||^2, also at probe slot
-// q * P + j (the scan's value of a row is ||q'||^2 + ||r||^2 - 2 q'.r with
+// q * P + j, where (FP8) pdq takes ||q' - s_e code|| (the scan's value of a row is ||q'||^2 + ||r||^2 - 2 q'.r with
 // r = x - c_l).  blockIdx.x is the list, whose centroid stays in registers
 // (4 consecutive columns per lane and 128-column block, NI blocks) while the
 // warps of its gridDim.y CTAs stride over its entries: no search for an
@@ -391,7 +413,8 @@ __global__ void __launch_bounds__(256) gather_residual_kernel(const float* __res
                                                               const int64_t* __restrict__ list_qoff, int P,
                                                               const float* __restrict__ cent, int64_t max_rows,
                                                               float* __restrict__ escale, float* __restrict__ ecd,
-                                                              float* __restrict__ pcd, void* __restrict__ G) {
+                                                              float* __restrict__ pcd, float* __restrict__ pdq,
+                                                              void* __restrict__ G) {
   chain_wait();
   const int lane = threadIdx.x & 31;
   const int l = blockIdx.x;
@@ -430,7 +453,9 @@ __global__ void __launch_bounds__(256) gather_residual_kernel(const float* __res
       pcd[static_cast<int64_t>(ent >> 16) * P + (ent & 0xffffu)] = sq;
     }
     const float inv = FP8 && m > 0.0f ? 448.0f / m : 1.0f;
-    if (FP8 && lane == 0) escale[e] = 1.0f / inv;
+    const float s = FP8 ? 1.0f / inv : 1.0f;
+    if (FP8 && lane == 0) escale[e] = s;
+    float er = 0.0f;
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const int col = 128 * i + 4 * lane;
@@ -439,11 +464,20 @@ __global__ void __launch_bounds__(256) gather_residual_kernel(const float* __res
         const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[i].x * inv, v[i].y * inv), __NV_SATFINITE, __NV_E4M3);
         const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[i].z * inv, v[i].w * inv), __NV_SATFINITE, __NV_E4M3);
         *reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(G) + e * kpad + col) = lo | (hi << 16);
+        const float2 a = from_e4m3x2(lo), b = from_e4m3x2(hi);
+        const float t0 = fmaf(-s, a.x, v[i].x), t1 = fmaf(-s, a.y, v[i].y);
+        const float t2 = fmaf(-s, b.x, v[i].z), t3 = fmaf(-s, b.y, v[i].w);
+        er = fmaf(t0, t0, fmaf(t1, t1, fmaf(t2, t2, fmaf(t3, t3, er))));
       } else {
         const __nv_bfloat162 p0 = __floats2bfloat162_rn(v[i].x, v[i].y), p1 = __floats2bfloat162_rn(v[i].z, v[i].w);
         *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(G) + e * kpad + col) =
             make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
       }
+    }
+    if (FP8) {
+      for (int o = 16; o > 0; o >>= 1) er += __shfl_xor_sync(0xffffffffu, er, o);
+      if (lane == 0)
+        pdq[static_cast<int64_t>(ent >> 16) * P + (ent & 0xffffu)] = er < 1e30f ? sqrtf(er) * 1.0001f : INFINITY;
     }
   }
 }
@@ -474,16 +508,25 @@ __device__ __forceinline__ int value_bin(float v, float vmin, float scale) {
 // |v - d| of a candidate row: v the scan's value, d the reference's sequential
 // FP32 distance, Q = ||q - c_l||, R = the list's largest residual norm.  BF16:
 // the terms of the bounded scan's error bound (k_tc.cu), the FP32 accumulation
-// scaled to kpad products.  E4M3: each operand within 2^-4 of its value (3
-// mantissa bits) plus 1e-4 of the norm (subnormals: half of 2^-9 of a scale of
-// max / 448, over at most 1024 columns), so the product within 2 * 0.0626 +
-// 0.0626^2 of Q R, and 2^-8 Q R per 128 products for the accumulation.
-__device__ __forceinline__ float cand_eps(float cd, float R, int d, int kpad, bool fp8) {
+// scaled to kpad products.
+__device__ __forceinline__ float cand_eps(float cd, float R, int d, int kpad) {
   const float Q = sqrtf(cd) * 1.0001f + 1e-30f;
   const float u = 5.9604645e-8f;  // 2^-24
   const float blocks = static_cast<float>((kpad + 127) / 128);
-  const float c1 = fp8 ? 0.1292f + 0.00390625f * blocks : 0.00390625f + 0.0009765625f * blocks + 1.52587890625e-5f;
+  const float c1 = 0.00390625f + 0.0009765625f * blocks + 1.52587890625e-5f;
   return 1.0625f * (2.0f * c1 * Q * R + (d + 3) * u * (R * R + Q * Q) + (d + 5) * u * (Q + R) * (Q + R)) + 1e-30f;
+}
+
+// The same for E4M3 operands q~ and r~, with dq = ||q' - q~|| and E = the list's
+// largest ||r - r~||, both measured: q~.r~ - q'.r = q~.(r~ - r) + (q~ - q').r is
+// within (Q + dq) E + dq R, the accumulation within 2^-8 (Q + dq) (R + E) per 128
+// products, and 2^-14 of that for the scales' and the residuals' rounding.
+__device__ __forceinline__ float cand_eps8(float cd, float R, float dq, float E, int d, int kpad) {
+  const float Q = sqrtf(cd) * 1.0001f + 1e-30f;
+  const float u = 5.9604645e-8f;  // 2^-24
+  const float blocks = static_cast<float>((kpad + 127) / 128);
+  const float t = (Q + dq) * E + dq * R + (0.00390625f * blocks + 6.103515625e-5f) * (Q + dq) * (R + E);
+  return 1.0625f * (2.0f * t + (d + 3) * u * (R * R + Q * Q) + (d + 5) * u * (Q + R) * (Q + R)) + 1e-30f;
 }
 
 // One CTA per query: the R smallest keys (v, position) of the query's
@@ -500,7 +543,9 @@ __device__ __forceinline__ float cand_eps(float cd, float R, int d, int kpad, bo
 // Of the R, those that the scan's error bound proves to be outside the k best
 // of the R are dropped: the first k candidates' largest upper bound U is at
 // least the k-th smallest distance, so a row with v - eps > U is not among the
-// k.  The others go out, m_out[q] of them, in any order.
+// k.  The others go out, m_out[q] of them, in any order; for an FP8 scan (pdq),
+// whose bound leaves most of the R, with their lower bounds v - eps, and the
+// candidates of the k smallest values first (first_out[q] of them).
 // EXACT (FP32 searches): instead of the R smallest, every row that the bound
 // allows among the k nearest: with e the largest eps over the query's lists,
 // the k-th smallest distance is at most v_k + e, so all of them have
@@ -510,9 +555,10 @@ template <bool EXACT>
 __global__ void __launch_bounds__(kSelectThreads)
     cand_select_kernel(const float* __restrict__ cand, const int64_t* __restrict__ seg,
                        const int32_t* __restrict__ probes, int P, int R, int k, const int64_t* __restrict__ list_off,
-                       const float* __restrict__ pcd, const float* __restrict__ rmax, int dpad, int kpad, int fp8,
-                       int cap, int64_t* __restrict__ out_rows, int* __restrict__ m_out,
-                       int* __restrict__ over_list, int* __restrict__ over_n) {
+                       const float* __restrict__ pcd, const float* __restrict__ rmax,
+                       const float* __restrict__ pdq, const float* __restrict__ emax8, int dpad, int kpad,
+                       int cap, int64_t* __restrict__ out_rows, float* __restrict__ out_lb, int* __restrict__ m_out,
+                       int* __restrict__ first_out, int* __restrict__ over_list, int* __restrict__ over_n) {
   chain_wait();
   extern __shared__ __align__(16) unsigned char smem_sel[];
   uint64_t* s_cand = reinterpret_cast<uint64_t*>(smem_sel);  // cap keys (a power of two >= 2 * pow2(R))
@@ -527,12 +573,17 @@ __global__ void __launch_bounds__(kSelectThreads)
   const float* src = cand + r0;
   const int32_t* prow = probes + static_cast<int64_t>(qi) * P;
   const float* cdrow = pcd + static_cast<int64_t>(qi) * P;
+  auto eps_of = [&](int j) {  // of the query's j-th probed list
+    const int l = prow[j];
+    return pdq ? cand_eps8(cdrow[j], rmax[l], pdq[static_cast<int64_t>(qi) * P + j], emax8[l], dpad, kpad)
+               : cand_eps(cdrow[j], rmax[l], dpad, kpad);
+  };
   float emax = 0.0f;
   if (EXACT) {
     // Every thread needs the largest eps: all warps form it alike.
     for (int j = lane; j < P; j += 32)
       if (prow[j] >= 0) {
-        const float e = cand_eps(cdrow[j], rmax[prow[j]], dpad, kpad, fp8 != 0);
+        const float e = eps_of(j);
         emax = e < 1e23f ? fmaxf(emax, e) : INFINITY;
       }
     for (int off = 16; off > 0; off >>= 1) emax = fmaxf(emax, __shfl_xor_sync(0xffffffffu, emax, off));
@@ -763,57 +814,78 @@ __global__ void __launch_bounds__(kSelectThreads)
     rank = lo;
     return pos - sq[lo];
   };
+  auto put = [&](int at, int64_t row, float lb) {
+    out_rows[static_cast<int64_t>(qi) * R + at] = row;
+    if (pdq) out_lb[static_cast<int64_t>(qi) * R + at] = lb;
+  };
   unsigned int ub = 0u;
   for (int i = tid; i < n; i += kSelectThreads) {
     const uint32_t vb = static_cast<uint32_t>(keys[i] >> 32);
     if (vb > vk) continue;
     int j;
-    locate(i, j);
-    const float t = __fadd_ru(ordered_to_float(vb), cand_eps(cdrow[j], rmax[prow[j]], dpad, kpad, fp8 != 0));
+    const int64_t off = locate(i, j);
+    const int64_t row = list_off[prow[j]] + off;
+    const float e = eps_of(j), t = __fadd_ru(ordered_to_float(vb), e);
     ub = max(ub, ordered_bits(t == t ? t : INFINITY));
+    if (pdq) put(atomicAdd(&s_cnt, 1), row, __fsub_rd(ordered_to_float(vb), e));
   }
   for (int off = 16; off > 0; off >>= 1) ub = max(ub, __shfl_xor_sync(0xffffffffu, ub, off));
   if (lane == 0 && ub) atomicMax(&s_hi, ub);
   __syncthreads();
   const float U = n < k ? INFINITY : ordered_to_float(s_hi);
+  const int first = s_cnt;
+  __syncthreads();
   for (int b0 = 0; b0 < n; b0 += kSelectThreads) {
     const int i = b0 + tid;
     bool keep = false;
     int64_t row = -1;
-    if (i < n) {
+    float lb = 0.0f;
+    if (i < n && !(pdq && static_cast<uint32_t>(keys[i] >> 32) <= vk)) {
       int j;
       const int64_t off = locate(i, j);
       const float v = ordered_to_float(static_cast<uint32_t>(keys[i] >> 32));
-      keep = !(__fsub_rd(v, cand_eps(cdrow[j], rmax[prow[j]], dpad, kpad, fp8 != 0)) > U);
+      lb = __fsub_rd(v, eps_of(j));
+      keep = !(lb > U);
       row = list_off[prow[j]] + off;
     }
     const unsigned bal = __ballot_sync(0xffffffffu, keep);
     int at = 0;
     if (lane == 0 && bal) at = atomicAdd(&s_cnt, __popc(bal));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
-    if (keep) out_rows[static_cast<int64_t>(qi) * R + at] = row;
+    if (keep) put(at, row, lb);
   }
   __syncthreads();
-  if (tid == 0) m_out[qi] = s_cnt;
+  if (tid == 0) {
+    m_out[qi] = s_cnt;
+    if (pdq) first_out[qi] = first;
+  }
 }
 
 // One CTA per query: exact distances of its m candidate rows (m[q] of the R
 // slots) with the reference's sequential unfused FP32 loop (the same
 // operations, in the same order, as exact_l2_seq), then the k best (distance,
-// row).  Thread t owns candidate t of each batch of kExactThreads rows; the
+// row).  With lower bounds (lbs) the rows of the k smallest values come first;
+// their largest distance is at least the k-th smallest, so of the other rows
+// only those whose lower bound is not above it follow (5000 FP8 queries, 400
+// candidates of 500 floats, with the measured rounding errors: 398 -> 269 rows a
+// query, 844 -> 521 us; BF16's bound leaves 124 without it).  Thread t owns candidate t of each batch of
+// kExactThreads rows; the
 // rows pass through shared memory kExChunk dimensions at a time, copied by
 // 16-byte cp.async in a ring of kExStages chunks so that the next chunks'
 // fetches overlap this one's sums, and each thread continues its own sum from
 // there.  Bound by the gathered rows (DRAM).
 __global__ void __launch_bounds__(kExactThreads)
-    cand_exact_kernel(const int64_t* __restrict__ rows, const int* __restrict__ m_in, int R, int k,
+    cand_exact_kernel(const int64_t* __restrict__ rows, const float* __restrict__ lbs, const int* __restrict__ m_in,
+                      const int* __restrict__ first_in, int R, int k,
                       const float* __restrict__ codes, const float* __restrict__ q, int dpad,
                       const int64_t* __restrict__ ids, float* __restrict__ D, int64_t* __restrict__ I) {
   chain_wait();
   extern __shared__ __align__(16) unsigned char smem_ex[];
   __shared__ int64_t s_rows[kExactThreads];
   const int qi = blockIdx.x, tid = threadIdx.x;
-  const int m = m_in[qi];
+  __shared__ int s_more;
+  __shared__ unsigned int s_far;
+  const int m = m_in[qi], first = lbs ? first_in[qi] : m;
   const int n2 = pow2_ceil(max(2, max(m, k)));
   uint64_t* s_ex = reinterpret_cast<uint64_t*>(smem_ex);
   float* s_q = reinterpret_cast<float*>(s_ex + pow2_ceil(R < 2 ? 2 : R));  // dpad
@@ -822,10 +894,19 @@ __global__ void __launch_bounds__(kExactThreads)
   for (int c = 4 * tid; c < dpad; c += 4 * kExactThreads)
     *reinterpret_cast<float4*>(s_q + c) = *reinterpret_cast<const float4*>(qrow + c);
   for (int i = tid; i < n2; i += kExactThreads) s_ex[i] = kEmpty;
+  if (tid == 0) {
+    s_more = 0;
+    s_far = 0u;
+  }
   const int nch = (dpad + kExChunk - 1) / kExChunk;
-  for (int b0 = 0; b0 < m; b0 += kExactThreads) {
-    const int nb = min(kExactThreads, m - b0);
-    const int64_t row = tid < nb ? rows[static_cast<int64_t>(qi) * R + b0 + tid] : -1;
+  // Rows [0, head) are all summed, then the total - head others, whose numbers
+  // wait in the places of their keys.
+  const int head = min(m, (first + kExactThreads - 1) / kExactThreads * kExactThreads);
+  int total = head;
+  for (int b0 = 0; b0 < total; b0 += kExactThreads) {
+    const int nb = min(kExactThreads, total - b0);
+    const int64_t row =
+        tid < nb ? rows[static_cast<int64_t>(qi) * R + (b0 < head ? b0 + tid : static_cast<int>(s_ex[b0 + tid]))] : -1;
     __syncthreads();  // the previous batch's readers are done
     s_rows[tid] = row;
     __syncthreads();
@@ -854,10 +935,23 @@ __global__ void __launch_bounds__(kExactThreads)
       }
     }
     cp_async_wait<0>();
-    if (tid < nb && acc < FLT_MAX) s_ex[b0 + tid] = make_key(acc, static_cast<uint32_t>(row));
+    if (tid < nb) s_ex[b0 + tid] = acc < FLT_MAX ? make_key(acc, static_cast<uint32_t>(row)) : kEmpty;
+    if (m > head && b0 < head) {
+      // (A distance is not negative: its bits are ordered.)
+      if (b0 + tid < first) atomicMax(&s_far, __float_as_uint(acc < FLT_MAX ? acc : INFINITY));
+      if (b0 + kExactThreads >= head) {
+        __syncthreads();
+        const float far = first < k ? INFINITY : __uint_as_float(s_far);
+        for (int i = head + tid; i < m; i += kExactThreads)
+          if (!(lbs[static_cast<int64_t>(qi) * R + i] > far)) s_ex[head + atomicAdd(&s_more, 1)] = static_cast<uint64_t>(i);
+        __syncthreads();
+        total = head + s_more;
+      }
+    }
   }
   __syncthreads();
-  block_bitonic_sort(s_ex, n2);
+  const int n3 = pow2_ceil(max(2, max(total, k)));
+  block_bitonic_sort(s_ex, n3);
   for (int j = tid; j < k; j += kExactThreads) {
     const uint64_t key = s_ex[j];
     const size_t o = static_cast<size_t>(qi) * k + j;
@@ -918,23 +1012,24 @@ void launch_cand_scan(const void* tmap_q, const void* tmap_x, const CandArgs& a,
 }
 
 void launch_fp8_codes(const float* codes, const int64_t* list_off, const float* cent, int nlist, int dpad, int kpad8,
-                      void* out, float* scale, float* rnorm, cudaStream_t st) {
+                      void* out, float* scale, float* rnorm, float* emax, cudaStream_t st) {
   if (nlist <= 0) return;
   HB_CHECK(kpad8 % 128 == 0 && dpad <= kpad8, HB_ERR_INVALID, "bad FP8 row length");
-  list_fp8_kernel<<<nlist, 256, 0, st>>>(codes, list_off, cent, dpad, kpad8, static_cast<uint8_t*>(out), scale, rnorm);
+  list_fp8_kernel<<<nlist, 256, 0, st>>>(codes, list_off, cent, dpad, kpad8, static_cast<uint8_t*>(out), scale, rnorm,
+                                          emax);
   HB_CUDA(cudaGetLastError());
 }
 
 void launch_gather_residual(const float* q, int dpad, int kpad, bool fp8, const int32_t* list_q,
                             const int64_t* list_qoff, int nlist, int P, const float* cent, int64_t max_rows,
-                            float* escale, float* ecd, float* pcd, void* G, cudaStream_t st) {
+                            float* escale, float* ecd, float* pcd, float* pdq, void* G, cudaStream_t st) {
   if (max_rows <= 0) return;
   HB_CHECK(kpad % (fp8 ? 128 : 64) == 0 && dpad <= kpad && kpad <= 1024, HB_ERR_INVALID, "bad residual padding");
   // About 16 CTAs per SM over all lists.
   const dim3 g(nlist, static_cast<unsigned>(std::max(1, std::min(64, 148 * 16 / nlist))));
   auto go = [&](auto f, auto ni) {
     launch_chain(gather_residual_kernel<decltype(f)::value, decltype(ni)::value>, g, 256, 0, st, q, dpad, kpad,
-                 list_q, list_qoff, P, cent, max_rows, escale, ecd, pcd, G);
+                 list_q, list_qoff, P, cent, max_rows, escale, ecd, pcd, pdq, G);
   };
   auto width = [&](auto f) {
     if (kpad <= 128) go(f, std::integral_constant<int, 1>{});
@@ -965,8 +1060,9 @@ void make_u8_tensor_map(void* tmap_out, const void* base, size_t rows, int row_b
 }
 
 void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* probes, int nq, int P, int R, int k,
-                        const int64_t* list_off, const float* pcd, const float* rmax, int dpad, int kpad, bool fp8,
-                        int64_t* rows, int* m_out, int* over_list, int* over_n, cudaStream_t st) {
+                        const int64_t* list_off, const float* pcd, const float* rmax, const float* pdq,
+                        const float* emax8, int dpad, int kpad, int64_t* rows, float* lb, int* m_out, int* first_out,
+                        int* over_list, int* over_n, cudaStream_t st) {
   if (nq <= 0) return;
   HB_CHECK(R >= 1 && R <= kCandMaxR && k >= 1 && k <= R, HB_ERR_INVALID, "candidate count out of range");
   // Compaction buffer: at least 2048 keys and four times the R kept; an exact
@@ -976,16 +1072,16 @@ void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* pr
   const size_t smem_sel = static_cast<size_t>(cap) * sizeof(uint64_t);
   auto go = [&](auto kernel) {
     HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_sel)));
-    launch_chain(kernel, nq, kSelectThreads, smem_sel, st, cand, seg, probes, P, R, k, list_off, pcd, rmax, dpad,
-                 kpad, fp8 ? 1 : 0, cap, rows, m_out, over_list, over_n);
+    launch_chain(kernel, nq, kSelectThreads, smem_sel, st, cand, seg, probes, P, R, k, list_off, pcd, rmax, pdq,
+                 emax8, dpad, kpad, cap, rows, lb, m_out, first_out, over_list, over_n);
   };
   if (exact) go(cand_select_kernel<true>);
   else go(cand_select_kernel<false>);
   HB_CUDA(cudaGetLastError());
 }
 
-void launch_cand_exact(const int64_t* rows, const int* m, int nq, int R, int k, const float* codes, const float* q,
-                       int dpad, const int64_t* ids, float* D, int64_t* I, cudaStream_t st) {
+void launch_cand_exact(const int64_t* rows, const float* lb, const int* m, const int* first, int nq, int R, int k,
+                       const float* codes, const float* q, int dpad, const int64_t* ids, float* D, int64_t* I, cudaStream_t st) {
   if (nq <= 0) return;
   HB_CHECK(R >= 1 && R <= kCandMaxR && k <= R, HB_ERR_INVALID, "candidate count out of range");
   const size_t smem_ex = static_cast<size_t>(pow2_ceil(R < 2 ? 2 : R)) * sizeof(uint64_t) +
@@ -993,7 +1089,7 @@ void launch_cand_exact(const int64_t* rows, const int* m, int nq, int R, int k, 
                              sizeof(float);
   HB_CUDA(cudaFuncSetAttribute(cand_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(smem_ex)));
-  launch_chain(cand_exact_kernel, nq, kExactThreads, smem_ex, st, rows, m, R, k, codes, q, dpad, ids, D, I);
+  launch_chain(cand_exact_kernel, nq, kExactThreads, smem_ex, st, rows, lb, m, first, R, k, codes, q, dpad, ids, D, I);
   HB_CUDA(cudaGetLastError());
 }
 
