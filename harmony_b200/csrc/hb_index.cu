@@ -58,19 +58,19 @@ constexpr double kAssignTcTrain = 5.0e8;
 constexpr double kAssignTcAdd = 5.0e9;
 // (query, row) pairs from which a plain FP32 search takes the bounded scan
 // instead of the exact scan; below it the exact scan's fewer kernels win.
-// k <= 32, lists of 300 to 1800 rows: 9.6e3 pairs 97 -> 96 us, 2.0e4 110 -> 91,
-// 6.2e4 158 -> 97; lists of 100 rows: 2.6e4 pairs 90 -> 99 us, 6.4e4 107 -> 92.
-// k 100: 2.4e4 pairs 119 -> 125 us, 3.9e4 140 -> 141 and 267 -> 137 (one query),
-// 9.6e4 169 -> 134.
-constexpr double kScreenPairs = 1.2e4, kScreenPairsShort = 4.0e4, kScreenPairsLargeK = 4.0e4;
+// Exact against bounded, k <= 32, lists of 300 to 1800 rows: 1.6e4 to 2.0e4
+// pairs 73 / 84 us, 2.8e4 68 / 71, 3.9e4 99 / 85, 7.1e4 82 / 72, 2.0e5 109 / 83;
+// lists of 100 rows: 6.4e4 pairs 72 / 72, 2.6e5 82 / 74.  k 100: 6.2e4 pairs 95 /
+// 105, 9.6e4 107 / 104 (16 queries) and 181 / 106 (4), 1.6e5 152 / 119.
+constexpr double kScreenPairs = 3.0e4, kScreenPairsShort = 6.0e4, kScreenPairsLargeK = 8.0e4;
 constexpr double kScreenPairsShortLargeK = 1.0e5;
 constexpr int kScreenLargeK = 32;
 constexpr double kScreenShortRows = 256.0;
-// d > 128, pairs x padded dimensions: 270k x 500 (527 rows a list) 5.3e3 pairs
-// 124 -> 127 us, 2.1e4 162 -> 128 (k 100: 169 -> 145, 224 -> 147); 100k x 200
-// 5.1e3 pairs 95 -> 104 us, 2.0e4 124 -> 111; lists of 100 rows, d 200: 1.6e4 pairs
-// 94 -> 107, 6.4e4 110 -> 110.
-constexpr double kScreenWideWork = 4.0e6, kScreenWideWorkShort = 1.3e7;
+// d > 128, pairs x padded dimensions, exact against candidate matrix: 270k x 500
+// (527 rows a list) 4.3e6 119 / 118 us (k 100: 119 / 134), 1.1e7 169 / 125 and
+// 138 / 123 (382 / 146, 206 / 142); 200k x 1000 5.0e6 121 / 132, 8.1e6 157 / 158,
+// 2.0e7 195 / 144; lists of 100 rows, d 200: 1.3e7 87 / 97, 5.4e7 118 / 105.
+constexpr double kScreenWideWork = 8.0e6, kScreenWideWorkShort = 3.0e7;
 constexpr int kOneStageQueries = 256;
 constexpr double kSeedSample = 256.0;
 constexpr int kScreenWideRows = 2048;  // rows re-ranked per query of a wide FP32 search; more go to the exact scan
@@ -679,15 +679,16 @@ class IndexCore {
   }
 
   // Both routes give the same rows; the FP32 matrix costs its nq * nlist
-  // distances, the tensor-core one four more launches (about 25 us) and the
-  // re-ranking of nq * Pm candidates.  Seconds per element-pair of each,
-  // measured (matrix 6.4e12 per second, re-ranking 1e12): 777 queries, 4096
-  // lists of 96 dimensions, nprobe 256 126 -> 110 us by the matrix, nprobe 10 59
-  // against 90; 10k queries, 1024 lists of 128, nprobe 256 644 -> 403, nprobe 64
-  // 198 against 273; one query, 4096 lists 53 -> 36.
+  // distances (1.25e-13 s per dimension of one against 1.5e-14 on the tensor
+  // cores), the tensor-core one four more launches (23 us) and the re-ranking of
+  // nq * Pm candidates (1.2e-12 s per dimension, its longer selection included).
+  // Matrix against tensor cores: 777 queries, 4096 lists of 96 dimensions, nprobe
+  // 10 59 against 53 us, 64 62 / 65, 256 73 / 121; 10k queries, 1024 lists of 128,
+  // nprobe 10 183 / 115, 64 200 / 190, 256 329 / 638; 2500 queries, 2048 lists of
+  // 128, nprobe 64 106 / 86, 256 143 / 238; one query, 4096 lists 23 / 45.
   bool coarse_tc_pays(int nq, int Pm) const {
     const double pair = static_cast<double>(nq) * dpad_;
-    return pair * nlist_ * 1.55e-13 > 25e-6 + pair * Pm * 1e-12;
+    return pair * nlist_ * 1.1e-13 > 23e-6 + pair * Pm * 1.2e-12;
   }
 
   int coarse_extra(int P) const { return coarse_margin_ >= 0 ? coarse_margin_ : std::max(16, P / 4); }
