@@ -587,6 +587,15 @@ __global__ void __launch_bounds__(kSelectThreads)
         emax = e < 1e23f ? fmaxf(emax, e) : INFINITY;
       }
     for (int off = 16; off > 0; off >>= 1) emax = fmaxf(emax, __shfl_xor_sync(0xffffffffu, emax, off));
+    // Outside the bound's range, whatever the values (all of them may have
+    // overflowed where exact distances are finite).
+    if (!(emax < 1e23f)) {
+      if (tid == 0) {
+        over_list[atomicAdd(over_n, 1)] = qi;
+        m_out[qi] = 0;
+      }
+      return;
+    }
   }
   // One pass where a sample bounds it: the want-th smallest of the row's first
   // kSample values (the nearest lists' rows) is at least the row's want-th
@@ -599,7 +608,7 @@ __global__ void __launch_bounds__(kSelectThreads)
   int n = 0;             // keys to re-rank
   uint32_t vk = 0u;      // the k-th smallest value among them (ordered bits; all of them when fewer)
   bool done = false;
-  if (want <= min(m, kSample) && (!EXACT || emax < 1e23f)) {
+  if (want <= min(m, kSample)) {
     const int ns = min(m, kSample);
     uint32_t* smp = reinterpret_cast<uint32_t*>(s_hist);
     for (int i = tid; i < ns; i += kSelectThreads) {
@@ -772,7 +781,7 @@ __global__ void __launch_bounds__(kSelectThreads)
           __syncthreads();
           C = need = s_cnt;
         }
-        if (EXACT && (C > R || !(emax < 1e23f))) {
+        if (EXACT && C > R) {
           if (tid == 0) {
             over_list[atomicAdd(over_n, 1)] = qi;
             m_out[qi] = 0;
