@@ -1075,6 +1075,7 @@ constexpr int kSeedRows = 256;
 constexpr int kSeedWarps = 8;
 constexpr int kSeedQ = 8;  // queries per pass: the N of an mma, a warp each
 constexpr int kSeedKeyStride = kSeedRows + 4;
+constexpr uint32_t kNoKey = 0xFFFFFFFFu;  // a row whose value is NaN, or no row
 static_assert(kSeedWarps * 32 == kSeedRows && kSeedQ == kSeedWarps, "32 rows and a query per warp");
 
 __device__ __forceinline__ void mma_bf16_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -1190,9 +1191,9 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
 #pragma unroll
         for (int u = 0; u < 4; ++u) {  // row r + 8 (u / 2), query 2 t + u % 2
           const int j = 2 * t + (u & 1);
-          if (j < nb)
-            s_keys[j * kSeedKeyStride + r + 8 * (u >> 1)] =
-                ordered_bits(s_cd[j] + fmaf(-2.0f, d[u], (u >> 1) ? nc : na));
+          const float w = j < nb ? s_cd[j] + fmaf(-2.0f, d[u], (u >> 1) ? nc : na) : 0.0f;
+          // (A NaN's own bits can order anywhere.)
+          if (j < nb) s_keys[j * kSeedKeyStride + r + 8 * (u >> 1)] = w == w ? ordered_bits(w) : kNoKey;
         }
       }
       __syncthreads();
@@ -1202,11 +1203,16 @@ __global__ void __launch_bounds__(kSeedWarps * 32, 4) seed_bound_kernel(
         uint32_t kth;
         uint32_t v[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < n ? keys[32 * i + lane] : 0xFFFFFFFFu;
-        if (k <= kSmallKth) kth = warp_kth_small8(v, k, lane);
+        for (int i = 0; i < 8; ++i) v[i] = 32 * i + lane < n ? keys[32 * i + lane] : kNoKey;
+        // Fewer than k rows with a value give no bound.
+        int real = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) real += v[i] != kNoKey ? 1 : 0;
+        if (static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<unsigned>(real))) < k) kth = kNoKey;
+        else if (k <= kSmallKth) kth = warp_kth_small8(v, k, lane);
         else kth = warp_kth_above(v, k, kBoundBits);
         // U = the k-th smallest w + eps(q, l): every one of those k rows has
-        // an upper bound at most that.
+        // an upper bound at most that (kNoKey is a NaN's: FLT_MAX).
         if (lane == 0)  // (by_query: the same CTA's initial store is ordered before by the barriers above)
           thr[qi] = ordered_bits(
               fminf(__fadd_ru(ordered_to_float(kth), pair_eps(s_cd[wib], rmax[l], dpad)), FLT_MAX));
