@@ -516,8 +516,9 @@ class Index:
         _check(self._L.hb_set_autotune_table(self._h, text.encode()))
 
     def set_wait_budget(self, cycles: int = 0) -> None:
-        """Clock cycles a device wait of the BF16 scan spends before giving up
-        (0: the default)."""
+        """Clock cycles a device wait of the BF16 scan (the search then raises) and
+        of the tensor-core assignment of train and add (which then use the exact
+        kernel) spends before giving up (0: the default)."""
         _check(self._L.hb_set_wait_budget(self._h, int(cycles)))
 
     def coarse_fallbacks(self) -> int:

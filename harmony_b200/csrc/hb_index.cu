@@ -345,6 +345,7 @@ class IndexCore {
   // in centroid order), dist (optional) its exact distance.
   void assign_rows(Assigner& as, const float* x, size_t n, int32_t* arg, float* dist) {
     const int dp = static_cast<int>(dpad_), nl = static_cast<int>(nlist_);
+    Scope sc(this, as.on ? "assign_tc" : "assign_exact");
     if (!as.on) {
       launch_l2_argmin(x, static_cast<int>(n), cent_.p, nl, dp, arg, dist, st_);
       ++launches_;
@@ -372,6 +373,7 @@ class IndexCore {
       a.exact_list = as.exact;
       a.ctl = as.ctl;
       a.err = as.err;
+      a.wait_budget = wait_budget_;
       a.arg = arg + b;
       a.dist = dist ? dist + b : nullptr;
       launches_ += launch_assign_tc(a, num_sms_, st_);

@@ -129,7 +129,8 @@ struct AssignArgs {
   void* pairs;           // scratch, n x 8 bytes
   int* exact_list;       // scratch, n
   int* ctl;              // scratch, 4 ints: pairs, exact points, max ||c - mu||^2 (bits)
-  int* err;              // non-zero after a bounded wait gave up
+  int* err;              // non-zero after a bounded wait gave up (arg then holds any centroids)
+  long long wait_budget; // clock cycles a bounded mbarrier wait spends before giving up
   int32_t* arg;          // out, n
   float* dist;           // out, n (optional): exact distance to the centroid
 };

@@ -23,6 +23,10 @@
 // of each difference) is far inside the split's 2^-18.  Points or centroids
 // too large for the bound (norms past 1e15) and NaN are decided exactly.
 //
+// Every mbarrier wait is bounded (AssignArgs::wait_budget cycles).  After one
+// that gave up every point still has a valid column, the error flag is set, and
+// the caller makes the assignments again with the exact kernel.
+//
 // Bound: the MMA chain (24 x 64 cycles per 128 x 128 tile at kpad 128) and the
 // epilogue (11 instructions per value, 128 lanes: 1408 cycles) are even; a
 // point tile stays in shared memory for its sweep over the centroids
@@ -98,7 +102,7 @@ __global__ void __launch_bounds__(kAThreads, 1)
                      const float* __restrict__ xnorm, int n, int kpad, const float* __restrict__ cnorm, int nlist,
                      float bscale, const int* __restrict__ cmax_bits, int32_t* __restrict__ arg,
                      int2* __restrict__ pairs, int* __restrict__ exact_list, int* __restrict__ ctl,
-                     int* __restrict__ err) {
+                     int* __restrict__ err, long long budget) {
   constexpr int ST = RES ? kResStages : kStrStages;
   constexpr uint32_t kStageBytes = RES ? kABlk : 4 * kABlk;
   extern __shared__ uint8_t smem_raw[];
@@ -142,7 +146,7 @@ __global__ void __launch_bounds__(kAThreads, 1)
       for (int p = blockIdx.x; ok && p < ptiles; p += gridDim.x, ++ia) {
         if (RES) {
           const int ab = static_cast<int>(ia & 1u);
-          if (!mbar_wait(&sh.aempty[ab], ((ia >> 1) & 1u) ^ 1u, err, 41)) break;
+          if (!mbar_wait(&sh.aempty[ab], ((ia >> 1) & 1u) ^ 1u, err, 41, budget)) break;
           mbar_arrive_expect_tx(&sh.afull[ab], a_bytes);
           for (int kb = 0; kb < 2 * nh; ++kb)
             tma_load_2d(smem + ab * a_bytes + static_cast<uint32_t>(kb) * kABlk, &tmap_x, kb * 64, p * kAT, &sh.afull[ab]);
@@ -151,7 +155,7 @@ __global__ void __launch_bounds__(kAThreads, 1)
           const int steps = RES ? 2 * nh : nh;
           for (int kb = 0; kb < steps; ++kb, ++it) {
             const uint32_t s = it % ST;
-            if (!mbar_wait(&sh.empty[s], ((it / ST) & 1u) ^ 1u, err, 42)) {
+            if (!mbar_wait(&sh.empty[s], ((it / ST) & 1u) ^ 1u, err, 42, budget)) {
               ok = false;
               break;
             }
@@ -192,20 +196,20 @@ __global__ void __launch_bounds__(kAThreads, 1)
     for (int p = blockIdx.x; ok && p < ptiles; p += gridDim.x, ++ia) {
       const uint32_t ab = ia & 1u;
       if (RES) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&sh.afull[ab], (ia >> 1) & 1u, err, 43));
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.afull[ab], (ia >> 1) & 1u, err, 43, budget));
         if (!ok) break;
         tc_fence_after();
       }
       for (int c = 0; c < ctiles; ++c, ++tile) {
         const uint32_t b = tile % kAAcc;
-        ok = __all_sync(0xffffffffu, mbar_wait(&sh.acce[b], ((tile / kAAcc) & 1u) ^ 1u, err, 44));
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.acce[b], ((tile / kAAcc) & 1u) ^ 1u, err, 44, budget));
         if (!ok) break;
         tc_fence_after();
         const uint32_t d = tm + b * kAT;
         const int steps = RES ? 2 * nh : nh;
         for (int kb = 0; kb < steps; ++kb, ++it) {
           const uint32_t s = it % ST;
-          ok = __all_sync(0xffffffffu, mbar_wait(&sh.full[s], (it / ST) & 1u, err, 45));
+          ok = __all_sync(0xffffffffu, mbar_wait(&sh.full[s], (it / ST) & 1u, err, 45, budget));
           if (!ok) break;
           tc_fence_after();
           const uint32_t sb = rbase + s * kStageBytes;
@@ -255,7 +259,7 @@ __global__ void __launch_bounds__(kAThreads, 1)
       t.reset();
       for (int c = 0; c < ctiles; ++c, ++tile) {
         const uint32_t b = tile % kAAcc;
-        if (ok) ok = mbar_wait(&sh.accf[b], (tile / kAAcc) & 1u, err, 46);
+        if (ok) ok = mbar_wait(&sh.accf[b], (tile / kAAcc) & 1u, err, 46, budget);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) continue;
         tc_fence_after();
@@ -298,6 +302,9 @@ __global__ void __launch_bounds__(kAThreads, 1)
         t.v3 = fminf(t.v3, sh.mv[2][pl]);
         const int q = p * kAT + pl;
         int state = -1;  // no point
+        // After a wait that gave up any centroid will do (the host asks for all
+        // of them again), but what follows indexes with it.
+        if (q < n && !ok) arg[q] = 0;
         if (q < n && ok) {
           const float xn = xnorm[q];
           const float d1 = fabsf(xn + t.v1);
@@ -468,14 +475,14 @@ int launch_assign_tc(const AssignArgs& a, int num_sms, cudaStream_t st) {
                                  static_cast<int>(smem)));
     assign_tc_kernel<true><<<grid, kAThreads, smem, st>>>(tx, tc, a.xnorm, a.n, kpad, a.cnorm, a.nlist, bscale,
                                                            a.ctl + 2, a.arg, static_cast<int2*>(a.pairs), a.exact_list,
-                                                           a.ctl, a.err);
+                                                           a.ctl, a.err, a.wait_budget);
   } else {
     const size_t smem = 1024 + static_cast<size_t>(kStrStages) * 4 * kABlk;
     HB_CUDA(cudaFuncSetAttribute(assign_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)));
     assign_tc_kernel<false><<<grid, kAThreads, smem, st>>>(tx, tc, a.xnorm, a.n, kpad, a.cnorm, a.nlist, bscale,
                                                             a.ctl + 2, a.arg, static_cast<int2*>(a.pairs),
-                                                            a.exact_list, a.ctl, a.err);
+                                                            a.exact_list, a.ctl, a.err, a.wait_budget);
   }
   HB_CUDA(cudaGetLastError());
   assign_pairs_kernel<<<std::min((a.n + 127) / 128, 8 * num_sms), 128, 0, st>>>(

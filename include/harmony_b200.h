@@ -225,7 +225,9 @@ int hb_set_autotune_table(hb_index* ix, const char* text);
 /* Clock cycles a device-side wait of the BF16 scan spends before it gives
  * up (no reference counterpart; cycles <= 0 restores the default, 2e9).  A
  * wait that gives up makes the search return HB_ERR_CUDA with "gave up
- * waiting" and leaves the index usable. */
+ * waiting" and leaves the index usable.  The same budget holds for the
+ * tensor-core assignment of hb_train and hb_add, which then make the same
+ * assignments with the exact kernel. */
 int hb_set_wait_budget(hb_index* ix, int64_t cycles);
 
 /* Queries of the most recent BF16 search (d <= 128, k <= 256) whose
