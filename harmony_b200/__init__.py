@@ -371,6 +371,7 @@ class Index:
             raise HarmonyError(1, "faiss training is not part of this build")
         p, keep = _ptr(codes, np.float32)
         t0 = time.perf_counter()
+        _wait_for_torch(self.stream, codes)
         _check(self._L.hb_train(self._h, int(n), p, int(lite)))
         self.trainTime = time.perf_counter() - t0
 
@@ -378,6 +379,7 @@ class Index:
         """Index::add (src/Index.cpp:581-698)."""
         p, keep = _ptr(codes, np.float32)
         t0 = time.perf_counter()
+        _wait_for_torch(self.stream, codes)
         _check(self._L.hb_add(self._h, int(n), p))
         self.addTime = time.perf_counter() - t0
 
@@ -533,6 +535,7 @@ class Index:
         """Train the per-query nprobe predictor on n training queries labelled by
         the exact search at nprobe = label_nprobe, calibrated to `target` recall."""
         p, keep = _ptr(queries, np.float32)
+        _wait_for_torch(self.stream, queries)
         _check(self._L.hb_train_probe_predictor(self._h, int(n), p, int(k), int(label_nprobe), float(target)))
 
     def probe_calibration(self):
