@@ -1638,7 +1638,9 @@ class IndexCore {
     } catch (const Error& e) {
       if (e.code != HB_ERR_NOMEM) throw;
       cudaGetLastError();
-      cbuf_.release();  // the exact scan's buffers need the memory
+      // The exact scan's buffers need the memory.  (The failed reserve has
+      // outdated every captured graph.)
+      cbuf_.release();
       cbuf_ub_.release();
       cand_.release();
       gq_.release();

@@ -54,8 +54,9 @@ void launch_chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cuda
 }
 #endif
 
-// Bumped on every device allocation of a DevBuf: CUDA graphs that captured
-// buffer addresses are valid only while it is unchanged.
+// Bumped on every device allocation of a DevBuf, before it is tried (the old
+// block is gone by then, whether there is a new one or not): CUDA graphs that
+// captured buffer addresses are valid only while it is unchanged.
 inline std::atomic<uint64_t>& devbuf_generation() {
   static std::atomic<uint64_t> g{0};
   return g;
@@ -80,9 +81,9 @@ struct DevBuf {
       release();
       size_t bytes = count * sizeof(T);
       if (bytes == 0) bytes = sizeof(T);
+      devbuf_generation().fetch_add(1);
       HB_CUDA(cudaMalloc(&p, bytes));
       n = count;
-      devbuf_generation().fetch_add(1);
     }
     return p;
   }
