@@ -394,6 +394,9 @@ class IndexCore {
   // ---- train: src/Index.cpp:381-425 + src/Clustering.cpp:14-152 ------------
 
   void train(size_t n, const float* x, bool lite) {
+    with_candidate_memory([&] { train_all(n, x, lite); });
+  }
+  void train_all(size_t n, const float* x, bool lite) {
     HB_CHECK(x || n == 0, HB_ERR_INVALID, "null training data");
     HB_CHECK(n >= nlist_, HB_ERR_INVALID, "train needs at least nlist points");
     HB_CHECK(n < (1ull << 31), HB_ERR_INVALID, "train supports fewer than 2^31 points");
@@ -502,6 +505,9 @@ class IndexCore {
 
   void add(size_t n, const float* x) {
     if (n == 0) return;  // the reference returns before touching the lists
+    with_candidate_memory([&] { add_all(n, x); });
+  }
+  void add_all(size_t n, const float* x) {
     HB_CHECK(x, HB_ERR_INVALID, "null data");
     HB_CHECK(n < (1ull << 32) - 1, HB_ERR_INVALID, "add supports fewer than 2^32 - 1 vectors");
     HB_CUDA(cudaSetDevice(device_));
@@ -971,7 +977,9 @@ class IndexCore {
     if (p.use_graph) {
       HB_CHECK(mode == SCAN_PLAIN && (p.mode == HB_MODE_ORIGINAL || p.mode == HB_MODE_BRUTE_FORCE) && nq <= bs,
                HB_ERR_INVALID, "graph search runs ORIGINAL / BRUTE_FORCE searches of one batch");
-      search_graph(static_cast<int>(nq), q, static_cast<int>(k), static_cast<int>(P), R, bf16, p, D, I);
+      with_candidate_memory([&] {
+        search_graph(static_cast<int>(nq), q, static_cast<int>(k), static_cast<int>(P), R, bf16, p, D, I);
+      });
       return;
     }
     for (size_t b0 = 0; b0 < nq; b0 += bs) {
@@ -979,26 +987,27 @@ class IndexCore {
       cut_b0_ = b0;
       float* Dd = D + b0 * k;
       int64_t* Id = I + b0 * k;
-      if (!dev_out) out_rows(nb, static_cast<int>(k), Dd, Id);
-      // Queries.
       const float* qsrc = q + b0 * d_;
-      if (dev_in && d_ == dpad_ && reinterpret_cast<uintptr_t>(qsrc) % 16 == 0) {
-        qp_ = qsrc;  // already padded rows, read only during this call
-      } else {
-        qpad_.reserve(static_cast<size_t>(nb) * dpad_);
-        stage_queries(qsrc, nb, dev_in);
-      }
-      begin_batch();
-      if (P == 0 || ntotal_ == 0) {
-        launch_fill_results(Dd, Id, static_cast<size_t>(nb) * k, st_);
-        ++launches_;
-      } else {
-        if (bf16)
+      with_candidate_memory([&] {
+        if (!dev_out) out_rows(nb, static_cast<int>(k), Dd, Id);
+        // Queries.
+        if (dev_in && d_ == dpad_ && reinterpret_cast<uintptr_t>(qsrc) % 16 == 0) {
+          qp_ = qsrc;  // already padded rows, read only during this call
+        } else {
+          qpad_.reserve(static_cast<size_t>(nb) * dpad_);
+          stage_queries(qsrc, nb, dev_in);
+        }
+        begin_batch();
+        if (P == 0 || ntotal_ == 0) {
+          launch_fill_results(Dd, Id, static_cast<size_t>(nb) * k, st_);
+          ++launches_;
+        } else if (bf16) {
           search_batch_bf16(nb, static_cast<int>(P), static_cast<int>(k), R, Dd, Id);
-        else
+        } else {
           search_batch(nb, static_cast<int>(P), static_cast<int>(k), mode, p.pruning != 0, need_tops, warm_lists,
                        warm_size, W, B, qblock, Dd, Id);
-      }
+        }
+      });
       finish_batch(nb, static_cast<int>(P), static_cast<int>(k), bf16, Dd, Id, D + b0 * k, I + b0 * k,
                    !dev_out && !is_device_ptr(D) && !is_device_ptr(I));
     }
@@ -1065,12 +1074,16 @@ class IndexCore {
     bool again = host_out && !pinned;
     if (bounded && err != 0) {
       // A wait of a screened FP32 batch gave up: the exact scan for all of it.
-      begin_batch();
-      scan_exact_from(nb, P, k, qp_, probes_.p, SCAN_PLAIN, false, nullptr, 1, 1, 0, Dd, Id);
+      with_candidate_memory([&] {
+        begin_batch();
+        scan_exact_from(nb, P, k, qp_, probes_.p, SCAN_PLAIN, false, nullptr, 1, 1, 0, Dd, Id);
+      });
       again = true;
     } else if (bounded && over > 0) {
-      begin_batch();
-      fix_overflow(nb, P, k, over, Dd, Id);
+      with_candidate_memory([&] {
+        begin_batch();
+        fix_overflow(nb, P, k, over, Dd, Id);
+      });
       again = true;
     }
     if (again) {
@@ -1139,7 +1152,8 @@ class IndexCore {
     }
     if (cut_mode_ == 2) {
       npqin_.reserve(static_cast<size_t>(nb));
-      HB_CUDA(cudaMemcpyAsync(npqin_.p, cut_src_, static_cast<size_t>(nb) * sizeof(int32_t), cudaMemcpyDefault, st_));
+      HB_CUDA(cudaMemcpyAsync(npqin_.p, p.nprobe_per_query, static_cast<size_t>(nb) * sizeof(int32_t),
+                              cudaMemcpyDefault, st_));
       cut_src_ = npqin_.p;
     }
     cut_b0_ = 0;
@@ -1638,14 +1652,44 @@ class IndexCore {
     } catch (const Error& e) {
       if (e.code != HB_ERR_NOMEM) throw;
       cudaGetLastError();
-      // The exact scan's buffers need the memory.  (The failed reserve has
-      // outdated every captured graph.)
-      cbuf_.release();
-      cbuf_ub_.release();
-      cand_.release();
-      gq_.release();
+      release_candidates();  // the exact scan's buffers need the memory
       return false;
     }
+  }
+
+  // The buffers that only scans through candidates need; their searches take
+  // them again.  (Called after a failed reserve, which has outdated every
+  // captured graph.)
+  bool holds_candidates() const {
+    return cbuf_.p || cbuf_ub_.p || cand_.p || cand_rows_.p || gq_.p || gq8_.p || pcd_.p || qcd8_.p || seg_.p;
+  }
+  void release_candidates() {
+    cbuf_.release();
+    cbuf_ub_.release();
+    cand_.release();
+    cand_rows_.release();
+    gq_.release();
+    gq8_.release();
+    pcd_.release();
+    qcd8_.release();
+    seg_.release();
+  }
+  // f(), and once more without the candidate buffers where it runs out of
+  // memory beside them (a screened search then goes on with the exact scan):
+  // what earlier searches keep is not to fail a call that fits without it.
+  template <class F>
+  void with_candidate_memory(F&& f) {
+    try {
+      f();
+      return;
+    } catch (const Error& e) {
+      if (e.code != HB_ERR_NOMEM || !holds_candidates()) throw;
+    }
+    cudaGetLastError();
+    HB_CUDA(cudaStreamSynchronize(st_));
+    release_candidates();
+    screen_ = false;
+    f();
   }
 
   bool screen_batch(int nb, int P, int k, float* Dd, int64_t* Id) {
@@ -2035,7 +2079,9 @@ class IndexCore {
       gq_.reserve(nqp * static_cast<size_t>(kpad_));
     }
     cand_.reserve(std::max<size_t>(static_cast<size_t>(nb) * cand_row_bound(P), 1));
-    cand_rows_.reserve((3 * static_cast<size_t>(nb) * R + 1) / 2);
+    // The rows, then (FP8) as many lower bounds.
+    const size_t nr = static_cast<size_t>(nb) * R;
+    cand_rows_.reserve(fp8 ? (3 * nr + 1) / 2 : nr);
     over_list_.reserve(static_cast<size_t>(nb));
   }
 

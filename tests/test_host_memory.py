@@ -55,7 +55,8 @@ class HostIndex:
 
     def close(self):
         self.L.hb_destroy(self.h)
-        assert self.L.fake_used() == 0 and self.L.fake_stale() == 0
+        self.h = ctypes.c_void_p()
+        assert self.L.fake_stale() == 0
 
 
 def test_graph_is_dropped_with_its_buffers(lib):
@@ -74,4 +75,67 @@ def test_graph_is_dropped_with_its_buffers(lib):
     ix.search(2000, 10)
     assert ix.launched("scan_exact") == 2
     ix.search(100, 10, Precision.BF16, graph=True)
+    ix.close()
+
+
+def test_exact_search_of_overflowing_queries_gets_the_candidates_memory(lib):
+    """The queries that a screened batch hands to the exact scan (or all of them
+    after a wait that gave up) find room where the batch alone would."""
+    for overflow, err in ((2000, 0), (0, 14)):
+        ix = HostIndex(lib, 64, 16, 8, 4000)
+        ix.search(2000, 100)
+        assert ix.launched("rerank") == 1 and ix.launched("scan_exact") == 0
+        lib.fake_overflow(overflow)
+        lib.fake_err(err)
+        ix.room(4 * MB)  # the exact scan's slots take 13
+        ix.search(2000, 100)
+        assert lib.fake_failures() == 1 and ix.launched("rerank") == 2 and ix.launched("scan_exact") == 1
+        # With room again, through the candidates again.
+        lib.fake_overflow(0)
+        lib.fake_err(0)
+        ix.room(1 << 30)
+        ix.search(2000, 100)
+        assert ix.launched("rerank") == 3 and ix.launched("scan_exact") == 1
+        ix.close()
+
+
+@pytest.mark.parametrize("d", [64, 144])
+@pytest.mark.parametrize("graph", [False, True])
+def test_kept_candidate_memory_fails_no_later_call(lib, d, graph):
+    ix = HostIndex(lib, d, 16, 8, 4000)
+    before = lib.fake_used()
+    ix.search(3000, 20)
+    kept = lib.fake_used() - before
+    assert kept > 64 * MB and ix.launched("scan_exact") == 0
+    # A search beyond the candidates' k: its slots (58 MB) and results.
+    ix.room(8 * MB)
+    ix.search(3000, 300, graph=graph)
+    assert ix.launched("scan_exact") >= 1 and lib.fake_failures() >= 1
+    assert lib.fake_used() - before < kept
+    ix.close()
+
+
+def test_screened_search_without_room_keeps_nothing_of_the_candidates(lib):
+    ix = HostIndex(lib, 144, 16, 8, 4000)
+    before = lib.fake_used()
+    ix.search(6000, 300)  # exact
+    exact_only = lib.fake_used() - before
+    ix.search(3000, 20)  # 24 MB of candidates, 49 of their rows, 9 of gathered queries
+    assert lib.fake_used() - before - exact_only > 64 * MB
+    ix.room(10 * MB)
+    ix.search(6000, 20)
+    assert lib.fake_failures() >= 1 and ix.launched("scan_exact") == 2
+    # (The small buffers have grown with the batch.)
+    assert lib.fake_used() - before - exact_only < 8 * MB
+    ix.close()
+
+
+def test_add_gets_the_candidates_memory(lib):
+    ix = HostIndex(lib, 64, 16, 8, 4000)
+    ix.search(4000, 20)
+    ix.room(16 * MB)
+    x = np.zeros((40_000, 64), np.float32)  # 10 MB, its copies and scratch
+    assert lib.hb_add(ix.h, x.shape[0], x.ctypes.data) == 0, lib.hb_last_error()
+    assert lib.fake_failures() >= 1
+    ix.search(4000, 20)
     ix.close()
