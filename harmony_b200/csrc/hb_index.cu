@@ -948,6 +948,21 @@ class IndexCore {
     }
 
     const bool dev_out = is_device_ptr(D) && is_device_ptr(I);
+    // Queries that the results are written over: a copy of all of them first
+    // (device rows are read in place until a batch's last kernel, and a call may
+    // take several batches).
+    DevBuf<float> q_copy;
+    const uintptr_t q0 = reinterpret_cast<uintptr_t>(q), q1 = q0 + nq * d_ * sizeof(float);
+    auto over_queries = [&](const void* out, size_t bytes) {
+      const uintptr_t o = reinterpret_cast<uintptr_t>(out);
+      return o < q1 && q0 < o + bytes;
+    };
+    if (!p.use_graph &&  // (a graph search is one batch of copied queries)
+        (over_queries(D, nq * k * sizeof(float)) || over_queries(I, nq * k * sizeof(int64_t)))) {
+      with_candidate_memory([&] { q_copy.reserve(nq * d_); });
+      HB_CUDA(cudaMemcpyAsync(q_copy.p, q, nq * d_ * sizeof(float), cudaMemcpyDefault, st_));
+      q = q_copy.p;
+    }
     const bool dev_in = is_device_ptr(q);
     size_t bs = std::min<size_t>(nq, batch_limit(P, k));
     if (cand_path_ && P > 0) bs = std::min(bs, cand_batch_limit(P));
