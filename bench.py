@@ -576,6 +576,13 @@ def run_reference(args):
         return None
     import shutil
     import oracle
+    if not oracle.RefIndex.available():
+        oracle.build(reference=True)
+    if not oracle.RefIndex.available():
+        print(json.dumps({"impl": "reference",
+                          "unavailable": f"the reference's library is not built and its sources are not in "
+                                         f"{oracle.REFERENCE_SRC}"}), flush=True)
+        return None
     k, nq = WORKLOAD["k"], WORKLOAD["nq"]
     d = tempfile.mkdtemp(prefix="hb_ref_", dir="/dev/shm" if os.path.isdir("/dev/shm") else None)
     try:
@@ -587,8 +594,6 @@ def run_reference(args):
             meta = json.load(f)
         test_np = np.load(os.path.join(d, "test.npy"))
         gt = np.load(os.path.join(d, "gt.npy"))
-        if not oracle.RefIndex.available():
-            oracle.build(reference=True)
         ref = oracle.RefIndex.load(os.path.join(d, "index"))
     finally:
         shutil.rmtree(d, ignore_errors=True)
