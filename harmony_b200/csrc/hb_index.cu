@@ -603,11 +603,18 @@ class IndexCore {
   void build_bf16() {
     bf16_ready_ = false;
     fp8_ready_ = false;
+    spare_ = nullptr;
+    spare_bytes_ = 0;
     kpad_ = static_cast<int>((d_ + 63) / 64 * 64);
     if (ntotal_ == 0) return;
     // Residuals to the list centroids: BF16(x - c_l), their FP32 norms and
     // each list's largest residual norm (the scans' error bound uses it).
-    codes_bf16_.reserve(ntotal_ * static_cast<size_t>(kpad_));
+    // (With room at the end for small batches' candidates: a block of their own
+    // costs the first of them more than its search, 0.4 ms for one MiB.)
+    const size_t code_bytes = (ntotal_ * static_cast<size_t>(kpad_) * 2 + 255) / 256 * 256;
+    codes_bf16_.reserve((code_bytes + std::min(kSpareBytes, code_bytes / 16)) / 2);
+    spare_ = reinterpret_cast<unsigned char*>(codes_bf16_.p) + code_bytes;
+    spare_bytes_ = codes_bf16_.n * 2 - code_bytes;
     rnorm_.reserve(ntotal_);
     rmax_.reserve(nlist_);
     launch_residual_bf16(codes_.p, list_off_.p, cent_.p, static_cast<int>(nlist_), ntotal_, static_cast<int>(dpad_), kpad_,
@@ -1726,8 +1733,14 @@ class IndexCore {
     cnt.reserve(nb);
     m.reserve(nb);
     over_list_.reserve(static_cast<size_t>(nb));
-    cbuf_.reserve(static_cast<size_t>(nb) * cap);
-    cbuf_ub_.reserve(static_cast<size_t>(nb) * cap);
+    const size_t n = static_cast<size_t>(nb) * cap;
+    Carver c{spare_};
+    c.take(w_.key, n);
+    c.take(w_.ub, n);
+    if (!spare_ || c.off > spare_bytes_) {
+      w_.key = cbuf_.reserve(n);
+      w_.ub = cbuf_ub_.reserve(n);
+    }
   }
 
   // The exact list scan and merge of nb queries (qpad, nb x dpad) over the
@@ -1884,8 +1897,8 @@ class IndexCore {
     a.work_counter = counter(0);
     a.thr = thr_.p;
     a.rmax = rmax_.p;
-    a.cand = cbuf_.p;
-    a.cand_ub = cbuf_ub_.p;
+    a.cand = w_.key;
+    a.cand_ub = w_.ub;
     a.cand_cnt = cnt;
     a.cap = cap;
     a.k = k;
@@ -1900,7 +1913,7 @@ class IndexCore {
       // Second stage: the other lists, appended to the same buffers.
       {
         Scope sc(this, "kth_bound");
-        launch_kth_bound(cbuf_ub_.p, cnt, cap, nb, k, thr_.p, st_);
+        launch_kth_bound(w_.ub, cnt, cap, nb, k, thr_.p, st_);
       }
       {
         Scope sc(this, "build_work");
@@ -1918,7 +1931,7 @@ class IndexCore {
     }
     {
       Scope sc(this, "rerank");
-      launch_rerank_bf16(cbuf_.p, cbuf_ub_.p, cnt, cap, nb, k, codes_.p, qp_, static_cast<int>(dpad_), ids_.p, Dd,
+      launch_rerank_bf16(w_.key, w_.ub, cnt, cap, nb, k, codes_.p, qp_, static_cast<int>(dpad_), ids_.p, Dd,
                          Id, over_list_.p, status_.p + kStOver, rr_m, st_);
     }
     launches_ += 2;  // scan, re-rank
@@ -2090,13 +2103,20 @@ class IndexCore {
     if (fp8) {
       qscale8_.reserve(nqp);
       gq8_.reserve(nqp * static_cast<size_t>(kpad8_));
-    } else {
-      gq_.reserve(nqp * static_cast<size_t>(kpad_));
     }
-    cand_.reserve(std::max<size_t>(static_cast<size_t>(nb) * cand_row_bound(P), 1));
+    const size_t nm = std::max<size_t>(static_cast<size_t>(nb) * cand_row_bound(P), 1);
     // The rows, then (FP8) as many lower bounds.
-    const size_t nr = static_cast<size_t>(nb) * R;
-    cand_rows_.reserve(fp8 ? (3 * nr + 1) / 2 : nr);
+    const size_t nr = fp8 ? (3 * static_cast<size_t>(nb) * R + 1) / 2 : static_cast<size_t>(nb) * R;
+    const size_t ng = fp8 ? 0 : nqp * static_cast<size_t>(kpad_);
+    Carver c{spare_};
+    c.take(w_.mat, nm);
+    c.take(w_.rows, nr);
+    c.take(w_.q, ng);
+    if (!spare_ || c.off > spare_bytes_) {
+      if (ng) w_.q = gq_.reserve(ng);
+      w_.mat = cand_.reserve(nm);
+      w_.rows = cand_rows_.reserve(nr);
+    }
     over_list_.reserve(static_cast<size_t>(nb));
   }
 
@@ -2108,7 +2128,7 @@ class IndexCore {
     // memory over them, and items stay short enough to balance the CTAs.
     const int cr = std::min(1024, std::max(128, chunk_rows_for(nb, P, 128)));
     const size_t nqp = static_cast<size_t>(nb) * P;
-    float* lb = reinterpret_cast<float*>(cand_rows_.p + static_cast<size_t>(nb) * R);  // after the rows
+    float* lb = reinterpret_cast<float*>(w_.rows + static_cast<size_t>(nb) * R);  // after the rows
     {
       Scope sc(this, "build_work");
       launches_ += launch_build_work(probes_.p, nb, P, list_off_.p, static_cast<int>(nlist_), cr, 128, list_cnt_.p,
@@ -2129,8 +2149,8 @@ class IndexCore {
       } else {
         launch_gather_residual(qp_, static_cast<int>(dpad_), kpad_, false, list_q_.p, list_qoff_.p,
                                static_cast<int>(nlist_), P, cent_.p, static_cast<int64_t>(nqp), nullptr, qcd8_.p,
-                               pcd_.p, nullptr, gq_.p, st_);
-        make_bf16_tensor_map(gqmap_, gq_.p, nqp, kpad_);
+                               pcd_.p, nullptr, w_.q, st_);
+        make_bf16_tensor_map(gqmap_, w_.q, nqp, kpad_);
       }
     }
     CandArgs a{};
@@ -2146,7 +2166,7 @@ class IndexCore {
     a.chunk_rows = cr;
     a.P = P;
     a.seg = seg_.p;
-    a.cand = cand_.p;
+    a.cand = w_.mat;
     a.err = (status_.p + kStErr);
     a.qcd = qcd8_.p;
     if (fp8) {
@@ -2162,14 +2182,14 @@ class IndexCore {
     }
     {
       Scope sc(this, "cand_select");
-      launch_cand_select(cand_.p, seg_.p, probes_.p, nb, P, R, k, list_off_.p, pcd_.p, rmax_.p,
+      launch_cand_select(w_.mat, seg_.p, probes_.p, nb, P, R, k, list_off_.p, pcd_.p, rmax_.p,
                          fp8 ? pcd_.p + nqp : nullptr, fp8 ? list_scale8_.p + nlist_ : nullptr,
-                         static_cast<int>(dpad_), a.kpad, cand_rows_.p, lb, cand_m_.p, cand_m_.p + nb,
+                         static_cast<int>(dpad_), a.kpad, w_.rows, lb, cand_m_.p, cand_m_.p + nb,
                          exact ? over_list_.p : nullptr, (status_.p + kStOver), st_);
     }
     {
       Scope sc(this, "cand_exact");
-      launch_cand_exact(cand_rows_.p, fp8 ? lb : nullptr, cand_m_.p, cand_m_.p + nb, nb, R, k, codes_.p, qp_,
+      launch_cand_exact(w_.rows, fp8 ? lb : nullptr, cand_m_.p, cand_m_.p + nb, nb, R, k, codes_.p, qp_,
                         static_cast<int>(dpad_), ids_.p, Dd, Id, st_);
     }
     launches_ += 6;  // segment lengths, their sum (a library kernel), gather, scan, selection, re-rank
@@ -2553,7 +2573,7 @@ class IndexCore {
   DevBuf<int> scr_cnt_, scr_m_;      // its counts (bf16_stats reports BF16 searches only)
   int last_nb_ = 0;
   DevBuf<uint64_t> cbuf_;
-  DevBuf<uint32_t> cbuf_ub_;  // each candidate's upper bound
+  DevBuf<uint32_t> cbuf_ub_;
   DevBuf<float> oq_, od_;
   DevBuf<int32_t> op_;
   DevBuf<int64_t> oi_;
@@ -2563,6 +2583,18 @@ class IndexCore {
   int last_overflow_ = 0;
   DevBuf<int32_t> kq_;
   DevBuf<uint16_t> codes_bf16_;
+  // The end of codes_bf16_'s block, and the candidate workspace of the batch at
+  // hand: there where it fits, else in blocks of its own.
+  static constexpr size_t kSpareBytes = size_t(16) << 20;
+  unsigned char* spare_ = nullptr;
+  size_t spare_bytes_ = 0;
+  struct {
+    uint64_t* key;   // bounded scan: candidate keys,
+    uint32_t* ub;    // their upper bounds
+    float* mat;      // candidate matrix: values,
+    int64_t* rows;   // rows to re-rank (FP8: then their lower bounds),
+    uint16_t* q;     // gathered BF16 queries
+  } w_{};
   DevBuf<float> tile_norm_, rnorm_, rmax_;
   DevBuf<int64_t> tile_off_;
   DevBuf<int32_t> probes1_;

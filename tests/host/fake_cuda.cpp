@@ -14,7 +14,7 @@
 
 namespace {
 std::map<uintptr_t, size_t> live;  // device allocations
-size_t used = 0, peak = 0, limit = ~size_t(0);
+size_t used = 0, largest = 0, limit = ~size_t(0);
 long long failures = 0, stale = 0, captures = 0, graph_launches = 0;
 int overflow_queries = 0, device_err = 0;
 bool capturing = false;
@@ -46,10 +46,16 @@ void fake_reset() {
   failures = stale = captures = graph_launches = 0;
   overflow_queries = device_err = 0;
   launches.clear();
-  peak = used;
+  largest = 0;
 }
 void fake_limit(size_t bytes) { limit = bytes; }
 size_t fake_used() { return used; }
+// The largest block asked for since the last reset, which this makes.
+size_t fake_largest() {
+  const size_t n = largest;
+  largest = 0;
+  return n;
+}
 long long fake_failures() { return failures; }
 long long fake_stale() { return stale; }
 long long fake_captures() { return captures; }
@@ -71,7 +77,7 @@ cudaError_t cudaMalloc(void** p, size_t n) {
   if (!*p) return cudaErrorMemoryAllocation;
   live[reinterpret_cast<uintptr_t>(*p)] = n;
   used += n;
-  peak = std::max(peak, used);
+  largest = std::max(largest, n);
   return cudaSuccess;
 }
 cudaError_t cudaFree(void* p) {

@@ -24,7 +24,7 @@ def lib(tmp_path_factory):
     L.hb_destroy.argtypes = [c.c_void_p]
     L.fake_limit.argtypes = [c.c_size_t]
     L.fake_launched.argtypes = [c.c_char_p]
-    for name in ("fake_used", "fake_failures", "fake_stale", "fake_captures", "fake_graph_launches"):
+    for name in ("fake_used", "fake_largest", "fake_failures", "fake_stale", "fake_captures", "fake_graph_launches"):
         getattr(L, name).restype = c.c_longlong
     return L
 
@@ -138,4 +138,17 @@ def test_add_gets_the_candidates_memory(lib):
     assert lib.hb_add(ix.h, x.shape[0], x.ctypes.data) == 0, lib.hb_last_error()
     assert lib.fake_failures() >= 1
     ix.search(4000, 20)
+    ix.close()
+
+
+@pytest.mark.parametrize("d,precision", [(64, Precision.FP32), (64, Precision.BF16), (144, Precision.FP32)])
+def test_small_first_batch_takes_no_large_block(lib, d, precision):
+    """A block of one MiB and more is mapped on its own, which costs the first
+    small batch on an index more than its search."""
+    ix = HostIndex(lib, d, 500, 17, 300_000)
+    assert lib.fake_largest() > MB
+    ix.search(33, 20, precision)
+    assert ix.launched("scan_exact") == 0 and lib.fake_largest() < MB
+    ix.search(400, 20, precision)  # (beyond the spare memory)
+    assert ix.launched("scan_exact") == 0 and lib.fake_largest() > MB
     ix.close()
