@@ -609,10 +609,11 @@ class IndexCore {
     if (ntotal_ == 0) return;
     // Residuals to the list centroids: BF16(x - c_l), their FP32 norms and
     // each list's largest residual norm (the scans' error bound uses it).
-    // (With room at the end for small batches' candidates: a block of their own
-    // costs the first of them more than its search, 0.4 ms for one MiB.)
+    // With room at the end for small batches' candidates: a block of their own
+    // costs the first of them more than its search (0.4 ms for a block of one
+    // MiB or more, and 3 us a MiB).
     const size_t code_bytes = (ntotal_ * static_cast<size_t>(kpad_) * 2 + 255) / 256 * 256;
-    codes_bf16_.reserve((code_bytes + std::min(kSpareBytes, code_bytes / 16)) / 2);
+    codes_bf16_.reserve((code_bytes + std::min(kSpareBytes, code_bytes)) / 2);
     spare_ = reinterpret_cast<unsigned char*>(codes_bf16_.p) + code_bytes;
     spare_bytes_ = codes_bf16_.n * 2 - code_bytes;
     rnorm_.reserve(ntotal_);
@@ -624,7 +625,12 @@ class IndexCore {
     // Residual norms in 128-row tiles per list (+inf past each list's end),
     // copied next to each accumulator by the scan.
     std::vector<int64_t> toff(nlist_ + 1, 0);
-    for (size_t l = 0; l < nlist_; ++l) toff[l + 1] = toff[l] + (host_off_[l + 1] - host_off_[l] + 127) / 128;
+    longest_list_ = 0;
+    for (size_t l = 0; l < nlist_; ++l) {
+      const int64_t n = host_off_[l + 1] - host_off_[l];
+      toff[l + 1] = toff[l] + (n + 127) / 128;
+      longest_list_ = std::max(longest_list_, n);
+    }
     tile_off_.reserve(nlist_ + 1);
     HB_CUDA(cudaMemcpyAsync(tile_off_.p, toff.data(), toff.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st_));
     tile_norm_.reserve(std::max<size_t>(static_cast<size_t>(toff[nlist_]) * 128, 1));
@@ -973,7 +979,8 @@ class IndexCore {
     const bool dev_in = is_device_ptr(q);
     size_t bs = std::min<size_t>(nq, batch_limit(P, k));
     if (cand_path_ && P > 0) bs = std::min(bs, cand_batch_limit(P));
-    size_t bounded_bs = std::max<size_t>(1, (size_t(1) << 30) / (static_cast<size_t>(filter_cap(k)) * 8));
+    const size_t bounded_cap = static_cast<size_t>(filter_cap(k, static_cast<int>(P)));
+    size_t bounded_bs = std::max<size_t>(1, (size_t(1) << 30) / (bounded_cap * 8));
     if (screen_wide_ && mode == SCAN_PLAIN && P > 0) {
       // A query's candidate row has to fit.
       const int64_t L = cand_row_bound(static_cast<int>(P));
@@ -1669,7 +1676,7 @@ class IndexCore {
       if (screen_wide_)
         cand_reserve(nb, P, kScreenWideRows, false);
       else
-        bounded_reserve(nb, filter_cap(k), scr_cnt_, scr_m_);
+        bounded_reserve(nb, filter_cap(k, P), scr_cnt_, scr_m_);
       return true;
     } catch (const Error& e) {
       if (e.code != HB_ERR_NOMEM) throw;
@@ -1683,14 +1690,10 @@ class IndexCore {
   // them again.  (Called after a failed reserve, which has outdated every
   // captured graph.)
   bool holds_candidates() const {
-    return cbuf_.p || cbuf_ub_.p || cand_.p || cand_rows_.p || gq_.p || gq8_.p || pcd_.p || qcd8_.p || seg_.p;
+    return cand_block_.p || gq8_.p || pcd_.p || qcd8_.p || seg_.p;
   }
   void release_candidates() {
-    cbuf_.release();
-    cbuf_ub_.release();
-    cand_.release();
-    cand_rows_.release();
-    gq_.release();
+    cand_block_.release();
     gq8_.release();
     pcd_.release();
     qcd8_.release();
@@ -1717,13 +1720,23 @@ class IndexCore {
   bool screen_batch(int nb, int P, int k, float* Dd, int64_t* Id) {
     screen_ = screen_reserve(nb, P, k);
     if (!screen_) return false;
-    const int cap = filter_cap(k);
+    const int cap = filter_cap(k, P);
     const int cr = std::max(128, chunk_rows_for(nb, P, 128));
     if (screen_wide_)
       cand_pipeline(nb, P, k, kScreenWideRows, false, true, Dd, Id);
     else
       filter_pipeline(nb, P, k, cap, cr, scan_bf16_stages(kpad_), scr_cnt_.p, scr_m_.p, kDefaultWaitBudget, Dd, Id);
     return true;
+  }
+
+  // The candidate workspace that lay_out takes: in the spare end of the BF16
+  // codes' block where it fits, else in a block of its own.
+  template <class F>
+  void candidate_block(F&& lay_out) {
+    Carver need{nullptr};
+    lay_out(need);
+    Carver c{need.off <= spare_bytes_ ? spare_ : cand_block_.reserve(need.off)};
+    lay_out(c);
   }
 
   // Per-batch buffers of the bounded scan (counts and re-ranked rows in the
@@ -1733,14 +1746,10 @@ class IndexCore {
     cnt.reserve(nb);
     m.reserve(nb);
     over_list_.reserve(static_cast<size_t>(nb));
-    const size_t n = static_cast<size_t>(nb) * cap;
-    Carver c{spare_};
-    c.take(w_.key, n);
-    c.take(w_.ub, n);
-    if (!spare_ || c.off > spare_bytes_) {
-      w_.key = cbuf_.reserve(n);
-      w_.ub = cbuf_ub_.reserve(n);
-    }
+    candidate_block([&](Carver& c) {
+      c.take(w_.key, static_cast<size_t>(nb) * cap);
+      c.take(w_.ub, static_cast<size_t>(nb) * cap);
+    });
   }
 
   // The exact list scan and merge of nb queries (qpad, nb x dpad) over the
@@ -1801,13 +1810,19 @@ class IndexCore {
   }
 
   // Candidate buffer per query of the bounded BF16 scan: room for 16 k
-  // candidates (at least 2048), rounded up to a power of two (the re-rank
-  // sorts a buffer in place); a query needing more is searched again with the
-  // exact scan.
+  // candidates (at least 4096, at most kRerankMaxCap), rounded up to a power of
+  // two (the re-rank sorts a buffer in place), and no more than its nprobe lists
+  // can hold; a query needing more is searched again with the exact scan.
   static int filter_cap(size_t k) {
     size_t c = 4096;
     while (c < 16 * k) c <<= 1;
     return static_cast<int>(std::min<size_t>(kRerankMaxCap, c));
+  }
+  int filter_cap(size_t k, int P) const {
+    const int64_t rows = std::max<int64_t>(P * longest_list_, static_cast<int64_t>(k));
+    int c = 2;
+    while (c < rows && c < filter_cap(k)) c <<= 1;
+    return c;
   }
 
   // BF16 search of one batch, equal to the exact FP32 scan bit for bit: exact
@@ -1823,7 +1838,7 @@ class IndexCore {
     }
     probes_.reserve(static_cast<size_t>(nb) * P);
     coarse_and_cut(nb, P);
-    const int cap = filter_cap(k);
+    const int cap = filter_cap(k, P);
     bounded_reserve(nb, cap, ccnt_, rr_m_);
     last_nb_ = nb;
     const int cr0 = std::max(128, chunk_rows_for(nb, P, 128));
@@ -1856,7 +1871,7 @@ class IndexCore {
     // the rows it saves (33 queries, 17 lists of 600 rows, k 20: 145 -> 126 us).
     const double probed = static_cast<double>(P) * static_cast<double>(ntotal_) / static_cast<double>(nlist_);
     const bool two_stage = k > kFilterTightK && P > 1 &&
-                           (nb > kOneStageQueries || probed * k / kSeedSample > 0.5 * cap);
+                           (nb > kOneStageQueries || probed * k / kSeedSample > 0.5 * filter_cap(k));
     const int32_t* probes_a = probes_.p;
     int P_a = P, cr_a = cr;
     if (two_stage) {
@@ -2108,15 +2123,11 @@ class IndexCore {
     // The rows, then (FP8) as many lower bounds.
     const size_t nr = fp8 ? (3 * static_cast<size_t>(nb) * R + 1) / 2 : static_cast<size_t>(nb) * R;
     const size_t ng = fp8 ? 0 : nqp * static_cast<size_t>(kpad_);
-    Carver c{spare_};
-    c.take(w_.mat, nm);
-    c.take(w_.rows, nr);
-    c.take(w_.q, ng);
-    if (!spare_ || c.off > spare_bytes_) {
-      if (ng) w_.q = gq_.reserve(ng);
-      w_.mat = cand_.reserve(nm);
-      w_.rows = cand_rows_.reserve(nr);
-    }
+    candidate_block([&](Carver& c) {
+      c.take(w_.mat, nm);
+      c.take(w_.rows, nr);
+      c.take(w_.q, ng);
+    });
     over_list_.reserve(static_cast<size_t>(nb));
   }
 
@@ -2542,9 +2553,6 @@ class IndexCore {
   alignas(64) unsigned char gqmap_[128];  // gathered BF16 queries of the candidate-matrix scan
   bool cand_path_ = false;
   DevBuf<int64_t> seg_;
-  DevBuf<uint16_t> gq_;
-  DevBuf<float> cand_;
-  DevBuf<int64_t> cand_rows_;
   DevBuf<float> pcd_;   // ||q - c_l||^2 per (query, probe rank); FP8: then the entries' rounding errors
   DevBuf<int> cand_m_;  // rows re-ranked per query, then how many of them come first
   // tensor-core coarse quantizer
@@ -2572,8 +2580,6 @@ class IndexCore {
   bool screen_wide_ = false;         // d > 128: through the candidate matrix
   DevBuf<int> scr_cnt_, scr_m_;      // its counts (bf16_stats reports BF16 searches only)
   int last_nb_ = 0;
-  DevBuf<uint64_t> cbuf_;
-  DevBuf<uint32_t> cbuf_ub_;
   DevBuf<float> oq_, od_;
   DevBuf<int32_t> op_;
   DevBuf<int64_t> oi_;
@@ -2584,10 +2590,12 @@ class IndexCore {
   DevBuf<int32_t> kq_;
   DevBuf<uint16_t> codes_bf16_;
   // The end of codes_bf16_'s block, and the candidate workspace of the batch at
-  // hand: there where it fits, else in blocks of its own.
+  // hand: there where it fits, else in a block of its own.
   static constexpr size_t kSpareBytes = size_t(16) << 20;
   unsigned char* spare_ = nullptr;
   size_t spare_bytes_ = 0;
+  int64_t longest_list_ = 0;
+  DevBuf<unsigned char> cand_block_;
   struct {
     uint64_t* key;   // bounded scan: candidate keys,
     uint32_t* ub;    // their upper bounds

@@ -141,14 +141,17 @@ def test_add_gets_the_candidates_memory(lib):
     ix.close()
 
 
-@pytest.mark.parametrize("d,precision", [(64, Precision.FP32), (64, Precision.BF16), (144, Precision.FP32)])
-def test_small_first_batch_takes_no_large_block(lib, d, precision):
+@pytest.mark.parametrize("d,n,nlist,nprobe,nq,precision", [
+    (64, 300_000, 500, 17, 33, Precision.FP32), (64, 300_000, 500, 17, 33, Precision.BF16),
+    (144, 300_000, 500, 17, 33, Precision.FP32), (128, 10_000, 100, 10, 100, Precision.FP32),
+    (500, 20_000, 100, 16, 200, Precision.FP32)])
+def test_small_first_batch_takes_no_large_block(lib, d, n, nlist, nprobe, nq, precision):
     """A block of one MiB and more is mapped on its own, which costs the first
     small batch on an index more than its search."""
-    ix = HostIndex(lib, d, 500, 17, 300_000)
+    ix = HostIndex(lib, d, nlist, nprobe, n)
     assert lib.fake_largest() > MB
-    ix.search(33, 20, precision)
+    ix.search(nq, 20, precision)
     assert ix.launched("scan_exact") == 0 and lib.fake_largest() < MB
-    ix.search(400, 20, precision)  # (beyond the spare memory)
-    assert ix.launched("scan_exact") == 0 and lib.fake_largest() > MB
+    ix.search(3000, 20, precision)  # (beyond the spare memory: one block)
+    assert ix.launched("scan_exact") == 0 and lib.fake_largest() > 16 * MB
     ix.close()
