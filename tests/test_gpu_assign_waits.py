@@ -39,3 +39,27 @@ def test_wait_that_gives_up(n, nlist, d, lite, tmp_path):
     c1, b1, t1, a1 = build(x, nlist, str(tmp_path / "ex.index"), 1, lite)
     assert t1 == {"assign_tc", "assign_exact"} and a1 == {"assign_tc", "assign_exact"}
     assert np.array_equal(c0, c1) and np.array_equal(b0, b1)
+
+
+@pytest.mark.parametrize("d", [100, 200])
+@pytest.mark.parametrize("kind", ["nonfinite", "huge", "tiny", "ties", "far"])
+def test_values_outside_the_bound(kind, d, tmp_path):
+    """Points and centroids that the tensor cores may not decide: both routes
+    build the same."""
+    rng = np.random.default_rng(d)
+    n, nlist = 120_001, 385
+    x = rng.integers(0, 64, size=(nlist, d))[rng.integers(0, nlist, n)] + rng.integers(-8, 9, size=(n, d))
+    x = x.astype(np.float32)
+    if kind == "nonfinite":
+        x[::1777, 3], x[::2991, 5], x[::3331, 7], x[::4001] = np.nan, np.inf, -np.inf, 3e38
+    elif kind in ("huge", "tiny"):
+        x *= np.float32(2.0 ** (56 if kind == "huge" else -70))
+    elif kind == "ties":
+        x = rng.integers(0, 2, size=(500, d)).astype(np.float32)[rng.integers(0, 500, n)]
+    else:
+        x += np.float32(2.0 ** 17)
+    c0, b0, t0, a0 = build(x, nlist, str(tmp_path / "tc.index"), 0, True)
+    assert t0 == {"assign_tc"} and "assign_tc" in a0
+    c1, b1, t1, a1 = build(x, nlist, str(tmp_path / "ex.index"), 1, True)
+    assert t1 == {"assign_tc", "assign_exact"}
+    assert np.array_equal(c0, c1, equal_nan=True) and np.array_equal(b0, b1)
