@@ -415,13 +415,15 @@ __global__ void __launch_bounds__(256) coarse_refine_kernel(const float* __restr
     if (cdist) cdist[static_cast<size_t>(qi) * P + j] = key == kEmpty ? FLT_MAX : key_dist(key);
   }
   if (lane == 0) {
-    bool exact = true;
-    if (Pmr < nlist) {
+    // A value past FLT_MAX is no candidate, but its exact distance may be
+    // below that (the norms' sum overflowed): then fewer than Pmr are here.
+    const float vlast = cval[static_cast<size_t>(qi) * Pm + Pmr - 1];
+    bool exact = vlast < FLT_MAX;
+    if (exact && Pmr < nlist) {
       // Outside the Pmr candidates every value is >= vlast, so every exact
       // distance there is >= vlast - bound.
-      const float vlast = cval[static_cast<size_t>(qi) * Pm + Pmr - 1];
       const uint64_t kp = buf[Pr - 1];
-      exact = kp != kEmpty && vlast < FLT_MAX;
+      exact = kp != kEmpty;
       if (exact) {
         const float mn = *cmaxnorm;
         const float bound = 4e-4f * sqrtf(qn) * mn + 2e-5f * (mn * mn + qn + fabsf(vlast)) + 1e-30f;
@@ -483,11 +485,11 @@ __global__ void __launch_bounds__(256) coarse_refine_block_kernel(
   if (tid == 0) {
     float qs = 0.0f;
     for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) qs += s_qn[w];
-    bool exact = true;
-    if (Pmr < nlist) {
-      const float vlast = cval[static_cast<size_t>(qi) * Pm + Pmr - 1];
+    const float vlast = cval[static_cast<size_t>(qi) * Pm + Pmr - 1];
+    bool exact = vlast < FLT_MAX;
+    if (exact && Pmr < nlist) {
       const uint64_t kp = s_blk[Pr - 1];
-      exact = kp != kEmpty && vlast < FLT_MAX;
+      exact = kp != kEmpty;
       if (exact) {
         const float mn = *cmaxnorm;
         const float bound = 4e-4f * sqrtf(qs) * mn + 2e-5f * (mn * mn + qs + fabsf(vlast)) + 1e-30f;
