@@ -48,7 +48,7 @@ WORKLOAD = {
 # ncu capture of a 3M x 128 / nlist 1229 / nprobe 40 launch: 866.8 MB for 764.6 MB
 # (profiles/scan_bf16_3m_ncu_full.md).  The traffic grows with the lists read, so the
 # bench scales it by each launch's algorithmic bytes.
-SCAN_TRAFFIC_RATIO = 1.134
+SCAN_TRAFFIC_RATIO = 1.346
 NPROBE_SWEEP = [1, 2, 3, 4, 5, 6, 8, 10, 12, 14, 16, 20, 24, 28, 32, 40, 48, 56, 64, 80, 96, 128, 160, 192, 256]
 
 
@@ -245,6 +245,36 @@ def time_arm(torch, ix, test, k, P, precision, steps, warmup, world, dist, learn
             "kernel_ms": {n: v[0] / steps for n, v in prof.items()}}
 
 
+def exact_scan(torch, ix, test, k, P, steps):
+    """Queries per second of the exact FP32 list scan alone (a plain FP32 search
+    of this size takes the bounded scan): hb_search_noalloc, which always runs
+    the exact kernels, 1000 queries a call (its scratch is fixed).  CUDA events
+    on the index stream."""
+    from harmony_b200 import lib
+    nq, per = test.shape[0], min(1000, test.shape[0])
+    ix.nprobe = P
+    D = torch.empty((nq, k), dtype=torch.float32, device="cuda")
+    I = torch.empty((nq, k), dtype=torch.int64, device="cuda")
+    stream = torch.cuda.ExternalStream(ix.stream)
+
+    def once():
+        for b in range(0, nq, per):
+            n = min(per, nq - b)
+            if lib().hb_search_noalloc(ix._h, n, test[b:].data_ptr(), k, D[b:].data_ptr(), I[b:].data_ptr()):
+                raise RuntimeError(lib().hb_last_error().decode())
+
+    torch.cuda.synchronize()
+    once()
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record(stream)
+    for _ in range(steps):
+        once()
+    e1.record(stream)
+    e1.synchronize()
+    ms = e0.elapsed_time(e1) / steps
+    return {"qps": round(nq / ms * 1e3, 1), "nprobe": P, "queries_per_call": per, "ms_per_step": round(ms, 3)}
+
+
 def run_ours(args):
     import torch
     import torch.distributed as dist
@@ -345,29 +375,37 @@ def run_ours(args):
         e2e_ms = float(t.item())
     e2e_recall = recall(Ih_np, gt, k)
 
-    # Parity at this configuration (untimed).  The BF16 arms against the exact
-    # FP32 scan over the same probe lists: the fixed-nprobe arm at its nprobe,
-    # the learned arm with the same predicted per-query nprobe (the predictor
-    # cuts the probe rows the same way for either precision).  The FP32 scan
-    # against the reference's own Index::search is checked on the CPU-baseline
-    # sample below.
+    # Parity at this configuration (untimed): every arm against the exact FP32
+    # scan over the same probe lists, the learned one with the same predicted
+    # per-query nprobe (the predictor cuts the probe rows the same way for either
+    # precision).  A k past 256 takes the exact scan, whose k nearest are the
+    # first columns.  The FP32 results against the reference's own Index::search
+    # are checked on the CPU-baseline sample below.
     def exact_fp32(P, learned=False, target=0.0):
         sp = ix.search_params
         sp.precision, sp.learned_probe, sp.learned_target = Precision.FP32, learned, target
         ix.nprobe = P
-        Dx = torch.empty((nq, k), dtype=torch.float32, device="cuda")
-        Ix = torch.empty((nq, k), dtype=torch.int64, device="cuda")
-        ix.search(nq, test, k, Dx, Ix)
-        return Dx.cpu().numpy(), Ix.cpu().numpy()
+        Dx = torch.empty((nq, 257), dtype=torch.float32, device="cuda")
+        Ix = torch.empty((nq, 257), dtype=torch.int64, device="cuda")
+        ix.profile(True)
+        ix.search(nq, test, 257, Dx, Ix)
+        kernels = ix.profile_read()
+        ix.profile(False)
+        assert "scan_exact" in kernels and "scan_bf16" not in kernels, kernels
+        return (np.ascontiguousarray(Dx[:, :k].cpu().numpy()), np.ascontiguousarray(Ix[:, :k].cpu().numpy()))
 
     Pf, Pb = arms["fp32"]["nprobe"], arms["bf16"]["nprobe"]
-    ref_b = outs["fp32"] if Pb == Pf else exact_fp32(Pb)
-    ok_b, n_b = parity_count(*outs["bf16"], *ref_b)
+    ref_f = exact_fp32(Pf)
+    ok_f, n_f = parity_count(*outs["fp32"], *ref_f)
+    ok_b, n_b = parity_count(*outs["bf16"], *(ref_f if Pb == Pf else exact_fp32(Pb)))
     ref_l = exact_fp32(256, learned=True, target=tgt)
     ok_l, n_l = parity_count(*outs["learned_bf16"], *ref_l)
+    ix.search_params.learned_probe = False
+    exact_arm = exact_scan(torch, ix, test, k, Pf, max(1, args.steps // 4))
     Dh, Ih = outs["learned_bf16"] if head is arms["learned_bf16"] else outs["bf16"]
     parity = {
         "rule": "per query: distances bit-identical, ids identical except among ties at the k-th distance",
+        "fp32_vs_exact_scan": {"nprobe": Pf, "identical": ok_f, "queries": n_f},
         "bf16_fixed_vs_fp32_exact": {"nprobe": Pb, "identical": ok_b, "queries": n_b},
         "learned_bf16_vs_learned_fp32_exact": {"identical": ok_l, "queries": n_l},
         "headline_max_rel_dist_err_vs_fp64": max_rel_err_vs_fp64(torch, base, test, Dh, Ih),
@@ -464,7 +502,9 @@ def run_ours(args):
                                   "recall_at_10": round(arms["bf16"]["recall_at_10"], 4),
                                   "ms_per_step": round(arms["bf16"]["ms_per_step"], 3),
                                   "kernel_ms_per_step": {n: round(v, 4) for n, v in arms["bf16"]["kernel_ms"].items()}},
+            "exact_fp32_scan": exact_arm,
             "speedup_vs_plain_fp32": round(head["qps"] / fp["qps"], 2),
+            "speedup_vs_exact_fp32_scan": round(head["qps"] / world / exact_arm["qps"], 2),
             "e2e": {"value": round(world * nq / (e2e_ms / 1e3), 1), "unit": "queries/s",
                     "h2d_bytes_per_step": nq * d * 4, "d2h_bytes_per_step": nq * k * 12,
                     "recall_at_10": round(e2e_recall, 4)},
