@@ -45,7 +45,7 @@ WORKLOAD = {
     "nb": 10_000_000, "d": 128, "nlist": 4096, "k": 10, "nq": 10_000,
 }
 # DRAM bytes (read + write) of one scan_bf16 launch over its algorithmic bytes, from the
-# ncu capture of a 3M x 128 / nlist 1229 / nprobe 40 launch: 866.8 MB for 764.6 MB
+# ncu capture of a 3M x 128 / nlist 1229 / nprobe 40 launch: 1029.3 MB for 764.6 MB
 # (profiles/scan_bf16_3m_ncu_full.md).  The traffic grows with the lists read, so the
 # bench scales it by each launch's algorithmic bytes.
 SCAN_TRAFFIC_RATIO = 1.346
@@ -456,7 +456,7 @@ def run_ours(args):
     fp = arms["fp32"]
     fp_pairs = int(sizes[ix.probe_lists(test.cpu().numpy(), fp["nprobe"])[0]].sum())
     fp_bytes_alg = fp_pairs * d * 4
-    fp_scan = fp["kernel_ms"].get("scan_exact", 0.0) / 1e3
+    fp_scan = 0.0 if "scan_bf16" in fp["kernel_ms"] else fp["kernel_ms"].get("scan_exact", 0.0) / 1e3
     clocks = clk.summary()
     sm_mhz = clocks.get("sm_mhz") or 1965.0
     # The exact scan's own roofline is the FP32 pipe, not HBM (each probed list
@@ -951,15 +951,30 @@ def run_c2(args):
                        "recall_at_100_first_1000": round(recall(outs[name][1][:ng], gt, k), 4)}
                 if stats:
                     arm["bounded_scan"] = stats
-                scan = kern.get("scan_exact" if prec == Precision.FP32 else "scan_bf16")
+                # The scan that served the arm (a plain FP32 search of this size takes
+                # the bounded BF16 one, and its few overflowing queries the exact).
+                bounded = "scan_bf16" in kern
+                scan = kern.get("scan_bf16" if bounded else "scan_exact")
                 if scan:
-                    elem = 2 if prec == Precision.BF16 else 4
-                    arm["scan_bytes_alg_gbs"] = round(pairs * d * elem / (scan / 1e3) / 1e9, 1)
-                    if prec == Precision.FP32:
+                    arm["scan_bytes_alg_gbs"] = round(pairs * d * (2 if bounded else 4) / (scan / 1e3) / 1e9, 1)
+                    if not bounded:
                         arm["scan_fp32_ops_per_s"] = 3.0 * pairs * d / (scan / 1e3)
                 row[name] = arm
-            ok, n = parity_count(*outs["bf16"], *outs["fp32"])
-            row["bf16_identical_to_fp32"] = {"identical": ok, "queries": n}
+            # Both arms against the exact scan (a k past 256 takes it; its k nearest
+            # are the first columns).
+            ix.search_params.precision = Precision.FP32
+            Dx = torch.empty((nq, 257), dtype=torch.float32, device="cuda")
+            Ix = torch.empty((nq, 257), dtype=torch.int64, device="cuda")
+            ix.search(nq, queries, 257, Dx, Ix)
+            e0.record(stream)
+            ix.search(nq, queries, 257, Dx, Ix)
+            e1.record(stream)
+            e1.synchronize()
+            row["exact_scan_k257_ms"] = round(e0.elapsed_time(e1), 3)
+            ref = (np.ascontiguousarray(Dx[:, :k].cpu().numpy()), np.ascontiguousarray(Ix[:, :k].cpu().numpy()))
+            for name in ("fp32", "bf16"):
+                ok, n = parity_count(*outs[name], *ref)
+                row[f"{name}_identical_to_exact_scan"] = {"identical": ok, "queries": n}
             # Largest relative error of the returned distances against FP64
             # recomputation, first 1000 queries.
             for name in ("fp32", "bf16"):

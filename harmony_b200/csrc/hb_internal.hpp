@@ -230,7 +230,6 @@ void launch_scatter_sorted(const float* x, const uint32_t* order, size_t n, int 
 void launch_list_offsets(const int32_t* assign, size_t n, int nlist, int64_t* list_off,
                          void* tmp, size_t tmp_bytes, cudaStream_t st);
 size_t list_offsets_tmp_bytes(int nlist);
-void launch_i64_to_i32(const int64_t* src, size_t n, int32_t* dst, cudaStream_t st);
 // Rows of w 32-bit words: dst[i] = src[idx[i]] (gather) / dst[idx[i]] = src[i]
 // (scatter), i < n.
 void launch_gather_words(const uint32_t* src, const int32_t* idx, int n, int w, uint32_t* dst, cudaStream_t st);
@@ -370,7 +369,6 @@ void launch_cand_select(const float* cand, const int64_t* seg, const int32_t* pr
                         int* over_list, int* over_n, cudaStream_t st);
 void launch_cand_exact(const int64_t* rows, const float* lb, const int* m, const int* first, int nq, int R, int k,
                        const float* codes, const float* q, int dpad, const int64_t* ids, float* D, int64_t* I, cudaStream_t st);
-void launch_to_bf16(const float* src, size_t n, int dpad, int kpad, void* dst, cudaStream_t st);
 void launch_scan_bf16(const void* tmap, const TcArgs& a, int num_sms, cudaStream_t st);
 // One thread waits on an mbarrier nothing arrives on, with a budget of
 // `budget` cycles: *err gets `code` and *waited the cycles spent (-1 if the
@@ -378,7 +376,6 @@ void launch_scan_bf16(const void* tmap, const TcArgs& a, int num_sms, cudaStream
 void launch_wait_selftest(long long budget, int code, int* err, long long* waited, cudaStream_t st);
 // *out = max over i of sqrt(norms[i]) (slightly rounded up), on the device.
 void launch_max_norm(const float* norms, size_t n, float* out, cudaStream_t st);
-// probes (nq x P) -> first column (nq x 1) and the rest (nq x (P-1)).
 
 // k_coarse_tc.cu: tensor-core coarse quantizer (3-term BF16 split) with an
 // exact FP32 finish; the probe rows equal the exact quantizer's.

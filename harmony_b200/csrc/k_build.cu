@@ -162,10 +162,6 @@ __global__ void histogram_kernel(const int32_t* __restrict__ assign, size_t n, i
   if (i < n) atomicAdd(reinterpret_cast<unsigned long long*>(&cnt[assign[i]]), 1ull);
 }
 
-__global__ void i64_to_i32_kernel(const int64_t* __restrict__ s, size_t n, int32_t* __restrict__ d) {
-  const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
-  if (i < n) d[i] = static_cast<int32_t>(s[i]);
-}
 __global__ void i32_to_i64_kernel(const int32_t* __restrict__ s, size_t n, int64_t* __restrict__ d) {
   const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (i < n) d[i] = static_cast<int64_t>(s[i]);
@@ -271,11 +267,6 @@ void launch_list_offsets(const int32_t* assign, size_t n, int nlist, int64_t* li
   HB_CUDA(cub::DeviceScan::ExclusiveSum(tmp, cub_bytes, cnt, list_off, static_cast<int64_t>(nlist) + 1, st));
 }
 
-void launch_i64_to_i32(const int64_t* src, size_t n, int32_t* dst, cudaStream_t st) {
-  if (!n) return;
-  i64_to_i32_kernel<<<grid_exact(n, 256), 256, 0, st>>>(src, n, dst);
-  HB_CUDA(cudaGetLastError());
-}
 void launch_i32_to_i64(const int32_t* src, size_t n, int64_t* dst, cudaStream_t st) {
   if (!n) return;
   i32_to_i64_kernel<<<grid_exact(n, 256), 256, 0, st>>>(src, n, dst);

@@ -1244,17 +1244,6 @@ __global__ void max_norm_kernel(const float* __restrict__ norms, size_t n, float
 
 __global__ void sqrt_inplace_kernel(float* v) { *v = sqrtf(*v) * 1.0001f; }
 
-__global__ void to_bf16_kernel(const float* __restrict__ src, size_t n, int dpad, int kpad,
-                               __nv_bfloat16* __restrict__ dst) {
-  const size_t total = n * static_cast<size_t>(kpad);
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const size_t r = i / kpad;
-    const int c = static_cast<int>(i - r * kpad);
-    dst[i] = __float2bfloat16_rn(c < dpad ? src[r * dpad + c] : 0.0f);
-  }
-}
-
 // Self-test of the bounded mbarrier wait: one thread initialises an mbarrier
 // that nothing ever arrives on and waits for its first phase with a budget of
 // `budget` clock cycles.  No copy or MMA is in flight, so giving up is the
@@ -1318,14 +1307,6 @@ void make_f32_store_map(void* tmap_out, const float* base, size_t rows, size_t c
                                     box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                     CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   HB_CHECK(r == CUDA_SUCCESS, HB_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-}
-
-void launch_to_bf16(const float* src, size_t n, int dpad, int kpad, void* dst, cudaStream_t st) {
-  if (!n) return;
-  size_t g = (n * kpad + 255) / 256;
-  if (g > 148u * 64u) g = 148u * 64u;
-  to_bf16_kernel<<<static_cast<unsigned>(g), 256, 0, st>>>(src, n, dpad, kpad, static_cast<__nv_bfloat16*>(dst));
-  HB_CUDA(cudaGetLastError());
 }
 
 void launch_scan_bf16(const void* tmap, const TcArgs& a, int num_sms, cudaStream_t st) {
