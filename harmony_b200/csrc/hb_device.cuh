@@ -77,7 +77,8 @@ __device__ __forceinline__ void block_bitonic_sort(uint64_t* s, int n) {
   }
 }
 
-// Monotone map of a float to uint32 (all signs), and its inverse.
+// Monotone map of a float to uint32 (all signs), and its inverse.  A NaN lands
+// anywhere: callers keep it out.
 __device__ __forceinline__ uint32_t ordered_bits(float f) {
   const uint32_t b = __float_as_uint(f);
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
@@ -86,12 +87,7 @@ __device__ __forceinline__ float ordered_to_float(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-// Squared L2 distance of one stored row and one query row (both padded to
-// dpad, a multiple of 4, with zeros) with the reference's sequential
-// unfused FP32 loop, src/utils.h:480-487: t = q - x, sum += t * t, each
-// operation rounded on its own, dimensions in order.  The zero padding adds
-// exact zeros.
-// The same loop continued from acc over dims [0, n) of x and qrow (n a
+// exact_l2_seq's loop continued from acc over dims [0, n) of x and qrow (n a
 // multiple of 4): running it over consecutive pieces of a row in order gives
 // the whole row's sum bit for bit.
 __device__ __forceinline__ float exact_l2_seq_from(float acc, const float* __restrict__ x,
@@ -113,6 +109,11 @@ __device__ __forceinline__ float exact_l2_seq_from(float acc, const float* __res
   return acc;
 }
 
+// Squared L2 distance of one stored row and one query row (both padded to
+// dpad, a multiple of 4, with zeros) with the reference's sequential
+// unfused FP32 loop, src/utils.h:480-487: t = q - x, sum += t * t, each
+// operation rounded on its own, dimensions in order.  The zero padding adds
+// exact zeros.
 __device__ __forceinline__ float exact_l2_seq(const float* __restrict__ x, const float* __restrict__ qrow, int dpad) {
   float acc = 0.0f;
 #pragma unroll 8

@@ -71,6 +71,12 @@ constexpr double kScreenShortRows = 256.0;
 // 138 / 123 (382 / 146, 206 / 142); 200k x 1000 5.0e6 121 / 132, 8.1e6 157 / 158,
 // 2.0e7 195 / 144; lists of 100 rows, d 200: 1.3e7 87 / 97, 5.4e7 118 / 105.
 constexpr double kScreenWideWork = 8.0e6, kScreenWideWorkShort = 3.0e7;
+// Queries up to which a batch with k > kFilterTightK may take one scan stage
+// (see filter_pipeline).  Two stages against one, BF16, 500 lists of 600 rows x
+// 100, nprobe 17, k 20: 33 queries 124 / 109 us, 128 139 / 111, 256 150 / 121, 512
+// 167 / 134; 1000 lists of 300 x 96, nprobe 8, k 100: 33 116 / 104, 256 141 / 125.
+// (Where the seed's bound is as good as there one stage stays ahead past 256
+// queries; a bound that is not costs each query its buffer and the exact scan.)
 constexpr int kOneStageQueries = 256;
 constexpr double kSeedSample = 256.0;
 constexpr int kScreenWideRows = 2048;  // rows re-ranked per query of a wide FP32 search; more go to the exact scan
@@ -578,9 +584,6 @@ class IndexCore {
     drop_graphs();
   }
 
-  // BF16 copy of the codes (rows padded to kpad = d rounded up to 64) and its
-  // TMA tensor map, for the tensor-core scans (the heap scan takes d <= 128,
-  // the candidate-matrix scan any d).
   // E4M3 copy of the codes for the FP8 candidate scan (rows padded to kpad8
   // = d rounded up to 128 bytes) with a per-list scale, built on the first
   // FP8 search after the lists change.
@@ -600,6 +603,9 @@ class IndexCore {
     fp8_ready_ = true;
   }
 
+  // BF16 copy of the codes (rows padded to kpad = d rounded up to 64) and its
+  // TMA tensor map, for the tensor-core scans (the bounded scan takes d <= 128,
+  // the candidate matrix any d).
   void build_bf16() {
     bf16_ready_ = false;
     fp8_ready_ = false;
@@ -886,8 +892,8 @@ class IndexCore {
     }
     HB_CHECK(p.seed_rows >= 0 && p.seed_rows <= 256, HB_ERR_INVALID, "seed_rows must be in [0, 256]");
     seed_rows_ = p.seed_rows > 0 ? p.seed_rows : 256;
-    // BF16 route: the bounded filter scan (exact result) for d <= 128 and
-    // k <= 256, else the candidate-matrix scan with a fixed re-rank width.
+    // BF16 route: the bounded scan (exact result) for d <= 128 and k <= 256,
+    // else the candidate-matrix scan with a fixed re-rank width.
     const int want_R = std::max(static_cast<int>(k), p.rerank_mult * static_cast<int>(k));
     int etv = 0, eqt = 0, eqg = 0;
     const bool exact_k = scan_exact_smem_bytes(static_cast<int>(d_), static_cast<int>(dpad_), static_cast<int>(k),
@@ -1828,9 +1834,10 @@ class IndexCore {
   // BF16 search of one batch, equal to the exact FP32 scan bit for bit: exact
   // coarse probes, per-query BF16 rows / error bounds, the list-major work
   // description, a per-query admission bound seeded from the nearest list,
-  // one tensor-core pass appending the rows under each query's bound, then
-  // the exact re-rank of the rows under W_k + 2 eps.  Queries whose candidate
-  // buffer overflowed are searched again with the exact scan.
+  // one tensor-core pass (two for k > kFilterTightK) appending the rows under
+  // each query's bound, then the exact re-rank of the rows whose lower bound is
+  // at most U.  Queries whose candidate buffer overflowed are searched again
+  // with the exact scan.
   void search_batch_bf16(int nb, int P, int k, int R, float* Dd, int64_t* Id) {
     if (cand_path_) {
       search_batch_cand(nb, P, k, R, Dd, Id);
@@ -1851,8 +1858,7 @@ class IndexCore {
     filter_pipeline(nb, P, k, cap, cr, stages, ccnt_.p, rr_m_.p, wait_budget_, Dd, Id);
   }
 
-  // The bounded scan of one batch after the coarse probes: per-query prep,
-  // work description (chunks of cr rows), seed bounds, the scan with a ring
+  // The bounded scan of one batch after the coarse probes: work description (chunks of cr rows), seed bounds, the scan with a ring
   // of `stages` B tiles, and the exact re-rank.  For k > kFilterTightK the
   // scan runs in two stages: every query's nearest list first, whose k-th
   // admitted value bounds the second stage over the other lists.  Every

@@ -329,7 +329,7 @@ struct CandArgs {
   int chunk_rows;           // multiple of 128
   int P;
   const int64_t* seg;       // nq x P + 1: start of each (query, probe rank) segment of `cand`
-  float* cand;              // candidate rows: ||x||^2 - 2 q~.x~, +inf padding
+  float* cand;              // candidate rows: qcd + ||x - c_l||^2 - 2 (q - c_l)~.(x - c_l)~, +inf padding
   int* err;
   int fp8;                  // 1: E4M3 residual operands (kpad = FP8 row bytes, a multiple of 128)
   const float* qscale;      // FP8: per list-major entry s_e (q - c_l ~ s_e * code)

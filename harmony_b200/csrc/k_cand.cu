@@ -1,11 +1,13 @@
-// BF16 tensor-core list scan through a candidate matrix, for the searches the
-// shared-memory heap scan (k_tc.cu) does not hold: vectors wider than 128
-// dimensions and more than 64 candidates per query.
+// Tensor-core list scan (BF16 or E4M3) through a candidate matrix, for the
+// searches that the bounded scan (k_tc.cu) does not serve: vectors wider than
+// 128 dimensions (plain FP32 searches with enough work among them), k > 256, and
+// FP8 at any size.
 //
-//  1. gather_queries_kernel writes, for every (list, query probing it) entry
-//     of the list-major work description, the query in BF16 (K = kpad, zero
-//     padded): one row per entry, so the queries of one work item are 128
-//     consecutive rows and reach the tensor cores by plain TMA tiles.
+//  1. gather_residual_kernel writes, for every (list, query probing it) entry
+//     of the list-major work description, the query's residual q - c_l in BF16
+//     or scaled E4M3 (K = kpad, zero padded): one row per entry, so the queries
+//     of one work item are 128 consecutive rows and reach the tensor cores by
+//     plain TMA tiles.
 //  2. cand_scan_kernel: persistent, one CTA per SM, 192 threads (4 epilogue
 //     warps, a TMA warp, an MMA warp).  Work items are (list, chunk of rows,
 //     group of <= 128 queries).  Up to eight 64-column K blocks of the group's
@@ -13,7 +15,8 @@
 //     item; for each 128-row tile of the chunk the TMA warp streams the row
 //     blocks (B) through a ring, the MMA warp issues tcgen05.mma M128 x N128 x
 //     K16 into one of four TMEM accumulators, and the epilogue (thread =
-//     query, TMEM lane) writes v = ||x||^2 - 2 q~.x~ of the tile's rows into
+//     query, TMEM lane) writes v = ||q - c_l||^2 + ||r||^2 - 2 (q - c_l)~.r~ of
+//     the tile's rows (r = x - c_l; ~: rounded to BF16 or E4M3) into
 //     the query's candidate row: the concatenation over its probes, in probe
 //     order, of one segment per probed list (the list's length rounded up to
 //     8; +inf past the end).  Wider queries stream beside the rows.
@@ -21,11 +24,10 @@
 //     (v, position) of its candidate row (unique keys, so the choice is
 //     deterministic), or all the rows that the scan's error bound allows, and
 //     maps each position back to its stored row.
-//  4. cand_exact_kernel: one CTA per query recomputes the R distances with
+//  4. cand_exact_kernel: one CTA per query recomputes their distances with
 //     the reference's sequential unfused FP32 loop and returns the k best
-//     (distance, row) -- the same rule as the heap scan's rerank, so whenever
-//     the true k nearest are among the R candidates the result equals the
-//     exact scan's.
+//     (distance, row) -- the bounded scan's re-rank's rule, so whenever the true
+//     k nearest are among the candidates the result equals the exact scan's.
 // Every mbarrier wait is bounded; on a timeout the kernel records an error
 // code, the roles stop, copies and MMAs in flight are waited for and TMEM is
 // freed.
