@@ -1693,12 +1693,12 @@ class IndexCore {
   }
 
   // The buffers that only scans through candidates need; their searches take
-  // them again.  (Called after a failed reserve, which has outdated every
-  // captured graph.)
+  // them again.  (The graphs captured with them go first.)
   bool holds_candidates() const {
     return cand_block_.p || gq8_.p || pcd_.p || qcd8_.p || seg_.p;
   }
   void release_candidates() {
+    drop_graphs();
     cand_block_.release();
     gq8_.release();
     pcd_.release();

@@ -16,7 +16,7 @@ namespace {
 std::map<uintptr_t, size_t> live;  // device allocations
 size_t used = 0, largest = 0, limit = ~size_t(0);
 long long failures = 0, stale = 0, captures = 0, graph_launches = 0;
-int overflow_queries = 0, device_err = 0;
+int overflow_queries = 0, device_err = 0, failing_copies = 0;
 bool capturing = false;
 std::vector<std::string> launches;
 // Buffers the launches of a captured graph were given.
@@ -44,7 +44,7 @@ extern "C" {
 void fake_reset() {
   limit = ~size_t(0);
   failures = stale = captures = graph_launches = 0;
-  overflow_queries = device_err = 0;
+  overflow_queries = device_err = failing_copies = 0;
   launches.clear();
   largest = 0;
 }
@@ -62,6 +62,7 @@ long long fake_captures() { return captures; }
 long long fake_graph_launches() { return graph_launches; }
 void fake_overflow(int queries) { overflow_queries = queries; }
 void fake_err(int code) { device_err = code; }
+void fake_fail_copies(int n) { failing_copies = n; }
 int fake_launched(const char* name) {
   return static_cast<int>(std::count(launches.begin(), launches.end(), std::string(name)));
 }
@@ -100,6 +101,7 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  if (failing_copies > 0) return --failing_copies, cudaErrorMemoryAllocation;
   if (!capturing) std::memmove(d, s, n);
   return cudaSuccess;
 }

@@ -78,6 +78,20 @@ def test_graph_is_dropped_with_its_buffers(lib):
     ix.close()
 
 
+def test_graph_is_dropped_where_something_else_runs_out(lib):
+    """Out of memory in a call that is no allocation of the library's: the
+    candidate buffers go all the same, and the graphs with them."""
+    ix = HostIndex(lib, 64, 16, 8, 4000)
+    ix.search(50, 300)  # (so that the second of these allocates nothing)
+    for _ in range(2):
+        ix.search(2000, 10, Precision.BF16, graph=True)
+    assert lib.fake_captures() == 1 and lib.fake_graph_launches() == 1
+    lib.fake_fail_copies(1)
+    ix.search(50, 300)
+    ix.search(2000, 10, Precision.BF16, graph=True)
+    ix.close()
+
+
 def test_exact_search_of_overflowing_queries_gets_the_candidates_memory(lib):
     """The queries that a screened batch hands to the exact scan (or all of them
     after a wait that gave up) find room where the batch alone would."""
