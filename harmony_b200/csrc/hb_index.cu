@@ -1858,11 +1858,11 @@ class IndexCore {
     filter_pipeline(nb, P, k, cap, cr, stages, ccnt_.p, rr_m_.p, wait_budget_, Dd, Id);
   }
 
-  // The bounded scan of one batch after the coarse probes: work description (chunks of cr rows), seed bounds, the scan with a ring
-  // of `stages` B tiles, and the exact re-rank.  For k > kFilterTightK the
-  // scan runs in two stages: every query's nearest list first, whose k-th
-  // admitted value bounds the second stage over the other lists.  Every
-  // (cr, stages) gives the same result.
+  // The bounded scan of one batch after the coarse probes: work description
+  // (chunks of cr rows), seed bounds, the scan with a ring of `stages` B tiles,
+  // and the exact re-rank.  For k > kFilterTightK the scan may run in two stages:
+  // every query's nearest list first, whose k-th admitted value bounds the second
+  // stage over the other lists.  Every (cr, stages) gives the same result.
   void filter_pipeline(int nb, int P, int k, int cap, int cr, int stages, int* cnt, int* rr_m, long long budget,
                        float* Dd, int64_t* Id) {
     list_cnt_.reserve(nlist_);
